@@ -15,8 +15,11 @@
 // only scale err). The estimate, the norms and the stopping test are double-float too (the FP64
 // pipes of GB300 are too slow to hold them), the test as |u|^2 |v|^2 <= eps^2 err. The terms live in a double-float pool while the recursion needs them; packing
 // rounds them to the FP32 per-leaf segments the matvec streams.
+#include <algorithm>
+#include <mutex>
+
 #include "common.cuh"
-#include "df64.cuh"
+#include "df2.cuh"
 #include "entry_df.cuh"
 #include "internal.h"
 
@@ -25,6 +28,11 @@ namespace ac3d {
 namespace {
 constexpr int kDfThreads = 256;
 constexpr int kDfWarps = kDfThreads / 32;
+constexpr int kSmallThreads = 128;  // CTAs of the 1-, 2- and 4-warp groups
+constexpr int kAllocTerms = 4;      // terms per allocation from the pool
+// Blocks are run by groups of W warps, W by the block's larger side: 1 up to 64, 2 up to 128, 4 up to
+// 256 (so that a thread owns at most two rows and two columns), 8 above.
+constexpr int kGroups = 4;
 }  // namespace
 
 struct AcaDfArgs {
@@ -35,13 +43,14 @@ struct AcaDfArgs {
   const DfElem* el;            // double-float quadrature points and normals (columns)
   const float4* tab;           // df_sincos table in global memory (copied to shared memory)
   const int4* blocks;
-  const int* order;
+  const int* order;            // blocks grouped by W = 8, 4, 2, 1
+  int split[kGroups];          // blocks per group
   df64 k;
   double eps;
   df64 eps2;       // eps^2 as a double-float (the stopping test)
   int maxk;
   int iter_cap;
-  cdf* pool;
+  df2* pool;       // terms u | v, complex double-floats packed as (re, im)
   long long pool_cap;
   unsigned long long* pool_used;
   long long* term_off;
@@ -51,13 +60,14 @@ struct AcaDfArgs {
   int zero_guard;  // boundary blocks: v kept when v_j == 0 and exactly-zero blocks skipped
 };
 
-// One out-of-line copy of the entry (its loops are not unrolled into the callers' unrolled
-// rows-per-lane loops; see entry_far_call in assemble.cu).
-__device__ __noinline__ cdf entry_df_call(df64 k, const DfPt* p, const DfElem* e, const float4* tab) {
-  return entry_df(k, p, e, tab);
+// The CTA's copy of the df_sincos table. A function's own shared variable, so that out-of-line code
+// reads it with shared-memory loads.
+__device__ __forceinline__ float4* s_table() {
+  __shared__ float4 s_tab[kDfTab];
+  return s_tab;
 }
-
-__device__ __forceinline__ void load_table(const float4* __restrict__ g, float4* s) {
+__device__ __forceinline__ void load_table(const float4* __restrict__ g) {
+  float4* s = s_table();
   for (int i = threadIdx.x; i < kDfTab; i += blockDim.x) s[i] = g[i];
   __syncthreads();
 }
@@ -90,14 +100,6 @@ __device__ __forceinline__ df64 shfl_df(df64 v, int src) {
   return {__shfl_sync(0xffffffffu, v.hi, src), __shfl_sync(0xffffffffu, v.lo, src)};
 }
 
-// Sum over the warp by butterfly; every lane ends with the same value (the double-float add is
-// commutative bit for bit: TwoSum's error term is exact).
-__device__ __forceinline__ df64 warp_sum_df(df64 v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = v + df64{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
-  return v;
-}
-
 // a * b of two FP32 values, exactly, as a double-float
 __device__ __forceinline__ df64 df_prod_ff(float a, float b) {
   float p, e;
@@ -112,170 +114,373 @@ __device__ __forceinline__ bool aca_converged(df64 uv, df64 err, df64 eps2) {
   return !df_is_zero(err) && !(uv > eps2 * err);
 }
 
-// (value, index) argmax over the warp: larger value wins, smaller index on ties
+// (value, index) argmax over the warp: larger value wins, smaller index on ties. Values are
+// non-negative double-floats, or -1 for a lane without one; three integer reductions on keys in
+// the values' order (-1 below 0, the low part with -0 = +0) instead of a butterfly of triples.
 __device__ __forceinline__ void warp_argmax_df(df64& val, int& idx) {
+  const unsigned hk = val.hi < 0.0f ? 0u : __float_as_uint(val.hi + 0.0f) + 1u;
+  const unsigned hm = __reduce_max_sync(0xffffffffu, hk);
+  const unsigned lb = __float_as_uint(val.lo + 0.0f);
+  const unsigned lk = hk == hm ? ((lb >> 31) ? ~lb : lb | 0x80000000u) : 0u;
+  const unsigned lm = __reduce_max_sync(0xffffffffu, lk);
+  const unsigned best = hk == hm && lk == lm ? (unsigned)idx : 0xffffffffu;
+  idx = (int)__reduce_min_sync(0xffffffffu, best);
+  val.hi = hm == 0u ? -1.0f : __uint_as_float(hm - 1u);
+  val.lo = __uint_as_float((lm >> 31) ? lm & 0x7fffffffu : ~lm);
+}
+
+// Sums of two double-floats over the warp by butterfly; every lane ends with the same values (the
+// double-float add is commutative bit for bit: TwoSum's error term is exact).
+__device__ __forceinline__ void warp_sum2_df(df64& x, df64& y) {
+  df2 v = df2_make(x, y);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const df64 ov{__shfl_xor_sync(0xffffffffu, val.hi, o), __shfl_xor_sync(0xffffffffu, val.lo, o)};
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    if (ov > val || (ov == val && oi < idx)) {
-      val = ov;
-      idx = oi;
+  for (int o = 16; o > 0; o >>= 1)
+    v = v + df2{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
+  x = df2_x(v);
+  y = df2_y(v);
+}
+
+// FP32 complex product of the leading parts (re, im): acc += a b
+__device__ __forceinline__ void lead_fma(float& re, float& im, f2 a, f2 b) {
+  re = fmaf(f2_x(a), f2_x(b), re);
+  re = fmaf(-f2_y(a), f2_y(b), re);
+  im = fmaf(f2_x(a), f2_y(b), im);
+  im = fmaf(f2_y(a), f2_x(b), im);
+}
+
+// The three quadrature-point pairs of cnt entries, 3 cnt items spread over the T threads of a
+// group: entry e is the pair (pts + e ps, el + e es), ps and es 0 or 1; item 3 e + h goes to
+// b0[3 e + h] (first point) and b1[3 e + h] (second point), shared-memory addresses. One out-of-line
+// copy serves every group width and both directions.
+__device__ __noinline__ void eval_items(df64 k, const DfPt* __restrict__ pts, int ps, const DfElem* __restrict__ el,
+                                        int es, int cnt, int tid, int T, uint32_t b0, uint32_t b1) {
+  const df2 kk = df2_dup(k);
+  const float4* tab = s_table();
+#pragma unroll 1
+  for (int it = tid; it < 3 * cnt; it += T) {
+    const int e = it / 3, h = it - 3 * e;
+    const DfItem d = entry_item(kk, pts + e * ps, el + e * es, h, tab);
+    asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(b0 + 16 * it), "l"(d.p0), "l"(d.e0) : "memory");
+    asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(b1 + 16 * it), "l"(d.p1), "l"(d.e1) : "memory");
+  }
+}
+__device__ __forceinline__ uint32_t shared_addr(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+// One step of the transposed butterfly below: of 2 N values, a lane keeps N (the upper ones in the
+// lanes with bit O set) and adds its partner's share of them.
+template <int N, int O>
+__device__ __forceinline__ void fold(float* v) {
+  const bool up = (threadIdx.x & O) != 0;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const float keep = up ? v[k + N] : v[k], give = up ? v[k] : v[k + N];
+    v[k] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+  }
+}
+
+// |u^T U_p| |v V_p^T| of the NT earlier terms p0 .. p0 + NT - 1 that exist (FP32 on the leading parts,
+// each dot product summed over rows l, l + 32, ... by lane l and then over the lanes in the order of
+// a xor butterfly) into prod[p]. uh, vh: leading parts of the new u and v, us and vs apart. The 4 NT
+// sums are folded together, half of them dropped from a lane at each step: 4 NT shuffles and
+// 5 - log2(4 NT) more instead of 20 NT.
+template <int NT>
+__device__ __forceinline__ void cross_terms(int p0, int nst, int m, int n, const f2* uh, int us, const f2* vh, int vs,
+                                            const df2* pool, const long long* toff, df64* prod) {
+  const int lane = threadIdx.x & 31;
+  float s[4 * NT];
+#pragma unroll
+  for (int k = 0; k < 4 * NT; k++) s[k] = 0.f;
+  const df2* P[NT];
+#pragma unroll
+  for (int t = 0; t < NT; t++) P[t] = pool + toff[min(p0 + t, nst - 1)];
+#pragma unroll(4 / NT)
+  for (int r = lane; r < m; r += 32) {
+    const f2 u = uh[r * us];
+#pragma unroll
+    for (int t = 0; t < NT; t++) lead_fma(s[4 * t], s[4 * t + 1], u, P[t][r].hi);
+  }
+#pragma unroll(4 / NT)
+  for (int c = lane; c < n; c += 32) {
+    const f2 v = vh[c * vs];
+#pragma unroll
+    for (int t = 0; t < NT; t++) lead_fma(s[4 * t + 2], s[4 * t + 3], v, P[t][m + c].hi);
+  }
+  // the butterfly's steps in its order: lanes 16 apart, 8, 4, 2, 1
+  if constexpr (NT == 4) {
+    fold<8, 16>(s);
+    fold<4, 8>(s);
+    fold<2, 4>(s);
+    fold<1, 2>(s);
+    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+  } else if constexpr (NT == 2) {
+    fold<4, 16>(s);
+    fold<2, 8>(s);
+    fold<1, 4>(s);
+    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 2);
+    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+  } else {
+    fold<2, 16>(s);
+    fold<1, 8>(s);
+    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 4);
+    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 2);
+    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+  }
+  // the 32 / NT lanes of a term hold Re, Im of u^T U, then Re, Im of v V^T, 8 / NT lanes each
+  constexpr int Q = 8 / NT;
+  const float im = __shfl_down_sync(0xffffffffu, s[0], Q);
+  const float a = sqrtf(s[0] * s[0] + im * im);
+  const float b = __shfl_down_sync(0xffffffffu, a, 2 * Q);
+  const int p = p0 + lane / (4 * Q);
+  if (lane % (4 * Q) == 0 && p < nst) prod[p] = df_prod_ff(a, b);
+}
+
+// Every earlier term, spread over the W warps of a group: as many at a time per warp as leave no
+// warp idle
+template <int W>
+__device__ __forceinline__ void cross_all(int w, int nst, int m, int n, const f2* uh, int us, const f2* vh, int vs,
+                                          const df2* pool, const long long* toff, df64* prod) {
+  if (W > 1 && nst <= W) {
+    for (int p = w; p < nst; p += W) cross_terms<1>(p, nst, m, n, uh, us, vh, vs, pool, toff, prod);
+  } else if (W > 1 && nst <= 2 * W) {
+    for (int p = 2 * w; p < nst; p += 2 * W) cross_terms<2>(p, nst, m, n, uh, us, vh, vs, pool, toff, prod);
+  } else {
+    for (int p = 4 * w; p < nst; p += 4 * W) cross_terms<4>(p, nst, m, n, uh, us, vh, vs, pool, toff, prod);
+  }
+}
+
+// 16 bytes from global to shared memory behind the entry evaluation; visible to the group after
+// cp_async_wait and the group's barrier
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ ulonglong2 lds_pair(uint32_t a) {
+  ulonglong2 v;
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(a) : "memory");
+  return v;
+}
+// Entry e from its items (the six points in order), less the earlier terms:
+// - sum_{p < nst} coef[p] * pool[toff[p] + off], four loads in flight. Out of line like eval_items:
+// the warps of an SM are at different places of the recursion, and its straight-line code in every
+// caller overran the instruction caches (21% of the stalls; 8.9 -> 7.9 ms on the 20480-triangle
+// relief). Loading a group of terms ahead of the arithmetic costs more instructions than it hides.
+__device__ __noinline__ df2 finish_entry(uint32_t b0, uint32_t b1, int e, uint32_t coef, uint32_t toff,
+                                         const df2* pool, int nst) {
+  df2 acc{f2_dup(0.0f), f2_dup(0.0f)};
+#pragma unroll 1
+  for (int h = 3 * e; h < 3 * e + 3; h++) {
+    const ulonglong2 x = lds_pair(b0 + 16 * h), y = lds_pair(b1 + 16 * h);
+    acc = df2_add_prod(x.x, x.y, acc);
+    acc = df2_add_prod(y.x, y.y, acc);
+  }
+  acc = entry_scale(acc);
+#pragma unroll 1
+  for (int p = 0; p < nst; p += 4) {
+    df2 a[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (p + u < nst) {
+        long long o;
+        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(o) : "r"(toff + 8 * (p + u)) : "memory");
+        a[u] = df2_ldc(pool + o);
+      }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (p + u < nst) {
+        const ulonglong2 c = lds_pair(coef + 16 * (p + u));
+        df2_cfms(acc, df2{c.x, c.y}, a[u]);
+      }
+  }
+  return acc;
+}
+
+// Synchronises the W warps of group `grp` of the CTA.
+template <int W>
+__device__ __forceinline__ void group_sync(int grp) {
+  if (W == 1)
+    __syncwarp();
+  else if (W == kDfWarps)
+    __syncthreads();
+  else {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(32 * W) : "memory");
+  }
+}
+
+// (value, index) argmax over the group, first index on ties; sv, si: W slots, free after the next
+// group_sync
+template <int W>
+__device__ __forceinline__ void group_argmax(df64& val, int& idx, df64* sv, int* si, int grp) {
+  warp_argmax_df(val, idx);
+  if (W == 1) return;
+  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) % W;
+  if (lane == 0) {
+    sv[w] = val;
+    si[w] = idx;
+  }
+  group_sync<W>(grp);
+  val = sv[0];
+  idx = si[0];
+#pragma unroll
+  for (int k = 1; k < W; k++)
+    if (sv[k] > val || (sv[k] == val && si[k] < idx)) {
+      val = sv[k];
+      idx = si[k];
     }
-  }
 }
 
-// acc -= sum_{p < nst} coef[p] * pool[toff[p] + off], two loads in flight
-__device__ __forceinline__ void sub_terms_df(cdf& acc, const cdf* coef, const cdf* __restrict__ pool,
-                                             const long long* toff, long long off, int nst) {
-  int p = 0;
-  for (; p + 2 <= nst; p += 2) {
-    const cdf a0 = pool[toff[p] + off], a1 = pool[toff[p + 1] + off];
-    cdf_fms(acc, coef[p], a0);
-    cdf_fms(acc, coef[p + 1], a1);
-  }
-  if (p < nst) cdf_fms(acc, coef[p], pool[toff[p] + off]);
-}
-
-// FP32 complex product of the leading parts: acc += a b
-__device__ __forceinline__ void lead_fma(float& re, float& im, const cdf& a, const cdf& b) {
-  re = fmaf(a.re.hi, b.re.hi, re);
-  re = fmaf(-a.im.hi, b.im.hi, re);
-  im = fmaf(a.re.hi, b.im.hi, im);
-  im = fmaf(a.im.hi, b.re.hi, im);
-}
+// Shared memory of one group of W <= 4 warps (the rows and columns fit in 64 W).
+template <int W>
+struct AcaGroup {
+  static constexpr int kTerms = W == 1 ? 64 : kWarpAcaTerms;  // terms < min(m, n)
+  ulonglong2 b0[96 * W], b1[96 * W];  // items of 32 W entries
+  df2 coef[kTerms];
+  df2 vs[64 * W];                     // the row residual
+  f2 uh[64 * W], vh[64 * W];          // leading parts of the new u and v
+  df64 su[64 * W], sv[64 * W];        // |u_r|^2, |v_c|^2
+  long long toff[kTerms];
+  df64 prod[kTerms];
+  df64 bv[2][W];
+  int bi[2][W];
+  long long base;
+  int ovf;
+};
+static_assert(sizeof(AcaGroup<1>) % 16 == 0 && sizeof(AcaGroup<2>) % 16 == 0 && sizeof(AcaGroup<4>) % 16 == 0,
+              "groups follow one another in shared memory");
 
 // ------------------------------------------------------------------------------------------
-// Warp per block (sides up to 32 LPL): lane l owns rows / columns l + 32 k, the current u and v
-// stay in registers, earlier terms are read from the pool.
+// W warps per block, sides up to 64 W: thread t owns rows and columns t and t + 32 W. The entries of a
+// row or column are evaluated as 3 items each (pairs of quadrature points) spread evenly over the
+// group's threads, because the sides rarely fill the threads: clusters halve from the root, so a
+// mesh's sides are about c, 2 c, 4 c, ... with 16 < c <= 32, and one entry per lane left up to half
+// of the lanes idle (20480 triangles: c = 20). Each entry is then finished by its owner. Sums are
+// taken in one order whatever W: rows and columns l, l + 32, ... by lane l, then the butterfly.
+//
+// Bound by the FP32 pipe (45-50% busy) and, beside it, by instruction supply and latency: the warps
+// are at different places of a long recursion. Four CTAs of 128 threads per SM (128 registers)
+// beat six (80 registers, spills) 4.9 to 6.2 ms on the 20480-triangle relief: more warps thrash L1 and
+// the instruction caches. With the 8-warp blocks' kernel the assembly takes 8.8 instead of 11.0 ms
+// there, 1.77 instead of 2.95 ms on 5280 triangles and 94 instead of 106 ms on 118680 (2 kHz), against
+// one warp per block with scalar arithmetic up to sides of 256.
 // ------------------------------------------------------------------------------------------
-template <int LPL>
-__global__ void __launch_bounds__(256, LPL == 8 ? 1 : 2) aca_df_warp_kernel(AcaDfArgs A, int nblocks) {
-  __shared__ float4 s_tab[kDfTab];
-  __shared__ __align__(16) unsigned char s_raw[8 * kWarpAcaTerms * (2 * sizeof(cdf) + sizeof(long long))];
-  load_table(A.tab, s_tab);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int bi = blockIdx.x * 8 + warp;
-  if (bi >= nblocks) return;
-  cdf* uq = reinterpret_cast<cdf*>(s_raw) + warp * kWarpAcaTerms;
-  cdf* vq = reinterpret_cast<cdf*>(s_raw) + (8 + warp) * kWarpAcaTerms;
-  long long* toff = reinterpret_cast<long long*>(s_raw + 16 * kWarpAcaTerms * sizeof(cdf)) + warp * kWarpAcaTerms;
-  const int b = A.order[bi];
+template <int W>
+__device__ __forceinline__ void aca_small(const AcaDfArgs& A, unsigned char* smem, int b) {
+  constexpr int T = 32 * W;
+  const int grp = (threadIdx.x >> 5) / W;
+  AcaGroup<W>& S = reinterpret_cast<AcaGroup<W>*>(smem)[grp];
+  const uint32_t b0 = shared_addr(S.b0), b1 = shared_addr(S.b1), coef = shared_addr(S.coef), toff = shared_addr(S.toff);
+  const int tid = threadIdx.x % T, lane = threadIdx.x & 31, gw = tid >> 5;
   const int4 q = A.blocks[b];
   const int rs = q.x, cs = q.z, m = q.y - q.x, n = q.w - q.z;
   int iter_lim = min(A.maxk, min(m - 1, n - 1));
   if (iter_lim < 0) iter_lim = 0;
-  if (iter_lim > kWarpAcaTerms) iter_lim = kWarpAcaTerms;  // the host routes only blocks that fit
+  if (iter_lim > AcaGroup<W>::kTerms) iter_lim = AcaGroup<W>::kTerms;  // the host routes only blocks that fit
 
+  // every warp of the group reaches the same verdict by itself
   if (iter_lim > 0 &&
       zero_block(A, rs, m, cs, n, lane, 32, [](bool ok) { return __all_sync(0xffffffffu, ok) != 0; })) {
-    if (lane == 0) {
+    if (tid == 0) {
       A.rank[b] = 0;
       if (A.passes) A.passes[b] = 0;
     }
     return;
   }
 
-  unsigned used_l = lane == 0 ? 1u : 0u;  // bit k: row lane + 32 k is used (row 0 first)
+  unsigned used = tid == 0 ? 1u : 0u;  // bit k: row tid + T k is used (row 0 first)
   df64 err{0.0f, 0.0f};
   int i = 0, iter = 0, nst = 0, npass = 0;
   bool need_alloc = true;
   long long base = 0;
-  cdf u_l[LPL], v_l[LPL];
+  int nfree = 0;
   while (iter < iter_lim) {
     if (need_alloc) {
-      unsigned long long bb = 0;
-      int ovf = 0;
-      if (lane == 0) {
-        const unsigned long long need = (unsigned long long)(m + n);
-        bb = atomicAdd(A.pool_used, need);
-        ovf = bb + need > (unsigned long long)A.pool_cap;
-        if (ovf) atomicOr(A.status, 1);
+      // a term's place in the pool; taken for several terms at a time (never more than the block
+      // can have), because every iteration would wait for the atomic's round trip
+      if (nfree == 0) {
+        nfree = min(kAllocTerms, iter_lim - iter);
+        if (tid == 0) {
+          const unsigned long long need = (unsigned long long)(m + n) * nfree;
+          const unsigned long long bb = atomicAdd(A.pool_used, need);
+          S.ovf = bb + need > (unsigned long long)A.pool_cap;
+          S.base = (long long)bb;
+          if (S.ovf) atomicOr(A.status, 1);
+        }
+        group_sync<W>(grp);
+        if (S.ovf) break;
+        base = S.base;
+      } else {
+        base += m + n;
       }
-      ovf = __shfl_sync(0xffffffffu, ovf, 0);
-      if (ovf) break;
-      base = (long long)__shfl_sync(0xffffffffu, bb, 0);
+      nfree--;
       need_alloc = false;
     }
     npass++;
-    cdf* unew = A.pool + base;
-    cdf* vnew = unew + m;
-    for (int p = lane; p < nst; p += 32) uq[p] = A.pool[toff[p] + i];
-    __syncwarp();
-    // row residual and column pivot
-    const DfPt* pi = A.pts + rs + i;
+    df2* unew = A.pool + base;
+    df2* vnew = unew + m;
+    // row residual v = M(i, :) - U(i, :) V and column pivot
+    for (int p = tid; p < nst; p += T) cp_async_16(coef + 16 * p, A.pool + S.toff[p] + i);
     df64 best{-1.0f, 0.0f};
     int bidx = 0;
-#pragma unroll
-    for (int kk = 0; kk < LPL; kk++) {
-      const int c = lane + 32 * kk;
+#pragma unroll 1
+    for (int c0 = 0; c0 < n; c0 += T) {
+      if (c0) group_sync<W>(grp);  // the first entries are finished
+      eval_items(A.k, A.pts + rs + i, 0, A.el + cs + c0, 1, min(T, n - c0), tid, T, b0, b1);
+      cp_async_wait();
+      group_sync<W>(grp);
+      const int c = c0 + tid;
       if (c < n) {
-        cdf v = entry_df_call(A.k, pi, A.el + cs + c, s_tab);
-        sub_terms_df(v, uq, A.pool, toff, (long long)m + c, nst);
-        v_l[kk] = v;
-        const df64 a = cdf_abs2(v);
+        const df2 v = finish_entry(b0, b1, tid, coef, toff, A.pool + m + c, nst);
+        df2_stc(&S.vs[c], v);
+        const df64 a = df2_abs2(v);
         if (a > best) {
           best = a;
           bidx = c;
         }
       }
     }
-    warp_argmax_df(best, bidx);
+    if (W == 1) __syncwarp();
+    group_argmax<W>(best, bidx, S.bv[0], S.bi[0], grp);
     const int j = bidx;
-    cdf mine = v_l[0];
-#pragma unroll
-    for (int kk = 1; kk < LPL; kk++)
-      if (kk == (j >> 5)) mine = v_l[kk];
-    const cdf vj{shfl_df(mine.re, j & 31), shfl_df(mine.im, j & 31)};
-    for (int p = lane; p < nst; p += 32) vq[p] = A.pool[toff[p] + m + j];
-    __syncwarp();
+    const cdf vj = df2_to_cdf(df2_ldc(&S.vs[j]));
+    for (int p = tid; p < nst; p += T) cp_async_16(coef + 16 * p, A.pool + S.toff[p] + m + j);
     const bool keep = df_is_zero(vj.re) && df_is_zero(vj.im);
     const CdfDivisor dv = keep ? CdfDivisor{cdf{}, 1.0f} : cdf_divisor(vj);
-    df64 vn{0.0f, 0.0f};
-#pragma unroll
-    for (int kk = 0; kk < LPL; kk++) {
-      const int c = lane + 32 * kk;
-      if (c < n) {
-        cdf v = v_l[kk];
-        if (!keep) v = cdf_divide(v, dv);
-        v_l[kk] = v;
-        vnew[c] = v;
-        vn += cdf_abs2(v);
-      }
+#pragma unroll 1
+    for (int c = tid; c < n; c += T) {
+      df2 v = df2_ldc(&S.vs[c]);
+      if (!keep) v = df2_cdivide(v, dv);
+      df2_stc(vnew + c, v);
+      S.vh[c] = v.hi;
+      S.sv[c] = df2_abs2(v);
     }
-    // column residual
-    df64 un{0.0f, 0.0f};
-#pragma unroll
-    for (int kk = 0; kk < LPL; kk++) {
-      const int r = lane + 32 * kk;
+    // column residual u = M(:, j) - U V(:, j)
+#pragma unroll 1
+    for (int r0 = 0; r0 < m; r0 += T) {
+      if (r0) group_sync<W>(grp);
+      eval_items(A.k, A.pts + rs + r0, 1, A.el + cs + j, 0, min(T, m - r0), tid, T, b0, b1);
+      cp_async_wait();
+      group_sync<W>(grp);
+      const int r = r0 + tid;
       if (r < m) {
-        cdf u = entry_df_call(A.k, A.pts + rs + r, A.el + cs + j, s_tab);
-        sub_terms_df(u, vq, A.pool, toff, (long long)r, nst);
-        u_l[kk] = u;
-        unew[r] = u;
-        un += cdf_abs2(u);
+        const df2 u = finish_entry(b0, b1, tid, coef, toff, A.pool + r, nst);
+        df2_stc(unew + r, u);
+        S.uh[r] = u.hi;
+        S.su[r] = df2_abs2(u);
       }
     }
-    // cross terms sum_q |u^T U_q| |v V_q^T| (FP32 on the leading parts, exact products summed as
-    // double-floats: all on the FP32 pipes)
+    group_sync<W>(grp);
+    // norms, every warp the same sums; cross terms sum_q |u^T U_q| |v V_q^T| (FP32 on the leading
+    // parts, exact products summed as double-floats), the earlier terms over the warps
+    df64 un{0.0f, 0.0f}, vn{0.0f, 0.0f};
+    for (int c = lane; c < n; c += 32) vn += S.sv[c];
+    for (int r = lane; r < m; r += 32) un += S.su[r];
+    warp_sum2_df(un, vn);
+    const df64 unt = un, vnt = vn;
+    cross_all<W>(gw, nst, m, n, S.uh, 1, S.vh, 1, A.pool, S.toff, S.prod);
+    group_sync<W>(grp);
     df64 dots{0.0f, 0.0f};
-    for (int p = 0; p < nst; p++) {
-      const cdf* Up = A.pool + toff[p];
-      const cdf* Vp = Up + m;
-      float udr = 0.f, udi = 0.f, vdr = 0.f, vdi = 0.f;
-#pragma unroll
-      for (int kk = 0; kk < LPL; kk++) {
-        const int r = lane + 32 * kk;
-        if (r < m) lead_fma(udr, udi, u_l[kk], Up[r]);
-        if (r < n) lead_fma(vdr, vdi, v_l[kk], Vp[r]);
-      }
-      udr = warp_sum(udr);
-      udi = warp_sum(udi);
-      vdr = warp_sum(vdr);
-      vdi = warp_sum(vdi);
-      dots += df_prod_ff(sqrtf(udr * udr + udi * udi), sqrtf(vdr * vdr + vdi * vdi));
-    }
-    const df64 unt = warp_sum_df(un), vnt = warp_sum_df(vn);
+    for (int p = 0; p < nst; p++) dots += S.prod[p];
     const df64 uv = unt * vnt;
     err += uv + df_ldexp(dots, 2.0f);
     if (aca_converged(uv, err, A.eps2)) break;
@@ -283,104 +488,69 @@ __global__ void __launch_bounds__(256, LPL == 8 ? 1 : 2) aca_df_warp_kernel(AcaD
     // next row pivot over unused rows
     best = df64{-1.0f, 0.0f};
     bidx = 0;
-#pragma unroll
-    for (int kk = 0; kk < LPL; kk++) {
-      const int r = lane + 32 * kk;
-      if (r < m && !((used_l >> kk) & 1u)) {
-        const df64 a = cdf_abs2(u_l[kk]);
+#pragma unroll 1
+    for (int kk = 0; kk < 2; kk++) {
+      const int r = tid + kk * T;
+      if (r < m && !((used >> kk) & 1u)) {
+        const df64 a = S.su[r];
         if (a > best) {
           best = a;
           bidx = r;
         }
       }
     }
-    warp_argmax_df(best, bidx);
+    if (!zero_term && tid == 0) {
+      S.toff[nst] = base;
+      A.term_off[(long long)b * A.maxk + nst] = base;
+    }
+    group_argmax<W>(best, bidx, S.bv[1], S.bi[1], grp);
     i = bidx;
-    if (lane == (i & 31)) used_l |= 1u << (i >> 5);
+    if (tid == (i % T)) used |= 1u << (i / T);
     if (!zero_term) {
-      if (lane == 0) {
-        toff[nst] = base;
-        A.term_off[(long long)b * A.maxk + nst] = base;
-      }
       nst++;
       need_alloc = true;
     }
     iter++;
-    __syncwarp();
+    if (W == 1) __syncwarp();
   }
-  if (lane == 0) {
+  if (tid == 0) {
     A.rank[b] = nst;
     if (A.passes) A.passes[b] = npass;
   }
 }
 
 // ------------------------------------------------------------------------------------------
-// One CTA per block (blocks with a side above 256).
+// One CTA per block (blocks with a side above 256, or more terms than the groups hold): thread t
+// owns rows and columns t + 256 k, kept in the pool. Sums: by thread, then over the warps.
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void block_argmax_df(df64& val, int& idx, df64* sv, int* si) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  warp_argmax_df(val, idx);
-  if (lane == 0) {
-    sv[w] = val;
-    si[w] = idx;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    df64 bv = sv[0];
-    int bi = si[0];
-    for (int k = 1; k < kDfWarps; k++)
-      if (sv[k] > bv || (sv[k] == bv && si[k] < bi)) {
-        bv = sv[k];
-        bi = si[k];
-      }
-    sv[0] = bv;
-    si[0] = bi;
-  }
-  __syncthreads();
-  val = sv[0];
-  idx = si[0];
-  __syncthreads();
+// Shared memory of a CTA block beside its coefficients, term offsets and used-row bits
+struct AcaCta {
+  ulonglong2 b0[3 * kDfThreads], b1[3 * kDfThreads];
+  df64 bv[2][kDfWarps];
+  int bi[2][kDfWarps];
+  df64 sd[2][kDfWarps];
+  long long base;
+  int ovf, pad;
+};
+static_assert(sizeof(AcaCta) % 16 == 0, "the coefficients follow");
+
+static size_t aca_cta_smem(int iter_cap, int max_rows) {
+  return sizeof(AcaCta) + (size_t)iter_cap * (sizeof(df2) + sizeof(long long) + sizeof(df64)) + (size_t)((max_rows + 31) / 32) * 4;
 }
 
-// Sum over the CTA: warp sums, then the warps' sums in order by thread 0; every thread gets it.
-__device__ __forceinline__ df64 block_sum_df(df64 v, df64* sd) {
-  v = warp_sum_df(v);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) sd[w] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    df64 s = sd[0];
-    for (int k = 1; k < kDfWarps; k++) s += sd[k];
-    sd[0] = s;
-  }
-  __syncthreads();
-  v = sd[0];
-  __syncthreads();
-  return v;
-}
-
-__global__ void __launch_bounds__(kDfThreads) aca_df_kernel(AcaDfArgs A) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ float4 s_tab[kDfTab];
-  __shared__ df64 s_rv[kDfWarps];
-  __shared__ int s_ri[kDfWarps];
-  __shared__ df64 s_d[kDfWarps];
-  __shared__ long long s_base;
-  __shared__ int s_flag;
-  load_table(A.tab, s_tab);
-
-  const int b = A.order[blockIdx.x];
+__device__ __forceinline__ void aca_cta(const AcaDfArgs& A, unsigned char* smem, int b) {
+  AcaCta& S = *reinterpret_cast<AcaCta*>(smem);
+  df2* coef = reinterpret_cast<df2*>(smem + sizeof(AcaCta));
+  long long* toff = reinterpret_cast<long long*>(coef + A.iter_cap);
+  df64* prod = reinterpret_cast<df64*>(toff + A.iter_cap);
+  unsigned* used = reinterpret_cast<unsigned*>(prod + A.iter_cap);
+  const uint32_t b0 = shared_addr(S.b0), b1 = shared_addr(S.b1), coef_a = shared_addr(coef), toff_a = shared_addr(toff);
   const int4 q = A.blocks[b];
   const int rs = q.x, cs = q.z, m = q.y - q.x, n = q.w - q.z;
   int iter_lim = min(A.maxk, min(m - 1, n - 1));
   if (iter_lim < 0) iter_lim = 0;
   if (iter_lim > A.iter_cap) iter_lim = A.iter_cap;  // host guarantees iter_cap >= every iter_lim
-
-  cdf* uq = reinterpret_cast<cdf*>(smem_raw);
-  cdf* vq = uq + A.iter_cap;
-  long long* toff = reinterpret_cast<long long*>(vq + A.iter_cap);
-  unsigned* used = reinterpret_cast<unsigned*>(toff + A.iter_cap);
-  const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, T = kDfThreads, lane = tid & 31, warp = tid >> 5;
 
   if (A.zero_guard && iter_lim > 0 &&
       zero_block(A, rs, m, cs, n, tid, T, [](bool ok) { return __syncthreads_and(ok) != 0; })) {
@@ -391,10 +561,8 @@ __global__ void __launch_bounds__(kDfThreads) aca_df_kernel(AcaDfArgs A) {
     return;
   }
 
-  for (int w = tid; w < (m + 31) / 32; w += T) used[w] = 0;
-  __syncthreads();
-  if (tid == 0) used[0] = 1u;
-  df64 err{0.0f, 0.0f};  // meaningful in thread 0
+  for (int w = tid; w < (m + 31) / 32; w += T) used[w] = w == 0 ? 1u : 0u;
+  df64 err{0.0f, 0.0f};
   int i = 0, iter = 0, nst = 0, npass = 0;
   bool need_alloc = true;
   __syncthreads();
@@ -404,84 +572,92 @@ __global__ void __launch_bounds__(kDfThreads) aca_df_kernel(AcaDfArgs A) {
       if (tid == 0) {
         const unsigned long long need = (unsigned long long)(m + n);
         const unsigned long long bb = atomicAdd(A.pool_used, need);
-        s_flag = (bb + need > (unsigned long long)A.pool_cap) ? 1 : 0;
-        s_base = (long long)bb;
-        if (s_flag) atomicOr(A.status, 1);
+        S.ovf = (bb + need > (unsigned long long)A.pool_cap) ? 1 : 0;
+        S.base = (long long)bb;
+        if (S.ovf) atomicOr(A.status, 1);
       }
       __syncthreads();
-      if (s_flag) break;
+      if (S.ovf) break;
       need_alloc = false;
     }
     npass++;
-    cdf* unew = A.pool + s_base;
-    cdf* vnew = unew + m;
-    for (int p = tid; p < nst; p += T) uq[p] = A.pool[toff[p] + i];
-    __syncthreads();
+    const long long base = S.base;
+    df2* unew = A.pool + base;
+    df2* vnew = unew + m;
+    for (int p = tid; p < nst; p += T) df2_stc(&coef[p], df2_ldc(A.pool + toff[p] + i));
 
     // row residual v = M(i, :) - U(i, :) V
-    const DfPt* pi = A.pts + rs + i;
     df64 best{-1.0f, 0.0f};
     int bidx = 0;
-    for (int c = tid; c < n; c += T) {
-      cdf v = entry_df_call(A.k, pi, A.el + cs + c, s_tab);
-      sub_terms_df(v, uq, A.pool, toff, (long long)m + c, nst);
-      vnew[c] = v;
-      const df64 a = cdf_abs2(v);
-      if (a > best) {
-        best = a;
-        bidx = c;
+    for (int c0 = 0; c0 < n; c0 += T) {
+      if (c0) __syncthreads();  // the previous entries are finished
+      eval_items(A.k, A.pts + rs + i, 0, A.el + cs + c0, 1, min(T, n - c0), tid, T, b0, b1);
+      __syncthreads();
+      const int c = c0 + tid;
+      if (c < n) {
+        const df2 v = finish_entry(b0, b1, tid, coef_a, toff_a, A.pool + m + c, nst);
+        df2_stc(vnew + c, v);
+        const df64 a = df2_abs2(v);
+        if (a > best) {
+          best = a;
+          bidx = c;
+        }
       }
     }
-    block_argmax_df(best, bidx, s_rv, s_ri);
+    group_argmax<kDfWarps>(best, bidx, S.bv[0], S.bi[0], 0);
     const int j = bidx;
-    const cdf vj = vnew[j];
-    for (int p = tid; p < nst; p += T) vq[p] = A.pool[toff[p] + m + j];
-    __syncthreads();
+    const cdf vj = df2_to_cdf(df2_ldc(vnew + j));
+    for (int p = tid; p < nst; p += T) df2_stc(&coef[p], df2_ldc(A.pool + toff[p] + m + j));
+    __syncthreads();  // v_j is read before it is divided
     const bool keep = A.zero_guard && df_is_zero(vj.re) && df_is_zero(vj.im);
     const CdfDivisor dv = keep ? CdfDivisor{cdf{}, 1.0f} : cdf_divisor(vj);
     df64 vn{0.0f, 0.0f};
     for (int c = tid; c < n; c += T) {
-      cdf v = vnew[c];
-      if (!keep) v = cdf_divide(v, dv);
-      vnew[c] = v;
-      vn += cdf_abs2(v);
+      df2 v = df2_ldc(vnew + c);
+      if (!keep) v = df2_cdivide(v, dv);
+      df2_stc(vnew + c, v);
+      vn += df2_abs2(v);
     }
 
     // column residual u = M(:, j) - U V(:, j)
     df64 un{0.0f, 0.0f};
-    for (int r = tid; r < m; r += T) {
-      cdf u = entry_df_call(A.k, A.pts + rs + r, A.el + cs + j, s_tab);
-      sub_terms_df(u, vq, A.pool, toff, (long long)r, nst);
-      unew[r] = u;
-      un += cdf_abs2(u);
+    for (int r0 = 0; r0 < m; r0 += T) {
+      if (r0) __syncthreads();
+      eval_items(A.k, A.pts + rs + r0, 1, A.el + cs + j, 0, min(T, m - r0), tid, T, b0, b1);
+      __syncthreads();
+      const int r = r0 + tid;
+      if (r < m) {
+        const df2 u = finish_entry(b0, b1, tid, coef_a, toff_a, A.pool + r, nst);
+        df2_stc(unew + r, u);
+        un += df2_abs2(u);
+      }
     }
     __syncthreads();
 
-    // cross terms (one warp per earlier stored term, FP32 on the leading parts, exact products
-    // summed as double-floats)
-    df64 dots{0.0f, 0.0f};
-    for (int p = warp; p < nst; p += kDfWarps) {
-      const cdf* Up = A.pool + toff[p];
-      const cdf* Vp = Up + m;
-      float udr = 0.f, udi = 0.f, vdr = 0.f, vdi = 0.f;
-      for (int r = lane; r < m; r += 32) lead_fma(udr, udi, unew[r], Up[r]);
-      for (int c = lane; c < n; c += 32) lead_fma(vdr, vdi, vnew[c], Vp[c]);
-      udr = warp_sum(udr);
-      udi = warp_sum(udi);
-      vdr = warp_sum(vdr);
-      vdi = warp_sum(vdi);
-      if (lane == 0) dots += df_prod_ff(sqrtf(udr * udr + udi * udi), sqrtf(vdr * vdr + vdi * vdi));
-    }
-    const df64 unt = block_sum_df(un, s_d);
-    const df64 vnt = block_sum_df(vn, s_d);
-    dots = block_sum_df(lane == 0 ? dots : df64{0.0f, 0.0f}, s_d);
-    if (tid == 0) {
-      const df64 uv = unt * vnt;
-      err += uv + df_ldexp(dots, 2.0f);
-      s_flag = aca_converged(uv, err, A.eps2) ? 1 : 0;
+    // cross terms and the norms; then the products in the order of one
+    // running sum per warp w over the terms w, w + 8, ..., and the eight sums in order
+    cross_all<kDfWarps>(warp, nst, m, n, &unew->hi, 2, &vnew->hi, 2, A.pool, toff, prod);
+    warp_sum2_df(un, vn);
+    if (lane == 0) {
+      S.sd[0][warp] = un;
+      S.sd[1][warp] = vn;
     }
     __syncthreads();
-    if (s_flag) break;
+    df64 unt = S.sd[0][0], vnt = S.sd[1][0];
+#pragma unroll 1
+    for (int k = 1; k < kDfWarps; k++) {
+      unt += S.sd[0][k];
+      vnt += S.sd[1][k];
+    }
+    df64 part{0.0f, 0.0f};
+    if (lane < kDfWarps)
+      for (int p = lane; p < nst; p += kDfWarps) part += prod[p];
+    df64 dots = shfl_df(part, 0);
+#pragma unroll 1
+    for (int k = 1; k < kDfWarps; k++) dots += shfl_df(part, k);
+    const df64 uv = unt * vnt;
+    err += uv + df_ldexp(dots, 2.0f);
+    if (aca_converged(uv, err, A.eps2)) break;
     const bool zero_term = df_is_zero(unt) || df_is_zero(vnt);
 
     // next row pivot: first max |u|^2 over unused rows
@@ -489,19 +665,19 @@ __global__ void __launch_bounds__(kDfThreads) aca_df_kernel(AcaDfArgs A) {
     bidx = 0;
     for (int r = tid; r < m; r += T) {
       if ((used[r >> 5] >> (r & 31)) & 1u) continue;
-      const df64 a = cdf_abs2(unew[r]);
+      const df64 a = df2_abs2(df2_ldc(unew + r));
       if (a > best) {
         best = a;
         bidx = r;
       }
     }
-    block_argmax_df(best, bidx, s_rv, s_ri);
+    group_argmax<kDfWarps>(best, bidx, S.bv[1], S.bi[1], 0);
     i = bidx;
     if (tid == 0) {
       used[i >> 5] |= 1u << (i & 31);
       if (!zero_term) {
-        toff[nst] = s_base;
-        A.term_off[(long long)b * A.maxk + nst] = s_base;
+        toff[nst] = base;
+        A.term_off[(long long)b * A.maxk + nst] = base;
       }
     }
     if (!zero_term) {
@@ -517,14 +693,43 @@ __global__ void __launch_bounds__(kDfThreads) aca_df_kernel(AcaDfArgs A) {
   }
 }
 
+__global__ void __launch_bounds__(kDfThreads, 2) aca_df_cta_kernel(AcaDfArgs A) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  load_table(A.tab);
+  aca_cta(A, smem_raw, A.order[blockIdx.x]);
+}
+
+// The blocks of sides up to 256 in one launch, longest first (the hardware dispatches CTAs in index
+// order): CTAs of one 4-warp, two 2-warp or four 1-warp groups.
+__global__ void __launch_bounds__(kSmallThreads, 4) aca_df_kernel(AcaDfArgs A) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  load_table(A.tab);
+  const int warp = threadIdx.x >> 5;
+  int cta = blockIdx.x;
+  const int* order = A.order + A.split[0];
+  if (cta < A.split[1]) return aca_small<4>(A, smem_raw, order[cta]);
+  cta -= A.split[1];
+  order += A.split[1];
+  const int n2 = (A.split[2] + 1) / 2;
+  if (cta < n2) {
+    const int bi = 2 * cta + warp / 2;
+    if (bi < A.split[2]) aca_small<2>(A, smem_raw, order[bi]);
+    return;
+  }
+  cta -= n2;
+  order += A.split[2];
+  const int bi = 4 * cta + warp;
+  if (bi < A.split[3]) aca_small<1>(A, smem_raw, order[bi]);
+}
+
 // ------------------------------------------------------------------------------------------
 // Near field: one CTA per block, one thread per entry, rounded to complex FP32.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) near_df_kernel(const DfPt* __restrict__ pts, const DfElem* __restrict__ el,
                                                       const float4* __restrict__ tab, const int4* __restrict__ blocks,
                                                       const long long* __restrict__ near_off, df64 k, cf* out) {
-  __shared__ float4 s_tab[kDfTab];
-  load_table(tab, s_tab);
+  load_table(tab);
+  const float4* s_tab = s_table();
   const int b = blockIdx.x;
   const int4 q = blocks[b];
   const int m = q.y - q.x, n = q.w - q.z;
@@ -532,8 +737,8 @@ __global__ void __launch_bounds__(256) near_df_kernel(const DfPt* __restrict__ p
   const int mn = m * n;
   for (int t = threadIdx.x; t < mn; t += blockDim.x) {
     const int c = t / m, r = t - c * m;
-    const cdf v = entry_df(k, pts + q.x + r, el + q.z + c, s_tab);
-    dst[t] = cf(v.re.hi, v.im.hi);
+    const df2 v = entry_df(k, pts + q.x + r, el + q.z + c, s_tab);
+    dst[t] = cf(f2_x(v.hi), f2_y(v.hi));
   }
 }
 
@@ -546,12 +751,31 @@ void launch_near_assembly_df(const DevGeometry& G, const DevPartition& DP, DevHM
   AC3D_CUDA(cudaGetLastError());
 }
 
-template <int LPL>
-static void aca_df_launch_warp(const AcaDfArgs& a, int nblocks, cudaStream_t s) {
-  if (nblocks <= 0) return;
-  note_launch();
-  aca_df_warp_kernel<LPL><<<(nblocks + 7) / 8, 256, 0, s>>>(a, nblocks);
-  AC3D_CUDA(cudaGetLastError());
+constexpr size_t kAcaSmemMax = 200 * 1024;
+
+// Blocks above 256 on s_large, the others on s_small.
+static void launch_aca_kernels(const AcaDfArgs& a, int max_rows, cudaStream_t s_large, cudaStream_t s_small) {
+  if (a.split[0] > 0) {
+    const size_t smem = aca_cta_smem(a.iter_cap, max_rows);
+    if (smem > kAcaSmemMax) throw Error(4, "ACA block too large for shared memory");
+    // once per process, to the largest size any launch uses: contexts on other threads launch with
+    // other sizes
+    static std::once_flag once;
+    std::call_once(once, [] {
+      AC3D_CUDA(cudaFuncSetAttribute(aca_df_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAcaSmemMax));
+    });
+    note_launch();
+    aca_df_cta_kernel<<<a.split[0], kDfThreads, smem, s_large>>>(a);
+    AC3D_CUDA(cudaGetLastError());
+  }
+  const int ctas = a.split[1] + (a.split[2] + 1) / 2 + (a.split[3] + 3) / 4;
+  if (ctas > 0) {
+    constexpr size_t smem = std::max({sizeof(AcaGroup<4>), 2 * sizeof(AcaGroup<2>), 4 * sizeof(AcaGroup<1>)});
+    static_assert(smem <= 48 * 1024, "no opt-in needed");
+    note_launch();
+    aca_df_kernel<<<ctas, kSmallThreads, smem, s_small>>>(a);
+    AC3D_CUDA(cudaGetLastError());
+  }
 }
 
 void launch_aca_df(const DevGeometry& G, const DevPartition& DP, DevHMat& H, double eps, int max_rows, cudaStream_t s,
@@ -559,37 +783,20 @@ void launch_aca_df(const DevGeometry& G, const DevPartition& DP, DevHMat& H, dou
   if (DP.na == 0) return;
   AcaDfArgs a{G.cen.as<double4>(), G.va.as<double4>(), G.eg64.as<ElemGeo<double>>(), G.cen_df.as<DfPt>(),
               G.el_df.as<DfElem>(), G.df_tab.as<float4>(), DP.blocks_a.as<int4>(), DP.aca_order.as<int>(),
-              df_from_double(H.k), eps, df_from_double(eps * eps), H.maxk, H.maxk, H.pool.as<cdf>(), H.pool_cap,
+              {DP.aca_split[0], DP.aca_split[1], DP.aca_split[2], DP.aca_split[3]},
+              df_from_double(H.k), eps, df_from_double(eps * eps), H.maxk, H.maxk, H.pool.as<df2>(), H.pool_cap,
               H.pool_used.as<unsigned long long>(), H.term_off.as<long long>(), H.rank.as<int>(),
               (int*)(H.pool_used.as<unsigned long long>() + 1), H.passes.as<int>(), 1};
-  // same grouping and stream split as launch_aca: CTA blocks, then warp blocks up to 256 / 128 / 64
-  const int* order = DP.aca_order.as<int>();
-  const int o1 = DP.aca_split[0], o2 = o1 + DP.aca_split[1], o3 = o2 + DP.aca_split[2];
-  if (DP.aca_split[0] > 0) {
-    const size_t smem = (size_t)a.iter_cap * (2 * sizeof(cdf) + sizeof(long long)) + (size_t)((max_rows + 31) / 32) * 4;
-    if (smem > 48 * 1024) {
-      if (smem > 200 * 1024) throw Error(4, "ACA block too large for shared memory");
-      AC3D_CUDA(cudaFuncSetAttribute(aca_df_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    }
-    note_launch();
-    aca_df_kernel<<<DP.aca_split[0], kDfThreads, smem, s>>>(a);
-    AC3D_CUDA(cudaGetLastError());
-  }
-  a.order = order + o1;
-  aca_df_launch_warp<8>(a, DP.aca_split[1], s_small);
-  a.order = order + o2;
-  aca_df_launch_warp<4>(a, DP.aca_split[2], s);
-  a.order = order + o3;
-  aca_df_launch_warp<2>(a, DP.aca_split[3], s_small);
+  launch_aca_kernels(a, max_rows, s, s_small);
 }
 
 // Receiver ACA (compute_ACA_listener, aca.cpp:84-134: one block of L receivers x Ne elements, no
 // zero guard) in double-float, then the terms converted in place to complex FP64 (same size).
-__global__ void cdf_to_cd_kernel(cdf* pool, const unsigned long long* used) {
+__global__ void df_to_cd_kernel(df2* pool, const unsigned long long* used) {
   const unsigned long long n = *used;
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (unsigned long long)gridDim.x * blockDim.x) {
-    const cdf v = pool[i];
+    const cdf v = df2_to_cdf(df2_ldc(pool + i));
     reinterpret_cast<cd*>(pool)[i] = cd(df_to_double(v.re), df_to_double(v.im));
   }
 }
@@ -600,18 +807,14 @@ void launch_listener_aca_df(const DevGeometry& G, const void* pts_df, int L, dou
   int iter_lim = std::min(maxk, std::min(L - 1, G.ne - 1));
   if (iter_lim < 1) iter_lim = 1;
   AcaDfArgs a{G.cen.as<double4>(), G.va.as<double4>(), G.eg64.as<ElemGeo<double>>(), (const DfPt*)pts_df,
-              G.el_df.as<DfElem>(), G.df_tab.as<float4>(), block, order, df_from_double(k), eps,
+              G.el_df.as<DfElem>(), G.df_tab.as<float4>(), block, order, {1, 0, 0, 0}, df_from_double(k), eps,
               df_from_double(eps * eps), maxk, iter_lim,
-              (cdf*)pool, pool_cap, used, term_off, rank, status, nullptr, 0};
-  const size_t smem = (size_t)iter_lim * (2 * sizeof(cdf) + sizeof(long long)) + (size_t)((L + 31) / 32) * 4;
-  if (smem > 200 * 1024) throw Error(4, "receiver ACA too large for shared memory (at most about 5000 receivers)");
-  if (smem > 48 * 1024)
-    AC3D_CUDA(cudaFuncSetAttribute(aca_df_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+              (df2*)pool, pool_cap, used, term_off, rank, status, nullptr, 0};
+  if (aca_cta_smem(iter_lim, L) > kAcaSmemMax)
+    throw Error(4, "receiver ACA too large for shared memory (at most about 5000 receivers)");
+  launch_aca_kernels(a, L, s, s);
   note_launch();
-  aca_df_kernel<<<1, kDfThreads, smem, s>>>(a);
-  AC3D_CUDA(cudaGetLastError());
-  note_launch();
-  cdf_to_cd_kernel<<<4 * device_sm_count(), 256, 0, s>>>((cdf*)pool, used);
+  df_to_cd_kernel<<<4 * device_sm_count(), 256, 0, s>>>((df2*)pool, used);
   AC3D_CUDA(cudaGetLastError());
 }
 

@@ -234,16 +234,16 @@ std::unique_ptr<DevHMat> assemble(ac3d_ctx* c, double k, int prec) {
       cudaStreamWaitEvent(c->stream, c->ev_join, 0);
     }
   } join_assembly{c};
-  if (H->pool_df)
-    launch_near_assembly_df(c->m->G, c->m->DP, *H, as);
-  else
+  const int na = c->m->DP.na;
+  if (!H->pool_df)
     launch_near_assembly(c->m->G, c->m->DP, *H, as);
+  else if (na == 0)
+    launch_near_assembly_df(c->m->G, c->m->DP, *H, as);
   H->err.alloc(16, s);
   AC3D_CUDA(cudaMemsetAsync(H->err.p, 0, 16, s));
   H->ticket.alloc(16, s);
   AC3D_CUDA(cudaMemsetAsync(H->ticket.p, 0, 16, s));
 
-  const int na = c->m->DP.na;
   H->rank.alloc((size_t)std::max(na, 1) * sizeof(int), s);
   H->passes.alloc((size_t)std::max(na, 1) * sizeof(int), s);
   H->t_off.alloc((size_t)(na + 1) * sizeof(int), s);
@@ -258,13 +258,16 @@ std::unique_ptr<DevHMat> assemble(ac3d_ctx* c, double k, int prec) {
       H->pool.alloc((size_t)cap * pool_es, s);
       H->pool_cap = cap;
       AC3D_CUDA(cudaMemsetAsync(H->pool_used.p, 0, 16, s));
-      // the ACA groups on the two assembly streams (the first after the near field)
+      // FP32 and FP64: the ACA groups on the two assembly streams (the first after the near field).
+      // Double-float: the ACA first, longest blocks first, and the near field behind its large
+      // blocks, whose short CTAs fill the SMs as the blocks run out
       AC3D_CUDA(cudaEventRecord(c->ev_fork, s));
       AC3D_CUDA(cudaStreamWaitEvent(as, c->ev_fork, 0));
       AC3D_CUDA(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-      if (H->pool_df)
+      if (H->pool_df) {
         launch_aca_df(c->m->G, c->m->DP, *H, c->aca_tol, c->m->P.max_rows, as, c->side);
-      else
+        if (attempt == 0) launch_near_assembly_df(c->m->G, c->m->DP, *H, as);
+      } else
         launch_aca(c->m->G, c->m->DP, *H, c->aca_tol, c->m->P.max_rows, as, c->side);
       AC3D_CUDA(cudaEventRecord(c->ev_join, c->side));
       AC3D_CUDA(cudaEventRecord(c->ev_join_asm, as));

@@ -238,12 +238,12 @@ struct CdfDivisor {
   cdf inv;  // conj(w) / |w|^2
   float sc;
 };
-__host__ __device__ __forceinline__ CdfDivisor cdf_divisor(cdf d) {
+__device__ __forceinline__ CdfDivisor cdf_divisor(cdf d) {
   const float a = fmaxf(fabsf(d.re.hi), fabsf(d.im.hi));
-  int e = 0;
-  frexpf(a, &e);
-  e = e < -126 ? -126 : (e > 126 ? 126 : e);
-  const float sc = ldexpf(1.0f, -e);
+  // 2^e from the exponent field (0 for subnormal values, which the clamp covers too)
+  int e = (int)(__float_as_uint(a) >> 23) - 126;
+  e = e > 126 ? 126 : e;
+  const float sc = __uint_as_float((unsigned)(127 - e) << 23);
   const cdf w{df_ldexp(d.re, sc), df_ldexp(d.im, sc)};
   const df64 r = df_rcp(cdf_abs2(w));
   return {{w.re * r, df_neg(w.im * r)}, sc};

@@ -11,6 +11,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "df2.cuh"
 #include "df64.cuh"
 
 namespace ac3d {
@@ -20,39 +21,67 @@ struct alignas(16) DfPt {
   float pad[2];
 };
 
+// Quadrature points 2 h and 2 h + 1 side by side: yq[h][d] = {hi, hi', lo, lo'} of coordinate d, so
+// that one 16-byte load fills the two register pairs of the packed arithmetic.
 struct alignas(16) DfElem {
-  df64 yq[6][3];
+  float4 yq[3][3];
   df64 n[3];
   float pad[2];
 };
 static_assert(sizeof(DfElem) == 176, "DfElem layout");
 static_assert(sizeof(DfPt) == 32, "DfPt layout");
 
-__host__ __device__ __forceinline__ cdf entry_df(df64 k, const DfPt* __restrict__ pp, const DfElem* __restrict__ ge,
-                                        const float4* __restrict__ tab) {
+__device__ __forceinline__ df2 df2_load(const float4* p) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  return {v.x, v.y};
+}
+
+// Contributions of the quadrature points 2 h and 2 h + 1 to an entry, as exact-product pairs: point
+// 2 h adds p0 + e0 and point 2 h + 1 adds p1 + e1 to (re, im).
+struct DfItem {
+  f2 p0, e0, p1, e1;
+};
+
+// Two quadrature points at once through the geometry, the phase and the weights: about 400 packed
+// operations, bound by the FP32 pipe (two clocks each).
+__device__ __forceinline__ DfItem entry_item(df2 kk, const DfPt* __restrict__ pp, const DfElem* __restrict__ ge, int h,
+                                             const float4* __restrict__ tab) {
   const DfPt p = *pp;
-  const df64 nx = ge->n[0], ny = ge->n[1], nz = ge->n[2];
-  df64 are{0.f, 0.f}, aim{0.f, 0.f};
+  const df2 rx = df2_dup(p.x) - df2_load(&ge->yq[h][0]);
+  const df2 ry = df2_dup(p.y) - df2_load(&ge->yq[h][1]);
+  const df2 rz = df2_dup(p.z) - df2_load(&ge->yq[h][2]);
+  const df2 r = df2_sqrt(df2_norm2_3(rx, ry, rz));
+  const df2 rinv = df2_rcp(r);
+  const df2 s = df2_fma(rz, df2_dup(ge->n[2]), df2_fma(ry, df2_dup(ge->n[1]), rx * df2_dup(ge->n[0])));
+  const df2 kr = kk * r;
+  df2 cs, sn;
+  df2_sincos(kr, tab, cs, sn);
+  const df64 w0 = df_from_double(quad_w(0)), w3 = df_from_double(quad_w(3));
+  const df2 w = df2_make(h < 2 ? w0 : w3, h < 1 ? w0 : w3);
+  const df2 f = (s * (rinv * df2_sqr(rinv))) * w;
+  // e^{-ikr}(1 + ikr) = (cs + kr sn) + i (kr cs - sn)
+  f2 pr, er, pi, ei;
+  df2_prod(f, df2_fma(kr, sn, cs), pr, er);
+  df2_prod(f, df2_fms(kr, cs, sn), pi, ei);
+  return {f2_make(f2_x(pr), f2_x(pi)), f2_make(f2_x(er), f2_x(ei)), f2_make(f2_y(pr), f2_y(pi)),
+          f2_make(f2_y(er), f2_y(ei))};
+}
+
+__device__ __forceinline__ df2 entry_scale(df2 acc) { return acc * df2_dup(df_from_double(0.5 / (4.0 * kPi))); }
+
+// The entry as (re, im): bit for bit the sum over the six points in order in scalar double-float
+// arithmetic.
+__device__ __forceinline__ df2 entry_df(df64 k, const DfPt* __restrict__ pp, const DfElem* __restrict__ ge,
+                                        const float4* __restrict__ tab) {
+  const df2 kk = df2_dup(k);
+  df2 acc{f2_dup(0.0f), f2_dup(0.0f)};
 #pragma unroll 1
-  for (int q = 0; q < 6; q++) {
-    const df64 rx = p.x - ge->yq[q][0];
-    const df64 ry = p.y - ge->yq[q][1];
-    const df64 rz = p.z - ge->yq[q][2];
-    const df64 r2 = df_norm2_3(rx, ry, rz);
-    const df64 r = df_sqrt(r2);
-    const df64 rinv = df_rcp(r);
-    const df64 s = df_fma(rz, nz, df_fma(ry, ny, rx * nx));
-    const df64 kr = k * r;
-    df64 cs, sn;
-    df_sincos(kr, tab, cs, sn);
-    const df64 w = q < 3 ? df_from_double(quad_w(0)) : df_from_double(quad_w(3));
-    const df64 f = (s * (rinv * df_sqr(rinv))) * w;
-    // e^{-ikr}(1 + ikr) = (cs + kr sn) + i (kr cs - sn)
-    are = df_fma(f, df_fma(kr, sn, cs), are);
-    aim = df_fma(f, df_fma(kr, cs, df_neg(sn)), aim);
+  for (int h = 0; h < 3; h++) {
+    const DfItem t = entry_item(kk, pp, ge, h, tab);
+    acc = df2_add_prod(t.p0, t.e0, acc);
+    acc = df2_add_prod(t.p1, t.e1, acc);
   }
-  const df64 scale = df_from_double(0.5 / (4.0 * kPi));
-  return {are * scale, aim * scale};
+  return entry_scale(acc);
 }
 
 }  // namespace ac3d

@@ -62,8 +62,12 @@ __global__ void geometry_kernel(const double* __restrict__ P, const int* __restr
   pd.pad[0] = pd.pad[1] = 0.f;
   cen_df[e] = pd;
   DfElem ed;
-  for (int q = 0; q < 6; q++)
-    for (int d = 0; d < 3; d++) ed.yq[q][d] = df_from_double(fma(quad_n(q), ac[d], fma(quad_m(q), ab[d], a[d])));
+  for (int h = 0; h < 3; h++)
+    for (int d = 0; d < 3; d++) {
+      const df64 u = df_from_double(fma(quad_n(2 * h), ac[d], fma(quad_m(2 * h), ab[d], a[d])));
+      const df64 v = df_from_double(fma(quad_n(2 * h + 1), ac[d], fma(quad_m(2 * h + 1), ab[d], a[d])));
+      ed.yq[h][d] = make_float4(u.hi, v.hi, u.lo, v.lo);
+    }
   ed.n[0] = df_from_double(n0);
   ed.n[1] = df_from_double(n1);
   ed.n[2] = df_from_double(n2);

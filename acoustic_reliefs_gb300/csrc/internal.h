@@ -185,7 +185,7 @@ constexpr int kWarpAcaTerms = 128;
 // An assembled H-matrix of (K - I/2) at one wavenumber.
 struct DevHMat {
   int prec = PREC_MIXED;  // storage: complex FP32 (mixed) or complex FP64
-  bool pool_df = false;   // mixed storage assembled in double-float: the ACA pool holds cdf terms
+  bool pool_df = false;   // mixed storage assembled in double-float: the ACA pool holds complex double-float terms
   double k = 0;
   int maxk = 100;
   DevBuf near;            // complex storage of all near blocks
@@ -238,7 +238,8 @@ void launch_near_assembly(const DevGeometry& G, const DevPartition& DP, DevHMat&
 void launch_aca(const DevGeometry& G, const DevPartition& DP, DevHMat& H, double eps, int max_rows, cudaStream_t s,
                 cudaStream_t s_small);
 // Mixed-precision assembly with double-float entries and ACA recursion (FP64-accurate entries,
-// pivots and ranks; FP32 storage): near field into H.near (cf), ACA terms into H.pool (cdf).
+// pivots and ranks; FP32 storage): near field into H.near (cf), ACA terms into H.pool (complex
+// double-floats, 16 bytes).
 void launch_near_assembly_df(const DevGeometry& G, const DevPartition& DP, DevHMat& H, cudaStream_t s);
 void launch_aca_df(const DevGeometry& G, const DevPartition& DP, DevHMat& H, double eps, int max_rows, cudaStream_t s,
                    cudaStream_t s_small);

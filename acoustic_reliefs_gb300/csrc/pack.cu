@@ -11,7 +11,7 @@
 // uses to sum a term's per-leaf partial dots. Offsets are prefix sums over the ranks computed on
 // the device in a fixed order, so packing is deterministic. The pool itself is not needed after.
 #include "common.cuh"
-#include "df64.cuh"
+#include "df2.cuh"
 #include "internal.h"
 
 namespace ac3d {
@@ -69,7 +69,7 @@ __global__ void leaf_scan_kernel(const int* __restrict__ leaf_start, int nleaf, 
 // double-float term of the mixed-precision assembly.
 template <typename R>
 __device__ __forceinline__ cplx<R> seg_value(const cplx<R>& v) { return v; }
-__device__ __forceinline__ cf seg_value(const cdf& v) { return cf(v.re.hi, v.im.hi); }
+__device__ __forceinline__ cf seg_value(const df2& v) { return cf(f2_x(v.hi), f2_y(v.hi)); }
 
 constexpr int kPackThreads = 256;
 constexpr int kPackChunk = 512;  // list entries per round of a leaf's scan
@@ -180,7 +180,7 @@ void launch_pack(const DevPartition& DP, DevHMat& H, bool cols, cudaStream_t s) 
   if (H.prec == PREC_FP64)
     pack_side<cd, double>(DP, H, cols, s);
   else if (H.pool_df)
-    pack_side<cdf, float>(DP, H, cols, s);
+    pack_side<df2, float>(DP, H, cols, s);
   else
     pack_side<cf, float>(DP, H, cols, s);
 }

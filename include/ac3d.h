@@ -283,6 +283,11 @@ const char* ac3d_version(void);
  * tcgen05.mma (TF32 operands split in three products, FP32 accumulation in tensor memory). No
  * reference counterpart. */
 int ac3d_tensor_selftest(const float* A, const float* B, int K, float* D);
+/* Self-check of the packed (two at a time) double-float arithmetic of the mixed-precision assembly:
+ * the number of inputs whose bits differ from the scalar arithmetic's. op 0: the reciprocal, 1: the
+ * square root, over every FP32 significand at five exponents; 2: the double-float operations on
+ * 2^20 pairs of values. No reference counterpart. */
+int ac3d_packed_selftest(int op, long long* mismatches);
 
 /* ---------------------------------------------------------------------------------------------
  * Request server. No reference counterpart: the reference solves one frequency at a time inside
