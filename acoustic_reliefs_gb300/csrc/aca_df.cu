@@ -261,12 +261,27 @@ __device__ __forceinline__ ulonglong2 lds_pair(uint32_t a) {
   return v;
 }
 // Entry e from its items (the six points in order), less the earlier terms:
-// - sum_{p < nst} coef[p] * pool[toff[p] + off], four loads in flight. Out of line like eval_items:
-// the warps of an SM are at different places of the recursion, and its straight-line code in every
-// caller overran the instruction caches (21% of the stalls; 8.9 -> 7.9 ms on the 20480-triangle
-// relief). Loading a group of terms ahead of the arithmetic costs more instructions than it hides.
+// - sum_{p < nst} coef[p] * pool[toff[p] + off], D loads in flight, with AHEAD under the arithmetic of the D
+// terms before (and the first under the items' sum). Out of line like eval_items: the warps of an SM
+// are at different places of the recursion, and its straight-line code in every caller overran the
+// instruction caches (21% of the stalls; 8.9 -> 7.9 ms on the 20480-triangle relief). There, loading
+// ahead costs more instructions than it hides; the one block of the receiver ACA has hundreds of
+// terms and nothing else to run.
+// (terms past the last one load the last one again: a load behind a branch waits for the ones before)
+template <int D>
+__device__ __forceinline__ void load_terms(df2 (&a)[D], const df2* pool, uint32_t toff, int p, int nst) {
+#pragma unroll
+  for (int u = 0; u < D; u++) {
+    long long o;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(o) : "r"(toff + 8 * min(p + u, nst - 1)) : "memory");
+    a[u] = df2_ldc(pool + o);
+  }
+}
+template <int D, bool AHEAD>
 __device__ __noinline__ df2 finish_entry(uint32_t b0, uint32_t b1, int e, uint32_t coef, uint32_t toff,
                                          const df2* pool, int nst) {
+  df2 a[D], nx[D];
+  if (AHEAD && nst > 0) load_terms<D>(a, pool, toff, 0, nst);
   df2 acc{f2_dup(0.0f), f2_dup(0.0f)};
 #pragma unroll 1
   for (int h = 3 * e; h < 3 * e + 3; h++) {
@@ -276,21 +291,18 @@ __device__ __noinline__ df2 finish_entry(uint32_t b0, uint32_t b1, int e, uint32
   }
   acc = entry_scale(acc);
 #pragma unroll 1
-  for (int p = 0; p < nst; p += 4) {
-    df2 a[4];
+  for (int p = 0; p < nst; p += D) {
+    load_terms<D>(AHEAD ? nx : a, pool, toff, AHEAD ? p + D : p, nst);
 #pragma unroll
-    for (int u = 0; u < 4; u++)
-      if (p + u < nst) {
-        long long o;
-        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(o) : "r"(toff + 8 * (p + u)) : "memory");
-        a[u] = df2_ldc(pool + o);
-      }
-#pragma unroll
-    for (int u = 0; u < 4; u++)
+    for (int u = 0; u < D; u++)
       if (p + u < nst) {
         const ulonglong2 c = lds_pair(coef + 16 * (p + u));
         df2_cfms(acc, df2{c.x, c.y}, a[u]);
       }
+    if (AHEAD) {
+#pragma unroll
+      for (int u = 0; u < D; u++) a[u] = nx[u];
+    }
   }
   return acc;
 }
@@ -430,7 +442,7 @@ __device__ __forceinline__ void aca_small(const AcaDfArgs& A, unsigned char* sme
       group_sync<W>(grp);
       const int c = c0 + tid;
       if (c < n) {
-        const df2 v = finish_entry(b0, b1, tid, coef, toff, A.pool + m + c, nst);
+        const df2 v = finish_entry<4, false>(b0, b1, tid, coef, toff, A.pool + m + c, nst);
         df2_stc(&S.vs[c], v);
         const df64 a = df2_abs2(v);
         if (a > best) {
@@ -463,7 +475,7 @@ __device__ __forceinline__ void aca_small(const AcaDfArgs& A, unsigned char* sme
       group_sync<W>(grp);
       const int r = r0 + tid;
       if (r < m) {
-        const df2 u = finish_entry(b0, b1, tid, coef, toff, A.pool + r, nst);
+        const df2 u = finish_entry<4, false>(b0, b1, tid, coef, toff, A.pool + r, nst);
         df2_stc(unew + r, u);
         S.uh[r] = u.hi;
         S.su[r] = df2_abs2(u);
@@ -595,7 +607,7 @@ __device__ __forceinline__ void aca_cta(const AcaDfArgs& A, unsigned char* smem,
       __syncthreads();
       const int c = c0 + tid;
       if (c < n) {
-        const df2 v = finish_entry(b0, b1, tid, coef_a, toff_a, A.pool + m + c, nst);
+        const df2 v = finish_entry<4, false>(b0, b1, tid, coef_a, toff_a, A.pool + m + c, nst);
         df2_stc(vnew + c, v);
         const df64 a = df2_abs2(v);
         if (a > best) {
@@ -627,7 +639,7 @@ __device__ __forceinline__ void aca_cta(const AcaDfArgs& A, unsigned char* smem,
       __syncthreads();
       const int r = r0 + tid;
       if (r < m) {
-        const df2 u = finish_entry(b0, b1, tid, coef_a, toff_a, A.pool + r, nst);
+        const df2 u = finish_entry<4, false>(b0, b1, tid, coef_a, toff_a, A.pool + r, nst);
         df2_stc(unew + r, u);
         un += df2_abs2(u);
       }
@@ -790,6 +802,288 @@ void launch_aca_df(const DevGeometry& G, const DevPartition& DP, DevHMat& H, dou
   launch_aca_kernels(a, max_rows, s, s_small);
 }
 
+// ------------------------------------------------------------------------------------------
+// One block over the whole GPU: the receiver ACA (L receivers x Ne elements, a single block of high
+// rank). A cooperative kernel; CTA c owns a contiguous range of the columns and one of the rows. An
+// iteration has three grid barriers: after the row (every CTA then finds the pivot among the CTAs'
+// best), after the divided row and the column, and after the cross terms (one warp per earlier
+// term and side) and the norms. The stopping test and the next row pivot are computed by every CTA
+// alike. Sums are taken in the order of aca_cta. Data that other SMs write in the iteration is read
+// past L1 (ld.cg); terms are a multiple of 128 bytes apart, so that no line of an earlier term holds
+// part of a later one.
+//
+// Bound by latency: of an iteration's 40 us (1297 receivers x 10680 elements, tolerance 1e-5, 135 to 168
+// terms) the chain over the earlier terms takes 15 us, the longest dot product 12 us, the barriers
+// 5 us, the entries 3 us. 5.9 ms instead of 168 ms by one CTA, which is where it began (146 ms with
+// the entries' items spread over its threads).
+// ------------------------------------------------------------------------------------------
+struct alignas(16) AcaBest {
+  df2 v;      // the entry
+  df64 a;     // |v|^2
+  int idx;
+  int pad;
+};
+
+struct AcaGridBufs {
+  unsigned long long* bar;  // arrivals, zero at launch
+  int* fail;                // a wait gave up
+  AcaBest* best;            // per CTA
+  df64* sq_v;               // |v_c|^2 (n)
+  df64* sq_u;               // |u_r|^2 (m)
+  df64* norm;               // |u|^2, |v|^2
+  float2* dots;             // per earlier term: u^T U_p, v V_p^T
+  int stride;               // entries between terms
+};
+
+constexpr uint32_t kGridSpin = 1u << 24;  // polls of an L2 line, seconds in all
+
+__device__ __forceinline__ bool aca_grid_sync(const AcaGridBufs& X) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const unsigned long long t = atomicAdd(X.bar, 1ull);
+    const unsigned long long target = (t / gridDim.x + 1) * (unsigned long long)gridDim.x;
+    volatile unsigned long long* c = X.bar;
+    int ok = 1;
+    uint32_t it = 0;
+    while (*c < target) {
+      if (++it > kGridSpin) {
+        ok = 0;
+        atomicExch(X.fail, 1);
+        break;
+      }
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+__device__ __forceinline__ df2 df2_ldcg(const df2* p) {
+  const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(p));
+  return {v.x, v.y};
+}
+__device__ __forceinline__ df64 df64_ldcg(const df64* p) {
+  const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+  return {v.x, v.y};
+}
+
+// sum_r a_r b_r of the leading parts, a new vector against an earlier term, by one warp: lane 0 gets the
+// real part, lane 16 the imaginary part
+__device__ __noinline__ float grid_dot(const df2* a, const df2* b, int len) {
+  const int lane = threadIdx.x & 31;
+  float s[2] = {0.f, 0.f};
+  constexpr int D = 32;  // pairs of loads in flight
+  for (int r0 = lane; r0 < len; r0 += 32 * D) {
+    f2 x[D], y[D];
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+      const int r = min(r0 + 32 * k, len - 1);
+      x[k] = __ldcg(&a[r].hi);
+      y[k] = b[r].hi;
+    }
+#pragma unroll
+    for (int k = 0; k < D; k++)
+      if (r0 + 32 * k < len) lead_fma(s[0], s[1], x[k], y[k]);
+  }
+  fold<1, 16>(s);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+  return s[0];
+}
+
+__global__ void __launch_bounds__(kDfThreads, 1) aca_df_grid_kernel(AcaDfArgs A, AcaGridBufs X) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  load_table(A.tab);
+  AcaCta& S = *reinterpret_cast<AcaCta*>(smem);
+  df2* coef = reinterpret_cast<df2*>(smem + sizeof(AcaCta));
+  long long* toff = reinterpret_cast<long long*>(coef + A.iter_cap);
+  df64* prod = reinterpret_cast<df64*>(toff + A.iter_cap);
+  unsigned* used = reinterpret_cast<unsigned*>(prod + A.iter_cap);
+  const uint32_t b0 = shared_addr(S.b0), b1 = shared_addr(S.b1), coef_a = shared_addr(coef), toff_a = shared_addr(toff);
+  const int4 q = A.blocks[A.order[0]];
+  const int rs = q.x, cs = q.z, m = q.y - q.x, n = q.w - q.z;
+  const int iter_lim = max(0, min(min(A.maxk, A.iter_cap), min(m - 1, n - 1)));
+  const int tid = threadIdx.x, T = kDfThreads, lane = tid & 31, warp = tid >> 5;
+  const int G = gridDim.x, cta = blockIdx.x;
+  const int pc = (n + G - 1) / G, pr = (m + G - 1) / G;
+  const int c_lo = min(n, cta * pc), c_hi = min(n, c_lo + pc), r_lo = min(m, cta * pr), r_hi = min(m, r_lo + pr);
+  for (int w = tid; w < (m + 31) / 32; w += T) used[w] = w == 0 ? 1u : 0u;
+  __syncthreads();
+  df64 err{0.0f, 0.0f};
+  int i = 0, nst = 0;
+  bool ok = true;
+  for (int iter = 0; iter < iter_lim; iter++) {
+    const long long base = (long long)nst * X.stride;
+    df2* unew = A.pool + base;
+    df2* vnew = unew + m;
+    // row residual of this CTA's columns
+    for (int p = tid; p < nst; p += T) df2_stc(&coef[p], df2_ldcg(A.pool + toff[p] + i));
+    df64 best{-1.0f, 0.0f};
+    df2 bv{0, 0};
+    int bidx = 0;
+    for (int c0 = c_lo; c0 < c_hi; c0 += T) {
+      if (c0 > c_lo) __syncthreads();
+      eval_items(A.k, A.pts + rs + i, 0, A.el + cs + c0, 1, min(T, c_hi - c0), tid, T, b0, b1);
+      __syncthreads();
+      const int c = c0 + tid;
+      if (c < c_hi) {
+        const df2 v = finish_entry<8, true>(b0, b1, tid, coef_a, toff_a, A.pool + m + c, nst);
+        df2_stc(vnew + c, v);
+        const df64 a = df2_abs2(v);
+        if (a > best) {
+          best = a;
+          bidx = c;
+          bv = v;
+        }
+      }
+    }
+    {
+      df64 val = best;
+      int idx = bidx;
+      group_argmax<kDfWarps>(val, idx, S.bv[0], S.bi[0], 0);
+      AcaBest* o = X.best + cta;
+      if (tid == 0) {
+        o->a = val;
+        o->idx = idx;
+      }
+      if (idx == bidx && !(best.hi < 0.0f)) df2_stc(&o->v, bv);  // the one thread that holds it
+    }
+    if (!(ok = aca_grid_sync(X))) break;
+    // column pivot: the best of the CTAs' bests
+    best = df64{-1.0f, 0.0f};
+    bidx = 0;
+    for (int k = tid; k < G; k += T) {
+      const df64 a = df64_ldcg(&X.best[k].a);
+      const int idx = __ldcg(&X.best[k].idx);
+      if (a > best) {  // ascending ranges: the first of equals is the smallest index
+        best = a;
+        bidx = idx;
+      }
+    }
+    group_argmax<kDfWarps>(best, bidx, S.bv[1], S.bi[1], 0);
+    const int j = bidx;
+    const cdf vj = df2_to_cdf(df2_ldcg(&X.best[min(G - 1, j / pc)].v));
+    for (int p = tid; p < nst; p += T) df2_stc(&coef[p], df2_ldcg(A.pool + toff[p] + m + j));
+    const bool keep = A.zero_guard && df_is_zero(vj.re) && df_is_zero(vj.im);
+    const CdfDivisor dv = keep ? CdfDivisor{cdf{}, 1.0f} : cdf_divisor(vj);
+    for (int c = c_lo + tid; c < c_hi; c += T) {
+      df2 v = df2_ldcg(vnew + c);
+      if (!keep) v = df2_cdivide(v, dv);
+      df2_stc(vnew + c, v);
+      X.sq_v[c] = df2_abs2(v);
+    }
+    // column residual of this CTA's rows
+    for (int r0 = r_lo; r0 < r_hi; r0 += T) {
+      if (r0 > r_lo) __syncthreads();
+      eval_items(A.k, A.pts + rs + r0, 1, A.el + cs + j, 0, min(T, r_hi - r0), tid, T, b0, b1);
+      __syncthreads();
+      const int r = r0 + tid;
+      if (r < r_hi) {
+        const df2 u = finish_entry<8, true>(b0, b1, tid, coef_a, toff_a, A.pool + r, nst);
+        df2_stc(unew + r, u);
+        X.sq_u[r] = df2_abs2(u);
+      }
+    }
+    if (!(ok = aca_grid_sync(X))) break;
+    // norms by the first CTA; cross terms by the warps of the others
+    if (cta == 0) {
+      df64 un{0.0f, 0.0f}, vn{0.0f, 0.0f};
+      for (int c0 = tid; c0 < n; c0 += 8 * T) {
+        df64 x[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          if (c0 + k * T < n) x[k] = df64_ldcg(X.sq_v + c0 + k * T);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          if (c0 + k * T < n) vn += x[k];
+      }
+      for (int r = tid; r < m; r += T) un += df64_ldcg(X.sq_u + r);
+      warp_sum2_df(un, vn);
+      if (lane == 0) {
+        S.sd[0][warp] = un;
+        S.sd[1][warp] = vn;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        un = S.sd[0][0];
+        vn = S.sd[1][0];
+        for (int k = 1; k < kDfWarps; k++) {
+          un += S.sd[0][k];
+          vn += S.sd[1][k];
+        }
+        X.norm[0] = un;
+        X.norm[1] = vn;
+      }
+    }
+    if (cta > 0 || G == 1) {
+      const int ng = max(1, G - 1), w0 = warp * ng + (G == 1 ? 0 : cta - 1), nw = ng * kDfWarps;  // over the SMs first
+      for (int t = w0; t < 2 * nst; t += nw) {
+        // the long sides first
+        const int p = t < nst ? t : t - nst;
+        const bool row = t < nst;
+        const int o0 = row ? m : 0;
+        const float d = grid_dot(unew + o0, A.pool + toff[p] + o0, row ? n : m);
+        float* o = reinterpret_cast<float*>(X.dots + 2 * p + (row ? 1 : 0));
+        if (lane == 0) o[0] = d;
+        if (lane == 16) o[1] = d;
+      }
+    }
+    if (!(ok = aca_grid_sync(X))) break;
+    // stopping test and next row pivot, alike in every CTA
+    const df64 unt = df64_ldcg(X.norm), vnt = df64_ldcg(X.norm + 1);
+    for (int p = tid; p < nst; p += T) {
+      const float2 u = __ldcg(X.dots + 2 * p), v = __ldcg(X.dots + 2 * p + 1);
+      prod[p] = df_prod_ff(sqrtf(u.x * u.x + u.y * u.y), sqrtf(v.x * v.x + v.y * v.y));
+    }
+    __syncthreads();
+    df64 part{0.0f, 0.0f};
+    if (lane < kDfWarps)
+      for (int p = lane; p < nst; p += kDfWarps) part += prod[p];
+    df64 dots = shfl_df(part, 0);
+#pragma unroll 1
+    for (int k = 1; k < kDfWarps; k++) dots += shfl_df(part, k);
+    const df64 uv = unt * vnt;
+    err += uv + df_ldexp(dots, 2.0f);
+    if (aca_converged(uv, err, A.eps2)) break;
+    const bool zero_term = df_is_zero(unt) || df_is_zero(vnt);
+    best = df64{-1.0f, 0.0f};
+    bidx = 0;
+    for (int r0 = tid; r0 < m; r0 += 8 * T) {
+      df64 x[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (r0 + k * T < m) x[k] = df64_ldcg(X.sq_u + r0 + k * T);
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const int r = r0 + k * T;
+        if (r < m && !((used[r >> 5] >> (r & 31)) & 1u) && x[k] > best) {
+          best = x[k];
+          bidx = r;
+        }
+      }
+    }
+    group_argmax<kDfWarps>(best, bidx, S.bv[0], S.bi[0], 0);
+    i = bidx;
+    if (tid == 0) {
+      used[i >> 5] |= 1u << (i & 31);
+      if (!zero_term) {
+        toff[nst] = base;
+        if (cta == 0) A.term_off[nst] = base;
+      }
+    }
+    if (!zero_term) nst++;
+    __syncthreads();
+  }
+  if (cta == 0 && tid == 0) {
+    A.rank[0] = nst;
+    *A.pool_used = (unsigned long long)nst * X.stride;
+    if (!ok) atomicOr(A.status, 2);
+  }
+}
+
 // Receiver ACA (compute_ACA_listener, aca.cpp:84-134: one block of L receivers x Ne elements, no
 // zero guard) in double-float, then the terms converted in place to complex FP64 (same size).
 __global__ void df_to_cd_kernel(df2* pool, const unsigned long long* used) {
@@ -801,18 +1095,50 @@ __global__ void df_to_cd_kernel(df2* pool, const unsigned long long* used) {
   }
 }
 
+// Entries of a receiver term in the pool: rounded up so that terms start on 128-byte lines.
+int listener_term_stride(int L, int ne) { return (L + ne + 7) & ~7; }
+
 void launch_listener_aca_df(const DevGeometry& G, const void* pts_df, int L, double k, double eps, int maxk,
                             void* pool, long long pool_cap, unsigned long long* used, long long* term_off, int* rank,
-                            int* status, const int4* block, const int* order, cudaStream_t s) {
+                            int* status, const int4* block, const int* order, DevBuf& scratch, cudaStream_t s) {
   int iter_lim = std::min(maxk, std::min(L - 1, G.ne - 1));
   if (iter_lim < 1) iter_lim = 1;
   AcaDfArgs a{G.cen.as<double4>(), G.va.as<double4>(), G.eg64.as<ElemGeo<double>>(), (const DfPt*)pts_df,
               G.el_df.as<DfElem>(), G.df_tab.as<float4>(), block, order, {1, 0, 0, 0}, df_from_double(k), eps,
               df_from_double(eps * eps), maxk, iter_lim,
               (df2*)pool, pool_cap, used, term_off, rank, status, nullptr, 0};
-  if (aca_cta_smem(iter_lim, L) > kAcaSmemMax)
+  const size_t smem = aca_cta_smem(iter_lim, L);
+  if (smem > kAcaSmemMax)
     throw Error(4, "receiver ACA too large for shared memory (at most about 5000 receivers)");
-  launch_aca_kernels(a, L, s, s);
+  static std::once_flag once;
+  std::call_once(once, [] {
+    AC3D_CUDA(cudaFuncSetAttribute(aca_df_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAcaSmemMax));
+  });
+  int per_sm = 0;
+  AC3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, aca_df_grid_kernel, kDfThreads, smem));
+  // about 64 columns (192 items) per CTA, at most one CTA per SM
+  const int grid = std::max(1, std::min((per_sm > 0 ? 1 : 0) * device_sm_count(), (G.ne + 63) / 64));
+  if (grid <= 2) {
+    // barriers would cost more than the columns: 0.30 against 0.23 ms with one CTA on 80 elements and
+    // 17 receivers; on 320 elements the grid is ahead (0.42 against 0.49 ms with 37 receivers)
+    launch_aca_kernels(a, L, s, s);
+    note_launch();
+    df_to_cd_kernel<<<4 * device_sm_count(), 256, 0, s>>>((df2*)pool, used);
+    AC3D_CUDA(cudaGetLastError());
+    return;
+  }
+  auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const size_t o_best = 256, o_v = o_best + up(grid * sizeof(AcaBest)), o_u = o_v + up((size_t)G.ne * sizeof(df64)),
+               o_n = o_u + up((size_t)L * sizeof(df64)), o_d = o_n + 256,
+               total = o_d + up((size_t)iter_lim * 2 * sizeof(float2));
+  scratch.alloc(total, s);
+  AC3D_CUDA(cudaMemsetAsync(scratch.p, 0, 256, s));
+  char* sp = (char*)scratch.p;
+  AcaGridBufs x{(unsigned long long*)sp, (int*)(sp + 8), (AcaBest*)(sp + o_best), (df64*)(sp + o_v), (df64*)(sp + o_u),
+                (df64*)(sp + o_n), (float2*)(sp + o_d), listener_term_stride(L, G.ne)};
+  void* args[] = {&a, &x};
+  note_launch();
+  AC3D_CUDA(cudaLaunchCooperativeKernel((const void*)aca_df_grid_kernel, dim3(grid), dim3(kDfThreads), args, smem, s));
   note_launch();
   df_to_cd_kernel<<<4 * device_sm_count(), 256, 0, s>>>((df2*)pool, used);
   AC3D_CUDA(cudaGetLastError());

@@ -931,7 +931,7 @@ void upload_receivers(ac3d_ctx* c, const double* L, int n, DevBuf& dst) {
 
 // Receiver matrix by ACA (reference mode, compute_ACA_listener, aca.cpp:84-134).
 struct ListenerLR {
-  DevBuf pool, toff, rank, used, blk, ord, pts, t;
+  DevBuf pool, toff, rank, used, blk, ord, pts, t, scratch;
   int L = 0, iter_lim = 0;
   int prec = PREC_MIXED;  // precision of the stored terms (the apply's arithmetic)
 };
@@ -946,7 +946,7 @@ std::unique_ptr<ListenerLR> listener_lr(ac3d_ctx* c, double k, const double* Lh,
   const bool df = c->prec != PREC_FP64 && c->assembly == AC3D_ASSEMBLY_DF;
   Q->prec = df ? PREC_FP64 : c->prec;
   const size_t cs = Q->prec == PREC_FP64 ? sizeof(cd) : sizeof(cf);
-  const long long cap = (long long)Q->iter_lim * (L + c->m->Ne);
+  const long long cap = (long long)Q->iter_lim * (df ? listener_term_stride(L, c->m->Ne) : L + c->m->Ne);
   Q->pool.alloc((size_t)cap * cs, s);
   Q->toff.alloc((size_t)Q->iter_lim * sizeof(long long), s);
   Q->rank.alloc(sizeof(int), s);
@@ -966,7 +966,11 @@ std::unique_ptr<ListenerLR> listener_lr(ac3d_ctx* c, double k, const double* Lh,
     upload(Q->pts, v, s);
     launch_listener_aca_df(c->m->G, Q->pts.p, L, k, c->q_tol, maxk, Q->pool.p, cap, Q->used.as<unsigned long long>(),
                            Q->toff.as<long long>(), Q->rank.as<int>(), (int*)(Q->used.as<unsigned long long>() + 1),
-                           Q->blk.as<int4>(), Q->ord.as<int>(), s);
+                           Q->blk.as<int4>(), Q->ord.as<int>(), Q->scratch, s);
+    unsigned long long used[2];
+    AC3D_CUDA(cudaMemcpyAsync(used, Q->used.p, 16, cudaMemcpyDeviceToHost, s));
+    AC3D_CUDA(cudaStreamSynchronize(s));
+    if ((int)(used[1] & 0xffffffffu) & 2) throw Error(AC3D_ERR_CUDA, "receiver ACA grid barrier timed out (bounded wait)");
     return Q;
   }
   if (c->prec == PREC_FP64) {

@@ -18,10 +18,12 @@ void launch_listener_aca(const DevGeometry& G, int prec, const void* pts, int L,
                          int* status, const int4* block, const int* order, cudaStream_t s);
 // The receiver ACA in double-float arithmetic (the mixed path's default assembly): pts_df holds L
 // double-float points (8 floats each: x, y, z as hi/lo pairs, two pad); the terms end up in the
-// pool as complex FP64.
+// pool as complex FP64, listener_term_stride(L, ne) entries apart. A cooperative kernel; status gets bit
+// 1 (value 2) if one of its bounded waits gave up. scratch is allocated on s and must outlive the launch.
+int listener_term_stride(int L, int ne);
 void launch_listener_aca_df(const DevGeometry& G, const void* pts_df, int L, double k, double eps, int maxk,
                             void* pool, long long pool_cap, unsigned long long* used, long long* term_off, int* rank,
-                            int* status, const int4* block, const int* order, cudaStream_t s);
+                            int* status, const int4* block, const int* order, DevBuf& scratch, cudaStream_t s);
 
 void launch_lr_apply(int prec, const void* pool, const long long* toff, const int* rank, int iter_lim, int L, int ne,
                      const cd* x, int trans, cd* t, cd* out, cudaStream_t s);

@@ -39,3 +39,20 @@ def test_aca_groups_match_oracle(oracle_lib, gpu_lib, leaf, nx):
     assert differ <= 1 + len(H.ranks) // 1000
     yo, _, _ = oracle_lib.solve_pressures(m, k, d, 1, Ls, 1e-4, 1e-4, 1e-9, listener="dense")
     assert np.linalg.norm(y - yo) / np.linalg.norm(yo) < 1e-4
+
+
+@pytest.mark.parametrize("nx,L", [(4, 17), (5, 2), (9, 3), (9, 181), (23, 700), (40, 37)])
+def test_receiver_aca_matches_oracle(oracle_lib, gpu_lib, nx, L):
+    """The receiver ACA by one CTA (128 panels) and over the GPU (ranges of columns and rows that do
+    not divide evenly, fewer receivers than CTAs): the oracle's receiver ACA product."""
+    R = meshes.relief(0.6, 0.6, 0.05, nx, 2, nx, 0, meshes.smooth_heightmap(16, 5))
+    Ls = meshes.semicircle(5.0, L) + np.random.default_rng(L).uniform(-0.2, 0.2, size=(L, 3))
+    f, d = 1200.0, np.array([0.2, -1.0, 0.1]) / np.linalg.norm([0.2, -1.0, 0.1])
+    bem = DiffBEM(32, 2.0, [f], 1, 1e-6, 1e-5, 1e-9, precision="mixed", incident=("plane", d), listener="aca")
+    bem.silent = True
+    bem.set_krylov("gmres")
+    bem.set_mesh(R.Ps, R.Es)
+    y = bem.pvals(f, Ls)
+    m = oracle_lib.Mesh(R.Ps, R.Es, 32, 2.0)
+    yo, _, _ = oracle_lib.solve_pressures(m, oracle_lib.wavenumber(f), d, 1, Ls, 1e-6, 1e-5, 1e-9, listener="aca")
+    assert np.linalg.norm(y - yo) / np.linalg.norm(yo) < 1e-4
