@@ -80,43 +80,48 @@ __global__ void far_reduce_kernel(const cd* __restrict__ partial, int L, int S, 
   y[l] = cd(sr, si);
 }
 
-// out_j = sum_l Q_lj vf_l  (plain transpose), receivers staged through shared memory
+// out_j = sum_l Q_lj vf_l (plain transpose). Bound by the entries' FP32 arithmetic once the GPU is full,
+// which one thread per element was not (5280 elements: 21 CTAs). A CTA takes kFTElems elements and
+// spreads the entries of kFTTile receivers over its threads; one thread per element then adds them in
+// receiver order (partial sums of kFFThreads receivers in R, their total in FP64). 5280 elements x
+// 181 receivers: 47 instead of 250 us.
+constexpr int kFTElems = 16, kFTTile = 128;
 template <typename R>
 __global__ void __launch_bounds__(kFFThreads) far_t_kernel(GeoView<R> G, const double4* __restrict__ recv, int L, R k,
                                                            const cd* __restrict__ vf, cd* out) {
-  __shared__ double4 sp[kFFThreads];
-  __shared__ cd sv[kFFThreads];
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ cplx<R> q[kFTTile][kFTElems + 1];
+  constexpr int kGroups = kFFThreads / kFTElems;
+  const int e = threadIdx.x % kFTElems, grp = threadIdx.x / kFTElems;
+  const int j = blockIdx.x * kFTElems + e;
   const bool ok = j < G.ne;
-  double4 va = make_double4(0, 0, 0, 0);
-  ElemGeo<R> g;
-  if (ok) {
-    va = G.va[j];
-    g = G.eg[j];
-  }
+  const double4 va = G.va[ok ? j : G.ne - 1];
+  const ElemGeo<R> g = G.eg[ok ? j : G.ne - 1];
   double sr = 0, si = 0;
-  for (int base = 0; base < L; base += kFFThreads) {
-    const int cnt = min(kFFThreads, L - base);
-    __syncthreads();
-    if (threadIdx.x < cnt) {
-      sp[threadIdx.x] = recv[base + threadIdx.x];
-      sv[threadIdx.x] = vf[base + threadIdx.x];
+  R ar = 0, ai = 0;
+  for (int base = 0; base < L; base += kFTTile) {
+    const int cnt = min(kFTTile, L - base);
+    __syncthreads();  // the previous tile is added up
+    for (int a = grp; a < cnt; a += kGroups) {
+      const double4 P = recv[base + a];
+      q[a][e] = entry_from_d<R>(k, (R)(P.x - va.x), (R)(P.y - va.y), (R)(P.z - va.z), g);
     }
     __syncthreads();
-    if (ok) {
-      R ar = 0, ai = 0;
+    if (grp == 0) {
       for (int a = 0; a < cnt; a++) {
-        const double4 P = sp[a];
-        cplx<R> q = entry_from_d<R>(k, (R)(P.x - va.x), (R)(P.y - va.y), (R)(P.z - va.z), g);
-        const R vr = (R)sv[a].re, vi = (R)sv[a].im;
-        ar += q.re * vr - q.im * vi;
-        ai += q.re * vi + q.im * vr;
+        const cplx<R> v = q[a][e];
+        const cd f = vf[base + a];
+        const R vr = (R)f.re, vi = (R)f.im;
+        ar += v.re * vr - v.im * vi;
+        ai += v.re * vi + v.im * vr;
       }
-      sr += ar;
-      si += ai;
+      if ((base + kFTTile) % kFFThreads == 0 || base + kFTTile >= L) {
+        sr += ar;
+        si += ai;
+        ar = ai = 0;
+      }
     }
   }
-  if (ok) out[j] = cd(sr, si);
+  if (ok && grp == 0) out[j] = cd(sr, si);
 }
 
 void launch_far_field(const DevGeometry& G, int prec, const double4* recv, int L, double k, const cd* x, cd* y,
@@ -137,7 +142,7 @@ void launch_far_field(const DevGeometry& G, int prec, const double4* recv, int L
 
 void launch_far_field_t(const DevGeometry& G, int prec, const double4* recv, int L, double k, const cd* vf, cd* out,
                         cudaStream_t s) {
-  const int nb = (G.ne + kFFThreads - 1) / kFFThreads;
+  const int nb = (G.ne + kFTElems - 1) / kFTElems;
   note_launch();
   if (prec == PREC_FP64)
     far_t_kernel<double><<<nb, kFFThreads, 0, s>>>(geo_view<double>(G), recv, L, k, vf, out);
