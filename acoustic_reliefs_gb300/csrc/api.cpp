@@ -600,6 +600,7 @@ void check_pipeline(ac3d_ctx* c, const DevHMat& H) {
 void solve_impl(ac3d_ctx* c, DevHMat& H, const cd* b, cd* x, bool tr);
 
 void solve(ac3d_ctx* c, DevHMat& H, const cd* b, cd* x, bool tr) {
+  if (tr) ensure_near_transposed(c->m->DP, H, c->stream);
   solve_impl(c, H, b, x, tr);
   check_pipeline(c, H);
 }
@@ -2071,8 +2072,9 @@ int ac3d_matvec_timing(ac3d_ctx* c, int iters, int transposed, double* ms, long 
   return guard(c, [&] {
     if (!c->last_H) throw Error(AC3D_ERR_STATE, "no H-matrix: call ac3d_pressures first");
     cudaStream_t s = c->stream;
-    const DevHMat& H = *c->last_H;
+    DevHMat& H = *c->last_H;
     ensure_work(c);
+    if (transposed) ensure_near_transposed(c->m->DP, H, s);
     // the variant the solve runs: FP64 vectors on the FP64 H-matrix; on the FP32 H-matrix FP32
     // vectors (GMRES) or FP64 vectors with their FP32 shadows (BiCGSTAB), FP32 arithmetic
     const int vec64 = H.prec == PREC_FP64 ? 1 : (c->krylov == AC3D_KRYLOV_GMRES ? 0 : 2);

@@ -492,20 +492,32 @@ __global__ void __launch_bounds__(kGatherThreads, AC3D_GATHER_MIN_CTAS) seg_gath
         AT tr[RPL], ti[RPL];
 #pragma unroll
         for (int jr = 0; jr < RPL; jr++) tr[jr] = ti[jr] = 0;
+        // near: the transposed copy, so that the lanes' columns of a row are consecutive (the blocks
+        // themselves would be read a line per lane); the rows of a warp's blocks in order, U loads in
+        // flight (as many as the 56 registers hold). Transposed matvec, before and after: 149.6 and
+        // 101.3 us on the 20480-triangle relief, 65.7 and 37.5 us on 5280 triangles
         for (int it = V.trn_ptr[leaf] + warp; it < V.trn_ptr[leaf + 1]; it += kWarps) {
           const int b = V.trn[it];
           const int4 blk = V.blocks_d[b];
           const int m = blk.y - blk.x;
           const cplx<AT>* xs = xm + blk.x;
+          const cplx<MT>* D = near + V.near_off[b];
+          constexpr int U = sizeof(AT) > 4 ? 2 : RPL > 2 ? 4 : 8;
+          for (int r0 = 0; r0 < m; r0 += U) {
 #pragma unroll
-          for (int jr = 0; jr < RPL; jr++) {
-            const int col = lane + 32 * jr;
-            if (col < R) {
-              const cplx<MT>* Dc = near + V.near_off[b] + (long long)col * m;
-              for (int r = 0; r < m; r++) {
-                const cplx<AT> zz = xs[r];
-                acc_mac(tr[jr], ti[jr], Dc[r], zz.re, zz.im);
+            for (int jr = 0; jr < RPL; jr++) {
+              const int col = min(lane + 32 * jr, R - 1);
+              cplx<MT> d[U];
+              cplx<AT> z[U];
+#pragma unroll
+              for (int u = 0; u < U; u++) {
+                const int r = min(r0 + u, m - 1);
+                d[u] = D[(long long)r * R + col];
+                z[u] = xs[r];
               }
+#pragma unroll
+              for (int u = 0; u < U; u++)
+                if (r0 + u < m) acc_mac(tr[jr], ti[jr], d[u], z[u].re, z[u].im);
             }
           }
         }
@@ -650,10 +662,11 @@ static void mv_t(const DevPartition& DP, const DevHMat& H, bool tr, const void* 
   v.a_kptr = DP.didx_ptr.as<int>();
   v.a_idx = DP.didx.as<int>();
   v.blocks_d = DP.blocks_d.as<int4>();
-  v.near_off = DP.near_off.as<long long>();
+  v.near_off = tr ? DP.near_off_t.as<long long>() : DP.near_off.as<long long>();
   v.trn_ptr = DP.tr_near_ptr.as<int>();
   v.trn = DP.tr_near.as<int>();
   v.err = H.err.as<int>();
+  if (tr && DP.nd > 0 && !H.nearT.p) throw Error(3, "internal: transposed near field not built");
   const cplx<MT>* useg = H.useg.as<cplx<MT>>();
   const cplx<MT>* vseg = H.vseg.as<cplx<MT>>();
   cplx<AT>* t = (cplx<AT>*)tvec;
@@ -697,7 +710,7 @@ static void mv_t(const DevPartition& DP, const DevHMat& H, bool tr, const void* 
   }
   const int P = std::min(DP.nleaf, nb * device_sm_count());
   launch_k(pdl && DP.na > 0, kern, dim3(P), dim3(kGatherThreads), kRingBytes, s, v, DP.nleaf,
-           (const cplx<MT>*)H.near.as<cplx<MT>>(),
+           (const cplx<MT>*)(tr ? H.nearT : H.near).as<cplx<MT>>(),
            tr ? vseg : useg, tc, (const cplx<VT>*)x, xm, (cplx<VT>*)y, (const cplx<VT>*)bminus,
            (const cplx<VT>*)ep.dot_a, (const cplx<VT>*)ep.dot_b, ep.partials, ep.red5, H.ticket.as<unsigned>(), done);
 

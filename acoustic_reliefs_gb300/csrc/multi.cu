@@ -990,13 +990,15 @@ static void mmv_rpl(const DevPartition& DP, const DevHMat& H, const MultiBufs& B
 
 // One CTA per near block: block b (m x n, column-major at near_off[b]) transposed to n x m
 // column-major at near_off_t[b]. Padding columns of the transposed segments stay zero.
+template <typename R>
 __global__ void near_transpose_kernel(const int4* __restrict__ blocks, const long long* __restrict__ off,
-                                      const long long* __restrict__ off_t, const cf* __restrict__ near, cf* nearT) {
+                                      const long long* __restrict__ off_t, const cplx<R>* __restrict__ near,
+                                      cplx<R>* nearT) {
   const int b = blockIdx.x;
   const int4 q = blocks[b];
   const int m = q.y - q.x, n = q.w - q.z;
-  const cf* src = near + off[b];
-  cf* dst = nearT + off_t[b];
+  const cplx<R>* src = near + off[b];
+  cplx<R>* dst = nearT + off_t[b];
   for (int t = threadIdx.x; t < m * n; t += blockDim.x) {
     const int r = t / n, c = t - r * n;
     dst[t] = src[c * m + r];
@@ -1005,14 +1007,19 @@ __global__ void near_transpose_kernel(const int4* __restrict__ blocks, const lon
 
 void ensure_near_transposed(const DevPartition& DP, DevHMat& H, cudaStream_t s) {
   if (H.nearT.p) return;
-  if (H.prec == PREC_FP64) throw Error(3, "internal: block matvec needs FP32 storage");
-  const size_t bytes = (size_t)std::max<int64_t>(DP.near_total_t, 2) * sizeof(cf);
+  const size_t bytes = (size_t)std::max<int64_t>(DP.near_total_t, 2) * (H.prec == PREC_FP64 ? sizeof(cd) : sizeof(cf));
   H.nearT.alloc(bytes, s);
   AC3D_CUDA(cudaMemsetAsync(H.nearT.p, 0, bytes, s));
   if (DP.nd == 0) return;
   note_launch();
-  near_transpose_kernel<<<DP.nd, 256, 0, s>>>(DP.blocks_d.as<int4>(), DP.near_off.as<long long>(),
-                                              DP.near_off_t.as<long long>(), H.near.as<cf>(), H.nearT.as<cf>());
+  if (H.prec == PREC_FP64)
+    near_transpose_kernel<double><<<DP.nd, 256, 0, s>>>(DP.blocks_d.as<int4>(), DP.near_off.as<long long>(),
+                                                        DP.near_off_t.as<long long>(), H.near.as<cd>(),
+                                                        H.nearT.as<cd>());
+  else
+    near_transpose_kernel<float><<<DP.nd, 256, 0, s>>>(DP.blocks_d.as<int4>(), DP.near_off.as<long long>(),
+                                                       DP.near_off_t.as<long long>(), H.near.as<cf>(),
+                                                       H.nearT.as<cf>());
   AC3D_CUDA(cudaGetLastError());
 }
 
