@@ -7,7 +7,7 @@
 // and dc/dh += A - B + C (adjoint.cpp:231). B is a dense all-pairs sweep over every element j
 // exactly as in the reference (it does not use the H-matrix). The first sum of B depends only on
 // the element i, so it is computed once per distinct element instead of once per incidence.
-// All sweeps are tiled (8 targets per CTA, element range split across CTAs) with per-thread
+// All sweeps are tiled (2 targets per CTA, element range split across CTAs) with per-thread
 // sums in the kernel precision and FP64 block/split reductions in a fixed order.
 #include "common.cuh"
 #include "internal.h"
@@ -18,7 +18,8 @@ namespace ac3d {
 namespace {
 constexpr int kAdjThreads = 256;
 constexpr int kAdjWarps = kAdjThreads / 32;
-constexpr int kTile = 8;
+constexpr int kTile = 8;   // targets per CTA that the element splits are sized for
+constexpr int kTile3 = 2;  // targets per CTA, few enough for their geometry to stay in registers
 }  // namespace
 
 template <typename R>
@@ -51,28 +52,28 @@ __global__ void __launch_bounds__(kAdjThreads) derA_kernel(GeoView<R> G, Adjoint
 // s1[touch * S + split] = sum_{j in split} x_j dM(c_i, tri_j)/dp_y, i = touch_elem[touch]
 template <typename R>
 __global__ void __launch_bounds__(kAdjThreads) derB_s1_kernel(GeoView<R> G, AdjointArgs a, cd* part, int S) {
-  __shared__ double sd[kAdjWarps][2 * kTile];
-  const int t0 = blockIdx.x * kTile, split = blockIdx.y;
+  __shared__ double sd[kAdjWarps][2 * kTile3];
+  const int t0 = blockIdx.x * kTile3, split = blockIdx.y;
   const int per = (G.ne + S - 1) / S;
   const int j0 = split * per, j1 = min(G.ne, j0 + per);
-  double4 C[kTile];
-  for (int p = 0; p < kTile; p++) C[p] = G.cen[a.touch_elem[min(t0 + p, a.ntouch - 1)]];
-  R ar[kTile], ai[kTile];
-  for (int p = 0; p < kTile; p++) ar[p] = ai[p] = 0;
+  double4 C[kTile3];
+  for (int p = 0; p < kTile3; p++) C[p] = G.cen[a.touch_elem[min(t0 + p, a.ntouch - 1)]];
+  R ar[kTile3], ai[kTile3];
+  for (int p = 0; p < kTile3; p++) ar[p] = ai[p] = 0;
   const R k = (R)a.k;
   for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
     const double4 va = G.va[j];
     const ElemGeo<R> g = G.eg[j];
     const R xr = (R)a.x[j].re, xi = (R)a.x[j].im;
-#pragma unroll 2
-    for (int p = 0; p < kTile; p++) {
+#pragma unroll
+    for (int p = 0; p < kTile3; p++) {
       cplx<R> d = dM_target<R>(k, (R)(C[p].x - va.x), (R)(C[p].y - va.y), (R)(C[p].z - va.z), g);
       ar[p] += d.re * xr - d.im * xi;
       ai[p] += d.re * xi + d.im * xr;
     }
   }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int p = 0; p < kTile; p++) {
+  for (int p = 0; p < kTile3; p++) {
     double vr = warp_sum((double)ar[p]), vi = warp_sum((double)ai[p]);
     if (lane == 0) {
       sd[w][2 * p] = vr;
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(kAdjThreads) derB_s1_kernel(GeoView<R> G, Adjo
     }
   }
   __syncthreads();
-  if (threadIdx.x < 2 * kTile) {
+  if (threadIdx.x < 2 * kTile3) {
     const int p = threadIdx.x >> 1;
     if (t0 + p < a.ntouch) {
       double s = 0;
@@ -91,52 +92,60 @@ __global__ void __launch_bounds__(kAdjThreads) derB_s1_kernel(GeoView<R> G, Adjo
   }
 }
 
-// s2[pair * S + split] = sum_{j in split} lmb_j dM(c_j, tri_i)/dq_{o,y}
+// s2[(3 touch + o) * S + split] = sum_{j in split} lmb_j dM(c_j, tri_i)/dq_{o,y}, i = touch_elem[touch]: all
+// three corners of an element together, since its incidences (one per differentiable corner) share
+// the distances and the kernel values. Bound by FP32 issue: 433 us on the 5280-triangle relief, 854 us
+// with a sweep per incidence.
 template <typename R>
 __global__ void __launch_bounds__(kAdjThreads) derB_s2_kernel(GeoView<R> G, AdjointArgs a, cd* part, int S) {
-  __shared__ double sd[kAdjWarps][2 * kTile];
-  const int t0 = blockIdx.x * kTile, split = blockIdx.y;
+  __shared__ double sd[kAdjWarps][6 * kTile3];
+  const int t0 = blockIdx.x * kTile3, split = blockIdx.y;
   const int per = (G.ne + S - 1) / S;
   const int j0 = split * per, j1 = min(G.ne, j0 + per);
-  double4 A[kTile];
-  ElemGeo<R> Eg[kTile];
-  int O[kTile];
-  for (int p = 0; p < kTile; p++) {
-    const int t = min(t0 + p, a.npairs - 1);
-    const int i = a.pair_elem[t];
+  double4 A[kTile3];
+  ElemGeo<R> Eg[kTile3];
+  for (int p = 0; p < kTile3; p++) {
+    const int i = a.touch_elem[min(t0 + p, a.ntouch - 1)];
     A[p] = G.va[i];
     Eg[p] = G.eg[i];
-    O[p] = a.pair_corner[t];
   }
-  R ar[kTile], ai[kTile];
-  for (int p = 0; p < kTile; p++) ar[p] = ai[p] = 0;
+  R ar[kTile3][3], ai[kTile3][3];
+  for (int p = 0; p < kTile3; p++)
+    for (int o = 0; o < 3; o++) ar[p][o] = ai[p][o] = 0;
   const R k = (R)a.k;
   for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
     const double4 c = G.cen[j];
     const R lr = (R)a.lmb[j].re, li = (R)a.lmb[j].im;
-#pragma unroll 2
-    for (int p = 0; p < kTile; p++) {
-      cplx<R> d = dM_source<R>(k, (R)(c.x - A[p].x), (R)(c.y - A[p].y), (R)(c.z - A[p].z), Eg[p], O[p]);
-      ar[p] += d.re * lr - d.im * li;
-      ai[p] += d.re * li + d.im * lr;
+#pragma unroll
+    for (int p = 0; p < kTile3; p++) {
+      cplx<R> d[3];
+      dM_source3<R>(k, (R)(c.x - A[p].x), (R)(c.y - A[p].y), (R)(c.z - A[p].z), Eg[p], d);
+#pragma unroll
+      for (int o = 0; o < 3; o++) {
+        ar[p][o] += d[o].re * lr - d[o].im * li;
+        ai[p][o] += d[o].re * li + d[o].im * lr;
+      }
     }
   }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int p = 0; p < kTile; p++) {
-    double vr = warp_sum((double)ar[p]), vi = warp_sum((double)ai[p]);
-    if (lane == 0) {
-      sd[w][2 * p] = vr;
-      sd[w][2 * p + 1] = vi;
+#pragma unroll
+  for (int p = 0; p < kTile3; p++)
+#pragma unroll
+    for (int o = 0; o < 3; o++) {
+      double vr = warp_sum((double)ar[p][o]), vi = warp_sum((double)ai[p][o]);
+      if (lane == 0) {
+        sd[w][6 * p + 2 * o] = vr;
+        sd[w][6 * p + 2 * o + 1] = vi;
+      }
     }
-  }
   __syncthreads();
-  if (threadIdx.x < 2 * kTile) {
-    const int p = threadIdx.x >> 1;
-    if (t0 + p < a.npairs) {
+  if (threadIdx.x < 6 * kTile3) {
+    const int p = threadIdx.x / 6, v = threadIdx.x % 6;
+    if (t0 + p < a.ntouch) {
       double s = 0;
       for (int ww = 0; ww < kAdjWarps; ww++) s += sd[ww][threadIdx.x];
-      double* dst = (double*)&part[(size_t)(t0 + p) * S + split];
-      dst[threadIdx.x & 1] = s;
+      double* dst = (double*)&part[(size_t)(3 * (t0 + p) + v / 2) * S + split];
+      dst[v & 1] = s;
     }
   }
 }
@@ -155,9 +164,10 @@ __global__ void adj_combine_kernel(AdjointArgs a, const double4* __restrict__ ce
       s1r += s1[(size_t)ti * S1 + s].re;
       s1i += s1[(size_t)ti * S1 + s].im;
     }
+    const size_t v = 3 * (size_t)ti + a.pair_corner[t];
     for (int s = 0; s < S2; s++) {
-      s2r += s2[(size_t)t * S2 + s].re;
-      s2i += s2[(size_t)t * S2 + s].im;
+      s2r += s2[v * S2 + s].re;
+      s2i += s2[v * S2 + s].im;
     }
     const cd li = a.lmb[i], xi = a.x[i];
     const double B = (s1r * li.re - s1i * li.im) + (s2r * xi.re - s2i * xi.im);
@@ -195,12 +205,13 @@ static void adjoint_t(const DevGeometry& G, const AdjointArgs& a, DevBuf& scratc
   int dev = 0, sms = 0;
   AC3D_CUDA(cudaGetDevice(&dev));
   AC3D_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // element splits: about eight CTAs per SM with kTile targets each, whatever the kernels' own tiles
   const int tiles1 = (a.ntouch + kTile - 1) / kTile, tiles2 = (a.npairs + kTile - 1) / kTile;
   auto pick = [&](int tiles) { return std::max(1, std::min(256, (sms * 8 + tiles - 1) / std::max(1, tiles))); };
   const int S1 = pick(tiles1), S2 = pick(tiles2);
   size_t bytesA = (size_t)a.npairs * sizeof(double);
   size_t bytes1 = (size_t)a.ntouch * S1 * sizeof(cd);
-  size_t bytes2 = (size_t)a.npairs * S2 * sizeof(cd);
+  size_t bytes2 = 3 * (size_t)a.ntouch * S2 * sizeof(cd);
   scratch.ensure(bytesA + bytes1 + bytes2 + 64, s);
   double* outA = scratch.as<double>();
   cd* s1 = (cd*)((char*)scratch.p + ((bytesA + 15) / 16) * 16);
@@ -210,10 +221,10 @@ static void adjoint_t(const DevGeometry& G, const AdjointArgs& a, DevBuf& scratc
   derA_kernel<R><<<(a.npairs * 32 + kAdjThreads - 1) / kAdjThreads, kAdjThreads, 0, s>>>(gv, a, outA);
   AC3D_CUDA(cudaGetLastError());
   note_launch();
-  derB_s1_kernel<R><<<dim3(tiles1, S1), kAdjThreads, 0, s>>>(gv, a, s1, S1);
+  derB_s1_kernel<R><<<dim3((a.ntouch + kTile3 - 1) / kTile3, S1), kAdjThreads, 0, s>>>(gv, a, s1, S1);
   AC3D_CUDA(cudaGetLastError());
   note_launch();
-  derB_s2_kernel<R><<<dim3(tiles2, S2), kAdjThreads, 0, s>>>(gv, a, s2, S2);
+  derB_s2_kernel<R><<<dim3((a.ntouch + kTile3 - 1) / kTile3, S2), kAdjThreads, 0, s>>>(gv, a, s2, S2);
   AC3D_CUDA(cudaGetLastError());
   note_launch();
   adj_combine_kernel<<<(a.HH + 127) / 128, 128, 0, s>>>(a, G.cen.as<double4>(), outA, s1, s2, S1, S2);
@@ -276,30 +287,32 @@ constexpr int bj() { return sizeof(R) == 4 ? 64 : 32; }  // elements per tile (F
 }  // namespace
 
 // s1[(i, r)] = sum_j x_r[j] dM(c_i, tri_j)/dp_y over the touched elements i (kind 0), or
-// s2[(pair, r)] = sum_j lmb_r[j] dM(c_j, tri_i)/dq_{o,y} over the incidences (i, o) (kind 1)
+// s2[(3 i + o, r)] = sum_j lmb_r[j] dM(c_j, tri_i)/dq_{o,y} over the corners o of the touched elements
+// i (kind 1; the corners of an element share the distances and kernel values, so a tile of 32 corners
+// evaluates its 11 or 12 elements once per j)
 template <typename R, int NR, int KIND>
 __global__ void __launch_bounds__(kAdjThreads) derB_tiled_kernel(GeoView<R> G, AdjointMultiArgs a, cd* part, int S) {
   static_assert(kBT * NR == 2 * kAdjThreads, "two (target, direction) sums per thread");
   constexpr int kBJ = bj<R>();
   __shared__ cplx<R> Dt[kBT][kBJ + 1];
   __shared__ cplx<R> Vt[kBJ][NR];
-  __shared__ double4 Tp[kBT];     // target point (kind 0: centroid of i) or vertex a of i (kind 1)
-  __shared__ ElemGeo<R> Tg[kBT];  // kind 1: geometry of i
-  __shared__ int To[kBT];         // kind 1: corner o
-  const int ntarget = KIND == 0 ? a.ntouch : a.npairs;
+  constexpr int kBE = KIND == 0 ? kBT : kBT / 3 + 2;  // elements of a tile of targets, at most
+  __shared__ double4 Tp[kBE];     // target point (kind 0: centroid of i) or vertex a of i (kind 1)
+  __shared__ ElemGeo<R> Tg[kBE];  // kind 1: geometry of i
+  const int ntarget = KIND == 0 ? a.ntouch : 3 * a.ntouch;
   const int t0 = blockIdx.x * kBT, split = blockIdx.y;
+  const int i0 = KIND == 0 ? t0 : t0 / 3;  // first touched element, and how many the tile meets
+  const int ni = KIND == 0 ? kBT : (min(t0 + kBT, ntarget) - 1) / 3 - i0 + 1;
   const int per = (G.ne + S - 1) / S;
   const int j0 = split * per, j1 = min(G.ne, j0 + per);
   const cd* vec = KIND == 0 ? a.x : a.lmb;
-  for (int p = threadIdx.x; p < kBT; p += blockDim.x) {
-    const int t = min(t0 + p, ntarget - 1);
+  for (int p = threadIdx.x; p < ni; p += blockDim.x) {
+    const int i = a.touch_elem[min(i0 + p, a.ntouch - 1)];
     if (KIND == 0) {
-      Tp[p] = G.cen[a.touch_elem[t]];
+      Tp[p] = G.cen[i];
     } else {
-      const int i = a.pair_elem[t];
       Tp[p] = G.va[i];
       Tg[p] = G.eg[i];
-      To[p] = a.pair_corner[t];
     }
   }
   const int p_acc = threadIdx.x / (NR / 2), r_acc = 2 * (threadIdx.x % (NR / 2));
@@ -307,20 +320,28 @@ __global__ void __launch_bounds__(kAdjThreads) derB_tiled_kernel(GeoView<R> G, A
   const R k = (R)a.k;
   for (int jt = j0; jt < j1; jt += kBJ) {
     __syncthreads();  // the previous tile is consumed (and the targets are staged)
-    for (int e = threadIdx.x; e < kBT * kBJ; e += blockDim.x) {
+    for (int e = threadIdx.x; e < ni * kBJ; e += blockDim.x) {
       const int p = e / kBJ, jj = e - p * kBJ, j = jt + jj;
-      cplx<R> d;
-      if (j < j1) {
-        if (KIND == 0) {
+      if (KIND == 0) {
+        cplx<R> d;
+        if (j < j1) {
           const double4 va = G.va[j];
           const ElemGeo<R> g = G.eg[j];
           d = dM_target<R>(k, (R)(Tp[p].x - va.x), (R)(Tp[p].y - va.y), (R)(Tp[p].z - va.z), g);
-        } else {
+        }
+        Dt[p][jj] = d;
+      } else {
+        cplx<R> d[3];
+        if (j < j1) {
           const double4 c = G.cen[j];
-          d = dM_source<R>(k, (R)(c.x - Tp[p].x), (R)(c.y - Tp[p].y), (R)(c.z - Tp[p].z), Tg[p], To[p]);
+          dM_source3<R>(k, (R)(c.x - Tp[p].x), (R)(c.y - Tp[p].y), (R)(c.z - Tp[p].z), Tg[p], d);
+        }
+#pragma unroll
+        for (int o = 0; o < 3; o++) {
+          const int row = 3 * (i0 + p) + o - t0;
+          if (row >= 0 && row < kBT) Dt[row][jj] = d[o];
         }
       }
-      Dt[p][jj] = d;
     }
     for (int e = threadIdx.x; e < kBJ * NR; e += blockDim.x) {
       const int jj = e / NR, r = e - jj * NR, j = jt + jj;
@@ -345,18 +366,24 @@ __global__ void __launch_bounds__(kAdjThreads) derB_tiled_kernel(GeoView<R> G, A
 
 // Per vertex h: sum over its incidences (CSR order), then over the directions, of
 // w_r (A_r - B_r + C_r), with C_r of the plane wave e^{-ik d_r.x} (sphere.h:22-26 along d_r).
+// One warp per vertex: lane r forms direction r's term of an incidence, the terms are added in order
+// (NR <= 32). One thread per vertex took 200 us on the 5280-triangle relief with 6 directions.
 template <int NR>
 __global__ void adj_combine_multi_kernel(AdjointMultiArgs a, const double4* __restrict__ cen,
                                          const double* __restrict__ outA, const cd* __restrict__ s1,
                                          const cd* __restrict__ s2, int S1, int S2, int ne) {
-  const int h = blockIdx.x * blockDim.x + threadIdx.x;
+  static_assert(NR <= 32, "a lane per direction");
+  const int h = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (h >= a.HH) return;
   double acc = 0;
   for (int t = a.h_off[h]; t < a.h_off[h + 1]; t++) {
     const int i = a.pair_elem[t];
     const int ti = a.pair_touch[t];
+    const size_t corner = 3 * (size_t)ti + a.pair_corner[t];
     const double4 c = cen[i];
-    for (int r = 0; r < a.nr; r++) {
+    double term = 0;
+    if (lane < a.nr) {
+      const int r = lane;
       double s1r = 0, s1i = 0, s2r = 0, s2i = 0;
       for (int s = 0; s < S1; s++) {
         const cd v = s1[((size_t)ti * NR + r) * S1 + s];
@@ -364,7 +391,7 @@ __global__ void adj_combine_multi_kernel(AdjointMultiArgs a, const double4* __re
         s1i += v.im;
       }
       for (int s = 0; s < S2; s++) {
-        const cd v = s2[((size_t)t * NR + r) * S2 + s];
+        const cd v = s2[(corner * NR + r) * S2 + s];
         s2r += v.re;
         s2i += v.im;
       }
@@ -375,10 +402,11 @@ __global__ void adj_combine_multi_kernel(AdjointMultiArgs a, const double4* __re
       sincos(ph, &sn, &cs);
       const double f = -a.k * a.dir[r][1] / 3.0;
       const double C = -(f * sn * li.re - f * cs * li.im);
-      acc += a.w[r] * (outA[(size_t)t * NR + r] - B + C);
+      term = outA[(size_t)t * NR + r] - B + C;
     }
+    for (int r = 0; r < a.nr; r++) acc += a.w[r] * __shfl_sync(0xffffffffu, term, r);
   }
-  a.grad[h] += acc;
+  if (lane == 0) a.grad[h] += acc;
 }
 
 template <typename R, int NR>
@@ -389,7 +417,7 @@ static void adjoint_multi_t(const DevGeometry& G, const AdjointMultiArgs& a, Dev
   const int S1 = pick(tiles1), S2 = pick(tiles2);
   const size_t bytesA = ((size_t)a.npairs * NR * sizeof(double) + 15) / 16 * 16;
   const size_t bytes1 = (size_t)a.ntouch * NR * S1 * sizeof(cd);
-  const size_t bytes2 = (size_t)a.npairs * NR * S2 * sizeof(cd);
+  const size_t bytes2 = 3 * (size_t)a.ntouch * NR * S2 * sizeof(cd);
   scratch.ensure(bytesA + bytes1 + bytes2 + 64, s);
   double* outA = scratch.as<double>();
   cd* s1 = (cd*)((char*)scratch.p + bytesA);
@@ -402,10 +430,10 @@ static void adjoint_multi_t(const DevGeometry& G, const AdjointMultiArgs& a, Dev
   derB_tiled_kernel<R, NR, 0><<<dim3(tiles1, S1), kAdjThreads, 0, s>>>(gv, a, s1, S1);
   AC3D_CUDA(cudaGetLastError());
   note_launch();
-  derB_tiled_kernel<R, NR, 1><<<dim3(tiles2, S2), kAdjThreads, 0, s>>>(gv, a, s2, S2);
+  derB_tiled_kernel<R, NR, 1><<<dim3((3 * a.ntouch + kBT - 1) / kBT, S2), kAdjThreads, 0, s>>>(gv, a, s2, S2);
   AC3D_CUDA(cudaGetLastError());
   note_launch();
-  adj_combine_multi_kernel<NR><<<(a.HH + 127) / 128, 128, 0, s>>>(a, G.cen.as<double4>(), outA, s1, s2, S1, S2, G.ne);
+  adj_combine_multi_kernel<NR><<<(a.HH + 3) / 4, 128, 0, s>>>(a, G.cen.as<double4>(), outA, s1, s2, S1, S2, G.ne);
   AC3D_CUDA(cudaGetLastError());
 }
 

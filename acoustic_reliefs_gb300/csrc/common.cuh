@@ -236,6 +236,36 @@ __device__ __forceinline__ cplx<R> dM_source(R k, R dx, R dy, R dz, const ElemGe
   return {are * scale, aim * scale};
 }
 
+// dM_source of the three corners at once: the distance, F and F' of a quadrature point are shared.
+template <typename R>
+__device__ __forceinline__ void dM_source3(R k, R dx, R dy, R dz, const ElemGeo<R>& g, cplx<R> (&out)[3]) {
+  R are[3] = {0, 0, 0}, aim[3] = {0, 0, 0};
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    const R m = (R)quad_m(q), n = (R)quad_n(q), w = (R)quad_w(q);
+    R rx = dx - m * g.ab[0] - n * g.ac[0];
+    R ry = dy - m * g.ab[1] - n * g.ac[1];
+    R rz = dz - m * g.ab[2] - n * g.ac[2];
+    R r = sqrt(rx * rx + ry * ry + rz * rz);
+    R Fre, Fim, dFre, dFim;
+    FdF<R>(k, r, Fre, Fim, dFre, dFim);
+    R s = rx * g.n[0] + ry * g.n[1] + rz * g.n[2];
+#pragma unroll
+    for (int o = 0; o < 3; o++) {
+      const R wx = o == 0 ? g.ab[0] - g.ac[0] : (o == 1 ? g.ac[0] : -g.ab[0]);
+      const R wz = o == 0 ? g.ab[2] - g.ac[2] : (o == 1 ? g.ac[2] : -g.ab[2]);
+      const R lam = o == 0 ? R(1) - m - n : (o == 1 ? m : n);
+      R c1 = -w * lam * ry * s / r;
+      R c2 = w * (-lam * g.n[1] + rx * wz - rz * wx);
+      are[o] += c1 * dFre + c2 * Fre;
+      aim[o] += c1 * dFim + c2 * Fim;
+    }
+  }
+  const R scale = (R)(0.5 / (4.0 * kPi));
+#pragma unroll
+  for (int o = 0; o < 3; o++) out[o] = {are[o] * scale, aim[o] * scale};
+}
+
 // ------------------------------------------------------------------------------------------
 // Reductions
 // ------------------------------------------------------------------------------------------
