@@ -13,6 +13,7 @@
 // with per-column scalars, FP64 dot products reduced in fixed order, and per-column convergence;
 // a column that has converged (or broken down) is frozen while the others continue.
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "common.cuh"
@@ -385,7 +386,10 @@ __global__ void __launch_bounds__(kMT, 1) mseg_dot_tc_kernel(SegView V, const un
   if (warp == 0) tmem_dealloc(tmem, 2 * NT);
 }
 
-// T[task][j] = sum over the task's block entries of P[kpos[e] + q][j], in leaf order.
+// T[task][j] = sum over the task's block entries of P[kpos[e] + q][j], in leaf order; a thread takes two
+// right-hand sides (16-byte loads, half the index loads). Bound by the latency of the chain of index
+// loads, P being 145 MB at 16 right-hand sides on the 20480-triangle relief: 92 us with one
+// right-hand side per thread, 56 us so.
 template <int NRB>
 __global__ void __launch_bounds__(256) mseg_reduce_kernel(const int* __restrict__ task_b,
                                                           const int* __restrict__ t_off, int ntask_cap,
@@ -395,243 +399,356 @@ __global__ void __launch_bounds__(256) mseg_reduce_kernel(const int* __restrict_
                                                           cf* __restrict__ T, const int* __restrict__ done) {
   if (done && *done) return;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int task = (int)(i / NRB), j = (int)(i % NRB);
+  const int task = (int)(i / (NRB / 2)), j = 2 * (int)(i % (NRB / 2));
   if (task >= ntask_cap || task >= *t_total) return;
   const int b = task_b[task];
   const int q = task - t_off[b];
-  float sr = 0, si = 0;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   const int e1 = ent_ptr[b + 1];
   int e = ent_ptr[b];
+  auto at = [&](int k) { return *reinterpret_cast<const float4*>(P + (size_t)(k + q) * NRB + j); };
+  auto add = [&](float4 v) {
+    s.x += v.x;
+    s.y += v.y;
+    s.z += v.z;
+    s.w += v.w;
+  };
   for (; e + 3 < e1; e += 4) {  // four independent loads in flight, summed in entry order
-    const int k0 = kpos[e], k1 = kpos[e + 1], k2 = kpos[e + 2], k3 = kpos[e + 3];
-    const cf v0 = P[(size_t)(k0 + q) * NRB + j], v1 = P[(size_t)(k1 + q) * NRB + j];
-    const cf v2 = P[(size_t)(k2 + q) * NRB + j], v3 = P[(size_t)(k3 + q) * NRB + j];
-    sr += v0.re;
-    si += v0.im;
-    sr += v1.re;
-    si += v1.im;
-    sr += v2.re;
-    si += v2.im;
-    sr += v3.re;
-    si += v3.im;
+    const float4 v0 = at(kpos[e]), v1 = at(kpos[e + 1]), v2 = at(kpos[e + 2]), v3 = at(kpos[e + 3]);
+    add(v0);
+    add(v1);
+    add(v2);
+    add(v3);
   }
-  for (; e < e1; e++) {
-    const cf v = P[(size_t)(kpos[e] + q) * NRB + j];
-    sr += v.re;
-    si += v.im;
-  }
-  T[(size_t)task * NRB + j] = cf(sr, si);
+  for (; e < e1; e++) add(at(kpos[e]));
+  *reinterpret_cast<float4*>(T + (size_t)task * NRB + j) = s;
 }
 
 // Gather pass: Y[rows][j] = -X/2 + near X[idx] + U T[idx], with per-column dot partials. Lane l
 // owns rows l + 32 q of the leaf and accumulates all NRB right-hand sides of them; warp w takes the
 // chunk columns w, w + 8, ..., so each segment element read from shared memory feeds 4 NRB FMAs
 // against the column's multiplier row (read as broadcast 16-byte loads). The warps' partial tiles
-// are summed once per leaf in fixed order. With every chunk's bulk copy each thread gathers (at
-// most) one 16-byte piece of a column's multiplier row (two of its nrb values) by cp.async into
-// the stage's multiplier buffer; the stage's mbarrier expects the copy bytes and one arrival per
-// thread, as in the single-vector gather pass.
+// are summed once per leaf in fixed order.
+//
+// Persistent and warp-specialised, as the single-vector gather pass: eight consumer warps, and one
+// producer warp that streams chunks of the CTA's leaves (a serpentine over the leaves by decreasing
+// work) through a ring: the chunk's bulk copy and its columns' multiplier rows (16-byte cp.async
+// pieces). Bound by FP32 issue: 64 FMAs and 9 shared-memory loads per column and warp at 16
+// right-hand sides, lanes 65% filled by leaves of 21 rows (102 us at full issue on the 20480-triangle
+// relief; 104 instructions per column and warp at 3.0 per clock and SM are issued). The chunks are
+// small (32 columns, 4 per warp), so a barrier of the whole CTA per chunk, one CTA per leaf, took
+// 252 us there; this takes 201 us (8 right-hand sides on 5280 triangles: 33 and 27 us). Packed FP32
+// pairs of right-hand sides (T stored in pairs) issued a fifth less and took 230 us: the pairs of
+// registers leave two CTAs per SM instead of three.
 template <int NRB, int RPL>
-__global__ void __launch_bounds__(kMT) mseg_gather_kernel(SegView V, const cf* __restrict__ near,
-                                                          const cf* __restrict__ lrseg, const cf* __restrict__ T,
-                                                          const cf* __restrict__ X, cf* __restrict__ Y,
-                                                          const cf* __restrict__ dot_a, const cf* __restrict__ dot_b,
-                                                          double* part, double* gpart, unsigned* tickets,
-                                                          double* red, const int* __restrict__ done) {
-  constexpr int CMAX = kMPieces / NRB;        // columns per chunk at most
-  constexpr int PPC = NRB / 2;                // 16-byte pieces per multiplier row
+struct MGather {
+  static constexpr int CMAX = kMPieces / NRB;                              // columns per chunk at most
+  static constexpr int kMatBytes = NRB == 16 && RPL == 1 ? kStageBytes / 2 : kStageBytes;  // 32 columns of 32 rows
+  static constexpr int kZBytes = kMPieces * sizeof(cf);
+  static constexpr int kRing = RPL == 1 ? (NRB == 16 ? 4 : 3) : 3;
+  static constexpr int kCtas = RPL == 1 ? 3 : 2;
+  static constexpr size_t kTile = 4ull * 32 * RPL * NRB * sizeof(cf);      // four partial tiles
+  static constexpr size_t smem() { return (size_t)kRing * (kMatBytes + kZBytes) + kTile; }
+};
+constexpr int kMGatherThreads = kMT + 32;
+
+// Barrier of the consumer warps (bounded; the producer keeps streaming).
+__device__ __forceinline__ bool mg_sync(uint64_t* bar, uint32_t& phase) {
+  mbar_arrive(bar);
+  const bool ok = mbar_wait_bounded(bar, phase);
+  phase ^= 1u;
+  return ok;
+}
+
+template <int NRB, int RPL>
+__global__ void __launch_bounds__(kMGatherThreads, MGather<NRB, RPL>::kCtas) mseg_gather_kernel(
+    SegView V, int nleaf, const cf* __restrict__ near, const cf* __restrict__ lrseg, const cf* __restrict__ T,
+    const cf* __restrict__ X, cf* __restrict__ Y, const cf* __restrict__ dot_a, const cf* __restrict__ dot_b,
+    double* part, double* gpart, unsigned* tickets, double* red, const int* __restrict__ done) {
+  using M = MGather<NRB, RPL>;
+  constexpr int PPC = NRB / 2;  // 16-byte pieces per multiplier row
+  constexpr int kSlots = M::kRing + 1;
   extern __shared__ __align__(128) unsigned char dsmem[];
-  auto stage = reinterpret_cast<unsigned char(*)[kStageBytes]>(dsmem);
-  __shared__ __align__(8) uint64_t full[kStages];
-  __shared__ __align__(16) unsigned char zraw[kStages * kMPieces * sizeof(cf)];
-  auto zbuf = reinterpret_cast<cf(*)[kMPieces]>(zraw);
+  unsigned char* mat = dsmem;
+  unsigned char* zb = dsmem + (size_t)M::kRing * M::kMatBytes;
+  cf* tile = reinterpret_cast<cf*>(zb + (size_t)M::kRing * M::kZBytes);
+  __shared__ __align__(8) uint64_t full[M::kRing], empty[M::kRing], cbar;
+  __shared__ int4 meta[M::kRing];  // leaf slot (-1: no more leaves), columns, first, last
+  __shared__ int4 slot[kSlots];    // position, first row, rows
+  __shared__ double sred[kMW][5][NRB];
+  __shared__ int s_fail;
+  __shared__ bool s_last;
   if (done && *done) return;
-  const int leaf = V.order[blockIdx.x];
-  const int ls = V.leaf_start[leaf], R = V.leaf_start[leaf + 1] - ls;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-
-  const int a_cols = V.a_kptr[leaf + 1] - V.a_kptr[leaf];
-  const int* a_idx = V.a_idx + V.a_kptr[leaf];
-  const int b_cols = V.b_kptr[leaf + 1] - V.b_kptr[leaf];
-  const int* b_idx = V.b_idx + V.b_kptr[leaf];
-  const cf* a_ptr = near + V.a_seg[leaf];
-  const cf* b_ptr = lrseg + V.b_seg[leaf];
-  const int cpc = min(CMAX, max(2, (int)(kStageBytes / sizeof(cf)) / R & ~1));
-  const int na = (a_cols + cpc - 1) / cpc, nb = (b_cols + cpc - 1) / cpc;
-  const int nch = na + nb;
-  struct Chunk {
-    const cf* src;
-    const int* idx;
-    const cf* z;
-    int ncols;
-  };
-  auto chunk = [&](int c) {
-    Chunk k;
-    if (c < na) {
-      const int c0 = c * cpc;
-      k.ncols = min(cpc, a_cols - c0);
-      k.src = a_ptr + (long long)c0 * R;
-      k.idx = a_idx + c0;
-      k.z = X;
-    } else {
-      const int c0 = (c - na) * cpc;
-      k.ncols = min(cpc, b_cols - c0);
-      k.src = b_ptr + (long long)c0 * R;
-      k.idx = b_idx + c0;
-      k.z = T;
-    }
-    return k;
-  };
-  // this thread's piece: column tid / PPC, values 2 (tid % PPC) and 2 (tid % PPC) + 1
-  const int pcol = tid / PPC, ppos = 2 * (tid % PPC);
-  auto col_index = [&](int c) {
-    if (c >= nch) return -1;
-    const Chunk k = chunk(c);
-    return pcol < k.ncols ? k.idx[pcol] : -1;
-  };
-  auto issue = [&](int c, int s, int zi) {
-    const Chunk k = chunk(c);
-    if (pcol < k.ncols) {
-      cf* dst = &zbuf[s][pcol * NRB + ppos];
-      if (zi >= 0) {
-        cp_async_elem<16>(dst, k.z + (size_t)zi * NRB + ppos);
-      } else {
-        dst[0] = cf();
-        dst[1] = cf();
-      }
-    }
-    cp_async_arrive_noinc(&full[s]);
-    if (tid == 0) {
-      const uint32_t bytes = (uint32_t)(k.ncols * R * sizeof(cf));
-      mbar_expect_tx(&full[s], bytes);
-      bulk_copy_g2s(stage[s], k.src, bytes, &full[s]);
-    }
-  };
-
+  const int P = gridDim.x;
   if (tid == 0) {
-    for (int st = 0; st < kStages; st++) mbar_init(&full[st], 1 + kMT);
+    for (int st = 0; st < M::kRing; st++) {
+      mbar_init(&full[st], 1 + 32);
+      mbar_init(&empty[st], kMW);
+    }
+    mbar_init(&cbar, kMT);
+    s_fail = 0;
     fence_barrier_init();
   }
   __syncthreads();
-  {
-    int zi[kStages];
-#pragma unroll
-    for (int c = 0; c < kStages; c++) zi[c] = col_index(c);
-#pragma unroll
-    for (int c = 0; c < kStages; c++)
-      if (c < nch) issue(c, c, zi[c]);
-  }
-  int next_zi = col_index(kStages);
 
-  float ar[RPL][NRB], ai[RPL][NRB];
+  if (warp == kMW) {
+    // ---- producer warp. Leaf geometry is loaded a leaf ahead and column indices a chunk ahead, so
+    // that their latency is not in the ring's way.
+    struct Leaf {
+      int li, ls, R, a_cols, b_cols, cpc, na, nch;
+      const cf *a_ptr, *b_ptr;
+      const int *a_idx, *b_idx;
+    };
+    auto leaf_at = [&](int n) {
+      Leaf L{-1, 0, 1, 0, 0, 2, 0, 1, nullptr, nullptr, nullptr, nullptr};
+      const long long li = (long long)n * P + ((n & 1) ? P - 1 - (int)blockIdx.x : (int)blockIdx.x);
+      if (li >= nleaf) return L;
+      const int leaf = V.order[li], ak = V.a_kptr[leaf], bk = V.b_kptr[leaf];
+      L.li = (int)li;
+      L.ls = V.leaf_start[leaf];
+      L.R = V.leaf_start[leaf + 1] - L.ls;
+      L.a_cols = V.a_kptr[leaf + 1] - ak;
+      L.b_cols = V.b_kptr[leaf + 1] - bk;
+      L.a_idx = V.a_idx + ak;
+      L.b_idx = V.b_idx + bk;
+      L.a_ptr = near + V.a_seg[leaf];
+      L.b_ptr = lrseg + V.b_seg[leaf];
+      L.cpc = min(M::CMAX, max(2, (int)(kStageBytes / sizeof(cf)) / L.R & ~1));
+      L.na = (L.a_cols + L.cpc - 1) / L.cpc;
+      L.nch = max(L.na + (L.b_cols + L.cpc - 1) / L.cpc, 1);  // a leaf without columns still gets one stage
+      return L;
+    };
+    int ix[M::CMAX / 32];  // the next chunk's column indices, one per lane
+    auto load_ix = [&](const Leaf& L, int c) {
+      const bool lr = c >= L.na;
+      const int c0 = (lr ? c - L.na : c) * L.cpc;
+      const int nc = min(L.cpc, (lr ? L.b_cols : L.a_cols) - c0);
+      const int* idx = (lr ? L.b_idx : L.a_idx) + c0;
+      if (L.li >= 0 && nc > 0) {
 #pragma unroll
-  for (int q = 0; q < RPL; q++)
-#pragma unroll
-    for (int jj = 0; jj < NRB; jj++) ar[q][jj] = ai[q][jj] = 0.f;
-  bool ok = true;
-  int c = 0;
-  for (; c < nch; c++) {
-    const int s = c % kStages;
-    if (!cta_wait(&full[s], (uint32_t)(c / kStages) & 1u)) {
-      ok = false;
-      break;
-    }
-    const int ncols = chunk(c).ncols;
-    const cf* S = (const cf*)stage[s];
-    const cf* Z = zbuf[s];
-    for (int cc = warp; cc < ncols; cc += kMW) {
-      const cf* col = S + cc * R;
-      cf u[RPL];
-#pragma unroll
-      for (int q = 0; q < RPL; q++) {
-        const int row = lane + 32 * q;
-        u[q] = row < R ? col[row] : cf();
+        for (int u = 0; u < M::CMAX / 32; u++) ix[u] = idx[min(lane + 32 * u, nc - 1)];
       }
-      const float4* z4 = reinterpret_cast<const float4*>(Z + cc * NRB);
-#pragma unroll
-      for (int jj = 0; jj < NRB / 2; jj++) {
-        const float4 zz = z4[jj];  // multipliers 2 jj and 2 jj + 1
-#pragma unroll
-        for (int q = 0; q < RPL; q++) {
-          ar[q][2 * jj] = fmaf(u[q].re, zz.x, ar[q][2 * jj]);
-          ar[q][2 * jj] = fmaf(-u[q].im, zz.y, ar[q][2 * jj]);
-          ai[q][2 * jj] = fmaf(u[q].re, zz.y, ai[q][2 * jj]);
-          ai[q][2 * jj] = fmaf(u[q].im, zz.x, ai[q][2 * jj]);
-          ar[q][2 * jj + 1] = fmaf(u[q].re, zz.z, ar[q][2 * jj + 1]);
-          ar[q][2 * jj + 1] = fmaf(-u[q].im, zz.w, ar[q][2 * jj + 1]);
-          ai[q][2 * jj + 1] = fmaf(u[q].re, zz.w, ai[q][2 * jj + 1]);
-          ai[q][2 * jj + 1] = fmaf(u[q].im, zz.z, ai[q][2 * jj + 1]);
+    };
+    bool failed = false;
+    long long seq = 0;
+    Leaf nxt = leaf_at(0);
+    load_ix(nxt, 0);
+    for (int n = 0; !failed; n++) {
+      const Leaf L = nxt;
+      const bool live = L.li >= 0;
+      if (live) nxt = leaf_at(n + 1);
+      if (lane == 0 && live) slot[n % kSlots] = make_int4(L.li, L.ls, L.R, 0);
+      for (int c = 0; c < L.nch; c++, seq++) {
+        const int s = (int)(seq % M::kRing);
+        if (seq >= M::kRing) {
+          const bool got =
+              __all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], (uint32_t)(seq / M::kRing - 1) & 1u));
+          if (!got) {
+            if (lane == 0) atomicExch(&s_fail, 1);
+            failed = true;
+            break;
+          }
         }
+        const bool lr = c >= L.na;
+        const int c0 = (lr ? c - L.na : c) * L.cpc;
+        const int ncols = live ? min(L.cpc, (lr ? L.b_cols : L.a_cols) - c0) : 0;
+        const cf* z = lr ? T : X;
+        if (lane == 0) {
+          meta[s] = make_int4(live ? n % kSlots : -1, ncols, c == 0, c == L.nch - 1);
+          const uint32_t bytes = (uint32_t)(ncols * L.R * sizeof(cf));
+          fence_proxy_async();
+          mbar_expect_tx(&full[s], bytes);  // zero bytes: a plain arrival
+          if (bytes)
+            bulk_copy_g2s(mat + (size_t)s * M::kMatBytes, (lr ? L.b_ptr : L.a_ptr) + (long long)c0 * L.R, bytes,
+                          &full[s]);
+        }
+        if (ncols > 0) {
+          // rounds of 32 pieces (a padding column is zero in the segment: it takes multiplier row 0)
+          cf* zs = reinterpret_cast<cf*>(zb + (size_t)s * M::kZBytes);
+#pragma unroll
+          for (int i = 0; i < M::CMAX * PPC / 32; i++) {
+            const int col = i * (32 / PPC) + lane / PPC, pos = 2 * (lane % PPC);
+            const int zi = max(__shfl_sync(0xffffffffu, ix[i * (32 / PPC) / 32], col & 31), 0);
+            if (col < ncols) cp_async_elem<16>(zs + col * NRB + pos, z + (size_t)zi * NRB + pos);
+          }
+        }
+        cp_async_arrive_noinc(&full[s]);
+        if (c + 1 < L.nch)
+          load_ix(L, c + 1);
+        else
+          load_ix(nxt, 0);
       }
-    }
-    __syncthreads();  // stage s and its multipliers are consumed
-    if (c + kStages < nch) {
-      fence_proxy_async();
-      const int zi = next_zi;
-      next_zi = col_index(c + kStages + 1);
-      issue(c + kStages, s, zi);
-    }
-  }
-  if (!ok) {
-    if (tid == 0) {
-      atomicExch(V.err, 1);
-      for (int cc = c; cc < min(nch, c + kStages); cc++)
-        mbar_wait_bounded(&full[cc % kStages], (uint32_t)(cc / kStages) & 1u);
+      if (!live) break;  // the end marker went out
     }
     cp_async_wait_all();
-    __syncthreads();
-  }
-  // sum the warps' tiles in fixed order through four slots in the ring memory (all stages are
-  // consumed): slot w = warp w + warp w + 4, then slot 0 + 1 + 2 + 3
-  cf* tile = (cf*)stage;
-  const int tsz = R * NRB;
-  __syncthreads();
-  for (int round = 0; round < 2; round++) {
-    if ((warp >> 2) == round) {
-      cf* dst = tile + (warp & 3) * tsz;
+    if (lane == 0)
+      for (long long cc = max(0LL, seq - M::kRing); cc < seq; cc++)
+        mbar_wait_bounded(&full[cc % M::kRing], (uint32_t)(cc / M::kRing) & 1u);
+  } else {
+    // ---- consumer warps
+    float ar[RPL][NRB], ai[RPL][NRB];
 #pragma unroll
-      for (int q = 0; q < RPL; q++) {
-        const int row = lane + 32 * q;
-        if (row < R) {
+    for (int q = 0; q < RPL; q++)
 #pragma unroll
-          for (int jj = 0; jj < NRB; jj++) {
-            cf v(ar[q][jj], ai[q][jj]);
-            if (round) v = cf(dst[row * NRB + jj].re + v.re, dst[row * NRB + jj].im + v.im);
-            dst[row * NRB + jj] = v;
+      for (int jj = 0; jj < NRB; jj++) ar[q][jj] = ai[q][jj] = 0.f;
+    int li = 0, ls = 0, R = 1;
+    uint32_t cphase = 0;
+    bool cok = true;
+    for (long long seq = 0;; seq++) {
+      const int s = (int)(seq % M::kRing);
+      const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], (uint32_t)(seq / M::kRing) & 1u));
+      if (!got) {
+        if (lane == 0) atomicExch(&s_fail, 1);
+        break;
+      }
+      const int4 mt = meta[s];
+      if (mt.x < 0) break;
+      if (mt.z) {
+        const int4 g = slot[mt.x];
+        li = g.x;
+        ls = g.y;
+        R = g.z;
+      }
+      const int ncols = mt.y;
+      const cf* S = reinterpret_cast<const cf*>(mat + (size_t)s * M::kMatBytes);
+      const cf* Z = reinterpret_cast<const cf*>(zb + (size_t)s * M::kZBytes);
+      // rows >= R are accumulated and not stored
+      const float4* z4 = reinterpret_cast<const float4*>(Z + warp * NRB);
+      const cf* up[RPL];
+#pragma unroll
+      for (int q = 0; q < RPL; q++) up[q] = S + warp * R + min(lane + 32 * q, R - 1);
+      const int ustep = kMW * R;
+      for (int cc = warp; cc < ncols; cc += kMW) {
+        cf u[RPL];
+#pragma unroll
+        for (int q = 0; q < RPL; q++) {
+          u[q] = *up[q];
+          up[q] += ustep;
+        }
+#pragma unroll
+        for (int jj = 0; jj < NRB / 2; jj++) {
+          const float4 zz = z4[jj];  // multipliers 2 jj and 2 jj + 1
+#pragma unroll
+          for (int q = 0; q < RPL; q++) {
+            ar[q][2 * jj] = fmaf(u[q].re, zz.x, ar[q][2 * jj]);
+            ar[q][2 * jj] = fmaf(-u[q].im, zz.y, ar[q][2 * jj]);
+            ai[q][2 * jj] = fmaf(u[q].re, zz.y, ai[q][2 * jj]);
+            ai[q][2 * jj] = fmaf(u[q].im, zz.x, ai[q][2 * jj]);
+            ar[q][2 * jj + 1] = fmaf(u[q].re, zz.z, ar[q][2 * jj + 1]);
+            ar[q][2 * jj + 1] = fmaf(-u[q].im, zz.w, ar[q][2 * jj + 1]);
+            ai[q][2 * jj + 1] = fmaf(u[q].re, zz.w, ai[q][2 * jj + 1]);
+            ai[q][2 * jj + 1] = fmaf(u[q].im, zz.z, ai[q][2 * jj + 1]);
+          }
+        }
+        z4 += kMW * NRB / 2;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
+      if (!mt.w) continue;
+      // ---- the leaf is complete: the warps' tiles in fixed order (slot w = warp w + warp w + 4, then
+      // slots 0 + 1 + 2 + 3)
+      const int tsz = R * NRB;
+      for (int round = 0; round < 2 && cok; round++) {
+        if ((warp >> 2) == round) {
+          cf* dst = tile + (warp & 3) * tsz;
+#pragma unroll
+          for (int q = 0; q < RPL; q++) {
+            const int row = lane + 32 * q;
+            if (row < R) {
+#pragma unroll
+              for (int jj = 0; jj < NRB; jj++) {
+                cf v(ar[q][jj], ai[q][jj]);
+                if (round) v = cf(dst[row * NRB + jj].re + v.re, dst[row * NRB + jj].im + v.im);
+                dst[row * NRB + jj] = v;
+              }
+            }
+          }
+        }
+        cok = mg_sync(&cbar, cphase);
+      }
+      if (!cok) break;
+#pragma unroll
+      for (int q = 0; q < RPL; q++)
+#pragma unroll
+        for (int jj = 0; jj < NRB; jj++) ar[q][jj] = ai[q][jj] = 0.f;
+      double d[5] = {0, 0, 0, 0, 0};
+      for (int i = tid; i < tsz; i += kMT) {  // column j = tid % NRB for every i of this thread
+        const int row = i / NRB;
+        const cf t0 = tile[i], t1 = tile[tsz + i], t2 = tile[2 * tsz + i], t3 = tile[3 * tsz + i];
+        const float sr = ((t0.re + t1.re) + t2.re) + t3.re, si = ((t0.im + t1.im) + t2.im) + t3.im;
+        const size_t e = (size_t)(ls + row) * NRB + i % NRB;
+        const cf xv = X[e];
+        const cf o(sr - 0.5f * xv.re, si - 0.5f * xv.im);
+        Y[e] = o;
+        if (part) {
+          const double oyr = o.re, oyi = o.im;
+          if (dot_a) {
+            const cf a = dot_a[e];
+            d[0] += (double)a.re * oyr + (double)a.im * oyi;
+            d[1] += (double)a.re * oyi - (double)a.im * oyr;
+          }
+          if (dot_b) {
+            const cf bb = dot_b[e];
+            d[2] += oyr * (double)bb.re + oyi * (double)bb.im;
+            d[3] += oyr * (double)bb.im - oyi * (double)bb.re;
+          }
+          d[4] += oyr * oyr + oyi * oyi;
+        }
+      }
+      if (part) {
+        // this leaf's partials at its position, then the two-level sum of grid_reduce with the leaves'
+        // positions in the place of CTAs
+#pragma unroll
+        for (int c = 0; c < 5; c++)
+#pragma unroll
+          for (int o = NRB; o < 32; o <<= 1) d[c] += __shfl_xor_sync(0xffffffffu, d[c], o);
+        if (lane < NRB)
+          for (int c = 0; c < 5; c++) sred[warp][c][lane] = d[c];
+        if (!(cok = mg_sync(&cbar, cphase))) break;
+        for (int v = tid; v < 5 * NRB; v += kMT) {
+          double a = 0;
+          for (int w = 0; w < kMW; w++) a += sred[w][v / NRB][v % NRB];
+          part[(size_t)li * 5 * NRB + v] = a;
+        }
+        const int g = li / kGroup, ng = (nleaf + kGroup - 1) / kGroup, gsize = min(kGroup, nleaf - g * kGroup);
+        __threadfence();
+        if (!(cok = mg_sync(&cbar, cphase))) break;
+        if (tid == 0) s_last = atomicAdd(&tickets[g], 1u) == (unsigned)(gsize - 1);
+        if (!(cok = mg_sync(&cbar, cphase))) break;
+        if (s_last) {
+          __threadfence();
+          for (int v = tid; v < 5 * NRB; v += kMT) {
+            double a = 0;
+#pragma unroll 8
+            for (int i = 0; i < gsize; i++) a += __ldcg(&part[(size_t)(g * kGroup + i) * 5 * NRB + v]);
+            gpart[(size_t)g * 5 * NRB + v] = a;
+          }
+          __threadfence();
+          if (!(cok = mg_sync(&cbar, cphase))) break;
+          if (tid == 0) {
+            tickets[g] = 0u;
+            s_last = atomicAdd(&tickets[ng], 1u) == (unsigned)(ng - 1);
+          }
+          if (!(cok = mg_sync(&cbar, cphase))) break;
+          if (s_last) {
+            __threadfence();
+            for (int v = tid; v < 5 * NRB; v += kMT) {
+              double a = 0;
+#pragma unroll 8
+              for (int i = 0; i < ng; i++) a += __ldcg(&gpart[(size_t)i * 5 * NRB + v]);
+              red[v] = a;
+            }
+            if (tid == 0) tickets[ng] = 0u;
           }
         }
       }
+      if (!(cok = mg_sync(&cbar, cphase))) break;  // the tiles, sred and s_last are free for the next leaf
     }
-    __syncthreads();
+    if (!cok && lane == 0) atomicExch(&s_fail, 1);
   }
-  double d[5] = {0, 0, 0, 0, 0};
-  for (int i = tid; i < tsz; i += kMT) {  // column j = tid % NRB for every i of this thread
-    const int row = i / NRB;
-    {
-      const cf t0 = tile[i], t1 = tile[tsz + i], t2 = tile[2 * tsz + i], t3 = tile[3 * tsz + i];
-      const float sr = ((t0.re + t1.re) + t2.re) + t3.re, si = ((t0.im + t1.im) + t2.im) + t3.im;
-      const size_t e = (size_t)(ls + row) * NRB + i % NRB;
-      const cf xv = X[e];
-      const cf o(sr - 0.5f * xv.re, si - 0.5f * xv.im);
-      Y[e] = o;
-      const double oyr = o.re, oyi = o.im;
-      if (dot_a) {
-        const cf a = dot_a[e];
-        d[0] += (double)a.re * oyr + (double)a.im * oyi;
-        d[1] += (double)a.re * oyi - (double)a.im * oyr;
-      }
-      if (dot_b) {
-        const cf bb = dot_b[e];
-        d[2] += oyr * (double)bb.re + oyi * (double)bb.im;
-        d[3] += oyr * (double)bb.im - oyi * (double)bb.re;
-      }
-      d[4] += oyr * oyr + oyi * oyi;
-    }
-  }
-  if (part) {
-    cta_partials<NRB>(d, part);
-    grid_reduce<5 * NRB>(part, gpart, tickets, red);
-  }
+  __syncthreads();
+  if (s_fail && tid == 0) atomicExch(V.err, 1);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -900,7 +1017,7 @@ template <int NRB, int RPL>
 static void set_multi_attrs() {
   AC3D_CUDA(cudaFuncSetAttribute(mseg_dot_kernel<NRB, RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMRing));
   AC3D_CUDA(cudaFuncSetAttribute(mseg_gather_kernel<NRB, RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kMRing));
+                                 (int)MGather<NRB, RPL>::smem()));
   AC3D_CUDA(cudaFuncSetAttribute(mseg_dot_kernel<NRB, RPL>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   AC3D_CUDA(cudaFuncSetAttribute(mseg_gather_kernel<NRB, RPL>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
 }
@@ -953,7 +1070,7 @@ static void mmv_t(const DevPartition& DP, const DevHMat& H, const MultiBufs& B, 
                                                                (const cf*)x, P, done);
     AC3D_CUDA(cudaGetLastError());
     note_launch();
-    const long long thr = H.task_cap * NRB;
+    const long long thr = H.task_cap * (NRB / 2);
     mseg_reduce_kernel<NRB><<<(int)((thr + 255) / 256), 256, 0, s>>>(
         H.task_b.as<int>(), H.t_off.as<int>(), (int)H.task_cap, H.t_off.as<int>() + DP.na,
         tr ? DP.blk_fw_ptr.as<int>() : DP.blk_tr_ptr.as<int>(), tr ? H.kpos_f.as<int>() : H.kpos_t.as<int>(), P,
@@ -970,9 +1087,18 @@ static void mmv_t(const DevPartition& DP, const DevHMat& H, const MultiBufs& B, 
   const cf* g_lr = tr ? H.vseg.as<cf>() : H.useg.as<cf>();
   double* g_part = dots ? B.partials : nullptr;
   double* g_gpart = B.partials + (size_t)std::max(DP.nleaf, 1184) * 5 * NRB;
-  mseg_gather_kernel<NRB, RPL><<<DP.nleaf, kMT, kMRing, s>>>(v, g_near, g_lr, T, (const cf*)x, (cf*)y,
-                                                              (const cf*)dot_a, (const cf*)dot_b, g_part, g_gpart,
-                                                              B.ticket, B.red, done);
+  constexpr size_t gsmem = MGather<NRB, RPL>::smem();
+  static std::atomic<int> per_sm{0};
+  int nb = per_sm.load();
+  if (!nb) {
+    AC3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, mseg_gather_kernel<NRB, RPL>, kMGatherThreads, gsmem));
+    nb = std::max(nb, 1);
+    per_sm.store(nb);
+  }
+  const int grid = std::min(DP.nleaf, nb * device_sm_count());
+  mseg_gather_kernel<NRB, RPL><<<grid, kMGatherThreads, gsmem, s>>>(v, DP.nleaf, g_near, g_lr, T, (const cf*)x, (cf*)y,
+                                                                    (const cf*)dot_a, (const cf*)dot_b, g_part, g_gpart,
+                                                                    B.ticket, B.red, done);
   if (DP.nleaf > 1024 * kGroup) throw Error(1, "block solves support at most 32768 leaf clusters");
   AC3D_CUDA(cudaGetLastError());
 }
