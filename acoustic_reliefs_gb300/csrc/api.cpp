@@ -11,6 +11,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <string>
 #include <unordered_map>
@@ -92,44 +93,96 @@ static std::vector<double> hemisphere(double radius, double ds) {
   return L;
 }
 
+// Device time between its construction and stop(), added to a statistic when the call ends
+// (resolve_timers): reading it at once would make the host wait between the phases of a call and
+// the device wait for the host's next launches.
 struct GpuTimer {
-  cudaEvent_t a = nullptr, b = nullptr;
-  cudaStream_t s;
-  explicit GpuTimer(cudaStream_t st) : s(st) {
-    AC3D_CUDA(cudaEventCreate(&a));
-    AC3D_CUDA(cudaEventCreate(&b));
-    AC3D_CUDA(cudaEventRecord(a, s));
+  ac3d_ctx* c;
+  PhaseTimer t;
+  explicit GpuTimer(ac3d_ctx* ctx) : c(ctx) {
+    AC3D_CUDA(cudaEventCreate(&t.a));
+    AC3D_CUDA(cudaEventCreate(&t.b));
+    AC3D_CUDA(cudaEventRecord(t.a, c->stream));
   }
-  double stop() {
-    AC3D_CUDA(cudaEventRecord(b, s));
-    AC3D_CUDA(cudaEventSynchronize(b));
-    float ms = 0;
-    AC3D_CUDA(cudaEventElapsedTime(&ms, a, b));
-    return ms;
+  GpuTimer(const GpuTimer&) = delete;
+  GpuTimer& operator=(const GpuTimer&) = delete;
+  void stop(double* acc) {
+    AC3D_CUDA(cudaEventRecord(t.b, c->stream));
+    t.acc = acc;
+    c->timers.push_back(t);
+    t = PhaseTimer{};
   }
   ~GpuTimer() {
-    if (a) cudaEventDestroy(a);
-    if (b) cudaEventDestroy(b);
+    if (t.a) cudaEventDestroy(t.a);
+    if (t.b) cudaEventDestroy(t.b);
   }
 };
 
-// A captured chunk of solver iterations as an executable graph. If enqueueing throws during the
-// capture, the capture is ended and its graph discarded, so the stream is usable again; the
-// executable graph is destroyed on every exit path after the stream has drained (an error may be
-// thrown while a launch is in flight).
-struct CapturedGraph {
-  cudaStream_t s;
+void drop_timers(ac3d_ctx* c) {
+  for (PhaseTimer& t : c->timers) {
+    cudaEventDestroy(t.a);
+    cudaEventDestroy(t.b);
+  }
+  c->timers.clear();
+}
+
+void resolve_timers(ac3d_ctx* c) {
+  for (PhaseTimer& t : c->timers) {
+    float ms = 0;
+    AC3D_CUDA(cudaEventSynchronize(t.b));
+    AC3D_CUDA(cudaEventElapsedTime(&ms, t.a, t.b));
+    *t.acc += ms;
+  }
+  drop_timers(c);
+}
+
+// On the way out of a failed call (a solve that did not converge keeps its phase times).
+void finish_timers(ac3d_ctx* c) {
+  try {
+    resolve_timers(c);
+  } catch (const Error&) {
+    cudaGetLastError();
+    drop_timers(c);
+  }
+}
+
+// Chunks of solver iterations: the first is enqueued directly, the later ones replay a graph captured
+// behind it. Capturing, instantiating and first launching a chunk took 0.45 to 0.55 ms and destroying
+// the executable graph 0.15 to 0.2 ms, with the device idle; now the device runs the direct chunk
+// meanwhile (a direct iteration costs it about 7 us more than a replayed one), a solve of one chunk
+// captures nothing, and a used graph is destroyed behind the next solve's first chunk. With the layout
+// of an assembly formed on the device (launch_leaf_layout), whole solves take 8.53 -> 7.78 ms on the
+// 5280-triangle relief, 1.65 -> 1.42 ms on the 1280-triangle sphere, 243 -> 238 ms on 118680 triangles.
+// If enqueueing throws during the capture, the capture is ended and its graph discarded, so the stream
+// is usable again.
+struct ChunkRunner {
+  static constexpr int kDirect = 1;
+  ac3d_ctx* c;
+  std::function<void()> enqueue;
   cudaGraphExec_t exec = nullptr;
   long long nodes = 0;  // kernels per launch
-  // host milliseconds spent capturing and instantiating are added to *ms_host
-  template <typename F>
-  CapturedGraph(cudaStream_t st, double* ms_host, F&& enqueue) : s(st) {
+  int launches = 0;
+  ChunkRunner(ac3d_ctx* ctx, std::function<void()> f) : c(ctx), enqueue(std::move(f)) {}
+  ChunkRunner(const ChunkRunner&) = delete;
+  ChunkRunner& operator=(const ChunkRunner&) = delete;
+  void launch() {
+    if (launches++ < kDirect) {
+      enqueue();
+      if (launches == 1) c->destroy_used_graphs();
+      return;
+    }
+    if (!exec) capture();
+    AC3D_CUDA(cudaGraphLaunch(exec, c->stream));
+    note_launch(nodes);
+  }
+  void capture() {
     const auto t0 = std::chrono::steady_clock::now();
-    struct Add {
+    struct Add {  // host milliseconds spent capturing and instantiating
       double* acc;
       std::chrono::steady_clock::time_point t0;
       ~Add() { *acc += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count(); }
-    } add{ms_host, t0};
+    } add{&c->stats.ms_graph, t0};
+    cudaStream_t s = c->stream;
     const long long before = t_kernel_launches;
     AC3D_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     try {
@@ -151,16 +204,10 @@ struct CapturedGraph {
     if (ei != cudaSuccess) exec = nullptr;
     AC3D_CUDA(ei);
   }
-  CapturedGraph(const CapturedGraph&) = delete;
-  CapturedGraph& operator=(const CapturedGraph&) = delete;
-  void launch() {
-    AC3D_CUDA(cudaGraphLaunch(exec, s));
-    note_launch(nodes);
-  }
-  ~CapturedGraph() {
+  ~ChunkRunner() {
     if (exec) {
-      cudaStreamSynchronize(s);
-      cudaGraphExecDestroy(exec);
+      cudaStreamSynchronize(c->stream);  // an error may be thrown while a launch is in flight
+      c->used_graphs.push_back(exec);
     }
   }
 };
@@ -173,17 +220,6 @@ struct ScopedEvent {
   ScopedEvent& operator=(const ScopedEvent&) = delete;
   ~ScopedEvent() {
     if (e) cudaEventDestroy(e);
-  }
-};
-
-struct GraphCache {
-  cudaGraphExec_t exec = nullptr;
-  const void* key_h = nullptr;
-  const void* key_x = nullptr;
-  bool tr = false;
-  int vec64 = 0;
-  ~GraphCache() {
-    if (exec) cudaGraphExecDestroy(exec);
   }
 };
 
@@ -250,14 +286,27 @@ std::unique_ptr<DevHMat> assemble(ac3d_ctx* c, double k, int prec) {
   AC3D_CUDA(cudaMemsetAsync(H->rank.p, 0, (size_t)std::max(na, 1) * sizeof(int), s));
   if (na > 0) {
     H->term_off.alloc((size_t)na * c->maxk * sizeof(long long), s);
-    H->pool_used.alloc(16, s);
+    // layout totals and the pool's counters, read back together (AsmTotals)
+    H->pool_used.alloc(sizeof(AsmTotals), s);
+    if (!c->h_totals) AC3D_CUDA(cudaMallocHost(&c->h_totals, sizeof(AsmTotals)));
+    const int nleaf = c->m->DP.nleaf;
+    for (DevBuf* kb : {&H->kseg_f, &H->kseg_t}) kb->alloc((size_t)(nleaf + 1) * sizeof(int), s);
+    for (DevBuf* sb : {&H->seg_f, &H->seg_t}) sb->alloc((size_t)(nleaf + 1) * sizeof(long long), s);
+    for (DevBuf* ob : {&H->order_rows, &H->order_cols}) ob->alloc((size_t)nleaf * sizeof(int), s);
+    const size_t tcap = (size_t)std::max<int64_t>(c->m->P.aca_term_cap, 1);
+    H->task_cap = (int64_t)tcap;
+    H->task_b.alloc(tcap * sizeof(int), s);
+    H->task_off.alloc(tcap * sizeof(long long), s);
+    DevBuf leaf_work;  // streamed columns per leaf, both sides
+    leaf_work.alloc(2 * (size_t)nleaf * sizeof(int), s);
+    const AsmTotals& tot = *c->h_totals;
     int64_t cap = c->m->pool_hint[prec];
     if (cap <= 0) cap = std::min<int64_t>(c->m->worst_pool, 16 * c->m->sum_mn);
     cap = std::max<int64_t>(cap, 1024);
     for (int attempt = 0;; attempt++) {
       H->pool.alloc((size_t)cap * pool_es, s);
       H->pool_cap = cap;
-      AC3D_CUDA(cudaMemsetAsync(H->pool_used.p, 0, 16, s));
+      AC3D_CUDA(cudaMemsetAsync(H->pool_used.p, 0, sizeof(AsmTotals), s));
       // FP32 and FP64: the ACA groups on the two assembly streams (the first after the near field).
       // Double-float: the ACA first, longest blocks first, and the near field behind its large
       // blocks, whose short CTAs fill the SMs as the blocks run out
@@ -273,108 +322,43 @@ std::unique_ptr<DevHMat> assemble(ac3d_ctx* c, double k, int prec) {
       AC3D_CUDA(cudaEventRecord(c->ev_join_asm, as));
       AC3D_CUDA(cudaStreamWaitEvent(s, c->ev_join, 0));
       AC3D_CUDA(cudaStreamWaitEvent(s, c->ev_join_asm, 0));
-      unsigned long long hu[2];
-      AC3D_CUDA(cudaMemcpyAsync(hu, H->pool_used.p, 16, cudaMemcpyDeviceToHost, s));
+      // ranks, segment layout and leaf orders on the device, so that the host waits once and reads
+      // totals only (on an overflowed pool the ranks are those of the terms that fit)
+      launch_rank_scan(c->m->DP, *H, s);
+      launch_leaf_layout(c->m->DP, *H, leaf_work.as<int>(), s);
+      AC3D_CUDA(cudaMemcpyAsync(c->h_totals, H->pool_used.p, sizeof(AsmTotals), cudaMemcpyDeviceToHost, s));
       AC3D_CUDA(cudaStreamSynchronize(s));
-      int status = (int)(hu[1] & 0xffffffffu);
-      if (!(status & 1)) {
-        H->pool_used_host = (int64_t)hu[0];
+      if (!(tot.status & 1)) {
+        H->pool_used_host = (int64_t)tot.pool_used;
         break;
       }
       if (cap >= c->m->worst_pool || attempt > 8) throw Error(AC3D_ERR_INTERNAL, "ACA pool overflow at worst-case size");
-      cap = std::min<int64_t>(c->m->worst_pool, std::max<int64_t>(cap * 2, (int64_t)hu[0]));
+      cap = std::min<int64_t>(c->m->worst_pool, std::max<int64_t>(cap * 2, (int64_t)tot.pool_used));
     }
     c->m->pool_hint[prec] = std::min<int64_t>(c->m->worst_pool, H->pool_used_host + H->pool_used_host / 8 + 4096);
-    const size_t tcap = (size_t)std::max<int64_t>(c->m->P.aca_term_cap, 1);
-    H->task_cap = (int64_t)tcap;
-    H->task_b.alloc(tcap * sizeof(int), s);
-    H->task_off.alloc(tcap * sizeof(long long), s);
-    launch_rank_scan(c->m->DP, *H, s);
     H->tvec.alloc(tcap * (prec == PREC_FP64 ? sizeof(cd) : sizeof(cf)), s);
     H->tvec64.alloc(tcap * sizeof(cd), s);
-    H->ranks_host.resize(na);
-    std::vector<int> passes(na);
-    AC3D_CUDA(cudaMemcpyAsync(H->ranks_host.data(), H->rank.p, na * sizeof(int), cudaMemcpyDeviceToHost, s));
-    AC3D_CUDA(cudaMemcpyAsync(passes.data(), H->passes.p, na * sizeof(int), cudaMemcpyDeviceToHost, s));
-    AC3D_CUDA(cudaStreamSynchronize(s));
-    int64_t lr = 0, ev = 0;
-    int mx = 0;
-    double sr = 0;
-    for (int b = 0; b < na; b++) {
-      int r = H->ranks_host[b];
-      const int* q = &c->m->P.approx[4 * b];
-      lr += (int64_t)r * ((q[1] - q[0]) + (q[3] - q[2]));
-      ev += (int64_t)passes[b] * ((q[1] - q[0]) + (q[3] - q[2]));
-      mx = std::max(mx, r);
-      sr += r;
-    }
-    H->lr_entries = lr;
-    H->aca_evaluated = ev;
-    c->stats.lr_entries = lr;
-    c->stats.aca_entries_evaluated = ev;
+    H->lr_entries = (int64_t)tot.lr_entries;
+    H->aca_evaluated = (int64_t)tot.aca_evaluated;
+    H->tc_bytes[0] = (int64_t)tot.tc_bytes[0];
+    H->tc_bytes[1] = (int64_t)tot.tc_bytes[1];
+    c->stats.lr_entries = H->lr_entries;
+    c->stats.aca_entries_evaluated = H->aca_evaluated;
     // per-leaf segments (U by row leaf, V by column leaf), then the pool is released
-    int64_t sum_rn = 0, kf = 0, kt = 0;
-    for (int b = 0; b < na; b++) sum_rn += (int64_t)H->ranks_host[b] * (c->m->P.approx[4 * b + 3] - c->m->P.approx[4 * b + 2]);
-    const int nleaf = c->m->DP.nleaf;
-    int64_t segf = 0, segt = 0;
-    for (int l = 0; l < nleaf; l++) {
-      const int Rl = c->m->P.leaf_start[l + 1] - c->m->P.leaf_start[l];
-      int K = 0;
-      for (int it = c->m->P.fw_lr_ptr[l]; it < c->m->P.fw_lr_ptr[l + 1]; it++) K += H->ranks_host[c->m->P.fw_lr[it]];
-      K += K & 1;
-      kf += K;
-      segf += (int64_t)K * Rl;
-      K = 0;
-      for (int it = c->m->P.tr_lr_ptr[l]; it < c->m->P.tr_lr_ptr[l + 1]; it++) K += H->ranks_host[c->m->P.tr_lr[it]];
-      K += K & 1;
-      kt += K;
-      segt += (int64_t)K * Rl;
-    }
-    H->kseg_f.alloc((size_t)(nleaf + 1) * sizeof(int), s);
-    H->kseg_t.alloc((size_t)(nleaf + 1) * sizeof(int), s);
-    H->seg_f.alloc((size_t)(nleaf + 1) * sizeof(long long), s);
-    H->seg_t.alloc((size_t)(nleaf + 1) * sizeof(long long), s);
-    H->useg.alloc((size_t)std::max<int64_t>(segf, 2) * cs, s);
-    H->vseg.alloc((size_t)std::max<int64_t>(segt, 2) * cs, s);
+    const int64_t kf = (int64_t)tot.columns[0], kt = (int64_t)tot.columns[1];
+    H->useg.alloc((size_t)std::max<int64_t>((int64_t)tot.entries[0], 2) * cs, s);
+    H->vseg.alloc((size_t)std::max<int64_t>((int64_t)tot.entries[1], 2) * cs, s);
     H->uidx.alloc((size_t)std::max<int64_t>(kf, 1) * sizeof(int), s);
     H->vidx.alloc((size_t)std::max<int64_t>(kt, 1) * sizeof(int), s);
     H->kpos_f.alloc((size_t)std::max<size_t>(c->m->P.fw_lr.size(), 1) * sizeof(int), s);
     H->kpos_t.alloc((size_t)std::max<size_t>(c->m->P.tr_lr.size(), 1) * sizeof(int), s);
     H->pbuf.alloc((size_t)std::max<int64_t>(std::max(kf, kt), 1) * sizeof(cd), s);
-    // leaves by decreasing streamed bytes: row leaves (near + U columns) for the forward gather and
-    // the transposed dot, column leaves (V columns; + transposed near) for the forward dot and the
-    // transposed gather. The hardware dispatches CTAs in index order, so this is
-    // longest-first list scheduling.
-    {
-      std::vector<int64_t> wr(nleaf), wc(nleaf);
-      std::vector<int> ord(nleaf);
-      for (int l = 0; l < nleaf; l++) {
-        const int Rl = c->m->P.leaf_start[l + 1] - c->m->P.leaf_start[l];
-        int64_t kr = c->m->P.didx_ptr[l + 1] - c->m->P.didx_ptr[l], kc = 0;
-        for (int it = c->m->P.fw_lr_ptr[l]; it < c->m->P.fw_lr_ptr[l + 1]; it++) kr += H->ranks_host[c->m->P.fw_lr[it]];
-        for (int it = c->m->P.tr_lr_ptr[l]; it < c->m->P.tr_lr_ptr[l + 1]; it++) kc += H->ranks_host[c->m->P.tr_lr[it]];
-        for (int it = c->m->P.tr_near_ptr[l]; it < c->m->P.tr_near_ptr[l + 1]; it++) {
-          const int* q = &c->m->P.direct[4 * c->m->P.tr_near[it]];
-          kc += q[1] - q[0];
-        }
-        wr[l] = kr * Rl;
-        wc[l] = kc * Rl;
-      }
-      auto sorted = [&](const std::vector<int64_t>& w) {
-        for (int l = 0; l < nleaf; l++) ord[l] = l;
-        std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return w[a] > w[b]; });
-        return ord;
-      };
-      upload(H->order_rows, sorted(wr), s);
-      upload(H->order_cols, sorted(wc), s);
-    }
     launch_pack(c->m->DP, *H, false, s);
     launch_pack(c->m->DP, *H, true, s);
     H->pool.release();
     H->term_off.release();
-    (void)sum_rn;
-    c->stats.max_rank = mx;
-    c->stats.mean_rank = sr / na;
+    c->stats.max_rank = (int)tot.max_rank;
+    c->stats.mean_rank = (double)tot.sum_rank / na;
   } else {
     // no admissible blocks: only the near field ran on the assembly stream
     AC3D_CUDA(cudaEventRecord(c->ev_join_asm, as));
@@ -407,10 +391,6 @@ std::unique_ptr<DevHMat> assemble(ac3d_ctx* c, double k, int prec) {
 // ------------------------------------------------------------------------------------------
 // Solve op(A) x = b (b, x FP64 device vectors of length Ne)
 // ------------------------------------------------------------------------------------------
-struct SolveCache {
-  std::vector<std::unique_ptr<GraphCache>> graphs;
-};
-
 void ensure_work(ac3d_ctx* c) {
   cudaStream_t s = c->stream;
   const size_t n = (size_t)c->m->Ne;
@@ -448,13 +428,13 @@ KrylovBufs bufs(ac3d_ctx* c, int vec64) {
   return B;
 }
 
-// Runs BiCGSTAB on the prepared buffers (B.b filled). Returns iterations; done flag in *done.
-int run_krylov(ac3d_ctx* c, const DevHMat& H, const KrylovBufs& B, bool tr, int vec64, double tol, int* done) {
+// Runs BiCGSTAB on the prepared buffers (B.b filled), g enqueueing its iterations. Returns iterations;
+// done flag in *done.
+int run_krylov(ac3d_ctx* c, const KrylovBufs& B, ChunkRunner& g, int vec64, double tol, int* done) {
   cudaStream_t s = c->stream;
   const int maxit = c->maxit > 0 ? c->maxit : 2 * c->m->Ne;
   krylov_enqueue_init(B, vec64, tol, maxit, s);
-  // capture one chunk of iterations as a graph and replay it until the state reports completion
-  CapturedGraph g(s, &c->stats.ms_graph, [&] { krylov_enqueue_iterations(B, c->m->DP, H, tr, vec64, c->chunk, s); });
+  // chunks of iterations until the state reports completion
   int launched = 0;
   const int max_launch = maxit / c->chunk + 2;
   // keep one chunk in flight while the host reads the previous state
@@ -535,14 +515,12 @@ void gmres_reset(const GmresBufs& G, cudaStream_t s) {
   AC3D_CUDA(cudaMemsetAsync(G.state, 0, G.nrb * sizeof(GState) + sizeof(GMulti), s));
 }
 
-// One GMRES cycle on op(A) d = b (complex FP64 device vectors): at most gm_restart iterations, in
-// the H-matrix's precision. Returns the iterations; the state's done code in *done.
-int run_gmres(ac3d_ctx* c, const DevHMat& H, const cd* b, cd* d, bool tr, double tol, int* done) {
+// One GMRES cycle on op(A) d = G.b (complex FP64 device vectors): at most gm_restart iterations, in
+// the H-matrix's precision, g enqueueing them. Returns the iterations; the state's done code in *done.
+int run_gmres(ac3d_ctx* c, const GmresBufs& G, ChunkRunner& g, cd* d, double tol, int* done) {
   cudaStream_t s = c->stream;
-  GmresBufs G = gmres_bufs(c, H, b);
   gmres_reset(G, s);
   gmres_enqueue_init(G, tol, s);
-  CapturedGraph g(s, &c->stats.ms_graph, [&] { gmres_enqueue_iterations(G, c->m->DP, H, tr, c->gm_chunk, s); });
   // keep one chunk in flight while the host reads the state after the previous one
   const int max_launch = (G.m + c->gm_chunk - 1) / c->gm_chunk + 1;
   int launched = 0;
@@ -622,10 +600,12 @@ void solve_gmres(ac3d_ctx* c, DevHMat& H, const cd* b, cd* x, bool tr) {
   AC3D_CUDA(cudaMemcpyAsync(&c->h_red[5], c->red.as<double>() + 4, sizeof(double), cudaMemcpyDeviceToHost, s));
   double bn2 = 0.0, rn2 = 0.0;
   int outer = 0, done = 0;
+  const GmresBufs G = gmres_bufs(c, H, c->r64.as<cd>());
+  ChunkRunner g(c, [&] { gmres_enqueue_iterations(G, c->m->DP, H, tr, c->gm_chunk, s); });
   while (outer < c->max_outer) {
     const double need = outer == 0 ? tol : tol * std::sqrt(bn2 / rn2);
     const double tin = fp64 ? 0.5 * need : std::max(c->inner_tol, 0.3 * need);
-    const int it = run_gmres(c, H, c->r64.as<cd>(), (cd*)B.x, tr, tin, &done);  // ends synchronised
+    const int it = run_gmres(c, G, g, (cd*)B.x, tin, &done);  // ends synchronised
     if (outer == 0) bn2 = c->h_red[5];
     c->stats.iterations += it;
     launch_add64(n, x, B.x, s);
@@ -652,7 +632,8 @@ void solve_impl(ac3d_ctx* c, DevHMat& H, const cd* b, cd* x, bool tr) {
   if (H.prec == PREC_FP64) {
     KrylovBufs B = bufs(c, 1);
     launch_copy64(n, b, B.b, s);
-    int it = run_krylov(c, H, B, tr, 1, tol, &done);
+    ChunkRunner g(c, [&] { krylov_enqueue_iterations(B, c->m->DP, H, tr, 1, c->chunk, s); });
+    int it = run_krylov(c, B, g, 1, tol, &done);
     launch_copy64(n, B.x, x, s);
     c->stats.iterations += it;
     c->stats.outer_steps += 1;
@@ -672,19 +653,20 @@ void solve_impl(ac3d_ctx* c, DevHMat& H, const cd* b, cd* x, bool tr) {
   KrylovBufs B = bufs(c, 2);
   launch_zero64(n, x, s);
   // x = 0: the first residual is b itself. |b|^2 is read back without a wait (the first inner
-  // tolerance does not depend on it), so the host captures the inner solve's graph while the
-  // device still runs the assembly.
+  // tolerance does not depend on it), so the host enqueues the inner solve while the device still
+  // runs the assembly.
   launch_copy64(n, b, c->r64.p, s);
   const int nb = launch_norm2_64(n, b, c->partials.as<double>(), s);
   launch_reduce5(c->partials.as<double>(), nb, c->red.as<double>(), s);
   AC3D_CUDA(cudaMemcpyAsync(&c->h_red[5], c->red.as<double>() + 4, sizeof(double), cudaMemcpyDeviceToHost, s));
   double bn2 = 0.0, rn2 = 0.0;
   int outer = 0;
+  ChunkRunner g(c, [&] { krylov_enqueue_iterations(B, c->m->DP, H, tr, 2, c->chunk, s); });
   while (outer < c->max_outer) {
     launch_copy64(n, c->r64.p, B.b, s);
     const double need = outer == 0 ? tol : tol * std::sqrt(bn2 / rn2);
     const double tin = std::max(c->inner_tol, 0.3 * need);
-    int it = run_krylov(c, H, B, tr, 2, tin, &done);  // ends with the stream synchronised
+    int it = run_krylov(c, B, g, 2, tin, &done);  // ends with the stream synchronised
     if (outer == 0) bn2 = c->h_red[5];
     c->stats.iterations += it;
     launch_add64(n, x, B.x, s);
@@ -706,21 +688,30 @@ struct BlockWork {
   DevBuf kv, parts, vparts, red, tick, pbuf, tbuf, tolb, state, r64, xcol, bcol, rcol, zcol;
 };
 
-int run_block_krylov(ac3d_ctx* c, const DevHMat& H, const MultiBufs& B, std::vector<int>& done) {
+// Launches chunks of a block solve until `flag`, read from the first 32 bytes of *state after each
+// chunk, is set. No chunk is kept in flight: the idle 16 or 8 iterations behind the last one would cost
+// more (about 12 us each) than the device's wait for the host between chunks (75 us).
+template <typename Flag>
+void run_block_chunks(ac3d_ctx* c, ChunkRunner& g, const void* state, int max_launch, Flag flag) {
+  cudaStream_t s = c->stream;
+  constexpr size_t kHead = 32;
+  static_assert(kHead <= sizeof(GState), "read into a pinned state");
+  if (!c->h_gstate) AC3D_CUDA(cudaMallocHost(&c->h_gstate, 2 * sizeof(GState)));
+  for (int k = 0; k < max_launch; k++) {
+    g.launch();
+    AC3D_CUDA(cudaMemcpyAsync(c->h_gstate, state, kHead, cudaMemcpyDeviceToHost, s));
+    AC3D_CUDA(cudaStreamSynchronize(s));
+    if (flag((const char*)c->h_gstate)) break;
+  }
+}
+
+int run_block_krylov(ac3d_ctx* c, const MultiBufs& B, ChunkRunner& g, std::vector<int>& done) {
   cudaStream_t s = c->stream;
   const int maxit = c->maxit > 0 ? c->maxit : 2 * B.n;
   mkrylov_enqueue_init(B, maxit, s);
-  {
-    CapturedGraph g(s, &c->stats.ms_graph, [&] { mkrylov_enqueue_iterations(B, c->m->DP, H, c->chunk, s); });
-    int head[4] = {0, 0, 0, 0};  // iter, maxit, done_all, nrb
-    const int max_launch = maxit / c->chunk + 2;
-    for (int launched = 0; launched < max_launch; launched++) {
-      g.launch();
-      AC3D_CUDA(cudaMemcpyAsync(head, B.state, sizeof(head), cudaMemcpyDeviceToHost, s));
-      AC3D_CUDA(cudaStreamSynchronize(s));
-      if (head[2]) break;
-    }
-  }
+  // the state starts with iter, maxit, done_all, nrb
+  run_block_chunks(c, g, B.state, maxit / c->chunk + 2, [](const char* h) { return ((const int*)h)[2] != 0; });
+  AC3D_CUDA(cudaStreamSynchronize(s));
   KStateM st;
   AC3D_CUDA(cudaMemcpy(&st, B.state, sizeof(KStateM), cudaMemcpyDeviceToHost));
   done.assign(B.nrb, 0);
@@ -733,27 +724,13 @@ int run_block_krylov(ac3d_ctx* c, const DevHMat& H, const MultiBufs& B, std::vec
 // tolerances B.tol): every iteration is one block matvec of all the columns' inputs, then each
 // column's Gram-Schmidt passes. Writes the FP32 block solution B.x; per-column done codes in
 // `done`. Returns the iterations of the longest cycle.
-int run_block_gmres(ac3d_ctx* c, const DevHMat& H, const MultiBufs& B, std::vector<int>& done) {
+int run_block_gmres(ac3d_ctx* c, const GmresBufs& G, const MultiBufs& B, ChunkRunner& g, std::vector<int>& done) {
   cudaStream_t s = c->stream;
-  GmresBufs G = gmres_bufs(c, H, B.b, B.nrb);
-  G.b32 = 1;
-  G.tolv = B.tol;
-  G.q = B.p;   // block vectors of the block solver, free during a GMRES batch
-  G.W = B.v;
-  G.W2 = B.s;  // nrb columns of n
   gmres_reset(G, s);
   gmres_enqueue_init(G, 1.0, s);
-  {
-    CapturedGraph g(s, &c->stats.ms_graph, [&] { gmres_enqueue_iterations_block(G, B, c->m->DP, H, c->gm_chunk, s); });
-    const int max_launch = (G.m + c->gm_chunk - 1) / c->gm_chunk + 1;
-    GMulti gm{};
-    for (int launched = 0; launched < max_launch; launched++) {
-      g.launch();
-      AC3D_CUDA(cudaMemcpyAsync(&gm, G.gm, sizeof(GMulti), cudaMemcpyDeviceToHost, s));
-      AC3D_CUDA(cudaStreamSynchronize(s));
-      if (gm.done_all) break;
-    }
-  }
+  static_assert(sizeof(GMulti) == 32, "read as one head");
+  run_block_chunks(c, g, G.gm, (G.m + c->gm_chunk - 1) / c->gm_chunk + 1,
+                   [](const char* h) { return ((const GMulti*)h)->done_all != 0; });
   gmres_enqueue_finish(G, B.x, s);
   std::vector<GState> st(G.nrb);
   GMulti gmf{};
@@ -793,18 +770,7 @@ MultiBufs block_bufs(ac3d_ctx* c, DevHMat& H, int nrb, BlockWork& W, bool tr) {
   if (tr) ensure_near_transposed(c->m->DP, H, s);
   const int n = c->m->Ne, nleaf = c->m->DP.nleaf;
   if (c->block_tc && nrb >= 8 && c->m->DP.max_leaf <= 32 && !(tr ? H.tcseg_f.p : H.tcseg_t.p)) {
-    // byte offsets of the split dot-pass segments: V by column leaf (A), U by row leaf (A^T)
-    const Partition& P = c->m->P;
-    const std::vector<int>& ptr = tr ? P.fw_lr_ptr : P.tr_lr_ptr;
-    const std::vector<int>& items = tr ? P.fw_lr : P.tr_lr;
-    std::vector<long long> off(nleaf + 1, 0);
-    for (int l = 0; l < nleaf; l++) {
-      int K = 0;
-      for (int it = ptr[l]; it < ptr[l + 1]; it++) K += H.ranks_host[items[it]];
-      K += K & 1;
-      off[l + 1] = off[l] + tc_segment_bytes(P.leaf_start[l + 1] - P.leaf_start[l], K);
-    }
-    build_tc_segments(c->m->DP, H, tr, off, s);
+    build_tc_segments(c->m->DP, H, tr, s);
     c->stats.hmat_bytes = (long long)H.bytes();  // the split segments are part of the H-matrix's footprint
   }
   const size_t blk32 = (size_t)n * nrb * sizeof(cf);
@@ -857,6 +823,22 @@ void solve_block(ac3d_ctx* c, DevHMat& H, int nrb, int nr, const cd* b64, cd* x6
   int outer = 0, iters = 0;
   std::vector<int> done;
   std::vector<double> tin(nrb, 1.0);
+  const bool gm = c->krylov == AC3D_KRYLOV_GMRES;
+  GmresBufs G;
+  if (gm) {
+    G = gmres_bufs(c, H, B.b, nrb);
+    G.b32 = 1;
+    G.tolv = B.tol;
+    G.q = B.p;   // block vectors of the block solver, free during a GMRES batch
+    G.W = B.v;
+    G.W2 = B.s;  // nrb columns of n
+  }
+  ChunkRunner g(c, [&] {
+    if (gm)
+      gmres_enqueue_iterations_block(G, B, c->m->DP, H, c->gm_chunk, s);
+    else
+      mkrylov_enqueue_iterations(B, c->m->DP, H, c->chunk, s);
+  });
   while (outer < c->max_outer) {
     bool any = false;
     for (int j = 0; j < nrb; j++) {
@@ -872,7 +854,7 @@ void solve_block(ac3d_ctx* c, DevHMat& H, int nrb, int nr, const cd* b64, cd* x6
     if (!any) break;
     AC3D_CUDA(cudaMemcpyAsync(W.tolb.p, tin.data(), nrb * sizeof(double), cudaMemcpyHostToDevice, s));
     launch_to32(n * nrb, W.r64.p, B.b, s);
-    iters += c->krylov == AC3D_KRYLOV_GMRES ? run_block_gmres(c, H, B, done) : run_block_krylov(c, H, B, done);
+    iters += gm ? run_block_gmres(c, G, B, g, done) : run_block_krylov(c, B, g, done);
     launch_add32(n * nrb, x64, B.x, s);
     for (int j = 0; j < nr; j++) {
       if (!(rn2[j] > tol * tol * bn2[j])) continue;
@@ -1001,19 +983,19 @@ std::unique_ptr<DevHMat> forward_one(ac3d_ctx* c, double f, const double4* recv,
                                      cd* y_out, bool keep, std::unique_ptr<ListenerLR>* q_keep) {
   cudaStream_t s = c->stream;
   const double k = wavenumber(f);
-  GpuTimer ta(s);
+  GpuTimer ta(c);
   auto H = assemble(c, k, c->prec);
-  c->stats.ms_assemble += ta.stop();
+  ta.stop(&c->stats.ms_assemble);
   ensure_work(c);
   // b = -incident field (the system is (K - I/2) x = -b, adjoint.cpp:95)
-  GpuTimer ts(s);
+  GpuTimer ts(c);
   launch_rhs(c->m->G, 1, k, c->src_kind, c->src, c->b64.p, s);
   launch_negate64(c->m->Ne, c->b64.p, s);
   solve(c, *H, c->b64.as<cd>(), x_out, false);
   c->stats.solves++;
-  c->stats.ms_solve += ts.stop();
+  ts.stop(&c->stats.ms_solve);
   if (y_out) {
-    GpuTimer tl(s);
+    GpuTimer tl(c);
     if (c->listener_mode == AC3D_LISTENER_ACA) {
       auto Q = listener_lr(c, k, Lh, L);
       listener_apply(c, *Q, x_out, y_out, false);
@@ -1021,7 +1003,7 @@ std::unique_ptr<DevHMat> forward_one(ac3d_ctx* c, double f, const double4* recv,
     } else {
       launch_far_field(c->m->G, c->prec, recv, L, k, x_out, y_out, c->ff_scratch, s);
     }
-    c->stats.ms_listener += tl.stop();
+    tl.stop(&c->stats.ms_listener);
   }
   if (!keep) H.reset();
   return H;
@@ -1057,7 +1039,7 @@ double band_eval(ac3d_ctx* c, double band, bool forward_only, double* grad_dev) 
   AC3D_CUDA(cudaStreamSynchronize(s));
   if (forward_only) return cval;
 
-  GpuTimer tadj(s);
+  GpuTimer tadj(c);
   vf.alloc((size_t)L * sizeof(cd), s);
   adjb.alloc((size_t)n * sizeof(cd), s);
   lmb.alloc((size_t)n * sizeof(cd), s);
@@ -1100,7 +1082,7 @@ double band_eval(ac3d_ctx* c, double band, bool forward_only, double* grad_dev) 
     launch_adjoint_terms(c->m->G, a, c->adj_scratch, s);
   }
   AC3D_CUDA(cudaStreamSynchronize(s));
-  c->stats.ms_adjoint += tadj.stop();
+  tadj.stop(&c->stats.ms_adjoint);
   return cval;
 }
 
@@ -1152,19 +1134,19 @@ double multi_eval(ac3d_ctx* c, const std::vector<double>& freqs, const std::vect
   };
   for (int fi = 0; fi < F; fi++) {
     const double k = wavenumber(freqs[fi]);
-    GpuTimer ta(s);
+    GpuTimer ta(c);
     auto H = assemble(c, k, c->prec);
-    c->stats.ms_assemble += ta.stop();
+    ta.stop(&c->stats.ms_assemble);
     // forward: b = -incident field (adjoint.cpp:95), one column per direction
-    GpuTimer ts(s);
+    GpuTimer ts(c);
     for (int d = 0; d < D; d++) {
       launch_rhs(c->m->G, 1, k, AC3D_INCIDENT_PLANE, &dirs[3 * d], ADJ.as<cd>() + (size_t)d * n, s);
       launch_negate64(n, ADJ.as<cd>() + (size_t)d * n, s);
     }
     solve_all(ADJ.as<cd>(), X.as<cd>(), *H, false);
-    c->stats.ms_solve += ts.stop();
+    ts.stop(&c->stats.ms_solve);
     // receivers, coefficient and adjoint right-hand side of each direction (adjoint.cpp:101-178)
-    GpuTimer tadj(s);
+    GpuTimer tadj(c);
     std::unique_ptr<ListenerLR> Q;
     if (c->listener_mode == AC3D_LISTENER_ACA) Q = listener_lr(c, k, c->Ls.data(), L);
     for (int d = 0; d < D; d++) {
@@ -1214,7 +1196,7 @@ double multi_eval(ac3d_ctx* c, const std::vector<double>& freqs, const std::vect
       launch_adjoint_terms_multi(c->m->G, a, c->adj_scratch, s);
     }
     AC3D_CUDA(cudaStreamSynchronize(s));
-    c->stats.ms_adjoint += tadj.stop();
+    tadj.stop(&c->stats.ms_adjoint);
   }
   coefs.assign((size_t)F * D, 0.0);
   AC3D_CUDA(cudaMemcpyAsync(coefs.data(), coef.p, (size_t)F * D * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1242,15 +1224,18 @@ int guard(ac3d_ctx* c, F&& f) {
     auto t0 = std::chrono::steady_clock::now();
     const long long l0 = t_kernel_launches;
     f();
+    resolve_timers(c);
     c->stats.ms_total = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     c->stats.kernel_launches = t_kernel_launches - l0;
     return AC3D_OK;
   } catch (const Error& e) {
     c->err = e.what();
     if (e.code == AC3D_ERR_CUDA) cudaGetLastError();
+    finish_timers(c);
     return e.code;
   } catch (const std::exception& e) {
     c->err = e.what();
+    finish_timers(c);
     return AC3D_ERR_INTERNAL;
   }
 }
@@ -1339,6 +1324,19 @@ std::shared_ptr<MeshState> build_mesh_state(const double* Ps, int V, const int32
     upload(DP.didx_t_ptr, mp->P.didx_t_ptr, s);
     upload(DP.didx_t, mp->P.didx_t, s);
     DP.near_total_t = mp->P.near_total_t;
+    {
+      // near columns a leaf streams: as row leaf (with its padding) and as column leaf
+      std::vector<int> wr(DP.nleaf), wc(DP.nleaf, 0);
+      for (int l = 0; l < DP.nleaf; l++) {
+        wr[l] = mp->P.didx_ptr[l + 1] - mp->P.didx_ptr[l];
+        for (int it = mp->P.tr_near_ptr[l]; it < mp->P.tr_near_ptr[l + 1]; it++) {
+          const int* q = &mp->P.direct[4 * mp->P.tr_near[it]];
+          wc[l] += q[1] - q[0];
+        }
+      }
+      upload(DP.near_cols_row, wr, s);
+      upload(DP.near_cols_col, wc, s);
+    }
     upload(DP.didx_ptr, mp->P.didx_ptr, s);
     upload(DP.didx, mp->P.didx, s);
     upload(DP.blk_fw_ptr, mp->P.blk_fw_ptr, s);
@@ -1436,6 +1434,8 @@ void ac3d_destroy(ac3d_ctx* c) {
   if (!c) return;
   cudaStream_t s = c->stream;
   if (s) cudaStreamSynchronize(s);
+  c->destroy_used_graphs();
+  drop_timers(c);
   // every device buffer is released on the context stream, so all of them go before the stream
   c->last_H.reset();
   DevBuf* bufs[] = {&c->kv, &c->kv32, &c->partials, &c->kstate, &c->red, &c->b64, &c->x64, &c->r64, &c->ff_scratch,
@@ -1705,9 +1705,9 @@ int ac3d_solve_multi(ac3d_ctx* c, double f, int kind, const double* vecs, int nr
     ensure_base_geometry(c);
     const double k = wavenumber(f);
     const int n = c->m->Ne;
-    GpuTimer ta(s);
+    GpuTimer ta(c);
     auto H = assemble(c, k, c->prec);
-    c->stats.ms_assemble += ta.stop();
+    ta.stop(&c->stats.ms_assemble);
     ensure_work(c);
     const double4* recv = c->Ls_dev.as<double4>();
     int nL = (int)c->Ls.size() / 3;
@@ -1719,7 +1719,7 @@ int ac3d_solve_multi(ac3d_ctx* c, double f, int kind, const double* vecs, int nr
     DevBuf ycol, b64, x64;
     ycol.alloc((size_t)nL * sizeof(cd), s);
     BlockWork W;
-    GpuTimer ts(s);
+    GpuTimer ts(c);
     for (int start = 0; start < nrhs; start += kMaxRhs) {
       const int nr = std::min(kMaxRhs, nrhs - start);
       const int nrb = nr <= 4 ? 4 : nr <= 8 ? 8 : 16;
@@ -1761,7 +1761,7 @@ int ac3d_solve_multi(ac3d_ctx* c, double f, int kind, const double* vecs, int nr
         AC3D_CUDA(cudaStreamSynchronize(s));
       }
     }
-    c->stats.ms_solve += ts.stop();
+    ts.stop(&c->stats.ms_solve);
     c->last_H = std::move(H);
     if (!c->stats.converged) throw Error(AC3D_ERR_NOT_CONVERGED, not_converged_message(c));
   });
@@ -2144,7 +2144,12 @@ int ac3d_get_ranks(ac3d_ctx* c, int32_t* ranks, int n) {
   if (!c || !ranks || n < 0) return AC3D_ERR_ARG;
   return guard(c, [&] {
     if (!c->last_H) throw Error(AC3D_ERR_STATE, "no H-matrix: call ac3d_pressures or ac3d_surface_values first");
-    const std::vector<int>& r = c->last_H->ranks_host;
+    std::vector<int>& r = c->last_H->ranks_host;
+    if (r.empty() && c->m->DP.na > 0) {  // fetched when asked for
+      r.resize(c->m->DP.na);
+      AC3D_CUDA(cudaMemcpyAsync(r.data(), c->last_H->rank.p, r.size() * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+      AC3D_CUDA(cudaStreamSynchronize(c->stream));
+    }
     if (n != (int)r.size())
       throw Error(AC3D_ERR_ARG, "expected " + std::to_string(r.size()) + " admissible blocks, got " + std::to_string(n));
     std::copy(r.begin(), r.end(), ranks);

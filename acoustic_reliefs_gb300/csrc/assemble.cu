@@ -520,27 +520,35 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? (LPL == 8 ? 2 : 4) : 1)
   }
 }
 
-__global__ void rank_scan_kernel(const int* __restrict__ rank, int na, int* t_off) {
-  __shared__ int sums[1024];
-  const int tid = threadIdx.x;
-  const int chunk = (na + 1023) / 1024;
-  const int s = min(na, tid * chunk), e = min(na, s + chunk);
+__global__ void __launch_bounds__(1024) rank_scan_kernel(const int* __restrict__ rank, int na, int* t_off) {
+  // a contiguous range per warp, its lanes side by side: 322 us with a range per thread on 358k blocks
+  __shared__ int sums[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int chunk = ((na + 31) / 32 + 31) & ~31;
+  const int s = min(na, warp * chunk), e = min(na, s + chunk);
   int acc = 0;
-  for (int i = s; i < e; i++) acc += rank[i];
-  sums[tid] = acc;
+#pragma unroll 4
+  for (int i = s + lane; i < e; i += 32) acc += rank[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) sums[warp] = acc;
   __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    int v = tid >= o ? sums[tid - o] : 0;
-    __syncthreads();
-    sums[tid] += v;
-    __syncthreads();
+  int base = 0;
+  for (int w = 0; w < warp; w++) base += sums[w];
+#pragma unroll 4
+  for (int i0 = s; i0 < e; i0 += 32) {
+    const int i = i0 + lane;
+    const int r = i < e ? rank[i] : 0;
+    int v = r;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += t;
+    }
+    if (i < e) t_off[i] = base + v - r;
+    base += __shfl_sync(0xffffffffu, v, 31);
   }
-  int base = tid ? sums[tid - 1] : 0;
-  for (int i = s; i < e; i++) {
-    t_off[i] = base;
-    base += rank[i];
-  }
-  if (tid == 1023) t_off[na] = sums[1023];
+  if (warp == 31 && lane == 0) t_off[na] = base;
 }
 
 template <typename R>

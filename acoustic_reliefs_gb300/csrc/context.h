@@ -34,10 +34,10 @@ struct ac3d_ctx {
   int maxit = 0;           // 0: twice the number of unknowns
   double inner_tol = 1e-6; // floor of the relative tolerance of each FP32 inner solve
   int max_outer = 10;
-  int chunk = 8;           // BiCGSTAB iterations per captured graph launch
+  int chunk = 8;           // BiCGSTAB iterations per chunk
   int krylov = AC3D_KRYLOV_BICGSTAB;  // inner solver of the single right-hand-side solves
   int gm_restart = 300;    // GMRES basis size: iterations per cycle before a restart
-  int gm_chunk = 16;       // GMRES iterations per captured graph launch
+  int gm_chunk = 16;       // GMRES iterations per chunk
   int maxk = 100;          // APPROX_ACA_MAX_K (constants.h:16)
   bool actual = false;     // use_actual: the coefficient / gradient calls run on the exact operator
 
@@ -79,11 +79,19 @@ struct ac3d_ctx {
   ac3d::KState* h_state = nullptr;  // pinned
   ac3d::GState* h_gstate = nullptr;  // pinned, two slots
   double* h_red = nullptr;    // pinned
+  ac3d::AsmTotals* h_totals = nullptr;  // pinned
+  std::vector<ac3d::PhaseTimer> timers;      // phases of the running call, read when it ends
+  std::vector<cudaGraphExec_t> used_graphs;  // executable graphs of finished solves, to be destroyed
+  void destroy_used_graphs() {
+    for (cudaGraphExec_t g : used_graphs) cudaGraphExecDestroy(g);
+    used_graphs.clear();
+  }
 
   ~ac3d_ctx() {
     if (h_state) cudaFreeHost(h_state);
     if (h_gstate) cudaFreeHost(h_gstate);
     if (h_red) cudaFreeHost(h_red);
+    if (h_totals) cudaFreeHost(h_totals);
   }
 };
 
@@ -98,6 +106,9 @@ double wavenumber(double f);  // k = 2 pi f / c, c = 344 m/s (helpers.h:8, const
 std::shared_ptr<MeshState> build_mesh_state(const double* Ps, int V, const int32_t* Es, int Ne, int cluster_size,
                                             double radius_factor, int maxk, cudaStream_t s);
 void ensure_work(ac3d_ctx* c);
+// Phase times of the call so far into the statistics (waits for the phases to end).
+void resolve_timers(ac3d_ctx* c);
+void finish_timers(ac3d_ctx* c);
 void reset_stats(ac3d_ctx* c);
 void upload_receivers(ac3d_ctx* c, const double* L, int n, DevBuf& dst);
 // One frequency on the context's mesh: assemble, solve, receivers (x_out: Ne, y_out: L complex

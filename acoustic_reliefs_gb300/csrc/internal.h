@@ -140,6 +140,7 @@ struct DevPartition {
   DevBuf fw_near_ptr, fw_near, fw_lr_ptr, fw_lr;
   DevBuf tr_near_ptr, tr_near, tr_lr_ptr, tr_lr;
   DevBuf near_off;                      // int64
+  DevBuf near_cols_row, near_cols_col;  // int: near columns a leaf streams as row and as column leaf
   DevBuf aca_order;                     // int
 };
 
@@ -182,6 +183,26 @@ enum Precision { PREC_MIXED = 0, PREC_FP64 = 1 };
 constexpr int kWarpAcaMaxDim = 256;
 constexpr int kWarpAcaTerms = 128;
 
+// Device time of a phase of a call: two recorded events and the statistic they go to.
+struct PhaseTimer {
+  cudaEvent_t a = nullptr, b = nullptr;
+  double* acc = nullptr;
+};
+
+// What the host reads of an assembly (device memory H.pool_used): the pool's counters (ACA kernels),
+// the block totals (rank_totals_kernel) and the segment sizes (leaf_scan_kernel), index 0 for the U
+// and 1 for the V segments.
+struct AsmTotals {
+  unsigned long long pool_used;
+  int status, pad;                      // bit 0: the pool overflowed
+  unsigned long long lr_entries;        // sum of rank (m + n)
+  unsigned long long aca_evaluated;     // sum of passes (m + n)
+  unsigned long long sum_rank, max_rank;
+  unsigned long long columns[2];        // segment columns (even per leaf)
+  unsigned long long entries[2];        // segment entries
+  unsigned long long tc_bytes[2];       // bytes of the split segments of the tensor-core dot pass
+};
+
 // An assembled H-matrix of (K - I/2) at one wavenumber.
 struct DevHMat {
   int prec = PREC_MIXED;  // storage: complex FP32 (mixed) or complex FP64
@@ -213,10 +234,11 @@ struct DevHMat {
   DevBuf tvec;            // intermediate V x per term (complex, vector precision)
   DevBuf tvec64;          // FP64 / double-float intermediate for refinement residuals
   DevBuf xdf;             // double-float copy of the residual matvec input (FP32 storage only)
-  DevBuf pool_used;       // unsigned long long
+  DevBuf pool_used;       // AsmTotals
   int64_t pool_cap = 0;
   int64_t pool_used_host = 0;
-  std::vector<int> ranks_host;
+  std::vector<int> ranks_host;  // fetched by ac3d_get_ranks
+  int64_t tc_bytes[2] = {0, 0};  // split segments of the U and the V side
   int64_t lr_entries = 0; // sum r (m + n)
   int64_t aca_evaluated = 0;  // entries ACA evaluated: sum passes (m + n)
   size_t bytes() const {
@@ -244,6 +266,9 @@ void launch_near_assembly_df(const DevGeometry& G, const DevPartition& DP, DevHM
 void launch_aca_df(const DevGeometry& G, const DevPartition& DP, DevHMat& H, double eps, int max_rows, cudaStream_t s,
                    cudaStream_t s_small);
 void launch_rank_scan(const DevPartition& DP, DevHMat& H, cudaStream_t s);
+// After launch_rank_scan: segment layout of both sides (kseg, seg), the leaves by decreasing streamed
+// bytes (order_rows, order_cols) and the totals of the assembly. leaf_work: 2 nleaf ints of scratch.
+void launch_leaf_layout(const DevPartition& DP, DevHMat& H, int* leaf_work, cudaStream_t s);
 // Packs the pool into the U segments (row leaves, cols = false) or V segments (column leaves).
 void launch_pack(const DevPartition& DP, DevHMat& H, bool cols, cudaStream_t s);
 

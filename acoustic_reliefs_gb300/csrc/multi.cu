@@ -190,9 +190,31 @@ constexpr size_t tc_dot_smem() {
   return tc_b_bytes<NRB>() + (size_t)kTcStages * kTcStageBytes;
 }
 
-// Bytes of a leaf's split segment: hi and lo parts of ceil8(K) rows of Kd floats.
-__host__ __device__ constexpr long long tc_leaf_bytes(int R, int K) {
-  return 8ll * ((2 * R + 7) & ~7) * ((K + 7) & ~7);
+// tc_off[l] = the prefix of the leaves' split segment bytes (one CTA)
+__global__ void __launch_bounds__(1024) tc_offset_kernel(const int* __restrict__ kseg,
+                                                         const int* __restrict__ leaf_start, int nleaf,
+                                                         long long* __restrict__ tc_off) {
+  __shared__ long long sb[1024];
+  const int tid = threadIdx.x;
+  const int chunk = (nleaf + 1023) / 1024;
+  const int s = min(nleaf, tid * chunk), e = min(nleaf, s + chunk);
+  auto bytes = [&](int l) { return tc_segment_bytes(leaf_start[l + 1] - leaf_start[l], kseg[l + 1] - kseg[l]); };
+  long long a = 0;
+  for (int l = s; l < e; l++) a += bytes(l);
+  sb[tid] = a;
+  __syncthreads();
+  for (int o = 1; o < 1024; o <<= 1) {
+    const long long v = tid >= o ? sb[tid - o] : 0;
+    __syncthreads();
+    sb[tid] += v;
+    __syncthreads();
+  }
+  a = tid ? sb[tid - 1] : 0;
+  for (int l = s; l < e; l++) {
+    tc_off[l] = a;
+    a += bytes(l);
+  }
+  if (tid == 1023) tc_off[nleaf] = sb[1023];
 }
 
 // One CTA per leaf: the leaf's segment (R x K column-major complex) into split TF32 tiles.
@@ -1149,17 +1171,17 @@ void ensure_near_transposed(const DevPartition& DP, DevHMat& H, cudaStream_t s) 
   AC3D_CUDA(cudaGetLastError());
 }
 
-void build_tc_segments(const DevPartition& DP, DevHMat& H, bool tr, const std::vector<long long>& off,
-                       cudaStream_t s) {
+void build_tc_segments(const DevPartition& DP, DevHMat& H, bool tr, cudaStream_t s) {
   DevBuf& tcs = tr ? H.tcseg_f : H.tcseg_t;
   DevBuf& tco = tr ? H.tcoff_f : H.tcoff_t;
   if (tcs.p) return;
   if (H.prec == PREC_FP64) throw Error(3, "internal: block matvec needs FP32 storage");
-  if ((int)off.size() != DP.nleaf + 1) throw Error(3, "internal: split segment offsets");
-  tco.alloc(off.size() * sizeof(long long), s);
-  // pageable source: the copy is staged before the call returns, so off may go away after it
-  AC3D_CUDA(cudaMemcpyAsync(tco.p, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice, s));
-  tcs.alloc((size_t)std::max<long long>(off.back(), 16), s);
+  tco.alloc((size_t)(DP.nleaf + 1) * sizeof(long long), s);
+  tcs.alloc((size_t)std::max<long long>(H.tc_bytes[tr ? 0 : 1], 16), s);
+  note_launch();
+  tc_offset_kernel<<<1, 1024, 0, s>>>((tr ? H.kseg_f : H.kseg_t).as<int>(), DP.leaf_start.as<int>(), DP.nleaf,
+                                      tco.as<long long>());
+  AC3D_CUDA(cudaGetLastError());
   if (DP.nleaf == 0) return;
   note_launch();
   tc_split_kernel<<<DP.nleaf, 256, 0, s>>>(tr ? H.useg.as<cf>() : H.vseg.as<cf>(),
@@ -1169,7 +1191,6 @@ void build_tc_segments(const DevPartition& DP, DevHMat& H, bool tr, const std::v
   AC3D_CUDA(cudaGetLastError());
 }
 
-long long tc_segment_bytes(int R, int K) { return tc_leaf_bytes(R, K); }
 
 
 void launch_mmatvec(const DevPartition& DP, const DevHMat& H, const MultiBufs& B, const void* x, void* y,

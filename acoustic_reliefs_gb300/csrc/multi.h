@@ -53,10 +53,11 @@ void launch_mmatvec(const DevPartition& DP, const DevHMat& H, const MultiBufs& B
 void ensure_near_transposed(const DevPartition& DP, DevHMat& H, cudaStream_t s);
 // Builds the TF32 hi / lo split of the dot-pass segments (V by column leaf for A, U by row leaf
 // for A^T with tr) that the tensor-core dot pass streams (once per H-matrix and orientation).
-// off: nleaf + 1 byte offsets, off[l + 1] - off[l] = tc_segment_bytes(R_l, K_l).
-void build_tc_segments(const DevPartition& DP, DevHMat& H, bool tr, const std::vector<long long>& off,
-                       cudaStream_t s);
-long long tc_segment_bytes(int R, int K);
+void build_tc_segments(const DevPartition& DP, DevHMat& H, bool tr, cudaStream_t s);
+// Bytes of a leaf's split segment: hi and lo parts of ceil8(K) rows of 2 R floats rounded up to 8.
+__host__ __device__ constexpr long long tc_segment_bytes(int R, int K) {
+  return 8ll * ((2 * R + 7) & ~7) * ((K + 7) & ~7);
+}
 void mkrylov_enqueue_init(const MultiBufs& B, int maxit, cudaStream_t s);
 void mkrylov_enqueue_iterations(const MultiBufs& B, const DevPartition& DP, const DevHMat& H, int count,
                                 cudaStream_t s);

@@ -10,45 +10,56 @@
 // kpos[e] is the segment column of the block's first term, which the reduce step of the matvec
 // uses to sum a term's per-leaf partial dots. Offsets are prefix sums over the ranks computed on
 // the device in a fixed order, so packing is deterministic. The pool itself is not needed after.
+#include <algorithm>
+
 #include "common.cuh"
 #include "df2.cuh"
 #include "internal.h"
+#include "multi.h"
 
 namespace ac3d {
 
-// Per leaf: K = sum of the ranks of its list, padded to even, into kseg[l] (a warp per leaf, the
+// Per leaf: raw[l] = sum of the ranks of its list, kseg[l] that padded to even (a warp per leaf, the
 // ranks summed by lanes; integer sums, so the order does not matter).
 __global__ void leaf_k_kernel(const int* __restrict__ rank, const int* __restrict__ ptr,
-                              const int* __restrict__ items, int nleaf, int* kseg) {
+                              const int* __restrict__ items, int nleaf, int* kseg, int* raw) {
   const int l = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (l >= nleaf) return;
   int K = 0;
   for (int it = ptr[l] + lane; it < ptr[l + 1]; it += 32) K += rank[items[it]];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) K += __shfl_xor_sync(0xffffffffu, K, o);
-  if (lane == 0) kseg[l] = K + (K & 1);
+  if (lane == 0) {
+    kseg[l] = K + (K & 1);
+    raw[l] = K;
+  }
 }
 
-// kseg[l] (holding K of leaf l) becomes the prefix of K, seg[l] the prefix of R K (one CTA).
-__global__ void leaf_scan_kernel(const int* __restrict__ leaf_start, int nleaf, int* kseg, long long* seg) {
-  __shared__ long long sk[1024], ss[1024];
+// kseg[l] (holding K of leaf l) becomes the prefix of K, seg[l] the prefix of R K (one CTA); the sums,
+// and the bytes of the split segments, to the totals of `side`.
+__global__ void leaf_scan_kernel(const int* __restrict__ leaf_start, int nleaf, int* kseg, long long* seg,
+                                 AsmTotals* tot, int side) {
+  __shared__ long long sk[1024], ss[1024], st[1024];
   const int tid = threadIdx.x;
   const int chunk = (nleaf + 1023) / 1024;
   const int s = min(nleaf, tid * chunk), e = min(nleaf, s + chunk);
-  long long ak = 0, as = 0;
+  long long ak = 0, as = 0, at = 0;
   for (int l = s; l < e; l++) {
-    const int K = kseg[l];
+    const int K = kseg[l], R = leaf_start[l + 1] - leaf_start[l];
     ak += K;
-    as += (long long)K * (leaf_start[l + 1] - leaf_start[l]);
+    as += (long long)K * R;
+    at += tc_segment_bytes(R, K);
   }
   sk[tid] = ak;
   ss[tid] = as;
+  st[tid] = at;
   __syncthreads();
   for (int o = 1; o < 1024; o <<= 1) {
-    long long vk = tid >= o ? sk[tid - o] : 0, vs = tid >= o ? ss[tid - o] : 0;
+    long long vk = tid >= o ? sk[tid - o] : 0, vs = tid >= o ? ss[tid - o] : 0, vt = tid >= o ? st[tid - o] : 0;
     __syncthreads();
     sk[tid] += vk;
     ss[tid] += vs;
+    st[tid] += vt;
     __syncthreads();
   }
   long long bk = tid ? sk[tid - 1] : 0, bs = tid ? ss[tid - 1] : 0;
@@ -62,7 +73,91 @@ __global__ void leaf_scan_kernel(const int* __restrict__ leaf_start, int nleaf, 
   if (tid == 1023) {
     kseg[nleaf] = (int)sk[1023];
     seg[nleaf] = ss[1023];
+    tot->columns[side] = (unsigned long long)sk[1023];
+    tot->entries[side] = (unsigned long long)ss[1023];
+    tot->tc_bytes[side] = (unsigned long long)st[1023];
   }
+}
+
+// Leaves by decreasing streamed entries: as row leaves (near + U columns: the forward gather and the
+// transposed dot; blockIdx.y 0) and as column leaves (V columns + transposed near: the forward dot
+// and the transposed gather; 1). The hardware dispatches CTAs in index order, so this is
+// longest-first list scheduling. A leaf's place is the number of leaves before it, ties in leaf order.
+__global__ void __launch_bounds__(256) leaf_order_kernel(const int* __restrict__ leaf_start, int nleaf,
+                                                         const int* __restrict__ raw,
+                                                         const int* __restrict__ near_row,
+                                                         const int* __restrict__ near_col, int* order_rows,
+                                                         int* order_cols) {
+  __shared__ long long sw[256];
+  const bool col = blockIdx.y != 0;
+  const int* lr = raw + (col ? nleaf : 0);
+  const int* near = col ? near_col : near_row;
+  auto work = [&](int l) { return (long long)(lr[l] + near[l]) * (leaf_start[l + 1] - leaf_start[l]); };
+  const int l = blockIdx.x * 256 + threadIdx.x;
+  const long long w = l < nleaf ? work(l) : 0;
+  int place = 0;
+  for (int base = 0; base < nleaf; base += 256) {
+    __syncthreads();
+    if (base + (int)threadIdx.x < nleaf) sw[threadIdx.x] = work(base + threadIdx.x);
+    __syncthreads();
+    const int cnt = min(256, nleaf - base);
+    for (int k = 0; k < cnt; k++) place += sw[k] > w || (sw[k] == w && base + k < l);
+  }
+  if (l < nleaf) (col ? order_cols : order_rows)[place] = l;
+}
+
+// Sums over the admissible blocks: rank (m + n), passes (m + n), rank, and the largest rank.
+__global__ void __launch_bounds__(256) rank_totals_kernel(const int* __restrict__ rank, const int* __restrict__ passes,
+                                                          const int4* __restrict__ blocks, int na, AsmTotals* tot) {
+  unsigned long long lr = 0, ev = 0, sr = 0;
+  int mx = 0;
+  for (int b = blockIdx.x * 256 + threadIdx.x; b < na; b += gridDim.x * 256) {
+    const int4 q = blocks[b];
+    const int mn = (q.y - q.x) + (q.w - q.z), r = rank[b];
+    lr += (unsigned long long)r * mn;
+    ev += (unsigned long long)passes[b] * mn;
+    sr += r;
+    mx = max(mx, r);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lr += __shfl_xor_sync(0xffffffffu, lr, o);
+    ev += __shfl_xor_sync(0xffffffffu, ev, o);
+    sr += __shfl_xor_sync(0xffffffffu, sr, o);
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&tot->lr_entries, lr);
+    atomicAdd(&tot->aca_evaluated, ev);
+    atomicAdd(&tot->sum_rank, sr);
+    atomicMax(&tot->max_rank, (unsigned long long)mx);
+  }
+}
+
+void launch_leaf_layout(const DevPartition& DP, DevHMat& H, int* leaf_work, cudaStream_t s) {
+  AsmTotals* tot = H.pool_used.as<AsmTotals>();
+  note_launch();
+  rank_totals_kernel<<<std::min((DP.na + 255) / 256, 2 * device_sm_count()), 256, 0, s>>>(
+      H.rank.as<int>(), H.passes.as<int>(), DP.blocks_a.as<int4>(), DP.na, tot);
+  AC3D_CUDA(cudaGetLastError());
+  for (int side = 0; side < 2; side++) {
+    DevBuf& kseg = side ? H.kseg_t : H.kseg_f;
+    DevBuf& seg = side ? H.seg_t : H.seg_f;
+    note_launch();
+    leaf_k_kernel<<<(DP.nleaf + 7) / 8, 256, 0, s>>>(
+        H.rank.as<int>(), side ? DP.tr_lr_ptr.as<int>() : DP.fw_lr_ptr.as<int>(),
+        side ? DP.tr_lr.as<int>() : DP.fw_lr.as<int>(), DP.nleaf, kseg.as<int>(), leaf_work + side * DP.nleaf);
+    AC3D_CUDA(cudaGetLastError());
+    note_launch();
+    leaf_scan_kernel<<<1, 1024, 0, s>>>(DP.leaf_start.as<int>(), DP.nleaf, kseg.as<int>(), seg.as<long long>(), tot,
+                                        side);
+    AC3D_CUDA(cudaGetLastError());
+  }
+  note_launch();
+  leaf_order_kernel<<<dim3((DP.nleaf + 255) / 256, 2), 256, 0, s>>>(
+      DP.leaf_start.as<int>(), DP.nleaf, leaf_work, DP.near_cols_row.as<int>(), DP.near_cols_col.as<int>(),
+      H.order_rows.as<int>(), H.order_cols.as<int>());
+  AC3D_CUDA(cudaGetLastError());
 }
 
 // Stored value of a pool entry: the entry itself, or the FP32 rounding (the leading part) of a
@@ -160,12 +255,6 @@ static void pack_side(const DevPartition& DP, DevHMat& H, bool cols, cudaStream_
   DevBuf& S = cols ? H.vseg : H.useg;
   DevBuf& idx = cols ? H.vidx : H.uidx;
   DevBuf& kpos = cols ? H.kpos_t : H.kpos_f;
-  note_launch();
-  leaf_k_kernel<<<(DP.nleaf + 7) / 8, 256, 0, s>>>(H.rank.as<int>(), ptr, items, DP.nleaf, kseg.as<int>());
-  AC3D_CUDA(cudaGetLastError());
-  note_launch();
-  leaf_scan_kernel<<<1, 1024, 0, s>>>(DP.leaf_start.as<int>(), DP.nleaf, kseg.as<int>(), seg.as<long long>());
-  AC3D_CUDA(cudaGetLastError());
   note_launch();
   pack_segments_kernel<P, R><<<DP.nleaf, kPackThreads, 0, s>>>(H.pool.as<P>(), H.task_off.as<long long>(),
                                                    H.t_off.as<int>(), H.rank.as<int>(), DP.blocks_a.as<int4>(),

@@ -146,6 +146,7 @@ void run_request(ac3d_server* S, ac3d_ctx* c, Request* r, MeshEntry& me) {
   AC3D_CUDA(cudaMemcpyAsync(r->out.data(), y.p, (size_t)L * sizeof(cd), cudaMemcpyDeviceToHost, s));
   AC3D_CUDA(cudaStreamSynchronize(s));
   y.release();
+  resolve_timers(c);
   const ac3d_stats& st = c->stats;
   r->info.hmat_bytes = st.hmat_bytes;
   r->info.lr_entries = st.lr_entries;
@@ -194,9 +195,11 @@ void worker(ac3d_server* S, int slot) {
       rc = e.code;
       msg = e.what();
       if (e.code == AC3D_ERR_CUDA) cudaGetLastError();
+      finish_timers(c);
     } catch (const std::exception& e) {
       rc = AC3D_ERR_INTERNAL;
       msg = e.what();
+      finish_timers(c);
     }
     c->m.reset();
     c->mesh_set = false;
