@@ -11,7 +11,8 @@
 // non-conjugated products); stop when sqrt(|u|^2 |v|^2 / err) <= eps, dropping the converging
 // term; next row pivot = first max of |u|^2 over rows not used yet. Each rank-1 term (u | v) is
 // bump-allocated from one pool with an atomic counter, so storage is proportional to the actual
-// ranks; the pool offset of term q of block b is term_off[b * maxk + q].
+// ranks; the pool offset of term q of block b is term_off[b * maxk + q]. The kernels here are those of
+// the FP32 assembly; FP64 and double-float ACA have their own (aca_f64.cu, aca_df.cu).
 #include "common.cuh"
 #include "internal.h"
 #include "listener.h"
@@ -295,8 +296,8 @@ __global__ void __launch_bounds__(kAcaThreads) aca_kernel(AcaArgs<R, P4> A) {
 // aca_kernel (pivot rules, stop rule, dropped converging term, zero terms not stored, exactly-zero
 // blocks skipped) with warp shuffles in place of block barriers. Lane l owns rows and columns
 // l + 32 k (k < LPL) and keeps the current term's u and v there in registers; the earlier terms
-// are read from the pool four at a time. Norms and cross terms are summed in the storage type R
-// (the FP64 path is unchanged); the error estimate is accumulated in FP64.
+// are read from the pool four at a time. Norms and cross terms are summed in the storage type R;
+// the error estimate is accumulated in FP64.
 // ------------------------------------------------------------------------------------------
 template <typename R>
 __device__ __forceinline__ void warp_argmax(R& val, int& idx) {
@@ -345,7 +346,7 @@ __device__ __forceinline__ void sub_terms(cplx<R>& acc, const cplx<R>* coef, con
 // Blocks of 129-256 rows (8 rows per lane) are few (less than one wave at 4 CTAs per SM), so
 // that variant takes the registers of 2 CTAs per SM and keeps its u / v rows unspilled.
 template <typename R, typename P4, int LPL>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? (LPL == 8 ? 2 : 4) : 1)
+__global__ void __launch_bounds__(256, LPL == 8 ? 2 : 4)
     aca_warp_kernel(AcaArgs<R, P4> A, int nblocks) {
   __shared__ __align__(16) unsigned char s_raw[8 * kWarpAcaTerms * (2 * sizeof(cplx<R>) + sizeof(long long))];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -616,17 +617,11 @@ static void aca_launch_t(const AcaArgs<R, P4>& a, int nblocks, int max_rows, cud
 void launch_aca(const DevGeometry& G, const DevPartition& DP, DevHMat& H, double eps, int max_rows, cudaStream_t s,
                 cudaStream_t s_small) {
   if (DP.na == 0) return;
-  int iter_cap = H.maxk;
   if (H.prec == PREC_FP64) {
-    AcaArgs<double, double4> a{geo_view<double>(G), DP.blocks_a.as<int4>(), DP.aca_order.as<int>(),
-                               G.cen.as<double4>(), H.k, eps, H.maxk, 1, iter_cap, H.pool.as<cd>(),
-                               H.pool_cap, H.pool_used.as<unsigned long long>(), H.term_off.as<long long>(),
-                               H.rank.as<int>(), (int*)(H.pool_used.as<unsigned long long>() + 1),
-                               H.passes.as<int>()};
-    aca_launch_all(a, DP, max_rows, s, s_small);
+    launch_aca_f64(G, DP, H, eps, max_rows, s, s_small);
   } else {
     AcaArgs<float, float4> a{geo_view<float>(G), DP.blocks_a.as<int4>(), DP.aca_order.as<int>(),
-                             G.cen32.as<float4>(), (float)H.k, eps, H.maxk, 1, iter_cap, H.pool.as<cf>(),
+                             G.cen32.as<float4>(), (float)H.k, eps, H.maxk, 1, H.maxk, H.pool.as<cf>(),
                              H.pool_cap, H.pool_used.as<unsigned long long>(), H.term_off.as<long long>(),
                              H.rank.as<int>(), (int*)(H.pool_used.as<unsigned long long>() + 1),
                              H.passes.as<int>()};
@@ -667,9 +662,8 @@ void launch_listener_aca(const DevGeometry& G, int prec, const void* pts, int L,
   int iter_lim = std::min(maxk, std::min(L - 1, G.ne - 1));
   if (iter_lim < 1) iter_lim = 1;
   if (prec == PREC_FP64) {
-    AcaArgs<double, double4> a{geo_view<double>(G), block, order, (const double4*)pts, k, eps, maxk, 0, iter_lim,
-                               (cd*)pool, pool_cap, used, term_off, rank, status, nullptr};
-    aca_launch_t(a, 1, L, s);
+    launch_listener_aca_f64(G, (const double4*)pts, L, k, eps, maxk, (cd*)pool, pool_cap, used, term_off, rank, status,
+                            block, order, s);
   } else {
     AcaArgs<float, float4> a{geo_view<float>(G), block, order, (const float4*)pts, (float)k, eps, maxk, 0,
                              iter_lim, (cf*)pool, pool_cap, used, term_off, rank, status, nullptr};

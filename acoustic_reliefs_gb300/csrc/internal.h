@@ -259,6 +259,9 @@ void launch_near_assembly(const DevGeometry& G, const DevPartition& DP, DevHMat&
 // Large blocks run on s, small blocks (one warp each) on s_small, which may be another stream.
 void launch_aca(const DevGeometry& G, const DevPartition& DP, DevHMat& H, double eps, int max_rows, cudaStream_t s,
                 cudaStream_t s_small);
+// The FP64 ones of launch_aca (aca_f64.cu); blocks with a side above 64 run on s.
+void launch_aca_f64(const DevGeometry& G, const DevPartition& DP, DevHMat& H, double eps, int max_rows, cudaStream_t s,
+                    cudaStream_t s_small);
 // Mixed-precision assembly with double-float entries and ACA recursion (FP64-accurate entries,
 // pivots and ranks; FP32 storage): near field into H.near (cf), ACA terms into H.pool (complex
 // double-floats, 16 bytes).

@@ -16,6 +16,9 @@ void launch_vf(const double* u, const cd* y, int L, cd* vf, cudaStream_t s);
 void launch_listener_aca(const DevGeometry& G, int prec, const void* pts, int L, double k, double eps, int maxk,
                          void* pool, long long pool_cap, unsigned long long* used, long long* term_off, int* rank,
                          int* status, const int4* block, const int* order, cudaStream_t s);
+void launch_listener_aca_f64(const DevGeometry& G, const double4* pts, int L, double k, double eps, int maxk, cd* pool,
+                             long long pool_cap, unsigned long long* used, long long* term_off, int* rank, int* status,
+                             const int4* block, const int* order, cudaStream_t s);
 // The receiver ACA in double-float arithmetic (the mixed path's default assembly): pts_df holds L
 // double-float points (8 floats each: x, y, z as hi/lo pairs, two pad); the terms end up in the
 // pool as complex FP64, listener_term_stride(L, ne) entries apart. A cooperative kernel; status gets bit
