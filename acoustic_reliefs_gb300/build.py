@@ -18,7 +18,7 @@ OUT_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(OUT_DIR, "libac3d.so")
 OBJ_DIR = os.path.join(HERE, "_build")
 
-SOURCES = ["api.cpp", "tree.cpp", "geometry.cu", "assemble.cu", "aca_df.cu", "aca_f64.cu", "matvec.cu", "pack.cu", "krylov.cu", "gmres.cu", "listener.cu",
+SOURCES = ["api.cpp", "tree.cpp", "geometry.cu", "assemble.cu", "aca_df.cu", "aca_f64.cu", "matvec.cu", "matvec64.cu", "pack.cu", "krylov.cu", "gmres.cu", "listener.cu",
            "adjoint.cu", "noalloc.cu", "serve.cpp", "multi.cu", "tcselftest.cu", "dfselftest.cu", "obj.cpp", "texmap.cu", "relief.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

@@ -286,6 +286,11 @@ struct MatvecEpilogue {
 };
 void launch_matvec(const DevPartition& DP, const DevHMat& H, int ne, bool transposed, int vec64,
                    const void* x, void* y, const void* b_minus, const MatvecEpilogue& ep, cudaStream_t s);
+// The passes on an FP64 H-matrix (matvec64.cu) and the reduce pass of it (matvec.cu)
+void launch_matvec_f64(const DevPartition& DP, const DevHMat& H, bool tr, const void* x, void* y, const void* bminus,
+                       const MatvecEpilogue& ep, const int* done, cudaStream_t s, bool pdl);
+void launch_reduce_f64(const DevPartition& DP, const DevHMat& H, bool tr, const void* p, void* t, const int* done,
+                       cudaStream_t s, bool pdl);
 int matvec_grid(const DevPartition& DP, bool transposed);
 int device_sm_count();
 // Looks up the allocation-free far field's fixed scratch on the current device (noalloc.cu), so

@@ -39,4 +39,25 @@ void launch_k(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sm
   AC3D_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
 }
 
+// Clusters of n CTAs (1 to 8), gridDim.x a multiple of n.
+template <typename... KArgs, typename... Args>
+void launch_clusters(bool pdl, unsigned n, void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
+                     Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = n;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
+  note_launch();
+  AC3D_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
+}
+
 }  // namespace ac3d

@@ -63,7 +63,7 @@ __device__ __forceinline__ void df_mac(df32& acc, float a, df32 z) {
   acc = df32(s.hi, __fadd_rn(acc.lo, __fadd_rn(s.lo, pe)));
 }
 
-// Accumulator arithmetic of the matvec passes: plain FP32 / FP64, or double-float.
+// Accumulator arithmetic of the matvec passes: plain FP32, or double-float.
 template <typename AT, typename MT>
 __device__ __forceinline__ void acc_mac(AT& ar, AT& ai, const cplx<MT>& a, const AT& zr, const AT& zi) {
   ar = fma((AT)a.re, zr, ar);
@@ -649,8 +649,20 @@ void prepare_matvec_kernels() {
     set_smem_attrs<float, float, float>();
     set_smem_attrs<float, double, df32>();
     set_smem_attrs<float, double, float>();
-    set_smem_attrs<double, double, double>();
   });
+}
+
+template <typename AT>
+static void launch_reduce(const DevPartition& DP, const DevHMat& H, bool tr, const cplx<AT>* p, cplx<AT>* t,
+                          const int* done, cudaStream_t s, bool pdl) {
+  launch_k(pdl, seg_reduce_kernel<AT>, dim3((int)((H.task_cap + 255) / 256)), dim3(256), 0, s, H.task_b.as<int>(),
+           H.t_off.as<int>(), (int)H.task_cap, H.t_off.as<int>() + DP.na,
+           tr ? DP.blk_fw_ptr.as<int>() : DP.blk_tr_ptr.as<int>(), tr ? H.kpos_f.as<int>() : H.kpos_t.as<int>(), p, t,
+           done);
+}
+void launch_reduce_f64(const DevPartition& DP, const DevHMat& H, bool tr, const void* p, void* t, const int* done,
+                       cudaStream_t s, bool pdl) {
+  launch_reduce<double>(DP, H, tr, (const cd*)p, (cd*)t, done, s, pdl);
 }
 
 template <typename MT, typename VT, typename AT, int RPL>
@@ -687,10 +699,7 @@ static void mv_t(const DevPartition& DP, const DevHMat& H, bool tr, const void* 
     d.order = tr ? H.order_rows.as<int>() : H.order_cols.as<int>();
     launch_k(pdl, seg_dot_kernel<MT, AT, RPL>, dim3(DP.nleaf), dim3(kThreads), kRingBytes, s, d,
              tr ? useg : vseg, xm, p, done);
-    launch_k(pdl, seg_reduce_kernel<AT>, dim3((int)((H.task_cap + 255) / 256)), dim3(256), 0, s,
-             H.task_b.as<int>(), H.t_off.as<int>(), (int)H.task_cap, H.t_off.as<int>() + DP.na,
-             tr ? DP.blk_fw_ptr.as<int>() : DP.blk_tr_ptr.as<int>(), tr ? H.kpos_f.as<int>() : H.kpos_t.as<int>(),
-             p, t, done);
+    launch_reduce<AT>(DP, H, tr, p, t, done, s, pdl);
   }
   v.b_seg = tr ? H.seg_t.as<long long>() : H.seg_f.as<long long>();
   v.b_kptr = tr ? H.kseg_t.as<int>() : H.kseg_f.as<int>();
@@ -731,7 +740,7 @@ static void mv_rpl(const DevPartition& DP, const DevHMat& H, bool tr, const void
     mv_t<MT, VT, AT, 8>(DP, H, tr, x, y, bminus, ep, done, tvec, s, x32, pdl);
 }
 
-// vec64: 0 FP32 vectors; 1 FP64 vectors (FP64 storage: FP64 arithmetic; FP32 storage: the
+// vec64: 0 FP32 vectors; 1 FP64 vectors (FP64 storage: FP64 arithmetic, matvec64.cu; FP32 storage: the
 // double-float residual); 2 FP64 vectors on FP32 storage with FP32 arithmetic, the multipliers
 // taken from the FP32 shadow x32 of x. pdl: launch the passes as programmatic dependents (the
 // kernel before the first pass then must follow the same protocol, see launch.cuh).
@@ -740,7 +749,7 @@ void launch_matvec_ex(const DevPartition& DP, const DevHMat& H, bool transposed,
                       const void* x32, bool pdl) {
   if (H.prec == PREC_FP64) {
     if (!vec64) throw Error(3, "internal: FP64 H-matrix needs FP64 vectors");
-    mv_rpl<double, double, double>(DP, H, transposed, x, y, b_minus, ep, done, H.tvec64.p, s, nullptr, pdl);
+    launch_matvec_f64(DP, H, transposed, x, y, b_minus, ep, done, s, pdl);
   } else if (vec64 == 2) {
     if (!x32) throw Error(3, "internal: FP32 shadow of the matvec input missing");
     mv_rpl<float, double, float>(DP, H, transposed, x, y, b_minus, ep, done, H.tvec.p, s, x32, pdl);
