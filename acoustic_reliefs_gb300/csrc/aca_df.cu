@@ -57,6 +57,7 @@ struct AcaDfArgs {
   int* rank;
   int* status;
   int* passes;     // per block: rows (and columns) evaluated, or null
+  unsigned* next;  // of each class of small blocks: the first one not taken
   int zero_guard;  // boundary blocks: v kept when v_j == 0 and exactly-zero blocks skipped
 };
 
@@ -78,19 +79,25 @@ __device__ __forceinline__ void load_table(const float4* __restrict__ g) {
 template <typename All>
 __device__ __forceinline__ bool zero_block(const AcaDfArgs& A, int rs, int m, int cs, int n, int t0, int step,
                                            All all) {
+  // the three planes together, the points first: almost every block fails there, after one round of loads
+  const double4 a0 = A.va[cs];
+  bool x = true, y = true, z = true;
+  for (int j = t0; j < n; j += step) {
+    const double4 a = A.va[cs + j];
+    x = x && a.x == a0.x;
+    y = y && a.y == a0.y;
+    z = z && a.z == a0.z;
+  }
+  for (int i = t0; i < m; i += step) {
+    const double4 p = A.cen[rs + i];
+    x = x && p.x == a0.x;
+    y = y && p.y == a0.y;
+    z = z && p.z == a0.z;
+  }
   for (int d = 0; d < 3; d++) {
-    const double4 a0 = A.va[cs];
-    const double v = d == 0 ? a0.x : (d == 1 ? a0.y : a0.z);
-    bool ok = true;
-    for (int j = t0; j < n && ok; j += step) {
-      const double4 a = A.va[cs + j];
-      const ElemGeo<double> g = A.eg[cs + j];
-      ok = (d == 0 ? a.x : (d == 1 ? a.y : a.z)) == v && g.ab[d] == 0.0 && g.ac[d] == 0.0;
-    }
-    for (int i = t0; i < m && ok; i += step) {
-      const double4 p = A.cen[rs + i];
-      ok = (d == 0 ? p.x : (d == 1 ? p.y : p.z)) == v;
-    }
+    bool ok = d == 0 ? x : (d == 1 ? y : z);
+    if (!all(ok)) continue;
+    for (int j = t0; j < n && ok; j += step) ok = A.eg[cs + j].ab[d] == 0.0 && A.eg[cs + j].ac[d] == 0.0;
     if (all(ok)) return true;
   }
   return false;
@@ -711,27 +718,40 @@ __global__ void __launch_bounds__(kDfThreads, 2) aca_df_cta_kernel(AcaDfArgs A) 
   aca_cta(A, smem_raw, A.order[blockIdx.x]);
 }
 
-// The blocks of sides up to 256 in one launch, longest first (the hardware dispatches CTAs in index
-// order): CTAs of one 4-warp, two 2-warp or four 1-warp groups.
+// The blocks next, next + 1, ... of a class by the CTA's groups, each as it gets free
+template <int W>
+__device__ __forceinline__ void run_groups(const AcaDfArgs& A, unsigned char* smem, const int* order, int count,
+                                           unsigned* next) {
+  __shared__ int s_block[kSmallThreads / 32];
+  const int grp = (threadIdx.x >> 5) / W, tid = threadIdx.x % (32 * W);
+  for (;;) {
+    if (tid == 0) {
+      const unsigned t = atomicAdd(next, 1u);
+      s_block[grp] = t < (unsigned)count ? order[t] : -1;
+    }
+    group_sync<W>(grp);
+    const int b = s_block[grp];
+    if (b < 0) break;
+    aca_small<W>(A, smem, b);
+    group_sync<W>(grp);  // the group's shared memory is free for the next block
+  }
+}
+
+// The blocks of sides up to 256 in one launch, longest first. As many CTAs as are resident take them,
+// first as one 4-warp group each, then as two 2-warp and four 1-warp groups: with four blocks to a
+// CTA that ends with the longest of them, 12.6 of 16 warps per SM were running (ACAW0 -> ACAW1 ms on the
+// 20480-triangle relief).
 __global__ void __launch_bounds__(kSmallThreads, 4) aca_df_kernel(AcaDfArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   load_table(A.tab);
-  const int warp = threadIdx.x >> 5;
-  int cta = blockIdx.x;
   const int* order = A.order + A.split[0];
-  if (cta < A.split[1]) return aca_small<4>(A, smem_raw, order[cta]);
-  cta -= A.split[1];
+  run_groups<4>(A, smem_raw, order, A.split[1], A.next);
+  __syncthreads();
   order += A.split[1];
-  const int n2 = (A.split[2] + 1) / 2;
-  if (cta < n2) {
-    const int bi = 2 * cta + warp / 2;
-    if (bi < A.split[2]) aca_small<2>(A, smem_raw, order[bi]);
-    return;
-  }
-  cta -= n2;
+  run_groups<2>(A, smem_raw, order, A.split[2], A.next + 1);
+  __syncthreads();
   order += A.split[2];
-  const int bi = 4 * cta + warp;
-  if (bi < A.split[3]) aca_small<1>(A, smem_raw, order[bi]);
+  run_groups<1>(A, smem_raw, order, A.split[3], A.next + 2);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -785,7 +805,7 @@ static void launch_aca_kernels(const AcaDfArgs& a, int max_rows, cudaStream_t s_
     constexpr size_t smem = std::max({sizeof(AcaGroup<4>), 2 * sizeof(AcaGroup<2>), 4 * sizeof(AcaGroup<1>)});
     static_assert(smem <= 48 * 1024, "no opt-in needed");
     note_launch();
-    aca_df_kernel<<<ctas, kSmallThreads, smem, s_small>>>(a);
+    aca_df_kernel<<<std::min(ctas, 4 * device_sm_count()), kSmallThreads, smem, s_small>>>(a);
     AC3D_CUDA(cudaGetLastError());
   }
 }
@@ -798,7 +818,7 @@ void launch_aca_df(const DevGeometry& G, const DevPartition& DP, DevHMat& H, dou
               {DP.aca_split[0], DP.aca_split[1], DP.aca_split[2], DP.aca_split[3]},
               df_from_double(H.k), eps, df_from_double(eps * eps), H.maxk, H.maxk, H.pool.as<df2>(), H.pool_cap,
               H.pool_used.as<unsigned long long>(), H.term_off.as<long long>(), H.rank.as<int>(),
-              (int*)(H.pool_used.as<unsigned long long>() + 1), H.passes.as<int>(), 1};
+              &H.pool_used.as<AsmTotals>()->status, H.passes.as<int>(), H.pool_used.as<AsmTotals>()->next, 1};
   launch_aca_kernels(a, max_rows, s, s_small);
 }
 
@@ -1106,7 +1126,7 @@ void launch_listener_aca_df(const DevGeometry& G, const void* pts_df, int L, dou
   AcaDfArgs a{G.cen.as<double4>(), G.va.as<double4>(), G.eg64.as<ElemGeo<double>>(), (const DfPt*)pts_df,
               G.el_df.as<DfElem>(), G.df_tab.as<float4>(), block, order, {1, 0, 0, 0}, df_from_double(k), eps,
               df_from_double(eps * eps), maxk, iter_lim,
-              (df2*)pool, pool_cap, used, term_off, rank, status, nullptr, 0};
+              (df2*)pool, pool_cap, used, term_off, rank, status, nullptr, nullptr, 0};
   const size_t smem = aca_cta_smem(iter_lim, L);
   if (smem > kAcaSmemMax)
     throw Error(4, "receiver ACA too large for shared memory (at most about 5000 receivers)");

@@ -200,6 +200,7 @@ struct AsmTotals {
   unsigned long long sum_rank, max_rank;
   unsigned long long columns[2];        // segment columns (even per leaf)
   unsigned long long entries[2];        // segment entries
+  unsigned next[4];                     // blocks taken, per class of small blocks (ACA kernel)
   unsigned long long tc_bytes[2];       // bytes of the split segments of the tensor-core dot pass
 };
 
