@@ -739,7 +739,7 @@ __device__ __forceinline__ void run_groups(const AcaDfArgs& A, unsigned char* sm
 
 // The blocks of sides up to 256 in one launch, longest first. As many CTAs as are resident take them,
 // first as one 4-warp group each, then as two 2-warp and four 1-warp groups: with four blocks to a
-// CTA that ends with the longest of them, 12.6 of 16 warps per SM were running (ACAW0 -> ACAW1 ms on the
+// CTA that ends with the longest of them, 12.6 of 16 warps per SM were running (4.94 -> 4.67 ms on the
 // 20480-triangle relief).
 __global__ void __launch_bounds__(kSmallThreads, 4) aca_df_kernel(AcaDfArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
