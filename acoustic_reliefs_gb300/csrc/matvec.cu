@@ -128,8 +128,10 @@ __global__ void __launch_bounds__(kThreads, 4) seg_dot_kernel(SegView V, const c
   const int ls = V.leaf_start[leaf], R = V.leaf_start[leaf + 1] - ls;
   const int k0 = V.b_kptr[leaf], K = V.b_kptr[leaf + 1] - k0;
   // a set done flag stays set for the rest of the solve, so reading it before the wait can only
-  // miss a flag that is being set (checked again after the wait)
-  if (K == 0 || (done && *(volatile const int*)done)) {
+  // miss a flag that is being set (checked again after the wait). The Givens step beside this pass
+  // may set it at any time, so the CTA votes: its threads must not part ways
+  const bool ended = __syncthreads_or(done && *(volatile const int*)done);
+  if (K == 0 || ended) {
     grid_dep_wait();
     grid_dep_launch();
     return;
@@ -142,7 +144,7 @@ __global__ void __launch_bounds__(kThreads, 4) seg_dot_kernel(SegView V, const c
   auto after_prefetch = [&]() -> bool {
     grid_dep_wait();
     grid_dep_launch();
-    if (done && *done) return false;
+    if (__syncthreads_or(done && *(volatile const int*)done)) return false;
 #pragma unroll
     for (int t = 0; t < RPG; t++) {
       const int row = g + G * t;
@@ -312,7 +314,8 @@ __global__ void __launch_bounds__(kGatherThreads, AC3D_GATHER_MIN_CTAS) seg_gath
   __shared__ int s_fail;
   __shared__ bool s_last;
   grid_dep_launch();  // as in the one-CTA-per-leaf pass
-  if (done && *done) {
+  // the vote of the CTA: the Givens step beside this pass may set the flag while its warps read it
+  if (__syncthreads_or(done && *(volatile const int*)done)) {
     grid_dep_wait();
     return;
   }

@@ -103,7 +103,8 @@ __global__ void __launch_bounds__(kMT) mseg_dot_kernel(SegView V, const cf* __re
   extern __shared__ __align__(128) unsigned char dsmem[];
   auto stage = reinterpret_cast<unsigned char(*)[kStageBytes]>(dsmem);
   __shared__ __align__(8) uint64_t full[kStages];
-  if (done && *done) return;
+  // the vote of the CTA: the Givens step beside this pass may set the flag while its warps read it
+  if (__syncthreads_or(done && *(volatile const int*)done)) return;
   const int leaf = V.order[blockIdx.x];
   const int ls = V.leaf_start[leaf], R = V.leaf_start[leaf + 1] - ls;
   const int k0 = V.b_kptr[leaf], K = V.b_kptr[leaf + 1] - k0;
@@ -265,7 +266,7 @@ __global__ void __launch_bounds__(kMT, 1) mseg_dot_tc_kernel(SegView V, const un
   __shared__ __align__(8) uint64_t full[kTcStages], empty[kTcStages], accf[2], acce[2];
   __shared__ uint32_t s_tmem;
   __shared__ int s_fail, s_issued, s_consumed;
-  if (done && *done) return;
+  if (__syncthreads_or(done && *(volatile const int*)done)) return;  // as in mseg_dot_kernel
   const int leaf = V.order[blockIdx.x];
   const int ls = V.leaf_start[leaf], R = V.leaf_start[leaf + 1] - ls;
   const int k0 = V.b_kptr[leaf], K = V.b_kptr[leaf + 1] - k0;
@@ -500,7 +501,7 @@ __global__ void __launch_bounds__(kMGatherThreads, MGather<NRB, RPL>::kCtas) mse
   __shared__ double sred[kMW][5][NRB];
   __shared__ int s_fail;
   __shared__ bool s_last;
-  if (done && *done) return;
+  if (__syncthreads_or(done && *(volatile const int*)done)) return;  // as in mseg_dot_kernel
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int P = gridDim.x;
   if (tid == 0) {
