@@ -338,6 +338,7 @@ std::unique_ptr<DevHMat> assemble(ac3d_ctx* c, double k, int prec) {
     c->m->pool_hint[prec] = std::min<int64_t>(c->m->worst_pool, H->pool_used_host + H->pool_used_host / 8 + 4096);
     H->tvec.alloc(tcap * (prec == PREC_FP64 ? sizeof(cd) : sizeof(cf)), s);
     H->tvec64.alloc(tcap * sizeof(cd), s);
+    H->tasks = (int64_t)tot.sum_rank;
     H->lr_entries = (int64_t)tot.lr_entries;
     H->aca_evaluated = (int64_t)tot.aca_evaluated;
     H->tc_bytes[0] = (int64_t)tot.tc_bytes[0];
@@ -790,7 +791,7 @@ MultiBufs block_bufs(ac3d_ctx* c, DevHMat& H, int nrb, BlockWork& W, bool tr) {
     AC3D_CUDA(cudaMemsetAsync(W.tick.p, 0, (1024 + 64) * sizeof(unsigned), s));
   }
   W.pbuf.ensure(std::max<size_t>(H.pbuf.bytes / sizeof(cd), 1) * nrb * sizeof(cf), s);
-  W.tbuf.ensure((size_t)std::max<int64_t>(H.task_cap, 1) * nrb * sizeof(cf), s);
+  W.tbuf.ensure((size_t)std::max<int64_t>(H.tasks, 1) * nrb * sizeof(cf), s);
   W.tolb.ensure((size_t)nrb * sizeof(double), s);
   W.state.ensure(sizeof(KStateM), s);
   B.partials = W.parts.as<double>();

@@ -232,6 +232,7 @@ struct DevHMat {
   DevBuf err;             // int: set by a kernel whose copy pipeline timed out
   DevBuf ticket;          // unsigned: gather-pass completion ticket (zero between launches)
   int64_t task_cap = 0;   // upper bound of the number of stored terms
+  int64_t tasks = 0;      // stored terms
   DevBuf tvec;            // intermediate V x per term (complex, vector precision)
   DevBuf tvec64;          // FP64 / double-float intermediate for refinement residuals
   DevBuf xdf;             // double-float copy of the residual matvec input (FP32 storage only)

@@ -188,7 +188,12 @@ __global__ void __launch_bounds__(kThreads, 4) seg_dot_kernel(SegView V, const c
 }
 
 // t[task] = sum over the leaf entries of the task's block of p[kpos[e] + q], in leaf order
-// (kpos is stored block-major, so a block's entries are consecutive).
+// (kpos is stored block-major, so a block's entries are consecutive). The grid covers the terms the
+// blocks could have: the gather pass may start when this pass's last CTA has, and behind the CTAs
+// that only return it does so when most sums are done. With a grid of the stored terms its streams
+// slowed the sums' loads: 97 instead of 85 us per matvec on the 20480-triangle relief, 164 instead
+// of 148 us on 34340; with the longer sums' entries in shared memory (cp.async) and the gather behind
+// the last sum, 85 and 145 us, but 56 instead of 54 us on 10980 and 35 instead of 34 us on 5280.
 template <typename AT>
 __global__ void __launch_bounds__(256) seg_reduce_kernel(const int* __restrict__ task_b,
                                                          const int* __restrict__ t_off, int ntask_cap,

@@ -412,18 +412,18 @@ __global__ void __launch_bounds__(kMT, 1) mseg_dot_tc_kernel(SegView V, const un
 // T[task][j] = sum over the task's block entries of P[kpos[e] + q][j], in leaf order; a thread takes two
 // right-hand sides (16-byte loads, half the index loads). Bound by the latency of the chain of index
 // loads, P being 145 MB at 16 right-hand sides on the 20480-triangle relief: 92 us with one
-// right-hand side per thread, 56 us so.
+// right-hand side per thread, 56 us so, 50 us with a grid of the stored terms alone and the places
+// of the next four entries under the loads of four.
 template <int NRB>
 __global__ void __launch_bounds__(256) mseg_reduce_kernel(const int* __restrict__ task_b,
-                                                          const int* __restrict__ t_off, int ntask_cap,
-                                                          const int* __restrict__ t_total,
+                                                          const int* __restrict__ t_off, int ntask,
                                                           const int* __restrict__ ent_ptr,
                                                           const int* __restrict__ kpos, const cf* __restrict__ P,
                                                           cf* __restrict__ T, const int* __restrict__ done) {
   if (done && *done) return;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int task = (int)(i / (NRB / 2)), j = 2 * (int)(i % (NRB / 2));
-  if (task >= ntask_cap || task >= *t_total) return;
+  if (task >= ntask) return;
   const int b = task_b[task];
   const int q = task - t_off[b];
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -436,12 +436,21 @@ __global__ void __launch_bounds__(256) mseg_reduce_kernel(const int* __restrict_
     s.z += v.z;
     s.w += v.w;
   };
+  int kk[4];
+  if (e + 3 < e1) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) kk[u] = kpos[e + u];
+  }
   for (; e + 3 < e1; e += 4) {  // four independent loads in flight, summed in entry order
-    const float4 v0 = at(kpos[e]), v1 = at(kpos[e + 1]), v2 = at(kpos[e + 2]), v3 = at(kpos[e + 3]);
-    add(v0);
-    add(v1);
-    add(v2);
-    add(v3);
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = at(kk[u]);
+    if (e + 7 < e1) {
+#pragma unroll
+      for (int u = 0; u < 4; u++) kk[u] = kpos[e + 4 + u];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) add(v[u]);
   }
   for (; e < e1; e++) add(at(kpos[e]));
   *reinterpret_cast<float4*>(T + (size_t)task * NRB + j) = s;
@@ -1093,9 +1102,9 @@ static void mmv_t(const DevPartition& DP, const DevHMat& H, const MultiBufs& B, 
                                                                (const cf*)x, P, done);
     AC3D_CUDA(cudaGetLastError());
     note_launch();
-    const long long thr = H.task_cap * (NRB / 2);
+    const long long thr = std::max<long long>(H.tasks, 1) * (NRB / 2);
     mseg_reduce_kernel<NRB><<<(int)((thr + 255) / 256), 256, 0, s>>>(
-        H.task_b.as<int>(), H.t_off.as<int>(), (int)H.task_cap, H.t_off.as<int>() + DP.na,
+        H.task_b.as<int>(), H.t_off.as<int>(), (int)H.tasks,
         tr ? DP.blk_fw_ptr.as<int>() : DP.blk_tr_ptr.as<int>(), tr ? H.kpos_f.as<int>() : H.kpos_t.as<int>(), P,
         T, done);
     AC3D_CUDA(cudaGetLastError());
