@@ -555,35 +555,59 @@ __global__ void __launch_bounds__(kGmThreads) k_gm_update(GmCols C, int m, int n
 // ------------------------------------------------------------------------------------------
 constexpr uint32_t kBarSpin = 1u << 22;  // polls (with a short sleep) before a barrier gives up
 
-// Grid-wide barrier over all CTAs of a cooperative launch (every CTA calls it the same number of
-// times). One 64-bit arrival counter that is never reset during a cycle: arrival ticket t belongs
-// to barrier instance t / total (no CTA arrives at the next instance before all have arrived at
-// this one), which is complete when the counter reaches (t / total + 1) total. One atomic per CTA
-// and a poll, instead of a count reset and a generation bump after the last arrival. Returns
-// false on every thread if this CTA's wait gave up (recorded in bar_fail).
-__device__ __forceinline__ bool gm_grid_barrier(GMulti* gm, unsigned total) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();  // this CTA's writes before its arrival
-    const unsigned long long t = atomicAdd(&gm->bar, 1ull);
-    const unsigned long long target = (t / total + 1) * (unsigned long long)total;
-    volatile unsigned long long* c = &gm->bar;
-    int ok = 1;
-    uint32_t it = 0;
-    while (*c < target) {
-      if (++it > kBarSpin) {
-        ok = 0;
-        atomicExch(&gm->bar_fail, 1);
-        break;
-      }
-      __nanosleep(20);
-    }
-    __threadfence();
-    s_ok = ok;
+// Grid-wide barrier over all CTAs of a cooperative launch (every CTA waits the same number of times).
+// One 64-bit arrival counter that is never reset during a cycle: a launch's barriers are complete when
+// it reaches the next multiples of the CTA count. The first of them follows from any value read
+// before this CTA's own arrival (none of the launch's barriers can be complete before that), so it
+// is read at the kernel's start and an arrival waits for no answer: the Gram-Schmidt kernel of 5280
+// elements took 15.2 us and takes 13.5, with the sums folded below it. wait
+// returns false on every thread if this CTA gave up (recorded in bar_fail).
+struct GmGridBar {
+  GMulti* gm;
+  unsigned total;
+  unsigned long long* next;  // thread 0's: the counter at the last complete barrier
+  __device__ __forceinline__ GmGridBar(GMulti* g, unsigned n) : gm(g), total(n) {
+    __shared__ unsigned long long s_next;
+    next = &s_next;
+    if (threadIdx.x == 0) s_next = *(volatile unsigned long long*)&gm->bar / total * total;
   }
-  __syncthreads();
-  return s_ok != 0;
+  __device__ __forceinline__ bool wait() {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const unsigned long long target = *next + total;
+      *next = target;
+      __threadfence();  // this CTA's writes before its arrival
+      asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(&gm->bar), "l"(1ull) : "memory");
+      volatile unsigned long long* c = &gm->bar;
+      int ok = 1;
+      uint32_t it = 0;
+      while (*c < target) {
+        if (++it > kBarSpin) {
+          ok = 0;
+          atomicExch(&gm->bar_fail, 1);
+          break;
+        }
+        __nanosleep(20);
+      }
+      __threadfence();
+      s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+  }
+};
+
+// One step of a transposed butterfly: of 2 N values, a lane keeps N (the upper ones in the lanes with
+// bit O set) and adds its partner's share of them. Steps 16, 8, ... give the bits of warp_sum.
+template <int N, int O, typename T>
+__device__ __forceinline__ void gm_fold(T* v) {
+  const bool up = (threadIdx.x & O) != 0;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const T keep = up ? v[k + N] : v[k], give = up ? v[k] : v[k + N];
+    v[k] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+  }
 }
 
 // Elements per lane per round of loads in gf_dot_partials: with FP32 vectors one round covers a
@@ -790,7 +814,7 @@ __global__ void __launch_bounds__(kGmThreads, sizeof(VT) == 4 ? 3 : 2) k_gm_fuse
   // update (it reads V_{j+1} only after this kernel has completed). Not with the Givens CTA: inside
   // a request server the early matvec CTAs would hold SM room that other requests' kernels need.
   const bool early = givens == 1;
-  const unsigned total = gridDim.x * gridDim.y;
+  GmGridBar bar(C.gm, gridDim.x * gridDim.y);
   GState* st = C.st + r;
   double* gd = C.gd + r * C.gds;
   V += r * C.Vs;
@@ -818,9 +842,9 @@ __global__ void __launch_bounds__(kGmThreads, sizeof(VT) == 4 ? 3 : 2) k_gm_fuse
   };
   // 1, 2: first-pass dots and their reduction
   if (work) gf_dot_partials<VT>(V, X, C.vs, lo, hi - lo, n, j, gd + L.part(), G);
-  ok = gm_grid_barrier(C.gm, total) && ok;
+  ok = bar.wait() && ok;
   if (work && ok) gf_reduce<VT>(gd, L, gd + L.part(), G, j, sj, 0);
-  ok = gm_grid_barrier(C.gm, total) && ok;
+  ok = bar.wait() && ok;
   if (work && ok) load_coef();
   VT a = 0;
   if (reorth) {
@@ -831,10 +855,10 @@ __global__ void __launch_bounds__(kGmThreads, sizeof(VT) == 4 ? 3 : 2) k_gm_fuse
       gf_dot_partials<VT>(V, W2, 1, lo, hi - lo, n, j, gd + L.part2(), G);
     }
     if (work && ok) gf_cta_sum<VT>(a, gd + L.npart() + blockIdx.x);
-    ok = gm_grid_barrier(C.gm, total) && ok;
+    ok = bar.wait() && ok;
     // 4: second-pass coefficients
     if (work && ok) gf_reduce<VT>(gd, L, gd + L.part2(), G, j, 1.0, 1);
-    ok = gm_grid_barrier(C.gm, total) && ok;
+    ok = bar.wait() && ok;
     if (early) grid_dep_launch();
     // 5: V_{j+1} = U - sum_k coef_k V_k
     if (work && ok) {
@@ -849,7 +873,7 @@ __global__ void __launch_bounds__(kGmThreads, sizeof(VT) == 4 ? 3 : 2) k_gm_fuse
       gf_cta_sum<VT>(a, gd + L.npart() + blockIdx.x);
     }
     // givens 1: k_gm_rotate reads the |.|^2 partials after this kernel has completed
-    if (givens != 1) ok = gm_grid_barrier(C.gm, total) && ok;
+    if (givens != 1) ok = bar.wait() && ok;
   }
   if (!run || (int)blockIdx.x != (givens == 2 ? G : 0)) return;
   if (!ok) {
@@ -900,15 +924,19 @@ __global__ void __launch_bounds__(kGmThreads) k_gm_rotate(GmCols C, int m, int L
 constexpr int kGdE = 2;
 
 // Per-CTA partial dots a_k = conj(V_k) . U and b_k = conj(V_k) . X (k < j) over [lo, lo + len)
-// of the block vectors U and X (stride xs), into pa / pb[(k G + c) 2]; each lane takes the
-// elements lane, lane + 32, ... in that order.
+// of the block vectors U and X (stride xs), into pa / pb[k G + c]; each lane takes the elements lane,
+// lane + 32, ... in that order. The vectors go last to first: the update takes them first to last, so
+// where a batch's bases exceed L2 (16 cycles of 20480 elements: from 50 vectors on) each pass begins
+// with what the other ended with.
 template <typename VT>
 __device__ __forceinline__ void gd_dot_partials(const cplx<VT>* __restrict__ V, const cplx<VT>* U,
                                                 const cplx<VT>* X, int xs, int lo, int len, int n, int j,
-                                                double* pa, double* pb, int G) {
+                                                cplx<VT>* pa, cplx<VT>* pb, int G) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int kb = 4 * warp; kb < j; kb += 4 * kGmWarps) {
-    VT ar[4] = {0, 0, 0, 0}, ai[4] = {0, 0, 0, 0}, br[4] = {0, 0, 0, 0}, bi[4] = {0, 0, 0, 0};
+  for (int kb = 4 * ((j - 1) / 4 - warp); kb >= 0 && j > 0; kb -= 4 * kGmWarps) {
+    VT acc[16];  // a and b of vector kb + q: 4 q + (Re a, Im a, Re b, Im b)
+#pragma unroll
+    for (int q = 0; q < 16; q++) acc[q] = 0;
     for (int t0 = 0; t0 < len; t0 += 32 * kGdE) {
       cplx<VT> v[kGdE][4], u[kGdE], x[kGdE];
 #pragma unroll
@@ -924,33 +952,26 @@ __device__ __forceinline__ void gd_dot_partials(const cplx<VT>* __restrict__ V, 
       for (int e = 0; e < kGdE; e++)
 #pragma unroll
         for (int q = 0; q < 4; q++) {  // conj(v) u and conj(v) x
-          ar[q] = fma(v[e][q].re, u[e].re, ar[q]);
-          ar[q] = fma(v[e][q].im, u[e].im, ar[q]);
-          ai[q] = fma(v[e][q].re, u[e].im, ai[q]);
-          ai[q] = fma(-v[e][q].im, u[e].re, ai[q]);
-          br[q] = fma(v[e][q].re, x[e].re, br[q]);
-          br[q] = fma(v[e][q].im, x[e].im, br[q]);
-          bi[q] = fma(v[e][q].re, x[e].im, bi[q]);
-          bi[q] = fma(-v[e][q].im, x[e].re, bi[q]);
+          VT* c = acc + 4 * q;
+          c[0] = fma(v[e][q].re, u[e].re, c[0]);
+          c[0] = fma(v[e][q].im, u[e].im, c[0]);
+          c[1] = fma(v[e][q].re, u[e].im, c[1]);
+          c[1] = fma(-v[e][q].im, u[e].re, c[1]);
+          c[2] = fma(v[e][q].re, x[e].re, c[2]);
+          c[2] = fma(v[e][q].im, x[e].im, c[2]);
+          c[3] = fma(v[e][q].re, x[e].im, c[3]);
+          c[3] = fma(-v[e][q].im, x[e].re, c[3]);
         }
     }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      ar[q] = warp_sum(ar[q]);
-      ai[q] = warp_sum(ai[q]);
-      br[q] = warp_sum(br[q]);
-      bi[q] = warp_sum(bi[q]);
-    }
-    if (lane == 0)
-#pragma unroll
-      for (int q = 0; q < 4; q++)
-        if (kb + q < j) {
-          const size_t o = ((size_t)(kb + q) * G + blockIdx.x) * 2;
-          pa[o] = (double)ar[q];
-          pa[o + 1] = (double)ai[q];
-          pb[o] = (double)br[q];
-          pb[o + 1] = (double)bi[q];
-        }
+    // lane 2 i ends with the sum of acc[i]
+    gm_fold<8, 16>(acc);
+    gm_fold<4, 8>(acc);
+    gm_fold<2, 4>(acc);
+    gm_fold<1, 2>(acc);
+    const VT sum = acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 1);
+    const VT im = __shfl_down_sync(0xffffffffu, sum, 2);
+    const int k = kb + lane / 8;
+    if (lane % 4 == 0 && k < j) (lane & 4 ? pb : pa)[(size_t)k * G + blockIdx.x] = cplx<VT>(sum, im);
   }
 }
 
@@ -958,14 +979,17 @@ __device__ __forceinline__ void gd_dot_partials(const cplx<VT>* __restrict__ V, 
 // sums the slots c, c + G, ... (a warp each) over the G per-CTA partials in CTA order.
 template <typename VT>
 __device__ __forceinline__ void gd_reduce(double* gd, const GmLayout& L, int G, int j) {
+  static_assert(sizeof(VT) == 4, "partials are FP32 pairs");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int sl = blockIdx.x + warp * G; sl <= 2 * j; sl += kGmWarps * G) {
     if (sl == 2 * j) {
       VT al = 0, br = 0, bi = 0;
+      const float* ab = reinterpret_cast<const float*>(gd + L.abpart());
+#pragma unroll 8
       for (int c = lane; c < G; c += 32) {
-        al += (VT)__ldcg(&gd[L.abpart() + 3 * c]);
-        br += (VT)__ldcg(&gd[L.abpart() + 3 * c + 1]);
-        bi += (VT)__ldcg(&gd[L.abpart() + 3 * c + 2]);
+        al += __ldcg(&ab[3 * c]);
+        br += __ldcg(&ab[3 * c + 1]);
+        bi += __ldcg(&ab[3 * c + 2]);
       }
       al = warp_sum(al);
       br = warp_sum(br);
@@ -979,11 +1003,13 @@ __device__ __forceinline__ void gd_reduce(double* gd, const GmLayout& L, int G, 
     }
     const bool isb = sl >= j;
     const int k = isb ? sl - j : sl;
-    const double* part = gd + (isb ? L.part2() : L.part());
+    const float2* part = reinterpret_cast<const float2*>(gd + (isb ? L.part2() : L.part()));
     VT sr = 0, si = 0;
+#pragma unroll 8
     for (int c = lane; c < G; c += 32) {
-      sr += (VT)__ldcg(&part[((size_t)k * G + c) * 2]);
-      si += (VT)__ldcg(&part[((size_t)k * G + c) * 2 + 1]);
+      const float2 v = __ldcg(&part[(size_t)k * G + c]);
+      sr += v.x;
+      si += v.y;
     }
     sr = warp_sum(sr);
     si = warp_sum(si);
@@ -1001,19 +1027,22 @@ __device__ __forceinline__ void gd_reduce(double* gd, const GmLayout& L, int G, 
 __device__ __forceinline__ void gd_scalars(const double* gd, const GmLayout& L, int j, double* sh) {
   if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
-  double aa = 0, abr = 0, abi = 0;
+  double t[4] = {0, 0, 0, 0};  // |a|^2, Re and Im of conj(a) b
+  const double al = __ldcg(&gd[L.ab()]), br = __ldcg(&gd[L.ab() + 1]), bi = __ldcg(&gd[L.ab() + 2]);
   for (int k = lane; k < j; k += 32) {
     const double ar = __ldcg(&gd[L.coef() + 2 * k]), ai = __ldcg(&gd[L.coef() + 2 * k + 1]);
     const double br = __ldcg(&gd[L.h2() + 2 * k]), bi = __ldcg(&gd[L.h2() + 2 * k + 1]);
-    aa += ar * ar + ai * ai;
-    abr += ar * br + ai * bi;  // conj(a) b
-    abi += ar * bi - ai * br;
+    t[0] += ar * ar + ai * ai;
+    t[1] += ar * br + ai * bi;
+    t[2] += ar * bi - ai * br;
   }
-  aa = warp_sum(aa);
-  abr = warp_sum(abr);
-  abi = warp_sum(abi);
+  // folded: 6 additions on the FP64 pipe (64 clocks each) in place of 15
+  gm_fold<2, 16>(t);
+  gm_fold<1, 8>(t);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) t[0] += __shfl_xor_sync(0xffffffffu, t[0], o);
+  const double aa = t[0], abr = __shfl_sync(0xffffffffu, t[0], 8), abi = __shfl_sync(0xffffffffu, t[0], 16);
   if (lane == 0) {
-    const double al = __ldcg(&gd[L.ab()]), br = __ldcg(&gd[L.ab() + 1]), bi = __ldcg(&gd[L.ab() + 2]);
     const double r2 = al - aa;
     const double ir2 = r2 > 0.0 ? gm_rcp(r2) : 0.0;
     sh[0] = r2;
@@ -1077,6 +1106,13 @@ __device__ __forceinline__ void gd_update(const double* gd, const GmLayout& L, i
                                           const cplx<VT>* X, cplx<VT>* U, int vs, int lo, int hi) {
   extern __shared__ __align__(16) unsigned char gsm[];
   __shared__ double sh[3];
+  double c0[4] = {0, 0, 0, 0};  // this thread's first coefficients, under the scalars
+  if (threadIdx.x < j) {
+    c0[0] = __ldcg(&gd[L.coef() + 2 * threadIdx.x]);
+    c0[1] = __ldcg(&gd[L.coef() + 2 * threadIdx.x + 1]);
+    c0[2] = __ldcg(&gd[L.h2() + 2 * threadIdx.x]);
+    c0[3] = __ldcg(&gd[L.h2() + 2 * threadIdx.x + 1]);
+  }
   gd_scalars(gd, L, j, sh);
   __syncthreads();
   const double r2 = sh[0];
@@ -1085,8 +1121,9 @@ __device__ __forceinline__ void gd_update(const double* gd, const GmLayout& L, i
   cplx<VT>* ca = reinterpret_cast<cplx<VT>*>(gsm);
   cplx<VT>* cb = ca + (m + 1);
   for (int k = threadIdx.x; k < j; k += blockDim.x) {
-    const double ar = __ldcg(&gd[L.coef() + 2 * k]), ai = __ldcg(&gd[L.coef() + 2 * k + 1]);
-    const double br = __ldcg(&gd[L.h2() + 2 * k]), bi = __ldcg(&gd[L.h2() + 2 * k + 1]);
+    const bool first = k == (int)threadIdx.x;
+    const double ar = first ? c0[0] : __ldcg(&gd[L.coef() + 2 * k]), ai = first ? c0[1] : __ldcg(&gd[L.coef() + 2 * k + 1]);
+    const double br = first ? c0[2] : __ldcg(&gd[L.h2() + 2 * k]), bi = first ? c0[3] : __ldcg(&gd[L.h2() + 2 * k + 1]);
     ca[k] = cplx<VT>((VT)ar, (VT)ai);
     cb[k] = cplx<VT>((VT)(br - (gr * ar - gi * ai)), (VT)(bi - (gr * ai + gi * ar)));
   }
@@ -1132,7 +1169,7 @@ __global__ void __launch_bounds__(kGmThreads, 3) k_gm_dcgs(GmCols C, int m, int 
   if (*(volatile const int*)&C.gm->done_all) return;
   const int r = blockIdx.y, G = (int)gridDim.x - (givens == 2 ? 1 : 0);
   const bool giv_cta = givens == 2 && (int)blockIdx.x == G;
-  const unsigned total = gridDim.x * gridDim.y;
+  GmGridBar bar(C.gm, gridDim.x * gridDim.y);
   GState* st = C.st + r;
   double* gd = C.gd + r * C.gds;
   V += r * C.Vs;
@@ -1151,7 +1188,8 @@ __global__ void __launch_bounds__(kGmThreads, 3) k_gm_dcgs(GmCols C, int m, int 
   bool ok = true;
   // 1: dots of the basis against u_j and w; |u_j|^2 and u_j^H w
   if (work) {
-    gd_dot_partials<VT>(V, U, X, C.vs, lo, hi - lo, n, j, gd + L.part(), gd + L.part2(), G);
+    gd_dot_partials<VT>(V, U, X, C.vs, lo, hi - lo, n, j, reinterpret_cast<cplx<VT>*>(gd + L.part()),
+                        reinterpret_cast<cplx<VT>*>(gd + L.part2()), G);
     VT al = 0, br = 0, bi = 0;
     for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
       const cplx<VT> u = U[(size_t)i * C.vs], x = X[(size_t)i * C.vs];
@@ -1172,13 +1210,13 @@ __global__ void __launch_bounds__(kGmThreads, 3) k_gm_dcgs(GmCols C, int m, int 
     if (threadIdx.x < 3) {
       VT t = 0;
       for (int w = 0; w < kGmWarps; w++) t += sw[threadIdx.x][w];
-      gd[L.abpart() + 3 * blockIdx.x + threadIdx.x] = (double)t;
+      reinterpret_cast<VT*>(gd + L.abpart())[3 * blockIdx.x + threadIdx.x] = t;
     }
   }
-  ok = gm_grid_barrier(C.gm, total) && ok;
+  ok = bar.wait() && ok;
   // 2: the sums
   if (work && ok) gd_reduce<VT>(gd, L, G, j);
-  ok = gm_grid_barrier(C.gm, total) && ok;
+  ok = bar.wait() && ok;
   if (givens == 1) grid_dep_launch();  // the next matvec reads u_{j+1} only after this kernel
   if (!run) return;
   if (!ok) {
