@@ -111,7 +111,7 @@ struct DotShape {
 };
 
 // Dot pass: p[kptr[leaf] + k] = sum_rows S[k][row] x[leaf rows] for every column k of the leaf's
-// low-rank segment (region B).
+// low-rank segment (region B), gridDim.y CTAs per leaf.
 template <typename MT, typename AT, int RPL>
 __global__ void __launch_bounds__(kThreads, 4) seg_dot_kernel(SegView V, const cplx<MT>* __restrict__ lrseg,
                                                            const cplx<AT>* __restrict__ xm, cplx<AT>* __restrict__ p,
@@ -126,7 +126,15 @@ __global__ void __launch_bounds__(kThreads, 4) seg_dot_kernel(SegView V, const c
   // stream in before the wait for the preceding kernel (which writes x and the done flag)
   const int leaf = V.order[blockIdx.x];
   const int ls = V.leaf_start[leaf], R = V.leaf_start[leaf + 1] - ls;
-  const int k0 = V.b_kptr[leaf], K = V.b_kptr[leaf + 1] - k0;
+  int k0 = V.b_kptr[leaf], K = V.b_kptr[leaf + 1] - k0;
+  const cplx<MT>* seg = lrseg + V.b_seg[leaf];
+  if (gridDim.y > 1) {  // this CTA's part of the columns, from an even one on (16-byte aligned copies)
+    const int lo = (int)((long long)K * blockIdx.y / gridDim.y) & ~1;
+    const int hi = blockIdx.y + 1 == gridDim.y ? K : (int)((long long)K * (blockIdx.y + 1) / gridDim.y) & ~1;
+    k0 += lo;
+    K = hi - lo;
+    seg += (long long)lo * R;
+  }
   // a set done flag stays set for the rest of the solve, so reading it before the wait can only
   // miss a flag that is being set (checked again after the wait). The Givens step beside this pass
   // may set it at any time, so the CTA votes: its threads must not part ways
@@ -154,7 +162,7 @@ __global__ void __launch_bounds__(kThreads, 4) seg_dot_kernel(SegView V, const c
     }
     return true;
   };
-  stream_leaf<MT>(stage, full, R, nullptr, 0, lrseg + V.b_seg[leaf], K, V.err, after_prefetch,
+  stream_leaf<MT>(stage, full, R, nullptr, 0, seg, K, V.err, after_prefetch,
                   [&](const cplx<MT>* S, int, int c0, int ncols, int, int, int) {
                     // two columns per lane in flight: j and j + STEP
                     for (int jb = warp * CPW; jb < ncols; jb += 2 * STEP) {
@@ -660,6 +668,20 @@ void prepare_matvec_kernels() {
   });
 }
 
+// CTAs per leaf of the dot pass (a column's dot is the same in any of them). Below two CTAs per SM
+// always more: 256 leaves of 5280 triangles 35.6 us a matvec with one CTA each and 31.0 with two, 64 leaves of
+// 1280 triangles 14.3 and 13.3 with eight. Up to a full wave of four per SM while a part keeps twice
+// the ring's bytes: 512 leaves of 10980 triangles (190 KB) 55.0 and 51.1 us with two, but four for
+// the 256 leaves of 5280 (150 KB) 34.7 us.
+static int dot_parts(int nleaf, size_t bytes) {
+  const int sms = device_sm_count();
+  int parts = 1;
+  while (parts < 8 && (nleaf * parts < 2 * sms ||
+                       (nleaf * parts < 4 * sms && bytes / ((size_t)nleaf * parts) >= 2 * kRingBytes)))
+    parts *= 2;
+  return parts;
+}
+
 template <typename AT>
 static void launch_reduce(const DevPartition& DP, const DevHMat& H, bool tr, const cplx<AT>* p, cplx<AT>* t,
                           const int* done, cudaStream_t s, bool pdl) {
@@ -705,7 +727,8 @@ static void mv_t(const DevPartition& DP, const DevHMat& H, bool tr, const void* 
     d.b_seg = tr ? H.seg_f.as<long long>() : H.seg_t.as<long long>();
     d.b_kptr = tr ? H.kseg_f.as<int>() : H.kseg_t.as<int>();
     d.order = tr ? H.order_rows.as<int>() : H.order_cols.as<int>();
-    launch_k(pdl, seg_dot_kernel<MT, AT, RPL>, dim3(DP.nleaf), dim3(kThreads), kRingBytes, s, d,
+    launch_k(pdl, seg_dot_kernel<MT, AT, RPL>, dim3(DP.nleaf, dot_parts(DP.nleaf, (tr ? H.useg : H.vseg).bytes)),
+             dim3(kThreads), kRingBytes, s, d,
              tr ? useg : vseg, xm, p, done);
     launch_reduce<AT>(DP, H, tr, p, t, done, s, pdl);
   }
