@@ -368,75 +368,105 @@ __global__ void __launch_bounds__(kGatherThreads, AC3D_GATHER_MIN_CTAS) seg_gath
   __syncthreads();
 
   if (warp == kWarps) {
-    // ---- producer warp: every leaf's chunks in order, with no gap between leaves
+    // ---- producer warp: every leaf's chunks in order, with no gap between leaves. Its own time per
+    // chunk bounds the pass on small meshes, so places advance by additions (no divisions per chunk) and
+    // the column indices are loaded a chunk ahead (the multipliers' addresses wait for them).
+    // Matvec, before and after: 30.9 and 29.5 us on 5280 triangles, 118 and 105 us on 10680 in 128
+    // leaves, 1019 and 1005 us on 118680
     bool waited = false, failed = false;
-    long long seq = 0;  // stage sequence number
-    LeafGeo nxt = leaf_geo(0);
-    for (int n = 0; !failed; n++) {
-      const LeafGeo cur = nxt;
-      if (cur.leaf >= 0) nxt = leaf_geo(n + 1);  // in flight while this leaf streams
-      const int leaf = cur.leaf, ls = cur.ls, R = cur.R, a_cols = cur.a_cols, b_cols = cur.b_cols;
-      const int cpc = leaf >= 0 ? min(kPCols, max(2, (int)(kStageBytes / sizeof(cplx<MT>)) / R & ~1)) : 2;
-      const int na = (a_cols + cpc - 1) / cpc, nb = (b_cols + cpc - 1) / cpc;
-      const int nch = leaf >= 0 ? max(na + nb, 1) : 1;  // a leaf with no columns still gets one stage
-      if (lane == 0 && leaf >= 0) {
-        slot_leaf[n % kLeafSlots] = leaf;
-        slot_ls[n % kLeafSlots] = ls;
-        slot_R[n % kLeafSlots] = R;
-      }
-      for (int c = 0; c < nch; c++, seq++) {
-        const int s = (int)(seq % kStages);
-        if (seq >= kStages) {
-          const bool got =
-              __all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], (uint32_t)(seq / kStages - 1) & 1u));
-          if (!got) {
-            if (lane == 0) atomicExch(&s_fail, 1);
-            failed = true;
-            break;
-          }
-        }
-        // chunk geometry
-        int ncols = 0;
-        const cplx<MT>* src = nullptr;
-        const int* idx = nullptr;
-        const cplx<AT>* z = nullptr;
-        if (leaf >= 0 && c < na) {
-          const int c0 = c * cpc;
-          ncols = min(cpc, a_cols - c0);
-          src = near + cur.a_seg + (long long)c0 * R;
-          idx = V.a_idx + cur.a_k + c0;
-          z = xm;
-        } else if (leaf >= 0 && c < na + nb) {
-          const int c0 = (c - na) * cpc;
-          ncols = min(cpc, b_cols - c0);
-          src = lrseg + cur.b_seg + (long long)c0 * R;
-          idx = V.b_idx + cur.b_k + c0;
-          z = t;
-        }
-        if (lane == 0) {
-          meta[s] = StageMeta{leaf >= 0 ? n % kLeafSlots : -1, ncols, c == 0, c == nch - 1};
-          const uint32_t bytes = (uint32_t)(ncols * R * sizeof(cplx<MT>));
-          fence_proxy_async();
-          mbar_expect_tx(&full[s], bytes);  // zero bytes: a plain arrival
-          if (bytes) bulk_copy_g2s(stage[s], src, bytes, &full[s]);
-        }
-        if (ncols > 0 && c >= na && !waited) {  // t comes from the preceding kernel
-          grid_dep_wait();
-          waited = true;
-        }
+    int st = 0, nissued = 0;
+    uint32_t ph = 1;  // of the empty barriers: a fresh one lets pass
+    int kk[kPProdCols];
+    auto load_idx = [&](const int* idx, int ncols) {
 #pragma unroll
-        for (int u = 0; u < kPProdCols; u++) {
-          const int col = lane + 32 * u;
-          if (col < ncols) cp_async_elem<sizeof(cplx<AT>)>(&zbuf[s][col], z + max(idx[col], 0));
-        }
-        cp_async_arrive_noinc(&full[s]);
+      for (int u = 0; u < kPProdCols; u++) kk[u] = lane + 32 * u < ncols ? idx[lane + 32 * u] : 0;
+    };
+    auto acquire = [&]() {
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&empty[st], ph))) {
+        if (lane == 0) atomicExch(&s_fail, 1);
+        failed = true;
       }
-      if (leaf < 0) break;  // the end marker went out
+      return !failed;
+    };
+    auto advance = [&]() {
+      nissued++;
+      if (++st == kStages) {
+        st = 0;
+        ph ^= 1u;
+      }
+    };
+    int slot = 0;
+    auto chunk_cols = [](const LeafGeo& o) { return min(kPCols, max(2, (int)(kStageBytes / sizeof(cplx<MT>)) / o.R & ~1)); };
+    LeafGeo nxt = leaf_geo(0);
+    int ncpc = nxt.leaf >= 0 ? chunk_cols(nxt) : 2;
+    load_idx(nxt.a_cols ? V.a_idx + nxt.a_k : V.b_idx + nxt.b_k, min(ncpc, nxt.a_cols ? nxt.a_cols : nxt.b_cols));
+    for (int n = 0; !failed && nxt.leaf >= 0; n++) {
+      const LeafGeo cur = nxt;
+      const int R = cur.R, cpc = ncpc;
+      nxt = leaf_geo(n + 1);  // in flight while this leaf streams
+      if (lane == 0) {
+        slot_leaf[slot] = cur.leaf;
+        slot_ls[slot] = cur.ls;
+        slot_R[slot] = R;
+      }
+      const bool two = cur.a_cols > 0 && cur.b_cols > 0;
+      bool first = true;
+      for (int region = cur.a_cols > 0 ? 0 : 1; region < 2 && !failed; region++) {
+        int left = region ? cur.b_cols : cur.a_cols;
+        if (region && left == 0 && cur.a_cols > 0) break;
+        const cplx<MT>* src = region ? lrseg + cur.b_seg : near + cur.a_seg;
+        const int* idx = region ? V.b_idx + cur.b_k : V.a_idx + cur.a_k;
+        const cplx<AT>* z = region ? t : xm;
+        // (a leaf with no columns still gets one stage)
+        do {
+          if (!acquire()) break;
+          const int ncols = min(cpc, left);
+          left -= ncols;
+          if (lane == 0) {
+            meta[st] = StageMeta{slot, ncols, first, left == 0 && (region || !two)};
+            const uint32_t bytes = (uint32_t)(ncols * R * sizeof(cplx<MT>));
+            fence_proxy_async();
+            mbar_expect_tx(&full[st], bytes);  // zero bytes: a plain arrival
+            if (bytes) bulk_copy_g2s(stage[st], src, bytes, &full[st]);
+          }
+          if (region && ncols > 0 && !waited) {  // t comes from the preceding kernel
+            grid_dep_wait();
+            waited = true;
+          }
+#pragma unroll
+          for (int u = 0; u < kPProdCols; u++) {
+            const int col = lane + 32 * u;
+            if (col < ncols) cp_async_elem<sizeof(cplx<AT>)>(&zbuf[st][col], z + max(kk[u], 0));
+          }
+          cp_async_arrive_noinc(&full[st]);
+          advance();
+          first = false;
+          src += (size_t)ncols * R;
+          idx += ncols;
+          if (left > 0) {
+            load_idx(idx, min(cpc, left));
+          } else if (region == 0 && two) {
+            load_idx(V.b_idx + cur.b_k, min(cpc, cur.b_cols));
+          } else if (nxt.leaf >= 0) {
+            ncpc = chunk_cols(nxt);
+            load_idx(nxt.a_cols ? V.a_idx + nxt.a_k : V.b_idx + nxt.b_k, min(ncpc, nxt.a_cols ? nxt.a_cols : nxt.b_cols));
+          }
+        } while (left > 0);
+      }
+      if (++slot == kLeafSlots) slot = 0;
+    }
+    if (!failed && acquire()) {  // the end marker
+      if (lane == 0) {
+        meta[st] = StageMeta{-1, 0, 1, 1};
+        mbar_expect_tx(&full[st], 0);
+      }
+      cp_async_arrive_noinc(&full[st]);
+      advance();
     }
     if (!waited) grid_dep_wait();
     cp_async_wait_all();
     if (lane == 0)
-      for (long long cc = max(0LL, seq - kStages); cc < seq; cc++)
+      for (int cc = max(0, nissued - kStages); cc < nissued; cc++)
         mbar_wait_bounded(&full[cc % kStages], (uint32_t)(cc / kStages) & 1u);
   } else {
     // ---- consumer warps
@@ -447,9 +477,12 @@ __global__ void __launch_bounds__(kGatherThreads, AC3D_GATHER_MIN_CTAS) seg_gath
     int leaf = -1, ls = 0, R = 0;
     uint32_t cphase = 0;
     bool cok = true;
-    for (long long seq = 0;; seq++) {
-      const int s = (int)(seq % kStages);
-      const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], (uint32_t)(seq / kStages) & 1u));
+    int s = kStages - 1;
+    uint32_t ph = 1;
+    for (;;) {
+      if (++s == kStages) s = 0;
+      if (s == 0) ph ^= 1u;
+      const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], ph));
       if (!got) {
         if (lane == 0) atomicExch(&s_fail, 1);
         break;
