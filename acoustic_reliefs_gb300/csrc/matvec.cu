@@ -110,18 +110,47 @@ struct DotShape {
   static constexpr int RPG = 32 * RPL / G;
 };
 
+// Barrier of the consumer warps only (the producer keeps streaming): every consumer thread arrives
+// on an mbarrier (release) and waits for the phase (acquire), with the bounded wait, so a failed
+// pipeline cannot leave threads blocked. Returns false if the phase did not complete.
+__device__ __forceinline__ bool consumer_sync(uint64_t* bar, uint32_t& phase) {
+  mbar_arrive(bar);
+  const bool ok = mbar_wait_bounded(bar, phase);
+  phase ^= 1u;
+  return ok;
+}
+
+// One step of a transposed butterfly: of 2 N values, a lane keeps N (the upper ones in the lanes with
+// bit O set) and adds its partner's share of them: the bits of the butterfly on each.
+template <int N, int O>
+__device__ __forceinline__ void dot_fold(float* v) {
+  const bool up = (threadIdx.x & O) != 0;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const float keep = up ? v[k + N] : v[k], give = up ? v[k] : v[k + N];
+    v[k] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+  }
+}
+
 // Dot pass: p[kptr[leaf] + k] = sum_rows S[k][row] x[leaf rows] for every column k of the leaf's
-// low-rank segment (region B), gridDim.y CTAs per leaf.
+// low-rank segment (region B), gridDim.y CTAs per leaf. As the gather pass, eight consumer warps and one
+// producer warp that streams the chunks, so that no barrier of the CTA stands between chunks, and sums over
+// the lanes folded (4 shuffles for 12). Matvec, before and after: 29.4 and 27.7 us on 5280 triangles, 84.0 and
+// 81.1 us on 20480, 145.8 and 143.0 us on 34340, 999 and 994 us on 118680.
 template <typename MT, typename AT, int RPL>
-__global__ void __launch_bounds__(kThreads, 4) seg_dot_kernel(SegView V, const cplx<MT>* __restrict__ lrseg,
-                                                           const cplx<AT>* __restrict__ xm, cplx<AT>* __restrict__ p,
-                                                           const int* __restrict__ done) {
+__global__ void __launch_bounds__(kThreads + 32, 4) seg_dot_kernel(SegView V, const cplx<MT>* __restrict__ lrseg,
+                                                                   const cplx<AT>* __restrict__ xm,
+                                                                   cplx<AT>* __restrict__ p,
+                                                                   const int* __restrict__ done) {
   constexpr int G = DotShape<RPL>::G, RPG = DotShape<RPL>::RPG;
   constexpr int CPW = 32 / G;             // columns per warp step
   constexpr int STEP = kWarps * CPW;      // columns per CTA step
   extern __shared__ __align__(128) unsigned char dsmem[];
   auto stage = reinterpret_cast<unsigned char(*)[kStageBytes]>(dsmem);
   __shared__ __align__(8) uint64_t full[kStages];
+  __shared__ __align__(8) uint64_t empty[kStages];
+  __shared__ __align__(8) uint64_t cbar;
+  __shared__ int s_stop;
   // the segments and the partition are not written by any kernel of a solve: the first stages
   // stream in before the wait for the preceding kernel (which writes x and the done flag)
   const int leaf = V.order[blockIdx.x];
@@ -135,6 +164,15 @@ __global__ void __launch_bounds__(kThreads, 4) seg_dot_kernel(SegView V, const c
     K = hi - lo;
     seg += (long long)lo * R;
   }
+  if (threadIdx.x == 0) {
+    for (int st = 0; st < kStages; st++) {
+      mbar_init(&full[st], 1);
+      mbar_init(&empty[st], kWarps);
+    }
+    mbar_init(&cbar, kThreads);
+    s_stop = 0;
+    fence_barrier_init();
+  }
   // a set done flag stays set for the rest of the solve, so reading it before the wait can only
   // miss a flag that is being set (checked again after the wait). The Givens step beside this pass
   // may set it at any time, so the CTA votes: its threads must not part ways
@@ -145,54 +183,116 @@ __global__ void __launch_bounds__(kThreads, 4) seg_dot_kernel(SegView V, const c
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cpc = max(2, (int)(kStageBytes / sizeof(cplx<MT>)) / R & ~1);  // columns per chunk, even
+  if (warp == kWarps) {
+    int st = 0, issued = 0;
+    uint32_t ph = 1;  // of the empty barriers: a fresh one lets pass
+    for (int c0 = 0; c0 < K; c0 += cpc) {
+      if (issued == kStages) {  // the ring is full: now the kernel before
+        grid_dep_wait();
+        grid_dep_launch();
+      }
+      const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&empty[st], ph));
+      if (!got && lane == 0) atomicExch(V.err, 1);
+      if (!got || *(volatile int*)&s_stop) break;
+      if (lane == 0) {
+        const uint32_t bytes = (uint32_t)(min(cpc, K - c0) * R * sizeof(cplx<MT>));
+        fence_proxy_async();
+        mbar_expect_tx(&full[st], bytes);
+        bulk_copy_g2s(stage[st], seg + (size_t)c0 * R, bytes, &full[st]);
+      }
+      issued++;
+      if (++st == kStages) {
+        st = 0;
+        ph ^= 1u;
+      }
+    }
+    if (issued <= kStages) {
+      grid_dep_wait();
+      grid_dep_launch();
+    }
+    // the copies land before the CTA exits
+    if (lane == 0)
+      for (int cc = max(0, issued - kStages); cc < issued; cc++)
+        mbar_wait_bounded(&full[cc % kStages], (uint32_t)(cc / kStages) & 1u);
+    return;
+  }
   const int g = lane % G, slot = lane / G;
   AT xr[RPG], xi[RPG];
-  init_ring(full);
   cplx<AT>* out = p + k0;
-  auto after_prefetch = [&]() -> bool {
-    grid_dep_wait();
-    grid_dep_launch();
-    if (__syncthreads_or(done && *(volatile const int*)done)) return false;
-#pragma unroll
-    for (int t = 0; t < RPG; t++) {
-      const int row = g + G * t;
-      const cplx<AT> v = row < R ? xm[ls + row] : cplx<AT>();
-      xr[t] = v.re;
-      xi[t] = v.im;
+  grid_dep_wait();
+  grid_dep_launch();
+  if (done) {  // the consumers' vote; the producer sees it when a stage is given back
+    if (*(volatile const int*)done) s_stop = 1;
+    uint32_t cph = 0;
+    if (!consumer_sync(&cbar, cph) || *(volatile int*)&s_stop) {
+      if (lane == 0) mbar_arrive(&empty[0]);
+      return;
     }
-    return true;
-  };
-  stream_leaf<MT>(stage, full, R, nullptr, 0, seg, K, V.err, after_prefetch,
-                  [&](const cplx<MT>* S, int, int c0, int ncols, int, int, int) {
-                    // two columns per lane in flight: j and j + STEP
-                    for (int jb = warp * CPW; jb < ncols; jb += 2 * STEP) {
-                      AT a[4];
+  }
 #pragma unroll
-                      for (int u = 0; u < 2; u++) {
-                        const int j = jb + slot + u * STEP;
-                        AT ar = 0, ai = 0;
-                        if (j < ncols) {
-                          const cplx<MT>* col = S + j * R;
+  for (int t = 0; t < RPG; t++) {
+    const int row = g + G * t;
+    const cplx<AT> v = row < R ? xm[ls + row] : cplx<AT>();
+    xr[t] = v.re;
+    xi[t] = v.im;
+  }
+  int st = 0;
+  uint32_t ph = 0;
+  for (int c0 = 0; c0 < K; c0 += cpc) {
+    const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&full[st], ph));
+    if (!got) {
+      if (lane == 0) atomicExch(V.err, 1);
+      break;
+    }
+    const cplx<MT>* S = (const cplx<MT>*)stage[st];
+    const int ncols = min(cpc, K - c0);
+    // two columns per lane in flight: j and j + STEP
+    for (int jb = warp * CPW; jb < ncols; jb += 2 * STEP) {
+      AT a[4];
 #pragma unroll
-                          for (int t = 0; t < RPG; t++) {
-                            const int row = g + G * t;
-                            if (row < R) acc_mac(ar, ai, col[row], xr[t], xi[t]);
-                          }
-                        }
-                        a[2 * u] = ar;
-                        a[2 * u + 1] = ai;
-                      }
+      for (int u = 0; u < 2; u++) {
+        const int j = jb + slot + u * STEP;
+        AT ar = 0, ai = 0;
+        if (j < ncols) {
+          const cplx<MT>* col = S + j * R;
 #pragma unroll
-                      for (int o = G / 2; o > 0; o >>= 1)
+          for (int t = 0; t < RPG; t++) {
+            const int row = g + G * t;
+            if (row < R) acc_mac(ar, ai, col[row], xr[t], xi[t]);
+          }
+        }
+        a[2 * u] = ar;
+        a[2 * u + 1] = ai;
+      }
+      const int j = jb + slot;
+      if constexpr (std::is_same<AT, float>::value) {
+        dot_fold<2, G / 2>(a);
+        dot_fold<1, G / 4>(a);
+        float v = a[0];
 #pragma unroll
-                        for (int u = 0; u < 4; u++) a[u] = acc_add(a[u], acc_shfl_xor(a[u], o));
-                      if (g == 0) {
-                        const int j = jb + slot;
-                        if (j < ncols) out[c0 + j] = cplx<AT>(a[0], a[1]);
-                        if (j + STEP < ncols) out[c0 + j + STEP] = cplx<AT>(a[2], a[3]);
-                      }
-                    }
-                  });
+        for (int o = G / 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        // the quarters of the column's lanes: Re, Im of column j, Re, Im of column j + STEP
+        const int jq = j + (g >= G / 2 ? STEP : 0);
+        if (g % (G / 4) == 0 && jq < ncols) reinterpret_cast<float*>(out + c0 + jq)[g / (G / 4) & 1] = v;
+      } else {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int u = 0; u < 4; u++) a[u] = acc_add(a[u], acc_shfl_xor(a[u], o));
+        if (g == 0) {
+          if (j < ncols) out[c0 + j] = cplx<AT>(a[0], a[1]);
+          if (j + STEP < ncols) out[c0 + j + STEP] = cplx<AT>(a[2], a[3]);
+        }
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[st]);
+    if (++st == kStages) {
+      st = 0;
+      ph ^= 1u;
+    }
+  }
 }
 
 // t[task] = sum over the leaf entries of the task's block of p[kpos[e] + q], in leaf order
@@ -290,16 +390,6 @@ constexpr int kLeafSlots = kStages + 1;      // leaves whose chunks can be in th
 struct StageMeta {
   int slot, ncols, first, last;  // slot < 0: no more leaves
 };
-
-// Barrier of the consumer warps only (the producer keeps streaming): every consumer thread arrives
-// on an mbarrier (release) and waits for the phase (acquire), with the bounded wait, so a failed
-// pipeline cannot leave threads blocked. Returns false if the phase did not complete.
-__device__ __forceinline__ bool consumer_sync(uint64_t* bar, uint32_t& phase) {
-  mbar_arrive(bar);
-  const bool ok = mbar_wait_bounded(bar, phase);
-  phase ^= 1u;
-  return ok;
-}
 
 template <typename MT, typename VT, typename AT, bool TRANS, int RPL>
 __global__ void __launch_bounds__(kGatherThreads, AC3D_GATHER_MIN_CTAS) seg_gather_persist_kernel(
@@ -761,7 +851,7 @@ static void mv_t(const DevPartition& DP, const DevHMat& H, bool tr, const void* 
     d.b_kptr = tr ? H.kseg_f.as<int>() : H.kseg_t.as<int>();
     d.order = tr ? H.order_rows.as<int>() : H.order_cols.as<int>();
     launch_k(pdl, seg_dot_kernel<MT, AT, RPL>, dim3(DP.nleaf, dot_parts(DP.nleaf, (tr ? H.useg : H.vseg).bytes)),
-             dim3(kThreads), kRingBytes, s, d,
+             dim3(kThreads + 32), kRingBytes, s, d,
              tr ? useg : vseg, xm, p, done);
     launch_reduce<AT>(DP, H, tr, p, t, done, s, pdl);
   }
