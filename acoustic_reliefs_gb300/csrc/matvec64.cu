@@ -242,8 +242,8 @@ void launch_matvec_f64(const DevPartition& DP, const DevHMat& H, bool tr, const 
                : DP.max_leaf <= 64 ? dot64_kernel<2>
                : DP.max_leaf <= 128 ? dot64_kernel<4>
                                     : dot64_kernel<8>;
-    int parts = 1;
-    while (parts < 32 && DP.nleaf * parts < 8 * sms) parts *= 2;
+    int parts = 1;  // a warp per 32 columns or so: 222 us a matvec against 229 with half of them (10620 triangles)
+    while (parts < 32 && DP.nleaf * parts < 16 * sms) parts *= 2;
     launch_k(pdl, dot, dim3(DP.nleaf, parts), dim3(kDotThreads), 0, s, d, tr ? useg : vseg, (const cd*)x, p, done);
     launch_reduce_f64(DP, H, tr, p, t, done, s, pdl);
   }
@@ -251,8 +251,14 @@ void launch_matvec_f64(const DevPartition& DP, const DevHMat& H, bool tr, const 
   v.b_kptr = (tr ? H.kseg_t : H.kseg_f).as<int>();
   v.b_idx = (tr ? H.vidx : H.uidx).as<int>();
   v.order = (tr ? H.order_cols : H.order_rows).as<int>();
+  // CTAs per leaf: up to two per SM always (128 leaves of 2720 triangles: 72 us a matvec with 1024 CTAs, 62 with
+  // 512), up to four while a CTA keeps 160 KB of the leaf (512 leaves of 10620 triangles: 238 us with
+  // 512 CTAs, 229 with 1024; 256 leaves of 5280: 109 us with 512, 114 with 1024, 156 with 256)
+  const size_t bytes = (tr ? H.nearT : H.near).bytes + (tr ? H.vseg : H.useg).bytes;
   unsigned parts = 1;
-  while (parts < 8 && DP.nleaf * (int)parts < 4 * sms) parts *= 2;
+  while (parts < 8 && (DP.nleaf * (int)parts < 2 * sms ||
+                       (DP.nleaf * (int)parts < 4 * sms && bytes / ((size_t)DP.nleaf * parts) >= 320 * 1024)))
+    parts *= 2;
   launch_clusters(pdl && DP.na > 0, parts, gather64_kernel, dim3(DP.nleaf * parts), dim3(kGatherThreads), s, v,
                   DP.nleaf, (tr ? H.nearT : H.near).as<cd>(), tr ? vseg : useg, t, (const cd*)x, (cd*)y,
                   (const cd*)bminus, (const cd*)ep.dot_a, (const cd*)ep.dot_b, ep.partials, ep.red5,
