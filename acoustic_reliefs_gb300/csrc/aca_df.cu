@@ -376,7 +376,7 @@ static_assert(sizeof(AcaGroup<1>) % 16 == 0 && sizeof(AcaGroup<2>) % 16 == 0 && 
 // of the lanes idle (20480 triangles: c = 20). Each entry is then finished by its owner. Sums are
 // taken in one order whatever W: rows and columns l, l + 32, ... by lane l, then the butterfly.
 //
-// Bound by the FP32 pipe (45-50% busy) and, beside it, by instruction supply and latency: the warps
+// Bound by the FP32 pipe (55% busy) and, beside it, by instruction supply and latency: the warps
 // are at different places of a long recursion. Four CTAs of 128 threads per SM (128 registers)
 // beat six (80 registers, spills) 4.9 to 6.2 ms on the 20480-triangle relief: more warps thrash L1 and
 // the instruction caches. With the 8-warp blocks' kernel the assembly takes 8.8 instead of 11.0 ms

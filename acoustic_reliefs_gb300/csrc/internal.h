@@ -211,7 +211,7 @@ struct DevHMat {
   double k = 0;
   int maxk = 100;
   DevBuf near;            // complex storage of all near blocks
-  DevBuf nearT;           // transposed near field (FP32; built on the first transposed block matvec)
+  DevBuf nearT;           // transposed near field (built before the first transposed matvec)
   DevBuf tcseg_f, tcseg_t;  // TF32 hi / lo split of the U / V segments (tensor-core block dot pass)
   DevBuf tcoff_f, tcoff_t;  // int64 [nleaf + 1]: byte offsets into tcseg_f / tcseg_t
   DevBuf pool;            // rank-1 terms (u | v) of all admissible blocks
