@@ -276,4 +276,32 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+// Sums of five values over the warp into dst[0..4], each with the bits of warp_sum: folded, so that they
+// take 9 additions on the FP64 pipe (64 clocks each) instead of 25. any = false (the same for the
+// warp): every lane's values are zero.
+template <int N, int O>
+__device__ __forceinline__ void fold_pairs(double* v) {
+  const bool up = (threadIdx.x & O) != 0;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const double keep = up ? v[k + N] : v[k], give = up ? v[k] : v[k + N];
+    v[k] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+  }
+}
+__device__ __forceinline__ void warp_sum5(const double* d, double* dst, bool any) {
+  const int lane = threadIdx.x & 31;
+  if (!any) {
+    if (lane < 5) dst[lane] = 0.0;
+    return;
+  }
+  double v[8] = {d[0], d[1], d[2], d[3], d[4], 0.0, 0.0, 0.0};
+  fold_pairs<4, 16>(v);
+  fold_pairs<2, 8>(v);
+  fold_pairs<1, 4>(v);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  const int k = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+  if ((lane & 3) == 0 && k < 5) dst[k] = v[0];
+}
+
 }  // namespace ac3d

@@ -182,10 +182,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3) gather64_kernel(
       d[4] = yr * yr + yi * yi;
     }
     if (partials) {
-      for (int i = 0; i < 5; i++) {
-        d[i] = warp_sum(d[i]);
-        if (lane == 0) sdot[warp][i] = d[i];
-      }
+      warp_sum5(d, sdot[warp], 32 * warp < R);
       __syncthreads();
       if (tid < 5) {
         double sum = 0;
@@ -206,9 +203,7 @@ __global__ void __launch_bounds__(kGatherThreads, 3) gather64_kernel(
       double acc[5] = {0, 0, 0, 0, 0};
       for (int l = tid; l < nleaf; l += kGatherThreads)
         for (int i = 0; i < 5; i++) acc[i] += __ldcg(&partials[(size_t)l * 5 + i]);
-      for (int i = 0; i < 5; i++) acc[i] = warp_sum(acc[i]);
-      if (lane == 0)
-        for (int i = 0; i < 5; i++) sdot[warp][i] = acc[i];
+      warp_sum5(acc, sdot[warp], 32 * warp < nleaf);
       __syncthreads();
       if (tid < 5) {
         double sum = 0;
