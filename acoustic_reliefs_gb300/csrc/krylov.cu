@@ -20,9 +20,10 @@ constexpr int kVecWarps = kVecThreads / 32;
 }  // namespace
 
 // What bounds the vector kernels on small meshes is FP64 latency (an instruction takes 64 clocks, a
-// division some 15 of them): sums are folded, each total is formed by one thread, the divisions of a
-// complex quotient run side by side on lanes, and the vectors are loaded under the scalars. 1280 triangles:
-// kf_p 8.0 -> 4.0, kf_s 4.5 -> 3.5, kf_xr 12.3 -> 7.7 us of a 64 us iteration.
+// division some 15 of them): sums are folded, each total is formed by one thread and omega's two
+// divisions run on two lanes. 1280 triangles: kf_xr 12.3 -> 7.9 us of a 64 us iteration. The complex
+// quotients stay with one thread and the loads behind them: in other shapes of the code the compiler
+// contracts their products otherwise, and a mixed solve then ends on another iterate.
 __device__ __forceinline__ void write_partials(double* d, double* partials) {
   __shared__ double sd[kVecWarps][5];
   warp_sum5(d, sd[threadIdx.x >> 5], true);
@@ -94,20 +95,22 @@ __global__ void k_scalar_init(KState* st, const double* partials, int n, double 
   }
 }
 
-// (ar + i ai) / (br + i bi) by one warp, a quotient per four lanes (lanes 4 q .. 4 q + 3 pass the same
-// operands); cr and ci are valid in every lane of the four
 __device__ __forceinline__ void cdivd(double ar, double ai, double br, double bi, double& cr, double& ci) {
-  const int lane = threadIdx.x & 31, j = lane & 3, q = lane & ~3;
-  const double s = fabs(br) + fabs(bi);
-  const double t = (j == 0 ? br : j == 1 ? bi : j == 2 ? ar : ai) / s;
-  const double xr = __shfl_sync(0xffffffffu, t, q), xi = __shfl_sync(0xffffffffu, t, q + 1);
-  const double yr = __shfl_sync(0xffffffffu, t, q + 2), yi = __shfl_sync(0xffffffffu, t, q + 3);
-  const double d = xr * xr + xi * xi;
-  const double nr = yr * xr + yi * xi, ni = yi * xr - yr * xi;
-  const double c = (j & 1 ? ni : nr) / d;
-  cr = __shfl_sync(0xffffffffu, c, q);
-  ci = __shfl_sync(0xffffffffu, c, q + 1);
+  double s = fabs(br) + fabs(bi);
+  double xr = br / s, xi = bi / s, yr = ar / s, yi = ai / s;
+  double d = xr * xr + xi * xi;
+  cr = (yr * xr + yi * xi) / d;
+  ci = (yi * xr - yr * xi) / d;
 }
+
+
+
+
+
+
+
+
+
 
 // ------------------------------------------------------------------------------------------
 // Fused iteration: every CTA of a vector kernel reduces the partials itself (same order, same
@@ -121,7 +124,6 @@ struct RhoStep {
   int done;
 };
 
-// by one warp, the same in every lane
 __device__ __forceinline__ RhoStep rho_step(const KState* st, const double* s) {
   RhoStep o{};
   o.rr = s[4];
@@ -144,12 +146,9 @@ __device__ __forceinline__ RhoStep rho_step(const KState* st, const double* s) {
     o.rho_im = 0.0;
     return o;
   }
-  const bool second = (threadIdx.x & 4) != 0;
-  double qr, qi;
-  cdivd(second ? st->alpha_re : o.rho_re, second ? st->alpha_im : o.rho_im, second ? st->omega_re : st->rho_re,
-        second ? st->omega_im : st->rho_im, qr, qi);
-  const double q1r = __shfl_sync(0xffffffffu, qr, 0), q1i = __shfl_sync(0xffffffffu, qi, 0);
-  const double q2r = __shfl_sync(0xffffffffu, qr, 4), q2i = __shfl_sync(0xffffffffu, qi, 4);
+  double q1r, q1i, q2r, q2i;
+  cdivd(o.rho_re, o.rho_im, st->rho_re, st->rho_im, q1r, q1i);
+  cdivd(st->alpha_re, st->alpha_im, st->omega_re, st->omega_im, q2r, q2i);
   o.beta_re = q1r * q2r - q1i * q2i;
   o.beta_im = q1r * q2i + q1i * q2r;
   return o;
@@ -165,19 +164,7 @@ __global__ void __launch_bounds__(kVecThreads) kf_p(KState* st, const double* pa
   if (st->done) return;
   // the scalars once per CTA (FP64 division is slow): every CTA gets the same values
   __shared__ RhoStep so;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  cplx<VT> ri, pi, vi;
-  auto load = [&]() {
-    if (i >= n) return;
-    ri = r[i];
-    pi = p[i];
-    vi = v[i];
-  };
-  load();
-  if (threadIdx.x < 32) {
-    const RhoStep w = rho_step(st, st->rsum);
-    if (threadIdx.x == 0) so = w;
-  }
+  if (threadIdx.x == 0) so = rho_step(st, st->rsum);
   __syncthreads();
   const RhoStep o = so;
   (void)partials;
@@ -191,13 +178,15 @@ __global__ void __launch_bounds__(kVecThreads) kf_p(KState* st, const double* pa
   }
   const VT br = (VT)o.beta_re, bi = (VT)o.beta_im;
   const VT wr = (VT)(o.restart ? 1.0 : st->omega_re), wi = (VT)(o.restart ? 0.0 : st->omega_im);
-  for (; i < n; i += gridDim.x * blockDim.x, load()) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const cplx<VT> ri = r[i];
     cplx<VT> pn;
     if (o.restart) {
       rhat[i] = ri;
       pn = ri;
       v[i] = cplx<VT>();
     } else {
+      const cplx<VT> pi = p[i], vi = v[i];
       const VT tr = pi.re - (wr * vi.re - wi * vi.im);
       const VT ti = pi.im - (wr * vi.im + wi * vi.re);
       pn = cplx<VT>(ri.re + br * tr - bi * ti, ri.im + br * ti + bi * tr);
@@ -223,24 +212,10 @@ __global__ void __launch_bounds__(kVecThreads) kf_s(KState* st, const double* re
   grid_dep_launch();
   if (st->done) return;
   __shared__ double sa[3];
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  cplx<VT> ri, vi;
-  auto load = [&]() {
-    if (i >= n) return;
-    ri = r[i];
-    vi = v[i];
-  };
-  load();
-  if (threadIdx.x < 32) {
+  if (threadIdx.x == 0) {
     const double d0 = red5[0], d1 = red5[1];
-    const bool zero = d0 == 0.0 && d1 == 0.0;
-    double cr = 0, ci = 0;
-    if (!zero) cdivd(st->rho_new_re, st->rho_new_im, d0, d1, cr, ci);
-    if (threadIdx.x == 0) {
-      sa[0] = cr;
-      sa[1] = ci;
-      sa[2] = zero ? 1.0 : 0.0;
-    }
+    sa[2] = (d0 == 0.0 && d1 == 0.0) ? 1.0 : 0.0;
+    if (sa[2] == 0.0) cdivd(st->rho_new_re, st->rho_new_im, d0, d1, sa[0], sa[1]);
   }
   __syncthreads();
   if (sa[2] != 0.0) {
@@ -249,7 +224,8 @@ __global__ void __launch_bounds__(kVecThreads) kf_s(KState* st, const double* re
   }
   const double ar = sa[0], ai = sa[1];
   const VT a_r = (VT)ar, a_i = (VT)ai;
-  for (; i < n; i += gridDim.x * blockDim.x, load()) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const cplx<VT> ri = r[i], vi = v[i];
     const cplx<VT> si(ri.re - (a_r * vi.re - a_i * vi.im), ri.im - (a_r * vi.im + a_i * vi.re));
     s[i] = si;
     if (s32) s32[i] = cf((float)si.re, (float)si.im);
@@ -271,17 +247,6 @@ __global__ void __launch_bounds__(kVecThreads) kf_xr(KState* st, const double* r
   if (st->done) return;
   __shared__ double sw[2];
   __shared__ bool s_last;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  cplx<VT> pi, si, ti, hi, xi;
-  auto load = [&]() {
-    if (i >= n) return;
-    pi = p[i];
-    si = s[i];
-    ti = t[i];
-    hi = rhat[i];
-    xi = x[i];
-  };
-  load();
   if (threadIdx.x < 2) {
     const double d4 = red5[4];
     sw[threadIdx.x] = d4 > 0.0 ? red5[2 + threadIdx.x] / d4 : 0.0;
@@ -291,7 +256,9 @@ __global__ void __launch_bounds__(kVecThreads) kf_xr(KState* st, const double* r
   const double ar_d = st->alpha_new_re, ai_d = st->alpha_new_im;
   const VT ar = (VT)ar_d, ai = (VT)ai_d, wr = (VT)wr_d, wi = (VT)wi_d;
   double d[5] = {0, 0, 0, 0, 0};
-  for (; i < n; i += gridDim.x * blockDim.x, load()) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const cplx<VT> pi = p[i], si = s[i], ti = t[i], hi = rhat[i];
+    cplx<VT> xi = x[i];
     xi.re += (ar * pi.re - ai * pi.im) + (wr * si.re - wi * si.im);
     xi.im += (ar * pi.im + ai * pi.re) + (wr * si.im + wi * si.re);
     x[i] = xi;
