@@ -31,6 +31,7 @@ struct AcaF64Args {
   const int* order;
   double k, eps, eps2;            // eps^2, -1 for eps < 0
   int maxk, zero_guard, iter_cap;
+  int wide;                       // every block in the order of the wide ones (below)
   int chunk;                      // entries evaluated at a time: T, or what shared memory leaves room for
   cd* pool;
   long long pool_cap;
@@ -97,7 +98,7 @@ __device__ __noinline__ void f64_items(double k, const double4* __restrict__ pts
 
 // Entry e from its items, less the earlier terms, four loads in flight.
 __device__ __forceinline__ cd f64_finish(const F64Item* items, int e, const cd* coef, const long long* toff,
-                                         const cd* pool, int nst) {
+                                         const cd* pool, int nst, bool swap = false) {
   double re = 0, im = 0;
 #pragma unroll 1
   for (int it = 6 * e; it < 6 * e + 6; it++) {
@@ -114,7 +115,7 @@ __device__ __forceinline__ cd f64_finish(const F64Item* items, int e, const cd* 
     for (int u = 0; u < 4; u++) a[u] = pool[toff[min(p + u, nst - 1)]];
 #pragma unroll
     for (int u = 0; u < 4; u++)
-      if (p + u < nst) cfms(acc, coef[p + u], a[u]);
+      if (p + u < nst) cfms(acc, swap ? a[u] : coef[p + u], swap ? coef[p + u] : a[u]);
   }
   return acc;
 }
@@ -161,6 +162,9 @@ __global__ void __launch_bounds__(T) aca_f64_kernel(AcaF64Args A) {
   const int4 q = A.blocks[b];
   const int rs = q.x, cs = q.z, m = q.y - q.x, n = q.w - q.z;
   const int iter_lim = max(0, min(min(A.maxk, A.iter_cap), min(m - 1, n - 1)));
+  // column residuals of wide blocks multiply term by coefficient, those of the others coefficient by term: the
+  // order of the two products in the imaginary part, and so the last bits, as assemble.cu has them
+  const bool wide = A.wide || m > kWarpAcaMaxDim || n > kWarpAcaMaxDim;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   // exactly-zero block: all panels in one axis-aligned plane that holds every target point (see aca_kernel)
@@ -250,7 +254,7 @@ __global__ void __launch_bounds__(T) aca_f64_kernel(AcaF64Args A) {
       __syncthreads();
       const int r = r0 + tid;
       if (tid < C && r < m) {
-        const cd u = f64_finish(items, tid, coef, toff, A.pool + r, nst);
+        const cd u = f64_finish(items, tid, coef, toff, A.pool + r, nst, wide);
         unew[r] = u;
         un += abs2(u);
       }
@@ -358,7 +362,7 @@ void launch_aca_f64(const DevGeometry& G, const DevPartition& DP, DevHMat& H, do
                     cudaStream_t s_small) {
   if (DP.na == 0) return;
   AcaF64Args a{G.va.as<double4>(), G.eg64.as<ElemGeo<double>>(), G.cen.as<double4>(), G.cen.as<double4>(),
-               DP.blocks_a.as<int4>(), nullptr, H.k, eps, eps < 0 ? -1.0 : eps * eps, H.maxk, 1, H.maxk, 0, H.pool.as<cd>(), H.pool_cap,
+               DP.blocks_a.as<int4>(), nullptr, H.k, eps, eps < 0 ? -1.0 : eps * eps, H.maxk, 1, H.maxk, H.maxk > kWarpAcaTerms, 0, H.pool.as<cd>(), H.pool_cap,
                H.pool_used.as<unsigned long long>(), H.term_off.as<long long>(), H.rank.as<int>(),
                (int*)(H.pool_used.as<unsigned long long>() + 1), H.passes.as<int>()};
   // aca_order: blocks above 256, then up to 256, 128 and 64
@@ -373,7 +377,7 @@ void launch_listener_aca_f64(const DevGeometry& G, const double4* pts, int L, do
                              const int4* block, const int* order, cudaStream_t s) {
   const int iter_lim = std::max(1, std::min(maxk, std::min(L - 1, G.ne - 1)));
   AcaF64Args a{G.va.as<double4>(), G.eg64.as<ElemGeo<double>>(), G.cen.as<double4>(), pts, block, nullptr, k,
-               eps, eps < 0 ? -1.0 : eps * eps, maxk, 0, iter_lim, 0, pool, pool_cap, used, term_off, rank, status, nullptr};
+               eps, eps < 0 ? -1.0 : eps * eps, maxk, 0, iter_lim, 1, 0, pool, pool_cap, used, term_off, rank, status, nullptr};
   aca_f64_launch<256>(a, order, 1, L, s);
 }
 

@@ -35,13 +35,18 @@ __device__ __forceinline__ void mac64(double& re, double& im, const cd& a, const
   im = fma(a.im, z.re, im);
 }
 
+// Sums have the order of the FP32 kernels' layout (G0 lanes per column in the dot pass; warps and
+// column slots in the gather), so that a solve ends on the same iterate whatever the layout.
+
 // p[kptr[leaf] + k] = sum over the leaf's rows of S[k][row] x[row]. G lanes per column (1 up to 32
 // rows, so that a lane has at most 32), gridDim.y CTAs per leaf, whose warps take 32 / G columns in turn.
-template <int G>
+// Rows g, g + G0, ... are summed apart for every g, then pairs G0 / 2 apart, G0 / 4, ...
+template <int G, int G0>
 __global__ void __launch_bounds__(kDotThreads, 6) dot64_kernel(SegView V, const cd* __restrict__ lrseg,
                                                                const cd* __restrict__ x, cd* __restrict__ p,
                                                                const int* __restrict__ done) {
-  __shared__ cd xs[kMaxRows];
+  __shared__ __align__(16) unsigned char xraw[kMaxRows * sizeof(cd)];
+  cd* xs = reinterpret_cast<cd*>(xraw);
   const int leaf = V.order[blockIdx.x];
   const int ls = V.leaf_start[leaf], R = V.leaf_start[leaf + 1] - ls;
   const int k0 = V.b_kptr[leaf], K = V.b_kptr[leaf + 1] - k0;
@@ -52,28 +57,32 @@ __global__ void __launch_bounds__(kDotThreads, 6) dot64_kernel(SegView V, const 
   if (__syncthreads_or(skip)) return;
   const int lane = threadIdx.x & 31, g = lane % G;
   const cd* seg = lrseg + V.b_seg[leaf];
-  constexpr int CW = 32 / G, U = 4;
+  constexpr int CW = 32 / G, NA = G0 / G;
   const int warp = blockIdx.y * (kDotThreads / 32) + (threadIdx.x >> 5), nw = gridDim.y * (kDotThreads / 32);
   for (int c0 = warp * CW; c0 < K; c0 += nw * CW) {
     const int c = c0 + lane / G;
     const cd* col = seg + (long long)min(c, K - 1) * R;
-    double re[2] = {0, 0}, im[2] = {0, 0};
-    cd a[U];
+    double re[NA], im[NA];
 #pragma unroll
-    for (int u = 0; u < U; u++) a[u] = col[min(g + u * G, R - 1)];
-    for (int r0 = g; r0 < R; r0 += U * G) {
-      cd b[U];
+    for (int u = 0; u < NA; u++) re[u] = im[u] = 0;
+    for (int r0 = g; r0 < R; r0 += G0) {
+      cd a[NA];
 #pragma unroll
-      for (int u = 0; u < U; u++) b[u] = col[min(r0 + (U + u) * G, R - 1)];
+      for (int u = 0; u < NA; u++) a[u] = col[min(r0 + u * G, R - 1)];
 #pragma unroll
-      for (int u = 0; u < U; u++)
-        if (r0 + u * G < R) mac64(re[u & 1], im[u & 1], a[u], xs[r0 + u * G]);
-#pragma unroll
-      for (int u = 0; u < U; u++) a[u] = b[u];
+      for (int u = 0; u < NA; u++)
+        if (r0 + u * G < R) mac64(re[u], im[u], a[u], xs[r0 + u * G]);
     }
-    double sr = re[0] + re[1], si = im[0] + im[1];
 #pragma unroll
-    for (int o = 1; o < G; o <<= 1) {
+    for (int h = NA / 2; h > 0; h >>= 1)
+#pragma unroll
+      for (int u = 0; u < h; u++) {
+        re[u] += re[u + h];
+        im[u] += im[u + h];
+      }
+    double sr = re[0], si = im[0];
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
       sr += __shfl_xor_sync(0xffffffffu, sr, o);
       si += __shfl_xor_sync(0xffffffffu, si, o);
     }
@@ -81,83 +90,100 @@ __global__ void __launch_bounds__(kDotThreads, 6) dot64_kernel(SegView V, const 
   }
 }
 
-// Thread (group g, row r) of a segment's columns g, g + G, ... of steps [s0, s1)
-__device__ __forceinline__ void gather_steps(double& re, double& im, const cd* __restrict__ seg, int K,
-                                             const int* __restrict__ idx, const cd* __restrict__ z, int R, int G,
-                                             int g, int tid, int s0, int s1) {
+// Thread (class k of NC, row r): the columns k, k + NC, ... of every chunk of cpc columns
+template <int NC>
+__device__ __forceinline__ void gather_class(double& re, double& im, const cd* __restrict__ seg, int K,
+                                             const int* __restrict__ idx, const cd* __restrict__ z, int R, int cpc,
+                                             int k, int r) {
   constexpr int U = 4;
-  for (int s = s0; s < s1; s += U) {
+  int c0 = 0, j = k;
+  auto next = [&]() {
+    while (c0 < K && j >= min(cpc, K - c0)) {
+      c0 += cpc;
+      j = k;
+    }
+    const int c = c0 < K ? c0 + j : -1;
+    j += NC;
+    return c;
+  };
+  for (int c = next(); c >= 0;) {
+    int cc[U], jx[U];
     cd a[U], v[U];
-    int j[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const int c = min((s + u) * G + g, K - 1);
-      j[u] = max(idx[c], 0);  // padding columns are zero and take any multiplier
-      a[u] = seg[(long long)c * R + tid];
+      cc[u] = c;
+      if (c >= 0) c = next();
     }
 #pragma unroll
-    for (int u = 0; u < U; u++) v[u] = z[j[u]];
+    for (int u = 0; u < U; u++) {
+      jx[u] = max(idx[max(cc[u], 0)], 0);  // padding columns are zero and take any multiplier
+      a[u] = seg[(long long)max(cc[u], 0) * R + r];
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) v[u] = z[jx[u]];
 #pragma unroll
     for (int u = 0; u < U; u++)
-      if (s + u < s1 && (s + u) * G + g < K) mac64(re, im, a[u], v[u]);
+      if (cc[u] >= 0) mac64(re, im, a[u], v[u]);
   }
 }
 
 // y[leaf rows] = -x/2 + S_A x[a_idx] + S_B t[b_idx], or b - that, with the optional dot partials of
-// seg_gather_persist_kernel. A cluster of CTAs per leaf shares its columns; the first one adds their row sums in
-// order and finishes the leaf. The near part runs before the wait for the reduce pass.
+// seg_gather_persist_kernel. The NC column classes are that kernel's (warp, slot) pairs: a cluster of S CTAs
+// holds them all, NC / S each with a thread per row. Every CTA adds its warps' slots, the first one the warps in
+// order, and finishes the leaf. The near part runs before the wait for the reduce pass.
+template <int NC, int S>
 __global__ void __launch_bounds__(kGatherThreads, 3) gather64_kernel(
     SegView V, int nleaf, const cd* __restrict__ near, const cd* __restrict__ lrseg, const cd* __restrict__ t,
     const cd* __restrict__ x, cd* __restrict__ y, const cd* __restrict__ bminus, const cd* __restrict__ dot_a,
     const cd* __restrict__ dot_b, double* partials, double* red5, unsigned* ticket, const int* __restrict__ done) {
-  constexpr int W = kGatherThreads / 32;
-  __shared__ cd part[kGatherThreads];
-  __shared__ cd rows[kMaxRows];
+  constexpr int W = 8, GP = NC / S, SL = NC / W, LW = GP / SL;  // slots per warp, warps per CTA
+  static_assert(GP % SL == 0 && LW * S == W, "a CTA holds whole warps");
+  __shared__ __align__(16) unsigned char praw[kGatherThreads * sizeof(cd)];
+  __shared__ __align__(16) unsigned char rraw[LW * kGatherThreads / GP * sizeof(cd)];
+  cd* part = reinterpret_cast<cd*>(praw);
+  cd* rows = reinterpret_cast<cd*>(rraw);
   __shared__ double sdot[W][5];
   __shared__ bool s_last;
   __shared__ int s_skip;
   grid_dep_launch();
   const cg::cluster_group cl = cg::this_cluster();
-  const int S = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int rank = (int)cl.block_rank();
   const int leaf = V.order[blockIdx.x / S];
   const int ls = V.leaf_start[leaf], R = V.leaf_start[leaf + 1] - ls;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5;
   // the flag may be set while this kernel runs: a thread that sees it skips its sums, but not the barriers,
   // and its cluster writes nothing
   const bool skip = done && *(volatile const int*)done;
-  const int G = kGatherThreads / R, g = tid / R, r = tid - g * R;
+  // two warps per CTA are one from either end: the first classes of a chunk have a column more
+  const int g = tid / R, r = tid - g * R, k = (g < SL ? rank : W - 1 - rank) * SL + g % SL;
+  const int cpc = min(128, max(2, (int)(kStageBytes / sizeof(cd)) / R & ~1));  // columns per chunk of its ring
   double re = 0, im = 0;
-  const int ak = V.a_kptr[leaf], ac = V.a_kptr[leaf + 1] - ak, na = (ac + G - 1) / G;
-  if (!skip && g < G && ac > 0)
-    gather_steps(re, im, near + V.a_seg[leaf], ac, V.a_idx + ak, x, R, G, g, r, na * rank / S,
-                 na * (rank + 1) / S);
-  const int bk = V.b_kptr[leaf], bc = V.b_kptr[leaf + 1] - bk, nb = (bc + G - 1) / G;
+  const int ak = V.a_kptr[leaf], ac = V.a_kptr[leaf + 1] - ak;
+  if (!skip && g < GP) gather_class<NC>(re, im, near + V.a_seg[leaf], ac, V.a_idx + ak, x, R, cpc, k, r);
+  const int bk = V.b_kptr[leaf], bc = V.b_kptr[leaf + 1] - bk;
   grid_dep_wait();
-  if (!skip && g < G && bc > 0)
-    gather_steps(re, im, lrseg + V.b_seg[leaf], bc, V.b_idx + bk, t, R, G, g, r, (int)((long long)nb * rank / S),
-                 (int)((long long)nb * (rank + 1) / S));
-  part[tid] = cd(re, im);
+  if (!skip && g < GP) gather_class<NC>(re, im, lrseg + V.b_seg[leaf], bc, V.b_idx + bk, t, R, cpc, k, r);
+  if (g < GP) part[tid] = cd(re, im);
   bool any = __syncthreads_or(skip);
   if (tid == 0) s_skip = any;
-  if (tid < R) {
-    double sr = part[tid].re, si = part[tid].im;
-    for (int i = 1; i < G; i++) {
-      sr += part[i * R + tid].re;
-      si += part[i * R + tid].im;
-    }
-    rows[tid] = cd(sr, si);
+  if (tid < LW * R) {
+    const cd* q = part + (size_t)(tid / R) * SL * R + tid % R;
+    cd v = q[0];
+    if constexpr (SL == 2) v = cd(v.re + q[R].re, v.im + q[R].im);
+    if constexpr (SL == 4)
+      v = cd((v.re + q[R].re) + (q[2 * R].re + q[3 * R].re), (v.im + q[R].im) + (q[2 * R].im + q[3 * R].im));
+    rows[tid] = v;
   }
-  if (S > 1) {
-    cl.sync();
-    if (rank == 0)
-      for (int i = 1; i < S; i++) any |= *cl.map_shared_rank(&s_skip, i) != 0;
-  }
+  cl.sync();
+  if (rank == 0)
+    for (int i = 1; i < S; i++) any |= *cl.map_shared_rank(&s_skip, i) != 0;
   if (rank == 0 && !any) {
     double d[5] = {0, 0, 0, 0, 0};
     if (tid < R) {
-      double sr = rows[tid].re, si = rows[tid].im;
-      for (int i = 1; i < S; i++) {
-        const cd v = cl.map_shared_rank(rows, i)[tid];
+      double sr = 0, si = 0;
+      for (int i = 0; i < W; i++) {
+        const bool own = LW == 1 || i < S;
+        const cd v = cl.map_shared_rank(rows, own ? i : W - 1 - i)[(own ? 0 : R) + tid];
         sr += v.re;
         si += v.im;
       }
@@ -171,27 +197,27 @@ __global__ void __launch_bounds__(kGatherThreads, 3) gather64_kernel(
       y[ls + tid] = cd(yr, yi);
       if (dot_a) {
         const cd a = dot_a[ls + tid];
-        d[0] = a.re * yr + a.im * yi;
-        d[1] = a.re * yi - a.im * yr;
+        d[0] += a.re * yr + a.im * yi;
+        d[1] += a.re * yi - a.im * yr;
       }
       if (dot_b) {
         const cd b = dot_b[ls + tid];
-        d[2] = yr * b.re + yi * b.im;
-        d[3] = yr * b.im - yi * b.re;
+        d[2] += yr * b.re + yi * b.im;
+        d[3] += yr * b.im - yi * b.re;
       }
-      d[4] = yr * yr + yi * yi;
+      d[4] += yr * yr + yi * yi;
     }
     if (partials) {
       warp_sum5(d, sdot[warp], 32 * warp < R);
       __syncthreads();
       if (tid < 5) {
         double sum = 0;
-        for (int w = 0; w < W; w++) sum += sdot[w][tid];
+        for (int w = 0; w < (int)blockDim.x / 32; w++) sum += sdot[w][tid];  // (warps from R / 32 on add 0)
         partials[(size_t)leaf * 5 + tid] = sum;
       }
     }
   }
-  if (S > 1) cl.sync();  // the row sums stay until they are read
+  cl.sync();  // the row sums stay until they are read
   if (rank == 0 && !any && partials && red5) {
     // the last leaf to finish reduces all partials in fixed order
     __threadfence();
@@ -200,10 +226,12 @@ __global__ void __launch_bounds__(kGatherThreads, 3) gather64_kernel(
     __syncthreads();
     if (s_last) {
       __threadfence();
-      double acc[5] = {0, 0, 0, 0, 0};
-      for (int l = tid; l < nleaf; l += kGatherThreads)
-        for (int i = 0; i < 5; i++) acc[i] += __ldcg(&partials[(size_t)l * 5 + i]);
-      warp_sum5(acc, sdot[warp], 32 * warp < nleaf);
+      for (int vt = tid; vt < 256; vt += blockDim.x) {  // in the order of 256 threads
+        double acc[5] = {0, 0, 0, 0, 0};
+        for (int l = vt; l < nleaf; l += 256)
+          for (int i = 0; i < 5; i++) acc[i] += __ldcg(&partials[(size_t)l * 5 + i]);
+        warp_sum5(acc, sdot[vt >> 5], (vt & ~31) < nleaf);
+      }
       __syncthreads();
       if (tid < 5) {
         double sum = 0;
@@ -233,10 +261,10 @@ void launch_matvec_f64(const DevPartition& DP, const DevHMat& H, bool tr, const 
     d.b_seg = (tr ? H.seg_f : H.seg_t).as<long long>();
     d.b_kptr = (tr ? H.kseg_f : H.kseg_t).as<int>();
     d.order = (tr ? H.order_rows : H.order_cols).as<int>();
-    auto dot = DP.max_leaf <= 32 ? dot64_kernel<1>
-               : DP.max_leaf <= 64 ? dot64_kernel<2>
-               : DP.max_leaf <= 128 ? dot64_kernel<4>
-                                    : dot64_kernel<8>;
+    auto dot = DP.max_leaf <= 32 ? dot64_kernel<1, 8>
+               : DP.max_leaf <= 64 ? dot64_kernel<2, 8>
+               : DP.max_leaf <= 128 ? dot64_kernel<4, 16>
+                                    : dot64_kernel<8, 32>;
     int parts = 1;  // a warp per 32 columns or so: 222 us a matvec against 229 with half of them (10620 triangles)
     while (parts < 32 && DP.nleaf * parts < 16 * sms) parts *= 2;
     launch_k(pdl, dot, dim3(DP.nleaf, parts), dim3(kDotThreads), 0, s, d, tr ? useg : vseg, (const cd*)x, p, done);
@@ -246,18 +274,20 @@ void launch_matvec_f64(const DevPartition& DP, const DevHMat& H, bool tr, const 
   v.b_kptr = (tr ? H.kseg_t : H.kseg_f).as<int>();
   v.b_idx = (tr ? H.vidx : H.uidx).as<int>();
   v.order = (tr ? H.order_cols : H.order_rows).as<int>();
-  // CTAs per leaf: up to two per SM always (128 leaves of 2720 triangles: 72 us a matvec with 1024 CTAs, 62 with
-  // 512), up to four while a CTA keeps 160 KB of the leaf (512 leaves of 10620 triangles: 238 us with
-  // 512 CTAs, 229 with 1024; 256 leaves of 5280: 109 us with 512, 114 with 1024, 156 with 256)
-  const size_t bytes = (tr ? H.nearT : H.near).bytes + (tr ? H.vseg : H.useg).bytes;
-  unsigned parts = 1;
-  while (parts < 8 && (DP.nleaf * (int)parts < 2 * sms ||
-                       (DP.nleaf * (int)parts < 4 * sms && bytes / ((size_t)DP.nleaf * parts) >= 320 * 1024)))
-    parts *= 2;
-  launch_clusters(pdl && DP.na > 0, parts, gather64_kernel, dim3(DP.nleaf * parts), dim3(kGatherThreads), s, v,
-                  DP.nleaf, (tr ? H.nearT : H.near).as<cd>(), tr ? vseg : useg, t, (const cd*)x, (cd*)y,
-                  (const cd*)bminus, (const cd*)ep.dot_a, (const cd*)ep.dot_b, ep.partials, ep.red5,
-                  H.ticket.as<unsigned>(), done);
+  auto gather = [&](auto kern, int classes, int ctas) {
+    const int threads = (classes / ctas * DP.max_leaf + 31) / 32 * 32;
+    launch_clusters(pdl && DP.na > 0, (unsigned)ctas, kern, dim3(DP.nleaf * ctas), dim3(threads), s, v, DP.nleaf,
+                    (tr ? H.nearT : H.near).as<cd>(), tr ? vseg : useg, t, (const cd*)x, (cd*)y, (const cd*)bminus,
+                    (const cd*)ep.dot_a, (const cd*)ep.dot_b, ep.partials, ep.red5, H.ticket.as<unsigned>(), done);
+  };
+  if (DP.max_leaf <= 32)
+    gather(gather64_kernel<32, 4>, 32, 4);
+  else if (DP.max_leaf <= 64)
+    gather(gather64_kernel<32, 8>, 32, 8);
+  else if (DP.max_leaf <= 128)
+    gather(gather64_kernel<16, 8>, 16, 8);
+  else
+    gather(gather64_kernel<8, 8>, 8, 8);
 }
 
 }  // namespace ac3d
