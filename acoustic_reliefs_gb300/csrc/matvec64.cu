@@ -2,14 +2,14 @@
 //
 // Bound by the FP64 pipe, not by memory: GB300 runs two FP64 lanes per clock and SM, so an element (four
 // multiply-adds, 16 bytes) takes 3 times as long to compute as to read, a warp instruction holds a
-// scheduler's pipe for 64 clocks, and lanes without an element cost as much as those with one. Leaves hold 16 to 32
-// elements (or their doubles), so lanes laid along a column's rows were a third empty and added
-// up over shuffles. Here the dot pass gives a lane a whole column (up to 32 rows of it), and the gather
-// pass gives a thread a row and every G-th column, G = 256 / R groups, which reads a segment as one
-// contiguous stream. At 64 clocks an instruction a few warps hide the loads, so these go from global
-// memory to registers. 5280-triangle relief, 2 kHz (170 MB): dot 107 -> 36 us, gather 128 ->
-// 68 us; 1280-triangle sphere in 16 leaves: gather 92 -> 19 us. The CTAs per leaf (up to 8, where the
-// leaves alone are fewer than four per SM) are what the sphere gains from.
+// scheduler's pipe for 64 clocks, and lanes without an element cost as much as those with one. Leaves hold 16 to
+// 32 elements (or their doubles), so lanes laid along a column's rows were a third empty and added
+// up over shuffles. Here the dot pass gives a lane a whole column (up to 32 rows of it), several CTAs a
+// leaf; the gather pass gives a thread a row of one column class (every 8th to 32nd column) and a leaf to a
+// cluster of 4 or 8 CTAs. At 64 clocks an instruction the other warps hide the loads, so these go from
+// global memory to registers (five CTAs per SM and two columns in flight: 123 us a matvec on 5280
+// triangles; three and four: 141; two and eight: 147). Matvec, against the FP32 layout: 248 -> 123 us on
+// 5280 triangles; gather on the sphere of 1280 triangles in 16 leaves: 92 -> 19 us.
 #include <algorithm>
 
 #include <cooperative_groups.h>
@@ -95,7 +95,7 @@ template <int NC>
 __device__ __forceinline__ void gather_class(double& re, double& im, const cd* __restrict__ seg, int K,
                                              const int* __restrict__ idx, const cd* __restrict__ z, int R, int cpc,
                                              int k, int r) {
-  constexpr int U = 4;
+  constexpr int U = 2;
   int c0 = 0, j = k;
   auto next = [&]() {
     while (c0 < K && j >= min(cpc, K - c0)) {
@@ -132,7 +132,7 @@ __device__ __forceinline__ void gather_class(double& re, double& im, const cd* _
 // holds them all, NC / S each with a thread per row. Every CTA adds its warps' slots, the first one the warps in
 // order, and finishes the leaf. The near part runs before the wait for the reduce pass.
 template <int NC, int S>
-__global__ void __launch_bounds__(kGatherThreads, 3) gather64_kernel(
+__global__ void __launch_bounds__(kGatherThreads, 5) gather64_kernel(
     SegView V, int nleaf, const cd* __restrict__ near, const cd* __restrict__ lrseg, const cd* __restrict__ t,
     const cd* __restrict__ x, cd* __restrict__ y, const cd* __restrict__ bminus, const cd* __restrict__ dot_a,
     const cd* __restrict__ dot_b, double* partials, double* red5, unsigned* ticket, const int* __restrict__ done) {
