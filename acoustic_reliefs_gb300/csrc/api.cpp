@@ -239,12 +239,24 @@ void require_mesh(ac3d_ctx* c) {
   if (!c->mesh_set) throw Error(AC3D_ERR_STATE, "No mesh set. Set one using set_mesh or precompute.");
 }
 
+// The context on an H-matrix's own mesh for the scope: set_mesh may have brought another one since the
+// H-matrix was assembled, with other block and leaf counts than its arrays have.
+struct MeshScope {
+  ac3d_ctx* c;
+  std::shared_ptr<MeshState> m;
+  MeshScope(ac3d_ctx* ctx, const std::shared_ptr<MeshState>& mesh) : c(ctx), m(ctx->m) { c->m = mesh; }
+  MeshScope(const MeshScope&) = delete;
+  MeshScope& operator=(const MeshScope&) = delete;
+  ~MeshScope() { c->m = m; }
+};
+
 // ------------------------------------------------------------------------------------------
 // Assembly
 // ------------------------------------------------------------------------------------------
 std::unique_ptr<DevHMat> assemble(ac3d_ctx* c, double k, int prec) {
   cudaStream_t s = c->stream;
   auto H = std::make_unique<DevHMat>();
+  H->mesh = c->m;
   H->prec = prec;
   H->pool_df = prec != PREC_FP64 && c->assembly == AC3D_ASSEMBLY_DF;
   H->k = k;
@@ -2074,6 +2086,7 @@ int ac3d_matvec_timing(ac3d_ctx* c, int iters, int transposed, double* ms, long 
     if (!c->last_H) throw Error(AC3D_ERR_STATE, "no H-matrix: call ac3d_pressures first");
     cudaStream_t s = c->stream;
     DevHMat& H = *c->last_H;
+    const MeshScope on_its_mesh(c, H.mesh);
     ensure_work(c);
     if (transposed) ensure_near_transposed(c->m->DP, H, s);
     // the variant the solve runs: FP64 vectors on the FP64 H-matrix; on the FP32 H-matrix FP32
@@ -2118,6 +2131,7 @@ int ac3d_block_matvec_timing(ac3d_ctx* c, int nrb, int iters, int transposed, do
     DevHMat& H = *c->last_H;
     if (H.prec == PREC_FP64) throw Error(AC3D_ERR_ARG, "block matvecs need the mixed-precision (FP32) H-matrix");
     cudaStream_t s = c->stream;
+    const MeshScope on_its_mesh(c, H.mesh);
     BlockWork W;
     MultiBufs B = block_bufs(c, H, nrb, W, transposed != 0);
     const size_t blk32 = (size_t)c->m->Ne * nrb * sizeof(cf);
@@ -2146,8 +2160,9 @@ int ac3d_get_ranks(ac3d_ctx* c, int32_t* ranks, int n) {
   return guard(c, [&] {
     if (!c->last_H) throw Error(AC3D_ERR_STATE, "no H-matrix: call ac3d_pressures or ac3d_surface_values first");
     std::vector<int>& r = c->last_H->ranks_host;
-    if (r.empty() && c->m->DP.na > 0) {  // fetched when asked for
-      r.resize(c->m->DP.na);
+    const int na = c->last_H->mesh->DP.na;
+    if (r.empty() && na > 0) {  // fetched when asked for
+      r.resize(na);
       AC3D_CUDA(cudaMemcpyAsync(r.data(), c->last_H->rank.p, r.size() * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
       AC3D_CUDA(cudaStreamSynchronize(c->stream));
     }

@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -206,6 +207,7 @@ struct AsmTotals {
 
 // An assembled H-matrix of (K - I/2) at one wavenumber.
 struct DevHMat {
+  std::shared_ptr<MeshState> mesh;  // whose partition its blocks are (a context may have another one by now)
   int prec = PREC_MIXED;  // storage: complex FP32 (mixed) or complex FP64
   bool pool_df = false;   // mixed storage assembled in double-float: the ACA pool holds complex double-float terms
   double k = 0;
