@@ -29,7 +29,6 @@ namespace {
 constexpr int kDfThreads = 256;
 constexpr int kDfWarps = kDfThreads / 32;
 constexpr int kSmallThreads = 128;  // CTAs of the 1-, 2- and 4-warp groups
-constexpr int kAllocTerms = 4;      // terms per allocation from the pool
 // Blocks are run by groups of W warps, W by the block's larger side: 1 up to 64, 2 up to 128, 4 up to
 // 256 (so that a thread owns at most two rows and two columns), 8 above.
 constexpr int kGroups = 4;
@@ -417,7 +416,7 @@ __device__ __forceinline__ void aca_small(const AcaDfArgs& A, unsigned char* sme
       // a term's place in the pool; taken for several terms at a time (never more than the block
       // can have), because every iteration would wait for the atomic's round trip
       if (nfree == 0) {
-        nfree = min(kAllocTerms, iter_lim - iter);
+        nfree = min(kAcaAllocTerms, iter_lim - iter);
         if (tid == 0) {
           const unsigned long long need = (unsigned long long)(m + n) * nfree;
           const unsigned long long bb = atomicAdd(A.pool_used, need);

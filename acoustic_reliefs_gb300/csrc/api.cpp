@@ -42,6 +42,7 @@ void DevBuf::alloc(size_t n, cudaStream_t stream) {
   s = stream;
   if (n == 0) n = 16;
   cudaError_t e = cudaMallocAsync(&p, n, s);
+  if (e != cudaSuccess) p = nullptr;
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     throw Error(AC3D_ERR_RESOURCE, "device allocation of " + std::to_string(n) + " bytes failed");
@@ -315,9 +316,20 @@ std::unique_ptr<DevHMat> assemble(ac3d_ctx* c, double k, int prec) {
     int64_t cap = c->m->pool_hint[prec];
     if (cap <= 0) cap = std::min<int64_t>(c->m->worst_pool, 16 * c->m->sum_mn);
     cap = std::max<int64_t>(cap, 1024);
+    // The double-float ACA takes a few terms' places at a time: on top of what its terms need, room for those
+    // that its blocks leave unused (at most 3 sum_mn, on average 1.5). Without it the first assembly of the
+    // 5280-triangle relief at 4.5 kHz (15.1 sum_mn of terms) overflowed and ran twice. Where the device has
+    // no room for them, the terms' own.
+    const int64_t spare = H->pool_df ? c->m->pool_spare : 0;
     for (int attempt = 0;; attempt++) {
-      H->pool.alloc((size_t)cap * pool_es, s);
-      H->pool_cap = cap;
+      H->pool_cap = std::min(std::max<int64_t>(c->m->worst_pool, 1024), cap + spare);
+      try {
+        H->pool.alloc((size_t)H->pool_cap * pool_es, s);
+      } catch (const Error& e) {
+        if (e.code != AC3D_ERR_RESOURCE || H->pool_cap <= cap) throw;
+        H->pool_cap = cap;
+        H->pool.alloc((size_t)cap * pool_es, s);
+      }
       AC3D_CUDA(cudaMemsetAsync(H->pool_used.p, 0, sizeof(AsmTotals), s));
       // FP32 and FP64: the ACA groups on the two assembly streams (the first after the near field).
       // Double-float: the ACA first, longest blocks first, and the near field behind its large
@@ -344,10 +356,12 @@ std::unique_ptr<DevHMat> assemble(ac3d_ctx* c, double k, int prec) {
         H->pool_used_host = (int64_t)tot.pool_used;
         break;
       }
-      if (cap >= c->m->worst_pool || attempt > 8) throw Error(AC3D_ERR_INTERNAL, "ACA pool overflow at worst-case size");
+      if (H->pool_cap >= c->m->worst_pool || attempt > 8) throw Error(AC3D_ERR_INTERNAL, "ACA pool overflow at worst-case size");
       cap = std::min<int64_t>(c->m->worst_pool, std::max<int64_t>(cap * 2, (int64_t)tot.pool_used));
     }
-    c->m->pool_hint[prec] = std::min<int64_t>(c->m->worst_pool, H->pool_used_host + H->pool_used_host / 8 + 4096);
+    // of the double-float ACA, the places of its passes
+    const int64_t need = H->pool_df ? std::min(H->pool_used_host, (int64_t)tot.aca_evaluated) : H->pool_used_host;
+    c->m->pool_hint[prec] = std::min<int64_t>(c->m->worst_pool, need + need / 8 + 4096);
     H->tvec.alloc(tcap * (prec == PREC_FP64 ? sizeof(cd) : sizeof(cf)), s);
     H->tvec64.alloc(tcap * sizeof(cd), s);
     H->tasks = (int64_t)tot.sum_rank;
@@ -1360,11 +1374,15 @@ std::shared_ptr<MeshState> build_mesh_state(const double* Ps, int V, const int32
     upload(DP.tr_pos, mp->P.tr_pos, s);
     mp->sum_mn = 0;
     mp->worst_pool = 0;
+    mp->pool_spare = 0;
     for (int b = 0; b < DP.na; b++) {
       const int* q = &mp->P.approx[4 * b];
       int m = q[1] - q[0], n = q[3] - q[2];
       mp->sum_mn += m + n;
-      mp->worst_pool += (int64_t)std::max(0, std::min(maxk, std::min(m - 1, n - 1))) * (m + n);
+      const int lim = std::max(0, std::min(maxk, std::min(m - 1, n - 1)));
+      mp->worst_pool += (int64_t)lim * (m + n);
+      if (std::max(m, n) <= kWarpAcaMaxDim && maxk <= kWarpAcaTerms)  // run by a group
+        mp->pool_spare += (int64_t)std::max(0, std::min(kAcaAllocTerms, lim) - 1) * (m + n);
     }
     mp->pool_hint[0] = mp->pool_hint[1] = 0;
     // geometry

@@ -170,7 +170,8 @@ struct MeshState {
   DevGeometry G;
   int64_t sum_mn = 0;      // sum over admissible blocks of m + n
   int64_t worst_pool = 0;  // ACA pool entries if every block reached its iteration limit
-  std::atomic<int64_t> pool_hint[2];  // per storage precision: pool size the last assembly needed
+  int64_t pool_spare = 0;  // entries that the double-float ACA may take and leave unused
+  std::atomic<int64_t> pool_hint[2];  // per storage precision: pool size the last assembly needed (without those)
   bool geom_base = false;  // G holds Ps0 (no heights applied)
   MeshState() {
     pool_hint[0] = 0;
@@ -183,6 +184,8 @@ enum Precision { PREC_MIXED = 0, PREC_FP64 = 1 };
 // Warp-per-block ACA: largest block side and largest number of iterations it handles.
 constexpr int kWarpAcaMaxDim = 256;
 constexpr int kWarpAcaTerms = 128;
+// The groups of the double-float ACA take the places of this many terms from the pool at a time.
+constexpr int kAcaAllocTerms = 4;
 
 // Device time of a phase of a call: two recorded events and the statistic they go to.
 struct PhaseTimer {

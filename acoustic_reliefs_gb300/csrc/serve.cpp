@@ -88,6 +88,11 @@ struct ac3d_server {
 namespace ac3d {
 namespace {
 
+// Bytes of the ACA pool beyond what the terms need; the assembly does without them if it has to.
+int64_t spare_bytes(const ac3d_server* S, const MeshEntry& me) {
+  return S->prec != AC3D_PREC_FP64 && S->assembly == AC3D_ASSEMBLY_DF ? me.m->pool_spare * 16 : 0;
+}
+
 // Device bytes a request may hold at its peak (assembly: near field, ACA pool and packed segments
 // coexist), from the partition and what earlier requests on the mesh needed.
 int64_t footprint(const ac3d_server* S, const MeshEntry& me, double f, int L) {
@@ -106,7 +111,7 @@ int64_t footprint(const ac3d_server* S, const MeshEntry& me, double f, int L) {
     work += ((int64_t)mm + 4) * m.Ne * (es == 16 ? 16 : 8) +
             (int64_t)gmres_scalar_doubles(mm, m.Ne) * 8 + 4096;
   }
-  return H + work;
+  return H + work + spare_bytes(S, me);
 }
 
 int admit_index(const ac3d_server* S) {
@@ -363,8 +368,9 @@ int ac3d_server_submit(ac3d_server* S, int mesh_id, double frequency, int kind, 
   }
   r->mesh = mesh_id;
   r->info.footprint_bytes = footprint(S, *S->meshes[mesh_id], frequency, L);
-  if (r->info.footprint_bytes > S->budget) {
-    S->err = "request needs an estimated " + std::to_string(r->info.footprint_bytes) +
+  const long long least = r->info.footprint_bytes - spare_bytes(S, *S->meshes[mesh_id]);
+  if (least > S->budget) {
+    S->err = "request needs an estimated " + std::to_string(least) +
              " device bytes, more than the server budget of " + std::to_string(S->budget);
     return AC3D_ERR_RESOURCE;
   }
