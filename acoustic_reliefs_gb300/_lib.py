@@ -86,6 +86,7 @@ SIGNATURES = {
     "ac3d_admit_next": (_I, [_P, _P, _I, ctypes.c_longlong, ctypes.c_longlong, _I]),
     "ac3d_tensor_selftest": (_I, [_P, _P, _I, _P]),
     "ac3d_packed_selftest": (_I, [_I, _P]),
+    "ac3d_transposed_selftest": (_I, [_P, _P]),
 }
 
 

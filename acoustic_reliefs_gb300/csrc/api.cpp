@@ -604,9 +604,28 @@ void check_pipeline(ac3d_ctx* c, const DevHMat& H) {
 
 void solve_impl(ac3d_ctx* c, DevHMat& H, const cd* b, cd* x, bool tr);
 
+// The transposed copy of the near field for single-vector passes. Where the device has no room for it they
+// read the blocks in place.
+void try_near_transposed(ac3d_ctx* c, DevHMat& H) {
+  try {
+    ensure_near_transposed(c->m->DP, H, c->stream);
+  } catch (const Error& e) {
+    if (e.code != AC3D_ERR_RESOURCE) throw;
+  }
+  c->stats.hmat_bytes = (long long)H.bytes();
+}
+
 void solve(ac3d_ctx* c, DevHMat& H, const cd* b, cd* x, bool tr) {
-  if (tr) ensure_near_transposed(c->m->DP, H, c->stream);
-  solve_impl(c, H, b, x, tr);
+  if (tr) try_near_transposed(c, H);
+  try {
+    solve_impl(c, H, b, x, tr);
+  } catch (const Error& e) {
+    // the copy may have taken the room of the solver's own buffers
+    if (e.code != AC3D_ERR_RESOURCE || !tr || !H.nearT.p) throw;
+    H.nearT.release();
+    c->stats.hmat_bytes = (long long)H.bytes();
+    solve_impl(c, H, b, x, tr);
+  }
   check_pipeline(c, H);
 }
 
@@ -798,8 +817,8 @@ MultiBufs block_bufs(ac3d_ctx* c, DevHMat& H, int nrb, BlockWork& W, bool tr) {
   const int n = c->m->Ne, nleaf = c->m->DP.nleaf;
   if (c->block_tc && nrb >= 8 && c->m->DP.max_leaf <= 32 && !(tr ? H.tcseg_f.p : H.tcseg_t.p)) {
     build_tc_segments(c->m->DP, H, tr, s);
-    c->stats.hmat_bytes = (long long)H.bytes();  // the split segments are part of the H-matrix's footprint
   }
+  c->stats.hmat_bytes = (long long)H.bytes();  // the copy and the split segments are part of the footprint
   const size_t blk32 = (size_t)n * nrb * sizeof(cf);
   W.kv.ensure(8 * blk32, s);
   MultiBufs B;
@@ -2106,7 +2125,7 @@ int ac3d_matvec_timing(ac3d_ctx* c, int iters, int transposed, double* ms, long 
     DevHMat& H = *c->last_H;
     const MeshScope on_its_mesh(c, H.mesh);
     ensure_work(c);
-    if (transposed) ensure_near_transposed(c->m->DP, H, s);
+    if (transposed) try_near_transposed(c, H);
     // the variant the solve runs: FP64 vectors on the FP64 H-matrix; on the FP32 H-matrix FP32
     // vectors (GMRES) or FP64 vectors with their FP32 shadows (BiCGSTAB), FP32 arithmetic
     const int vec64 = H.prec == PREC_FP64 ? 1 : (c->krylov == AC3D_KRYLOV_GMRES ? 0 : 2);
@@ -2187,6 +2206,40 @@ int ac3d_get_ranks(ac3d_ctx* c, int32_t* ranks, int n) {
     if (n != (int)r.size())
       throw Error(AC3D_ERR_ARG, "expected " + std::to_string(r.size()) + " admissible blocks, got " + std::to_string(n));
     std::copy(r.begin(), r.end(), ranks);
+  });
+}
+
+int ac3d_transposed_selftest(ac3d_ctx* c, long long* mismatches) {
+  if (!c || !mismatches) return AC3D_ERR_ARG;
+  return guard(c, [&] {
+    if (!c->last_H) throw Error(AC3D_ERR_STATE, "no H-matrix: call ac3d_pressures first");
+    cudaStream_t s = c->stream;
+    DevHMat& H = *c->last_H;
+    const MeshScope on_its_mesh(c, H.mesh);
+    const int n = c->m->Ne;
+    ensure_work(c);
+    ensure_near_transposed(c->m->DP, H, s);
+    DevBuf none, x32;
+    x32.alloc((size_t)n * sizeof(cf), s);
+    launch_to32(n, c->x64.p, x32.p, s);
+    long long bad = 0;
+    // every variant of the vectors: FP32, FP64, FP64 on FP32 arithmetic
+    for (int vec64 = H.prec == PREC_FP64 ? 1 : 0; vec64 <= (H.prec == PREC_FP64 ? 1 : 2); vec64++) {
+      const size_t es = vec64 ? sizeof(cd) : sizeof(cf);
+      const void* x = vec64 ? c->x64.p : x32.p;
+      std::vector<unsigned char> y[2];
+      for (int in_place = 0; in_place < 2; in_place++) {
+        if (in_place) std::swap(H.nearT, none);
+        launch_matvec_ex(c->m->DP, H, true, vec64, x, c->kv.p, nullptr, MatvecEpilogue{}, nullptr, s, x32.p, false);
+        if (in_place) std::swap(H.nearT, none);
+        y[in_place].resize(n * es);
+        AC3D_CUDA(cudaMemcpyAsync(y[in_place].data(), c->kv.p, n * es, cudaMemcpyDeviceToHost, s));
+        AC3D_CUDA(cudaStreamSynchronize(s));
+      }
+      for (int i = 0; i < n; i++) bad += std::memcmp(&y[0][i * es], &y[1][i * es], es) != 0;
+    }
+    check_pipeline(c, H);
+    *mismatches = bad;
   });
 }
 

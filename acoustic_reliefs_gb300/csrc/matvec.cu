@@ -392,11 +392,14 @@ constexpr int kPCols = 128;                  // multiplier columns per stage (ch
 constexpr int kPProdCols = kPCols / 32;      // per producer lane
 constexpr int kLeafSlots = kStages + 1;      // leaves whose chunks can be in the ring at once
 
+// The gather pass's directions: A x, and A^T x with the near field from its transposed copy or in place
+enum : int { kForward = 0, kTransposed = 1, kInPlace = 2 };
+
 struct StageMeta {
   int slot, ncols, first, last;  // slot < 0: no more leaves
 };
 
-template <typename MT, typename VT, typename AT, bool TRANS, int RPL>
+template <typename MT, typename VT, typename AT, int TRANS, int RPL>
 __global__ void __launch_bounds__(kGatherThreads, AC3D_GATHER_MIN_CTAS) seg_gather_persist_kernel(
     SegView V, int nleaf, const cplx<MT>* __restrict__ near, const cplx<MT>* __restrict__ lrseg,
     const cplx<AT>* __restrict__ t, const cplx<VT>* __restrict__ x, const cplx<AT>* __restrict__ xm,
@@ -636,10 +639,11 @@ __global__ void __launch_bounds__(kGatherThreads, AC3D_GATHER_MIN_CTAS) seg_gath
         AT tr[RPL], ti[RPL];
 #pragma unroll
         for (int jr = 0; jr < RPL; jr++) tr[jr] = ti[jr] = 0;
-        // near: the transposed copy, so that the lanes' columns of a row are consecutive (the blocks
-        // themselves would be read a line per lane); the rows of a warp's blocks in order, U loads in
-        // flight (as many as the 56 registers hold). Transposed matvec, before and after: 149.6 and
-        // 101.3 us on the 20480-triangle relief, 65.7 and 37.5 us on 5280 triangles
+        // near: the transposed copy, so that the lanes' columns of a row are consecutive; the rows of a
+        // warp's blocks in order, U loads in flight (as many as the 56 registers hold). The blocks
+        // themselves (kInPlace: the device has no room for the copy) are read a line per lane.
+        // Transposed matvec, from the blocks and from the copy: 149.6 and 101.3 us on the
+        // 20480-triangle relief, 65.7 and 37.5 us on 5280 triangles
         for (int it = V.trn_ptr[leaf] + warp; it < V.trn_ptr[leaf + 1]; it += kWarps) {
           const int b = V.trn[it];
           const int4 blk = V.blocks_d[b];
@@ -656,7 +660,7 @@ __global__ void __launch_bounds__(kGatherThreads, AC3D_GATHER_MIN_CTAS) seg_gath
 #pragma unroll
               for (int u = 0; u < U; u++) {
                 const int r = min(r0 + u, m - 1);
-                d[u] = D[(long long)r * R + col];
+                d[u] = D[TRANS == kInPlace ? (long long)col * m + r : (long long)r * R + col];
                 z[u] = xs[r];
               }
 #pragma unroll
@@ -768,7 +772,8 @@ static void set_smem_attrs_rpl() {
   // the largest shared-memory carveout, so that four CTAs of the ring size fit on an SM
   AC3D_CUDA(cudaFuncSetAttribute(seg_dot_kernel<MT, AT, RPL>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  100));
-  for (auto kern : {seg_gather_persist_kernel<MT, VT, AT, false, RPL>, seg_gather_persist_kernel<MT, VT, AT, true, RPL>}) {
+  for (auto kern : {seg_gather_persist_kernel<MT, VT, AT, kForward, RPL>, seg_gather_persist_kernel<MT, VT, AT, kTransposed, RPL>,
+                    seg_gather_persist_kernel<MT, VT, AT, kInPlace, RPL>}) {
     AC3D_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     AC3D_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRingBytes));
   }
@@ -828,11 +833,11 @@ static void mv_t(const DevPartition& DP, const DevHMat& H, bool tr, const void* 
   v.a_kptr = DP.didx_ptr.as<int>();
   v.a_idx = DP.didx.as<int>();
   v.blocks_d = DP.blocks_d.as<int4>();
-  v.near_off = tr ? DP.near_off_t.as<long long>() : DP.near_off.as<long long>();
+  const int mode = !tr ? kForward : H.nearT.p ? kTransposed : kInPlace;
+  v.near_off = mode == kTransposed ? DP.near_off_t.as<long long>() : DP.near_off.as<long long>();
   v.trn_ptr = DP.tr_near_ptr.as<int>();
   v.trn = DP.tr_near.as<int>();
   v.err = H.err.as<int>();
-  if (tr && DP.nd > 0 && !H.nearT.p) throw Error(3, "internal: transposed near field not built");
   const cplx<MT>* useg = H.useg.as<cplx<MT>>();
   const cplx<MT>* vseg = H.vseg.as<cplx<MT>>();
   cplx<AT>* t = (cplx<AT>*)tvec;
@@ -864,17 +869,19 @@ static void mv_t(const DevPartition& DP, const DevHMat& H, bool tr, const void* 
   // the gather reads x and the done flag before its wait, which needs the dot and reduce passes
   // between it and the kernel that wrote them; without low-rank blocks it is an ordinary launch
   // one resident wave: as many CTAs as fit on the device at once (each takes a share of the leaves)
-  auto kern = tr ? seg_gather_persist_kernel<MT, VT, AT, true, RPL> : seg_gather_persist_kernel<MT, VT, AT, false, RPL>;
-  static std::atomic<int> per_sm[2] = {{0}, {0}};
-  int nb = per_sm[tr].load();
+  auto kern = mode == kForward      ? seg_gather_persist_kernel<MT, VT, AT, kForward, RPL>
+              : mode == kTransposed ? seg_gather_persist_kernel<MT, VT, AT, kTransposed, RPL>
+                                    : seg_gather_persist_kernel<MT, VT, AT, kInPlace, RPL>;
+  static std::atomic<int> per_sm[3] = {{0}, {0}, {0}};
+  int nb = per_sm[mode].load();
   if (!nb) {
     AC3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, kGatherThreads, kRingBytes));
     nb = std::max(nb, 1);
-    per_sm[tr].store(nb);
+    per_sm[mode].store(nb);
   }
   const int P = std::min(DP.nleaf, nb * device_sm_count());
   launch_k(pdl && DP.na > 0, kern, dim3(P), dim3(kGatherThreads), kRingBytes, s, v, DP.nleaf,
-           (const cplx<MT>*)(tr ? H.nearT : H.near).as<cplx<MT>>(),
+           (const cplx<MT>*)(mode == kTransposed ? H.nearT : H.near).as<cplx<MT>>(),
            tr ? vseg : useg, tc, (const cplx<VT>*)x, xm, (cplx<VT>*)y, (const cplx<VT>*)bminus,
            (const cplx<VT>*)ep.dot_a, (const cplx<VT>*)ep.dot_b, ep.partials, ep.red5, H.ticket.as<unsigned>(), done);
 

@@ -127,11 +127,35 @@ __device__ __forceinline__ void gather_class(double& re, double& im, const cd* _
   }
 }
 
+// gather_class of a leaf's near columns in A^T without their transposed copy (the device has no room for
+// it): column c of the segment is a row of one of the near blocks that have the leaf's columns, in their
+// order; the walk over the columns and so the order of the sums are the same.
+template <int NC>
+__device__ __forceinline__ void gather_near_in_place(double& re, double& im, const SegView& V, int leaf,
+                                                     const cd* __restrict__ near, const cd* __restrict__ x, int R,
+                                                     int cpc, int k, int r) {
+  int it = V.trn_ptr[leaf], before = 0;  // the block, and the columns before it
+  const int end = V.trn_ptr[leaf + 1], K = V.a_kptr[leaf + 1] - V.a_kptr[leaf];
+  for (int c0 = 0; c0 < K; c0 += cpc)
+    for (int c = c0 + k; c < min(c0 + cpc, K); c += NC) {
+      int4 q;
+      int m = 0;
+      for (; it < end; it++, before += m) {
+        q = V.blocks_d[V.trn[it]];
+        m = q.y - q.x;
+        if (c < before + m) break;
+      }
+      if (it == end) return;  // the padding column
+      const int i = c - before;
+      mac64(re, im, near[V.near_off[V.trn[it]] + (long long)r * m + i], x[q.x + i]);
+    }
+}
+
 // y[leaf rows] = -x/2 + S_A x[a_idx] + S_B t[b_idx], or b - that, with the optional dot partials of
 // seg_gather_persist_kernel. The NC column classes are that kernel's (warp, slot) pairs: a cluster of S CTAs
 // holds them all, NC / S each with a thread per row. Every CTA adds its warps' slots, the first one the warps in
 // order, and finishes the leaf. The near part runs before the wait for the reduce pass.
-template <int NC, int S>
+template <int NC, int S, bool IN_PLACE>
 __global__ void __launch_bounds__(kGatherThreads, 5) gather64_kernel(
     SegView V, int nleaf, const cd* __restrict__ near, const cd* __restrict__ lrseg, const cd* __restrict__ t,
     const cd* __restrict__ x, cd* __restrict__ y, const cd* __restrict__ bminus, const cd* __restrict__ dot_a,
@@ -159,7 +183,12 @@ __global__ void __launch_bounds__(kGatherThreads, 5) gather64_kernel(
   const int cpc = min(128, max(2, (int)(kStageBytes / sizeof(cd)) / R & ~1));  // columns per chunk of its ring
   double re = 0, im = 0;
   const int ak = V.a_kptr[leaf], ac = V.a_kptr[leaf + 1] - ak;
-  if (!skip && g < GP) gather_class<NC>(re, im, near + V.a_seg[leaf], ac, V.a_idx + ak, x, R, cpc, k, r);
+  if (!skip && g < GP) {
+    if constexpr (IN_PLACE)
+      gather_near_in_place<NC>(re, im, V, leaf, near, x, R, cpc, k, r);
+    else
+      gather_class<NC>(re, im, near + V.a_seg[leaf], ac, V.a_idx + ak, x, R, cpc, k, r);
+  }
   const int bk = V.b_kptr[leaf], bc = V.b_kptr[leaf + 1] - bk;
   grid_dep_wait();
   if (!skip && g < GP) gather_class<NC>(re, im, lrseg + V.b_seg[leaf], bc, V.b_idx + bk, t, R, cpc, k, r);
@@ -250,7 +279,11 @@ void launch_matvec_f64(const DevPartition& DP, const DevHMat& H, bool tr, const 
   v.a_seg = (tr ? DP.near_seg_t : DP.near_seg).as<long long>();
   v.a_kptr = (tr ? DP.didx_t_ptr : DP.didx_ptr).as<int>();
   v.a_idx = (tr ? DP.didx_t : DP.didx).as<int>();
-  if (tr && DP.nd > 0 && !H.nearT.p) throw Error(3, "internal: transposed near field not built");
+  const bool in_place = tr && !H.nearT.p;
+  v.blocks_d = DP.blocks_d.as<int4>();
+  v.near_off = DP.near_off.as<long long>();
+  v.trn_ptr = DP.tr_near_ptr.as<int>();
+  v.trn = DP.tr_near.as<int>();
   const cd* useg = H.useg.as<cd>();
   const cd* vseg = H.vseg.as<cd>();
   cd* t = H.tvec64.as<cd>();
@@ -277,17 +310,17 @@ void launch_matvec_f64(const DevPartition& DP, const DevHMat& H, bool tr, const 
   auto gather = [&](auto kern, int classes, int ctas) {
     const int threads = (classes / ctas * DP.max_leaf + 31) / 32 * 32;
     launch_clusters(pdl && DP.na > 0, (unsigned)ctas, kern, dim3(DP.nleaf * ctas), dim3(threads), s, v, DP.nleaf,
-                    (tr ? H.nearT : H.near).as<cd>(), tr ? vseg : useg, t, (const cd*)x, (cd*)y, (const cd*)bminus,
+                    (tr && !in_place ? H.nearT : H.near).as<cd>(), tr ? vseg : useg, t, (const cd*)x, (cd*)y, (const cd*)bminus,
                     (const cd*)ep.dot_a, (const cd*)ep.dot_b, ep.partials, ep.red5, H.ticket.as<unsigned>(), done);
   };
   if (DP.max_leaf <= 32)
-    gather(gather64_kernel<32, 4>, 32, 4);
+    gather(in_place ? gather64_kernel<32, 4, true> : gather64_kernel<32, 4, false>, 32, 4);
   else if (DP.max_leaf <= 64)
-    gather(gather64_kernel<32, 8>, 32, 8);
+    gather(in_place ? gather64_kernel<32, 8, true> : gather64_kernel<32, 8, false>, 32, 8);
   else if (DP.max_leaf <= 128)
-    gather(gather64_kernel<16, 8>, 16, 8);
+    gather(in_place ? gather64_kernel<16, 8, true> : gather64_kernel<16, 8, false>, 16, 8);
   else
-    gather(gather64_kernel<8, 8>, 8, 8);
+    gather(in_place ? gather64_kernel<8, 8, true> : gather64_kernel<8, 8, false>, 8, 8);
 }
 
 }  // namespace ac3d

@@ -52,8 +52,10 @@ typedef struct ac3d_stats {
   long long near_entries, lr_entries; /* stored complex entries */
   double mean_rank;
   int max_rank;
-  long long hmat_bytes;     /* device bytes of the last H-matrix (including the split segments of
-                               tensor-core block matvecs once they are built) */
+  long long hmat_bytes;     /* device bytes of the last H-matrix, including the split segments of
+                               tensor-core block matvecs and, from the first transposed (adjoint)
+                               solve on, the transposed copy of its near field (as large as the near
+                               field; single-vector solves do without it where it does not fit) */
   int solves;               /* linear solves in the call */
   int iterations;           /* Krylov iterations, summed over solves and refinement steps */
   int outer_steps;          /* refinement steps (mixed precision) summed over solves */
@@ -288,6 +290,10 @@ int ac3d_tensor_selftest(const float* A, const float* B, int K, float* D);
  * square root, over every FP32 significand at five exponents; 2: the double-float operations on
  * 2^20 pairs of values. No reference counterpart. */
 int ac3d_packed_selftest(int op, long long* mismatches);
+/* Self-check of the transposed matvec on the last H-matrix: the number of elements of A^T x (x the last
+ * solution) whose bits differ between the near field read from its transposed copy and in place, over
+ * the vector variants of the H-matrix's precision. No reference counterpart. */
+int ac3d_transposed_selftest(ac3d_ctx* ctx, long long* mismatches);
 
 /* ---------------------------------------------------------------------------------------------
  * Request server. No reference counterpart: the reference solves one frequency at a time inside
