@@ -135,6 +135,17 @@ void resolve_timers(ac3d_ctx* c) {
     *t.acc += ms;
   }
   drop_timers(c);
+  if (c->q_pending) {
+    c->q_pending = false;
+    if (cudaStreamQuery(c->stream) != cudaSuccess) {  // (behind the phases there is nothing to wait for)
+      cudaGetLastError();
+      AC3D_CUDA(cudaStreamSynchronize(c->stream));
+    }
+    if (*c->h_q_status & 2) {
+      AC3D_CUDA(cudaMemsetAsync(c->q_status.p, 0, 16, c->stream));
+      throw Error(AC3D_ERR_CUDA, "receiver ACA grid barrier timed out (bounded wait)");
+    }
+  }
 }
 
 // On the way out of a failed call (a solve that did not converge keeps its phase times).
@@ -993,13 +1004,17 @@ std::unique_ptr<ListenerLR> listener_lr(ac3d_ctx* c, double k, const double* Lh,
         v[8 * i + 2 * d + 1] = (float)(Lh[3 * i + d] - (double)hi);
       }
     upload(Q->pts, v, s);
+    // the status is read when the call ends (resolve_timers)
+    if (!c->q_status.p) {
+      c->q_status.alloc(16, s);
+      AC3D_CUDA(cudaMemsetAsync(c->q_status.p, 0, 16, s));
+    }
+    if (!c->h_q_status) AC3D_CUDA(cudaMallocHost(&c->h_q_status, sizeof(int)));
     launch_listener_aca_df(c->m->G, Q->pts.p, L, k, c->q_tol, maxk, Q->pool.p, cap, Q->used.as<unsigned long long>(),
-                           Q->toff.as<long long>(), Q->rank.as<int>(), (int*)(Q->used.as<unsigned long long>() + 1),
-                           Q->blk.as<int4>(), Q->ord.as<int>(), Q->scratch, s);
-    unsigned long long used[2];
-    AC3D_CUDA(cudaMemcpyAsync(used, Q->used.p, 16, cudaMemcpyDeviceToHost, s));
-    AC3D_CUDA(cudaStreamSynchronize(s));
-    if ((int)(used[1] & 0xffffffffu) & 2) throw Error(AC3D_ERR_CUDA, "receiver ACA grid barrier timed out (bounded wait)");
+                           Q->toff.as<long long>(), Q->rank.as<int>(), c->q_status.as<int>(), Q->blk.as<int4>(),
+                           Q->ord.as<int>(), Q->scratch, s);
+    AC3D_CUDA(cudaMemcpyAsync(c->h_q_status, c->q_status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    c->q_pending = true;
     return Q;
   }
   if (c->prec == PREC_FP64) {
@@ -1490,7 +1505,7 @@ void ac3d_destroy(ac3d_ctx* c) {
   c->last_H.reset();
   DevBuf* bufs[] = {&c->kv, &c->kv32, &c->partials, &c->kstate, &c->red, &c->b64, &c->x64, &c->r64, &c->ff_scratch,
                     &c->adj_scratch, &c->tmp_recv, &c->Ls_dev, &c->d_h_off, &c->d_pair_elem, &c->d_pair_corner,
-                    &c->d_pair_touch, &c->d_touch, &c->gm};
+                    &c->d_pair_touch, &c->d_touch, &c->gm, &c->q_status};
   for (DevBuf* b : bufs) b->release();
   c->m.reset();  // a mesh shared with other contexts stays alive until its last user goes
   c->m_dense.reset();

@@ -80,6 +80,9 @@ struct ac3d_ctx {
   ac3d::GState* h_gstate = nullptr;  // pinned, two slots
   double* h_red = nullptr;    // pinned
   ac3d::AsmTotals* h_totals = nullptr;  // pinned
+  ac3d::DevBuf q_status;       // int: status of the receiver ACAs since it was last read
+  int* h_q_status = nullptr;   // pinned copy
+  bool q_pending = false;      // a receiver ACA of the running call has not been checked
   std::vector<ac3d::PhaseTimer> timers;      // phases of the running call, read when it ends
   std::vector<cudaGraphExec_t> used_graphs;  // executable graphs of finished solves, to be destroyed
   void destroy_used_graphs() {
@@ -92,6 +95,7 @@ struct ac3d_ctx {
     if (h_gstate) cudaFreeHost(h_gstate);
     if (h_red) cudaFreeHost(h_red);
     if (h_totals) cudaFreeHost(h_totals);
+    if (h_q_status) cudaFreeHost(h_q_status);
   }
 };
 
@@ -106,7 +110,8 @@ double wavenumber(double f);  // k = 2 pi f / c, c = 344 m/s (helpers.h:8, const
 std::shared_ptr<MeshState> build_mesh_state(const double* Ps, int V, const int32_t* Es, int Ne, int cluster_size,
                                             double radius_factor, int maxk, cudaStream_t s);
 void ensure_work(ac3d_ctx* c);
-// Phase times of the call so far into the statistics (waits for the phases to end).
+// Phase times of the call so far into the statistics (waits for the phases to end), and the status of
+// its receiver ACAs.
 void resolve_timers(ac3d_ctx* c);
 void finish_timers(ac3d_ctx* c);
 void reset_stats(ac3d_ctx* c);
