@@ -1131,13 +1131,14 @@ static void mmv_t(const DevPartition& DP, const DevHMat& H, const MultiBufs& B, 
   mseg_gather_kernel<NRB, RPL><<<grid, kMGatherThreads, gsmem, s>>>(v, DP.nleaf, g_near, g_lr, T, (const cf*)x, (cf*)y,
                                                                     (const cf*)dot_a, (const cf*)dot_b, g_part, g_gpart,
                                                                     B.ticket, B.red, done);
-  if (DP.nleaf > 1024 * kGroup) throw Error(1, "block solves support at most 32768 leaf clusters");
   AC3D_CUDA(cudaGetLastError());
 }
 
 template <int NRB>
 static void mmv_rpl(const DevPartition& DP, const DevHMat& H, const MultiBufs& B, const void* x, void* y,
                     const void* dot_a, const void* dot_b, const int* done, cudaStream_t s) {
+  // (the groups' partial sums and tickets end there)
+  if (DP.nleaf > 1024 * kGroup) throw Error(1, "block solves support at most 32768 leaf clusters");
   if (DP.max_leaf <= 32)
     mmv_t<NRB, 1>(DP, H, B, x, y, dot_a, dot_b, done, s);
   else if (DP.max_leaf <= 64)

@@ -1,10 +1,10 @@
 """Block solves where the gather pass's tiles, rings and chunks differ: leaves of 2 to 64 elements (one and
-two rows per lane), 4, 8 and 16 right-hand sides, no low-rank blocks, both directions."""
+two rows per lane), 4, 8 and 16 right-hand sides, no low-rank blocks, both directions, the leaf limit."""
 import numpy as np
 import pytest
 
 from acoustic_reliefs_gb300 import meshes
-from acoustic_reliefs_gb300.acoustics3d import DiffBEM
+from acoustic_reliefs_gb300.acoustics3d import AC3DError, DiffBEM
 from tests import cases
 
 pytestmark = pytest.mark.gpu
@@ -57,3 +57,15 @@ def test_transposed_block_solve_matches_single_solves(gpu_lib, leaf, factor, nd)
     assert abs(loss - (1 - np.mean([c for c, _ in singles]))) < 1e-6
     gref = -np.mean([s for _, s in singles], axis=0)
     assert np.linalg.norm(g - gref) / np.linalg.norm(gref) < 1e-4
+
+
+@pytest.mark.parametrize("method", ["gmres", "bicgstab"])
+def test_more_leaves_than_supported_are_refused(gpu_lib, method):
+    """33852 leaves of one triangle (the passes' reduction has room for 32768): refused before a launch."""
+    R = meshes.relief(0.6, 0.6, 0.05, 91, 1, 91, 0, meshes.smooth_heightmap(16, 5))
+    bem = DiffBEM(1, 0.2, [500.0], 1, 1e-3, 1e-3, 1e-6, precision="mixed")
+    bem.silent = True
+    bem.set_krylov(method)
+    bem.set_mesh(R.Ps, R.Es)
+    with pytest.raises(AC3DError, match="32768 leaf clusters"):
+        bem.pvals_multi(500.0, _dirs(2, 1), meshes.semicircle(5.0, 9))
