@@ -541,24 +541,29 @@ __device__ __forceinline__ void aca_small(const AcaDfArgs& A, unsigned char* sme
 // One CTA per block (blocks with a side above 256, or more terms than the groups hold): thread t
 // owns rows and columns t + 256 k, kept in the pool. Sums: by thread, then over the warps.
 // ------------------------------------------------------------------------------------------
-// Shared memory of a CTA block beside its coefficients, term offsets and used-row bits
+// Shared memory of a CTA block beside its coefficients, term offsets and used-row bits; C entries are
+// evaluated at a time, kDfThreads or half as many
+template <int C>
 struct AcaCta {
-  ulonglong2 b0[3 * kDfThreads], b1[3 * kDfThreads];
+  ulonglong2 b0[3 * C], b1[3 * C];
   df64 bv[2][kDfWarps];
   int bi[2][kDfWarps];
   df64 sd[2][kDfWarps];
   long long base;
   int ovf, pad;
 };
-static_assert(sizeof(AcaCta) % 16 == 0, "the coefficients follow");
+static_assert(sizeof(AcaCta<kDfThreads>) % 16 == 0 && sizeof(AcaCta<kDfThreads / 2>) % 16 == 0,
+              "the coefficients follow");
 
+template <int C>
 static size_t aca_cta_smem(int iter_cap, int max_rows) {
-  return sizeof(AcaCta) + (size_t)iter_cap * (sizeof(df2) + sizeof(long long) + sizeof(df64)) + (size_t)((max_rows + 31) / 32) * 4;
+  return sizeof(AcaCta<C>) + (size_t)iter_cap * (sizeof(df2) + sizeof(long long) + sizeof(df64)) + (size_t)((max_rows + 31) / 32) * 4;
 }
 
+template <int C>
 __device__ __forceinline__ void aca_cta(const AcaDfArgs& A, unsigned char* smem, int b) {
-  AcaCta& S = *reinterpret_cast<AcaCta*>(smem);
-  df2* coef = reinterpret_cast<df2*>(smem + sizeof(AcaCta));
+  AcaCta<C>& S = *reinterpret_cast<AcaCta<C>*>(smem);
+  df2* coef = reinterpret_cast<df2*>(smem + sizeof(AcaCta<C>));
   long long* toff = reinterpret_cast<long long*>(coef + A.iter_cap);
   df64* prod = reinterpret_cast<df64*>(toff + A.iter_cap);
   unsigned* used = reinterpret_cast<unsigned*>(prod + A.iter_cap);
@@ -607,13 +612,13 @@ __device__ __forceinline__ void aca_cta(const AcaDfArgs& A, unsigned char* smem,
     // row residual v = M(i, :) - U(i, :) V
     df64 best{-1.0f, 0.0f};
     int bidx = 0;
-    for (int c0 = 0; c0 < n; c0 += T) {
+    for (int c0 = 0; c0 < n; c0 += C) {
       if (c0) __syncthreads();  // the previous entries are finished
-      eval_items(A.k, A.pts + rs + i, 0, A.el + cs + c0, 1, min(T, n - c0), tid, T, b0, b1);
+      eval_items(A.k, A.pts + rs + i, 0, A.el + cs + c0, 1, min(C, n - c0), tid, T, b0, b1);
       __syncthreads();
-      const int c = c0 + tid;
-      if (c < n) {
-        const df2 v = finish_entry<4, false>(b0, b1, tid, coef_a, toff_a, A.pool + m + c, nst);
+      const int e = C == kDfThreads ? tid : tid - c0 % T, c = c0 + e;  // (thread t owns t, t + T, ...)
+      if (e >= 0 && e < C && c < n) {
+        const df2 v = finish_entry<4, false>(b0, b1, e, coef_a, toff_a, A.pool + m + c, nst);
         df2_stc(vnew + c, v);
         const df64 a = df2_abs2(v);
         if (a > best) {
@@ -639,13 +644,13 @@ __device__ __forceinline__ void aca_cta(const AcaDfArgs& A, unsigned char* smem,
 
     // column residual u = M(:, j) - U V(:, j)
     df64 un{0.0f, 0.0f};
-    for (int r0 = 0; r0 < m; r0 += T) {
+    for (int r0 = 0; r0 < m; r0 += C) {
       if (r0) __syncthreads();
-      eval_items(A.k, A.pts + rs + r0, 1, A.el + cs + j, 0, min(T, m - r0), tid, T, b0, b1);
+      eval_items(A.k, A.pts + rs + r0, 1, A.el + cs + j, 0, min(C, m - r0), tid, T, b0, b1);
       __syncthreads();
-      const int r = r0 + tid;
-      if (r < m) {
-        const df2 u = finish_entry<4, false>(b0, b1, tid, coef_a, toff_a, A.pool + r, nst);
+      const int e = C == kDfThreads ? tid : tid - r0 % T, r = r0 + e;
+      if (e >= 0 && e < C && r < m) {
+        const df2 u = finish_entry<4, false>(b0, b1, e, coef_a, toff_a, A.pool + r, nst);
         df2_stc(unew + r, u);
         un += df2_abs2(u);
       }
@@ -711,10 +716,11 @@ __device__ __forceinline__ void aca_cta(const AcaDfArgs& A, unsigned char* smem,
   }
 }
 
+template <int C>
 __global__ void __launch_bounds__(kDfThreads, 2) aca_df_cta_kernel(AcaDfArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   load_table(A.tab);
-  aca_cta(A, smem_raw, A.order[blockIdx.x]);
+  aca_cta<C>(A, smem_raw, A.order[blockIdx.x]);
 }
 
 // The blocks next, next + 1, ... of a class by the CTA's groups, each as it gets free
@@ -782,21 +788,42 @@ void launch_near_assembly_df(const DevGeometry& G, const DevPartition& DP, DevHM
   AC3D_CUDA(cudaGetLastError());
 }
 
-constexpr size_t kAcaSmemMax = 200 * 1024;
+// What a CTA can have beside the static shared memory of these kernels (the table, a few words).
+constexpr size_t kAcaSmemMax = 227 * 1024 - kDfTab * sizeof(float4) - 256;
+// The blocks that are taken: 40 bytes a term and a bit a row in 200 KB, or all of a CTA's in 200 KB. The
+// first kind fits with half of the entries at a time; with kDfThreads all do but those of 1.57 million rows
+// and more.
+constexpr size_t kAcaBlockMax = 200 * 1024;
+static_assert(sizeof(AcaCta<kDfThreads / 2>) + kAcaBlockMax <= kAcaSmemMax, "every block that is taken fits");
+
+// kernels[1] (half of the entries at a time) where kernels[0] does not fit; false: not taken
+template <typename K>
+static bool pick_aca_kernel(const K (&kernels)[2], int iter_cap, int max_rows, K& kernel, size_t& smem) {
+  smem = aca_cta_smem<kDfThreads>(iter_cap, max_rows);
+  if ((size_t)iter_cap * 40 + (size_t)((max_rows + 31) / 32) * 4 > kAcaBlockMax && smem > kAcaBlockMax) return false;
+  kernel = kernels[0];
+  if (smem > kAcaSmemMax) {
+    smem = aca_cta_smem<kDfThreads / 2>(iter_cap, max_rows);
+    kernel = kernels[1];
+  }
+  return true;
+}
 
 // Blocks above 256 on s_large, the others on s_small.
 static void launch_aca_kernels(const AcaDfArgs& a, int max_rows, cudaStream_t s_large, cudaStream_t s_small) {
   if (a.split[0] > 0) {
-    const size_t smem = aca_cta_smem(a.iter_cap, max_rows);
-    if (smem > kAcaSmemMax) throw Error(4, "ACA block too large for shared memory");
+    static void (*const kernels[2])(AcaDfArgs) = {aca_df_cta_kernel<kDfThreads>, aca_df_cta_kernel<kDfThreads / 2>};
+    void (*kernel)(AcaDfArgs);
+    size_t smem;
+    if (!pick_aca_kernel(kernels, a.iter_cap, max_rows, kernel, smem)) throw Error(4, "ACA block too large for shared memory");
     // once per process, to the largest size any launch uses: contexts on other threads launch with
     // other sizes
     static std::once_flag once;
     std::call_once(once, [] {
-      AC3D_CUDA(cudaFuncSetAttribute(aca_df_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAcaSmemMax));
+      for (auto k : kernels) AC3D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAcaSmemMax));
     });
     note_launch();
-    aca_df_cta_kernel<<<a.split[0], kDfThreads, smem, s_large>>>(a);
+    kernel<<<a.split[0], kDfThreads, smem, s_large>>>(a);
     AC3D_CUDA(cudaGetLastError());
   }
   const int ctas = a.split[1] + (a.split[2] + 1) / 2 + (a.split[3] + 3) / 4;
@@ -913,11 +940,12 @@ __device__ __noinline__ float grid_dot(const df2* a, const df2* b, int len) {
   return s[0];
 }
 
+template <int C>
 __global__ void __launch_bounds__(kDfThreads, 1) aca_df_grid_kernel(AcaDfArgs A, AcaGridBufs X) {
   extern __shared__ __align__(16) unsigned char smem[];
   load_table(A.tab);
-  AcaCta& S = *reinterpret_cast<AcaCta*>(smem);
-  df2* coef = reinterpret_cast<df2*>(smem + sizeof(AcaCta));
+  AcaCta<C>& S = *reinterpret_cast<AcaCta<C>*>(smem);
+  df2* coef = reinterpret_cast<df2*>(smem + sizeof(AcaCta<C>));
   long long* toff = reinterpret_cast<long long*>(coef + A.iter_cap);
   df64* prod = reinterpret_cast<df64*>(toff + A.iter_cap);
   unsigned* used = reinterpret_cast<unsigned*>(prod + A.iter_cap);
@@ -943,12 +971,12 @@ __global__ void __launch_bounds__(kDfThreads, 1) aca_df_grid_kernel(AcaDfArgs A,
     df64 best{-1.0f, 0.0f};
     df2 bv{0, 0};
     int bidx = 0;
-    for (int c0 = c_lo; c0 < c_hi; c0 += T) {
+    for (int c0 = c_lo; c0 < c_hi; c0 += C) {
       if (c0 > c_lo) __syncthreads();
-      eval_items(A.k, A.pts + rs + i, 0, A.el + cs + c0, 1, min(T, c_hi - c0), tid, T, b0, b1);
+      eval_items(A.k, A.pts + rs + i, 0, A.el + cs + c0, 1, min(C, c_hi - c0), tid, T, b0, b1);
       __syncthreads();
       const int c = c0 + tid;
-      if (c < c_hi) {
+      if (tid < C && c < c_hi) {
         const df2 v = finish_entry<8, true>(b0, b1, tid, coef_a, toff_a, A.pool + m + c, nst);
         df2_stc(vnew + c, v);
         const df64 a = df2_abs2(v);
@@ -995,12 +1023,12 @@ __global__ void __launch_bounds__(kDfThreads, 1) aca_df_grid_kernel(AcaDfArgs A,
       X.sq_v[c] = df2_abs2(v);
     }
     // column residual of this CTA's rows
-    for (int r0 = r_lo; r0 < r_hi; r0 += T) {
+    for (int r0 = r_lo; r0 < r_hi; r0 += C) {
       if (r0 > r_lo) __syncthreads();
-      eval_items(A.k, A.pts + rs + r0, 1, A.el + cs + j, 0, min(T, r_hi - r0), tid, T, b0, b1);
+      eval_items(A.k, A.pts + rs + r0, 1, A.el + cs + j, 0, min(C, r_hi - r0), tid, T, b0, b1);
       __syncthreads();
       const int r = r0 + tid;
-      if (r < r_hi) {
+      if (tid < C && r < r_hi) {
         const df2 u = finish_entry<8, true>(b0, b1, tid, coef_a, toff_a, A.pool + r, nst);
         df2_stc(unew + r, u);
         X.sq_u[r] = df2_abs2(u);
@@ -1126,15 +1154,17 @@ void launch_listener_aca_df(const DevGeometry& G, const void* pts_df, int L, dou
               G.el_df.as<DfElem>(), G.df_tab.as<float4>(), block, order, {1, 0, 0, 0}, df_from_double(k), eps,
               df_from_double(eps * eps), maxk, iter_lim,
               (df2*)pool, pool_cap, used, term_off, rank, status, nullptr, nullptr, 0};
-  const size_t smem = aca_cta_smem(iter_lim, L);
-  if (smem > kAcaSmemMax)
+  static void (*const kernels[2])(AcaDfArgs, AcaGridBufs) = {aca_df_grid_kernel<kDfThreads>, aca_df_grid_kernel<kDfThreads / 2>};
+  void (*kernel)(AcaDfArgs, AcaGridBufs);
+  size_t smem;
+  if (!pick_aca_kernel(kernels, iter_lim, L, kernel, smem))
     throw Error(4, "receiver ACA too large for shared memory (at most about 5000 receivers)");
   static std::once_flag once;
   std::call_once(once, [] {
-    AC3D_CUDA(cudaFuncSetAttribute(aca_df_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAcaSmemMax));
+    for (auto k : kernels) AC3D_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAcaSmemMax));
   });
   int per_sm = 0;
-  AC3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, aca_df_grid_kernel, kDfThreads, smem));
+  AC3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kDfThreads, smem));
   // about 64 columns (192 items) per CTA, at most one CTA per SM
   const int grid = std::max(1, std::min((per_sm > 0 ? 1 : 0) * device_sm_count(), (G.ne + 63) / 64));
   if (grid <= 2) {
@@ -1157,7 +1187,7 @@ void launch_listener_aca_df(const DevGeometry& G, const void* pts_df, int L, dou
                 (df64*)(sp + o_n), (float2*)(sp + o_d), listener_term_stride(L, G.ne)};
   void* args[] = {&a, &x};
   note_launch();
-  AC3D_CUDA(cudaLaunchCooperativeKernel((const void*)aca_df_grid_kernel, dim3(grid), dim3(kDfThreads), args, smem, s));
+  AC3D_CUDA(cudaLaunchCooperativeKernel((const void*)kernel, dim3(grid), dim3(kDfThreads), args, smem, s));
   note_launch();
   df_to_cd_kernel<<<4 * device_sm_count(), 256, 0, s>>>((df2*)pool, used);
   AC3D_CUDA(cudaGetLastError());
