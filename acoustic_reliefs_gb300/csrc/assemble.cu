@@ -12,7 +12,10 @@
 // term; next row pivot = first max of |u|^2 over rows not used yet. Each rank-1 term (u | v) is
 // bump-allocated from one pool with an atomic counter, so storage is proportional to the actual
 // ranks; the pool offset of term q of block b is term_off[b * maxk + q]. The kernels here are those of
-// the FP32 assembly; FP64 and double-float ACA have their own (aca_f64.cu, aca_df.cu).
+// the FP32 assembly and of long FP64 receiver blocks; FP64 and double-float ACA have their own (aca_f64.cu,
+// aca_df.cu).
+#include <mutex>
+
 #include "common.cuh"
 #include "internal.h"
 #include "listener.h"
@@ -605,10 +608,15 @@ static void aca_launch_all(AcaArgs<R, P4> a, const DevPartition& DP, int max_row
 template <typename R, typename P4>
 static void aca_launch_t(const AcaArgs<R, P4>& a, int nblocks, int max_rows, cudaStream_t s) {
   size_t smem = (size_t)a.iter_cap * (2 * sizeof(cplx<R>) + sizeof(long long)) + (size_t)((max_rows + 31) / 32) * 4;
-  if (smem > 48 * 1024) {
-    if (smem > 227 * 1024) throw Error(4, "ACA block too large for shared memory");
-    AC3D_CUDA(cudaFuncSetAttribute(aca_kernel<R, P4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  }
+  if (smem > 227 * 1024) throw Error(4, "ACA block too large for shared memory");
+  // once per process, to the largest size any launch can use: contexts on other threads launch with others
+  static std::once_flag once;
+  std::call_once(once, [] {
+    cudaFuncAttributes at{};
+    AC3D_CUDA(cudaFuncGetAttributes(&at, aca_kernel<R, P4>));
+    AC3D_CUDA(cudaFuncSetAttribute(aca_kernel<R, P4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   227 * 1024 - (int)at.sharedSizeBytes));
+  });
   note_launch();
   aca_kernel<R, P4><<<nblocks, kAcaThreads, smem, s>>>(a);
   AC3D_CUDA(cudaGetLastError());
@@ -654,7 +662,12 @@ void launch_rank_scan(const DevPartition& DP, DevHMat& H, cudaStream_t s) {
 
 // ------------------------------------------------------------------------------------------
 // Listener ACA (compute_ACA_listener, aca.cpp:84-134): one block of L receivers x Ne elements,
-// maxk 5000, no zero guard. Rows are receiver points.
+// maxk 5000, no zero guard. Rows are receiver points. In FP64, rows and columns of up to 1024 entries
+// together have their quadrature points spread over the CTA (aca_f64.cu), which fills its threads on the
+// short side; longer ones fill them with an entry each, and the items' way through shared memory costs more.
+// With the points spread, and with an entry per thread: 2.04 and 2.31 ms on 216 elements and 37 receivers,
+// 0.451 and 0.469 ms on 744 and 5; 3.20 and 3.17 ms on 744 and 300, 46.9 and 45.0 ms on 2664 and 300, 40.7
+// and 37.4 ms on 7016 and 37.
 // ------------------------------------------------------------------------------------------
 void launch_listener_aca(const DevGeometry& G, int prec, const void* pts, int L, double k, double eps, int maxk,
                          void* pool, long long pool_cap, unsigned long long* used, long long* term_off, int* rank,
@@ -662,8 +675,14 @@ void launch_listener_aca(const DevGeometry& G, int prec, const void* pts, int L,
   int iter_lim = std::min(maxk, std::min(L - 1, G.ne - 1));
   if (iter_lim < 1) iter_lim = 1;
   if (prec == PREC_FP64) {
-    launch_listener_aca_f64(G, (const double4*)pts, L, k, eps, maxk, (cd*)pool, pool_cap, used, term_off, rank, status,
-                            block, order, s);
+    if (L + G.ne <= 1024) {
+      launch_listener_aca_f64(G, (const double4*)pts, L, k, eps, maxk, (cd*)pool, pool_cap, used, term_off, rank,
+                              status, block, order, s);
+      return;
+    }
+    AcaArgs<double, double4> a{geo_view<double>(G), block, order, (const double4*)pts, k, eps, maxk, 0,
+                               iter_lim, (cd*)pool, pool_cap, used, term_off, rank, status, nullptr};
+    aca_launch_t(a, 1, L, s);
   } else {
     AcaArgs<float, float4> a{geo_view<float>(G), block, order, (const float4*)pts, (float)k, eps, maxk, 0,
                              iter_lim, (cf*)pool, pool_cap, used, term_off, rank, status, nullptr};
