@@ -641,7 +641,7 @@ __global__ void __launch_bounds__(kGatherThreads, AC3D_GATHER_MIN_CTAS) seg_gath
         for (int jr = 0; jr < RPL; jr++) tr[jr] = ti[jr] = 0;
         // near: the transposed copy, so that the lanes' columns of a row are consecutive; the rows of a
         // warp's blocks in order, U loads in flight (as many as the 56 registers hold). The blocks
-        // themselves (kInPlace: the device has no room for the copy) are read a line per lane.
+        // themselves (kInPlace: the device has no room for the copy) are read a column per lane.
         // Transposed matvec, from the blocks and from the copy: 149.6 and 101.3 us on the
         // 20480-triangle relief, 65.7 and 37.5 us on 5280 triangles
         for (int it = V.trn_ptr[leaf] + warp; it < V.trn_ptr[leaf + 1]; it += kWarps) {
@@ -650,6 +650,20 @@ __global__ void __launch_bounds__(kGatherThreads, AC3D_GATHER_MIN_CTAS) seg_gath
           const int m = blk.y - blk.x;
           const cplx<AT>* xs = xm + blk.x;
           const cplx<MT>* D = near + V.near_off[b];
+          if constexpr (TRANS == kInPlace) {
+#pragma unroll
+            for (int jr = 0; jr < RPL; jr++) {
+              const int col = lane + 32 * jr;
+              if (col < R) {
+                const cplx<MT>* Dc = D + (long long)col * m;
+                for (int r = 0; r < m; r++) {
+                  const cplx<AT> zz = xs[r];
+                  acc_mac(tr[jr], ti[jr], Dc[r], zz.re, zz.im);
+                }
+              }
+            }
+            continue;
+          }
           constexpr int U = sizeof(AT) > 4 ? 2 : RPL > 2 ? 4 : 8;
           for (int r0 = 0; r0 < m; r0 += U) {
 #pragma unroll
@@ -660,7 +674,7 @@ __global__ void __launch_bounds__(kGatherThreads, AC3D_GATHER_MIN_CTAS) seg_gath
 #pragma unroll
               for (int u = 0; u < U; u++) {
                 const int r = min(r0 + u, m - 1);
-                d[u] = D[TRANS == kInPlace ? (long long)col * m + r : (long long)r * R + col];
+                d[u] = D[(long long)r * R + col];
                 z[u] = xs[r];
               }
 #pragma unroll
