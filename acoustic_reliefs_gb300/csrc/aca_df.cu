@@ -1167,9 +1167,10 @@ void launch_listener_aca_df(const DevGeometry& G, const void* pts_df, int L, dou
   AC3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kDfThreads, smem));
   // about 64 columns (192 items) per CTA, at most one CTA per SM
   const int grid = std::max(1, std::min((per_sm > 0 ? 1 : 0) * device_sm_count(), (G.ne + 63) / 64));
-  if (grid <= 2) {
-    // barriers would cost more than the columns: 0.30 against 0.23 ms with one CTA on 80 elements and
-    // 17 receivers; on 320 elements the grid is ahead (0.42 against 0.49 ms with 37 receivers)
+  if (grid <= 2 || L + G.ne <= 384) {
+    // barriers would cost more than the entries. By the grid and by one CTA: 0.33 and 0.24 ms on 180
+    // elements and 37 receivers, 0.30 and 0.23 on 240 and 37, 0.09 and 0.08 on 384 and 5; the same on 308 and
+    // 37 (0.29, 0.30) and on 240 and 181; 0.29 and 0.36 on 468 and 37, 0.44 and 0.73 on 140 and 1297
     launch_aca_kernels(a, L, s, s);
     note_launch();
     df_to_cd_kernel<<<4 * device_sm_count(), 256, 0, s>>>((df2*)pool, used);
