@@ -747,9 +747,11 @@ struct BlockWork {
 
 // Launches chunks of a block solve until `flag`, read from the first 32 bytes of *state after each
 // chunk, is set. No chunk is kept in flight: the idle 16 or 8 iterations behind the last one would cost
-// more (about 12 us each) than the device's wait for the host between chunks (75 us).
+// more (about 12 us each) than the device's wait for the host between chunks (75 us). So a graph captured
+// for the second chunk leaves the device idle; `more` says that the solve will have one, and the graph is
+// captured while the device runs the first.
 template <typename Flag>
-void run_block_chunks(ac3d_ctx* c, ChunkRunner& g, const void* state, int max_launch, Flag flag) {
+void run_block_chunks(ac3d_ctx* c, ChunkRunner& g, const void* state, int max_launch, bool more, Flag flag) {
   cudaStream_t s = c->stream;
   constexpr size_t kHead = 32;
   static_assert(kHead <= sizeof(GState), "read into a pinned state");
@@ -757,17 +759,22 @@ void run_block_chunks(ac3d_ctx* c, ChunkRunner& g, const void* state, int max_la
   for (int k = 0; k < max_launch; k++) {
     g.launch();
     AC3D_CUDA(cudaMemcpyAsync(c->h_gstate, state, kHead, cudaMemcpyDeviceToHost, s));
+    if (more && !g.exec) g.capture();
     AC3D_CUDA(cudaStreamSynchronize(s));
     if (flag((const char*)c->h_gstate)) break;
   }
 }
 
-int run_block_krylov(ac3d_ctx* c, const MultiBufs& B, ChunkRunner& g, std::vector<int>& done) {
+// tol: the tightest of the columns'. Below 1e-5 a solve takes more than a chunk of 8 iterations (21 on 84
+// triangles, 22 on 240 at 3e-7); above, small ones often do not. Three directions, without and with the graph
+// captured behind the first chunk: 1.64 and 1.50 ms on 240 triangles at 3e-7 and 300 Hz; 1.18 and 1.22 ms at
+// 3e-4, where the one chunk is all.
+int run_block_krylov(ac3d_ctx* c, const MultiBufs& B, ChunkRunner& g, double tol, std::vector<int>& done) {
   cudaStream_t s = c->stream;
   const int maxit = c->maxit > 0 ? c->maxit : 2 * B.n;
   mkrylov_enqueue_init(B, maxit, s);
   // the state starts with iter, maxit, done_all, nrb
-  run_block_chunks(c, g, B.state, maxit / c->chunk + 2, [](const char* h) { return ((const int*)h)[2] != 0; });
+  run_block_chunks(c, g, B.state, maxit / c->chunk + 2, tol < 1e-5, [](const char* h) { return ((const int*)h)[2] != 0; });
   AC3D_CUDA(cudaStreamSynchronize(s));
   KStateM st;
   AC3D_CUDA(cudaMemcpy(&st, B.state, sizeof(KStateM), cudaMemcpyDeviceToHost));
@@ -786,7 +793,7 @@ int run_block_gmres(ac3d_ctx* c, const GmresBufs& G, const MultiBufs& B, ChunkRu
   gmres_reset(G, s);
   gmres_enqueue_init(G, 1.0, s);
   static_assert(sizeof(GMulti) == 32, "read as one head");
-  run_block_chunks(c, g, G.gm, (G.m + c->gm_chunk - 1) / c->gm_chunk + 1,
+  run_block_chunks(c, g, G.gm, (G.m + c->gm_chunk - 1) / c->gm_chunk + 1, false,
                    [](const char* h) { return ((const GMulti*)h)->done_all != 0; });
   gmres_enqueue_finish(G, B.x, s);
   std::vector<GState> st(G.nrb);
@@ -911,7 +918,8 @@ void solve_block(ac3d_ctx* c, DevHMat& H, int nrb, int nr, const cd* b64, cd* x6
     if (!any) break;
     AC3D_CUDA(cudaMemcpyAsync(W.tolb.p, tin.data(), nrb * sizeof(double), cudaMemcpyHostToDevice, s));
     launch_to32(n * nrb, W.r64.p, B.b, s);
-    iters += gm ? run_block_gmres(c, G, B, g, done) : run_block_krylov(c, B, g, done);
+    const double tightest = *std::min_element(tin.begin(), tin.end());
+    iters += gm ? run_block_gmres(c, G, B, g, done) : run_block_krylov(c, B, g, tightest, done);
     launch_add32(n * nrb, x64, B.x, s);
     for (int j = 0; j < nr; j++) {
       if (!(rn2[j] > tol * tol * bn2[j])) continue;
