@@ -45,7 +45,6 @@ struct AcaDfArgs {
   const int* order;            // blocks grouped by W = 8, 4, 2, 1
   int split[kGroups];          // blocks per group
   df64 k;
-  double eps;
   df64 eps2;       // eps^2 as a double-float (the stopping test)
   int maxk;
   int iter_cap;
@@ -842,7 +841,7 @@ void launch_aca_df(const DevGeometry& G, const DevPartition& DP, DevHMat& H, dou
   AcaDfArgs a{G.cen.as<double4>(), G.va.as<double4>(), G.eg64.as<ElemGeo<double>>(), G.cen_df.as<DfPt>(),
               G.el_df.as<DfElem>(), G.df_tab.as<float4>(), DP.blocks_a.as<int4>(), DP.aca_order.as<int>(),
               {DP.aca_split[0], DP.aca_split[1], DP.aca_split[2], DP.aca_split[3]},
-              df_from_double(H.k), eps, df_from_double(eps * eps), H.maxk, H.maxk, H.pool.as<df2>(), H.pool_cap,
+              df_from_double(H.k), df_from_double(eps * eps), H.maxk, H.maxk, H.pool.as<df2>(), H.pool_cap,
               H.pool_used.as<unsigned long long>(), H.term_off.as<long long>(), H.rank.as<int>(),
               &H.pool_used.as<AsmTotals>()->status, H.passes.as<int>(), H.pool_used.as<AsmTotals>()->next, 1};
   launch_aca_kernels(a, max_rows, s, s_small);
@@ -1151,7 +1150,7 @@ void launch_listener_aca_df(const DevGeometry& G, const void* pts_df, int L, dou
   int iter_lim = std::min(maxk, std::min(L - 1, G.ne - 1));
   if (iter_lim < 1) iter_lim = 1;
   AcaDfArgs a{G.cen.as<double4>(), G.va.as<double4>(), G.eg64.as<ElemGeo<double>>(), (const DfPt*)pts_df,
-              G.el_df.as<DfElem>(), G.df_tab.as<float4>(), block, order, {1, 0, 0, 0}, df_from_double(k), eps,
+              G.el_df.as<DfElem>(), G.df_tab.as<float4>(), block, order, {1, 0, 0, 0}, df_from_double(k),
               df_from_double(eps * eps), maxk, iter_lim,
               (df2*)pool, pool_cap, used, term_off, rank, status, nullptr, nullptr, 0};
   static void (*const kernels[2])(AcaDfArgs, AcaGridBufs) = {aca_df_grid_kernel<kDfThreads>, aca_df_grid_kernel<kDfThreads / 2>};

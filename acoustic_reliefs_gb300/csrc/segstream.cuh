@@ -139,7 +139,9 @@ struct SegView {
 // Iterates the chunks of the (up to two) regions of one leaf through the copy ring and calls
 // fn(stage_ptr, region, first_column, columns, next_region, next_first_column, next_columns) for
 // each chunk, all threads together (next_columns = 0 after the last chunk), so that the callback
-// can prefetch what the next chunk needs while it computes this one.
+// can prefetch what the next chunk needs while it computes this one. (The block dot pass has one region and
+// looks at nothing ahead; a function of one region made the compiler's code for it slower: 182 instead of
+// 174 us a block matvec of 16 right-hand sides on 7016 triangles in leaves of up to 64.)
 template <typename MT, typename F>
 __device__ __forceinline__ bool stream_leaf(unsigned char (*stage)[kStageBytes], uint64_t* full, int R,
                                             const cplx<MT>* a_ptr, int a_cols, const cplx<MT>* b_ptr, int b_cols,
