@@ -377,8 +377,8 @@ static_assert(sizeof(AcaGroup<1>) % 16 == 0 && sizeof(AcaGroup<2>) % 16 == 0 && 
 // Bound by the FP32 pipe (55% busy) and, beside it, by instruction supply and latency: the warps
 // are at different places of a long recursion. Four CTAs of 128 threads per SM (128 registers)
 // beat six (80 registers, spills) 4.9 to 6.2 ms on the 20480-triangle relief: more warps thrash L1 and
-// the instruction caches. With the 8-warp blocks' kernel the assembly takes 8.8 instead of 11.0 ms
-// there, 1.77 instead of 2.95 ms on 5280 triangles and 94 instead of 106 ms on 118680 (2 kHz), against
+// the instruction caches. With the 8-warp blocks' kernel the assembly takes 8.0 instead of 11.0 ms
+// there, 1.65 instead of 2.95 ms on 5280 triangles and 89 instead of 106 ms on 118680 (2 kHz), against
 // one warp per block with scalar arithmetic up to sides of 256.
 // ------------------------------------------------------------------------------------------
 template <int W>
@@ -857,9 +857,9 @@ void launch_aca_df(const DevGeometry& G, const DevPartition& DP, DevHMat& H, dou
 // past L1 (ld.cg); terms are a multiple of 128 bytes apart, so that no line of an earlier term holds
 // part of a later one.
 //
-// Bound by latency: of an iteration's 40 us (1297 receivers x 10680 elements, tolerance 1e-5, 135 to 168
-// terms) the chain over the earlier terms takes 15 us, the longest dot product 12 us, the barriers
-// 5 us, the entries 3 us. 5.9 ms instead of 168 ms by one CTA, which is where it began (146 ms with
+// Bound by latency: of an iteration's 37 us (1297 receivers x 10680 elements, tolerance 1e-5, 135 to 168
+// terms) the chain over the earlier terms takes some 14 us, the longest dot product 11 us, the barriers
+// 5 us, the entries 3 us. 5.6 ms instead of 168 ms by one CTA, which is where it began (146 ms with
 // the entries' items spread over its threads).
 // ------------------------------------------------------------------------------------------
 struct alignas(16) AcaBest {

@@ -163,8 +163,8 @@ void finish_timers(ac3d_ctx* c) {
 // the executable graph 0.15 to 0.2 ms, with the device idle; now the device runs the direct chunk
 // meanwhile (a direct iteration costs it about 7 us more than a replayed one), a solve of one chunk
 // captures nothing, and a used graph is destroyed behind the next solve's first chunk. With the layout
-// of an assembly formed on the device (launch_leaf_layout), whole solves take 8.53 -> 7.78 ms on the
-// 5280-triangle relief, 1.65 -> 1.42 ms on the 1280-triangle sphere, 243 -> 238 ms on 118680 triangles.
+// of an assembly formed on the device (launch_leaf_layout), whole solves went from 8.53 to 7.78 ms on the
+// 5280-triangle relief, from 1.65 to 1.42 ms on the 1280-triangle sphere.
 // If enqueueing throws during the capture, the capture is ended and its graph discarded, so the stream
 // is usable again.
 struct ChunkRunner {
@@ -547,7 +547,7 @@ GmresBufs gmres_bufs(ac3d_ctx* c, const DevHMat& H, const void* b, int nrb = 1) 
 }
 
 // Zero states (their tickets start at zero; each reducing pass leaves them at zero) and batch
-// completion count; no host wait, so the host captures the cycle's graph while the device runs
+// completion count; no host wait, so the host enqueues the cycle's first chunk while the device runs
 // the assembly.
 void gmres_reset(const GmresBufs& G, cudaStream_t s) {
   AC3D_CUDA(cudaMemsetAsync(G.state, 0, G.nrb * sizeof(GState) + sizeof(GMulti), s));

@@ -21,7 +21,7 @@ constexpr int kVecWarps = kVecThreads / 32;
 
 // What bounds the vector kernels on small meshes is FP64 latency (an instruction takes 64 clocks, a
 // division some 15 of them): sums are folded, each total is formed by one thread and omega's two
-// divisions run on two lanes. 1280 triangles: kf_xr 12.3 -> 7.9 us of a 64 us iteration. The complex
+// divisions run on two lanes. 1280 triangles: kf_xr 12.3 -> 7.9 us of an iteration that takes 56 us now. The complex
 // quotients stay with one thread and the loads behind them: in other shapes of the code the compiler
 // contracts their products otherwise, and a mixed solve then ends on another iterate.
 __device__ __forceinline__ void write_partials(double* d, double* partials) {

@@ -6,13 +6,15 @@
 //   U segment of a row leaf      : rows of the leaf of every admissible block above it, one column
 //                                  per rank-1 term;
 //   V segment of a column leaf   : columns of the leaf of every admissible block beside it.
-// Forward:    p = per-column dots of the V segments with x   (dot pass, one CTA per leaf)
+// Forward:    p = per-column dots of the V segments with x   (dot pass, one to eight CTAs per leaf)
 //             t[b, q] = sum over the column leaves of b of p (reduce, fixed leaf order)
-//             y = -x/2 + near x + U t                         (gather pass, one CTA per leaf)
-// Transpose:  the same with U and V swapped, plus the dense blocks read column-wise.
+//             y = -x/2 + near x + U t                         (gather pass, resident CTAs take the leaves)
+// Transpose:  the same with U and V swapped, the near field from its transposed copy or, where the device
+// has no room for that, from the blocks themselves.
 // Both passes stream their segments through shared memory with bulk async copies, so the bytes
-// in flight are set by the copy ring, not by how many loads a warp can issue. No atomics; every
-// sum has a fixed order, so results are bit-reproducible.
+// in flight are set by the copy ring, not by how many loads a warp can issue. Every sum has a fixed
+// order (atomics only count finished CTAs), so results are bit-reproducible. The FP64 H-matrix's
+// passes are in matvec64.cu; the reduce pass is common.
 #include <algorithm>
 #include <atomic>
 #include <mutex>
