@@ -857,10 +857,10 @@ void launch_aca_df(const DevGeometry& G, const DevPartition& DP, DevHMat& H, dou
 // past L1 (ld.cg); terms are a multiple of 128 bytes apart, so that no line of an earlier term holds
 // part of a later one.
 //
-// Bound by latency: of an iteration's 37 us (1297 receivers x 10680 elements, tolerance 1e-5, 135 to 168
-// terms) the chain over the earlier terms takes some 14 us, the longest dot product 11 us, the barriers
-// 5 us, the entries 3 us. 5.6 ms instead of 168 ms by one CTA, which is where it began (146 ms with
-// the entries' items spread over its threads).
+// Bound by latency: an iteration takes 37 us (1297 receivers x 10680 elements, tolerance 1e-5, 135 to 168
+// terms); when it was split up, at 40 us, the chain over the earlier terms took 15 us, the longest dot
+// product 12 us, the barriers 5 us, the entries 3 us. 5.6 ms instead of 168 ms by one CTA, which is where it
+// began (146 ms with the entries' items spread over its threads).
 // ------------------------------------------------------------------------------------------
 struct alignas(16) AcaBest {
   df2 v;      // the entry
