@@ -127,35 +127,49 @@ __device__ __forceinline__ void gather_class(double& re, double& im, const cd* _
   }
 }
 
-// gather_class of a leaf's near columns in A^T without their transposed copy (the device has no room for
-// it): column c of the segment is a row of one of the near blocks that have the leaf's columns, in their
-// order; the walk over the columns and so the order of the sums are the same.
-template <int NC>
-__device__ __forceinline__ void gather_near_in_place(double& re, double& im, const SegView& V, int leaf,
-                                                     const cd* __restrict__ near, const cd* __restrict__ x, int R,
-                                                     int cpc, int k, int r) {
-  int it = V.trn_ptr[leaf], before = 0;  // the block, and the columns before it
-  const int end = V.trn_ptr[leaf + 1], K = V.a_kptr[leaf + 1] - V.a_kptr[leaf];
-  for (int c0 = 0; c0 < K; c0 += cpc)
-    for (int c = c0 + k; c < min(c0 + cpc, K); c += NC) {
-      int4 q;
-      int m = 0;
-      for (; it < end; it++, before += m) {
-        q = V.blocks_d[V.trn[it]];
-        m = q.y - q.x;
-        if (c < before + m) break;
+// The gather pass's directions: A x, and A^T x with the near field from its transposed copy or, where the
+// device has no room for that, in place
+enum : int { kForward = 0, kTransposed = 1, kInPlace = 2 };
+
+// A^T: the near part of row r (a column of the near blocks that have the leaf's columns) that warp w of the FP32
+// layout's eight adds: of the blocks w, w + 8, ..., their rows in order.
+template <int DIR>
+__device__ __forceinline__ void near_transposed(double& re, double& im, const SegView& V, int leaf,
+                                                const cd* __restrict__ near, const cd* __restrict__ x, int R, int w,
+                                                int r) {
+  constexpr int U = 4;  // loads in flight
+  const int end = V.trn_ptr[leaf + 1];
+  for (int it = V.trn_ptr[leaf] + w; it < end; it += 8) {
+    const int b = V.trn[it];
+    const int4 q = V.blocks_d[b];
+    const int m = q.y - q.x, step = DIR == kInPlace ? 1 : R;
+    const cd* D = near + V.near_off[b] + (long long)r * (DIR == kInPlace ? m : 1);
+    const cd* xs = x + q.x;
+    int i = 0;
+    for (; i + U <= m; i += U, D += U * step) {
+      cd a[U], z[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        a[u] = D[u * step];
+        z[u] = xs[i + u];
       }
-      if (it == end) return;  // the padding column
-      const int i = c - before;
-      mac64(re, im, near[V.near_off[V.trn[it]] + (long long)r * m + i], x[q.x + i]);
+#pragma unroll
+      for (int u = 0; u < U; u++) mac64(re, im, a[u], z[u]);
     }
+#pragma unroll 1
+    for (; i < m; i++, D += step) mac64(re, im, *D, xs[i]);
+  }
 }
 
 // y[leaf rows] = -x/2 + S_A x[a_idx] + S_B t[b_idx], or b - that, with the optional dot partials of
 // seg_gather_persist_kernel. The NC column classes are that kernel's (warp, slot) pairs: a cluster of S CTAs
 // holds them all, NC / S each with a thread per row. Every CTA adds its warps' slots, the first one the warps in
-// order, and finishes the leaf. The near part runs before the wait for the reduce pass.
-template <int NC, int S, bool IN_PLACE>
+// order, and finishes the leaf. The near part runs before the wait for the reduce pass; in A^T it is summed
+// apart, by a thread per row and warp, and added to the warp's low-rank part, as the FP32 layout has it. (With
+// the near columns in the classes, as in A x, FP64 adjoint BiCGSTAB solves ended on other iterates. A^T x on
+// 5736 triangles in leaves of up to 32, 64, 128 and 256, in the FP32 layout, so, and in the classes: 287, 186,
+// 136 us; 450, 212, 177; 970, 255, 280; 1926, 316, 695.)
+template <int NC, int S, int DIR>
 __global__ void __launch_bounds__(kGatherThreads, 5) gather64_kernel(
     SegView V, int nleaf, const cd* __restrict__ near, const cd* __restrict__ lrseg, const cd* __restrict__ t,
     const cd* __restrict__ x, cd* __restrict__ y, const cd* __restrict__ bminus, const cd* __restrict__ dot_a,
@@ -181,13 +195,12 @@ __global__ void __launch_bounds__(kGatherThreads, 5) gather64_kernel(
   // two warps per CTA are one from either end: the first classes of a chunk have a column more
   const int g = tid / R, r = tid - g * R, k = (g < SL ? rank : W - 1 - rank) * SL + g % SL;
   const int cpc = min(128, max(2, (int)(kStageBytes / sizeof(cd)) / R & ~1));  // columns per chunk of its ring
-  double re = 0, im = 0;
-  const int ak = V.a_kptr[leaf], ac = V.a_kptr[leaf + 1] - ak;
-  if (!skip && g < GP) {
-    if constexpr (IN_PLACE)
-      gather_near_in_place<NC>(re, im, V, leaf, near, x, R, cpc, k, r);
-    else
-      gather_class<NC>(re, im, near + V.a_seg[leaf], ac, V.a_idx + ak, x, R, cpc, k, r);
+  double re = 0, im = 0, near_re = 0, near_im = 0;
+  if constexpr (DIR == kForward) {
+    const int ak = V.a_kptr[leaf], ac = V.a_kptr[leaf + 1] - ak;
+    if (!skip && g < GP) gather_class<NC>(re, im, near + V.a_seg[leaf], ac, V.a_idx + ak, x, R, cpc, k, r);
+  } else {
+    if (!skip && g < LW) near_transposed<DIR>(near_re, near_im, V, leaf, near, x, R, g ? W - 1 - rank : rank, r);
   }
   const int bk = V.b_kptr[leaf], bc = V.b_kptr[leaf + 1] - bk;
   grid_dep_wait();
@@ -201,6 +214,7 @@ __global__ void __launch_bounds__(kGatherThreads, 5) gather64_kernel(
     if constexpr (SL == 2) v = cd(v.re + q[R].re, v.im + q[R].im);
     if constexpr (SL == 4)
       v = cd((v.re + q[R].re) + (q[2 * R].re + q[3 * R].re), (v.im + q[R].im) + (q[2 * R].im + q[3 * R].im));
+    if constexpr (DIR != kForward) v = cd(v.re + near_re, v.im + near_im);
     rows[tid] = v;
   }
   cl.sync();
@@ -276,12 +290,12 @@ void launch_matvec_f64(const DevPartition& DP, const DevHMat& H, bool tr, const 
                        const MatvecEpilogue& ep, const int* done, cudaStream_t s, bool pdl) {
   SegView v = {};
   v.leaf_start = DP.leaf_start.as<int>();
-  v.a_seg = (tr ? DP.near_seg_t : DP.near_seg).as<long long>();
-  v.a_kptr = (tr ? DP.didx_t_ptr : DP.didx_ptr).as<int>();
-  v.a_idx = (tr ? DP.didx_t : DP.didx).as<int>();
-  const bool in_place = tr && !H.nearT.p;
+  v.a_seg = DP.near_seg.as<long long>();
+  v.a_kptr = DP.didx_ptr.as<int>();
+  v.a_idx = DP.didx.as<int>();
+  const int dir = !tr ? kForward : H.nearT.p ? kTransposed : kInPlace;
   v.blocks_d = DP.blocks_d.as<int4>();
-  v.near_off = DP.near_off.as<long long>();
+  v.near_off = (dir == kTransposed ? DP.near_off_t : DP.near_off).as<long long>();
   v.trn_ptr = DP.tr_near_ptr.as<int>();
   v.trn = DP.tr_near.as<int>();
   const cd* useg = H.useg.as<cd>();
@@ -310,17 +324,23 @@ void launch_matvec_f64(const DevPartition& DP, const DevHMat& H, bool tr, const 
   auto gather = [&](auto kern, int classes, int ctas) {
     const int threads = (classes / ctas * DP.max_leaf + 31) / 32 * 32;
     launch_clusters(pdl && DP.na > 0, (unsigned)ctas, kern, dim3(DP.nleaf * ctas), dim3(threads), s, v, DP.nleaf,
-                    (tr && !in_place ? H.nearT : H.near).as<cd>(), tr ? vseg : useg, t, (const cd*)x, (cd*)y, (const cd*)bminus,
+                    (dir == kTransposed ? H.nearT : H.near).as<cd>(), tr ? vseg : useg, t, (const cd*)x, (cd*)y, (const cd*)bminus,
                     (const cd*)ep.dot_a, (const cd*)ep.dot_b, ep.partials, ep.red5, H.ticket.as<unsigned>(), done);
   };
+#define AC3D_GATHER64(NC, S)                                              \
+  gather(dir == kForward      ? gather64_kernel<NC, S, kForward>          \
+         : dir == kTransposed ? gather64_kernel<NC, S, kTransposed>       \
+                              : gather64_kernel<NC, S, kInPlace>,         \
+         NC, S)
   if (DP.max_leaf <= 32)
-    gather(in_place ? gather64_kernel<32, 4, true> : gather64_kernel<32, 4, false>, 32, 4);
+    AC3D_GATHER64(32, 4);
   else if (DP.max_leaf <= 64)
-    gather(in_place ? gather64_kernel<32, 8, true> : gather64_kernel<32, 8, false>, 32, 8);
+    AC3D_GATHER64(32, 8);
   else if (DP.max_leaf <= 128)
-    gather(in_place ? gather64_kernel<16, 8, true> : gather64_kernel<16, 8, false>, 16, 8);
+    AC3D_GATHER64(16, 8);
   else
-    gather(in_place ? gather64_kernel<8, 8, true> : gather64_kernel<8, 8, false>, 8, 8);
+    AC3D_GATHER64(8, 8);
+#undef AC3D_GATHER64
 }
 
 }  // namespace ac3d
