@@ -1248,7 +1248,11 @@ __global__ void __launch_bounds__(kGmThreads) k_gm_dgivens(GmCols C, int m, int 
 
 // y = R^{-1} g over the completed columns, then coef_k = y_k s_k (one CTA). A chain of the columns: the
 // reciprocals are formed beforehand, the next column is loaded under this one's arithmetic (93
-// columns: 146 -> 65 us).
+// columns: 146 -> 65 us). The products are contracted as the compiler had them in the chain's former shape
+// (left to it, the last bits of FP64 solutions differ), so they are written out: g - a b.
+__device__ __forceinline__ Dc gm_step(Dc g, Dc a, Dc b) {
+  return dc(g.re - fma(a.re, b.re, -(a.im * b.im)), g.im - fma(a.re, b.im, a.im * b.re));
+}
 __global__ void __launch_bounds__(kGmThreads) k_gm_solve(GmCols C, int m, int G) {
   const GmLayout L{m, G};
   const GState* st = C.st + blockIdx.y;
@@ -1273,8 +1277,8 @@ __global__ void __launch_bounds__(kGmThreads) k_gm_solve(GmCols C, int m, int G)
     const Dc y = dc(gs[k].re * id[k], gs[k].im * id[k]);
     const Dc rk = r;  // this thread's entry of column k; the next column's under the arithmetic
     if (l0 < k - 1) r = entry(l0, k - 1);
-    if (l0 < k) gs[l0] = gs[l0] - rk * y;
-    for (int l = l0 + blockDim.x; l < k; l += blockDim.x) gs[l] = gs[l] - entry(l, k) * y;
+    if (l0 < k) gs[l0] = gm_step(gs[l0], rk, y);
+    for (int l = l0 + blockDim.x; l < k; l += blockDim.x) gs[l] = gm_step(gs[l], entry(l, k), y);
     __syncthreads();
   }
   for (int k = threadIdx.x; k < jj; k += blockDim.x) {

@@ -24,3 +24,17 @@ def test_pivots_of_equal_candidates(gpu_lib, i):
     x, want = bem.surface_vals(f), g[f"x{i}"]
     assert np.array_equal(bem.ranks(), g[f"rank{i}"])
     assert np.linalg.norm(x - want) < 1e-9 * np.linalg.norm(want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("i", range(5))
+def test_gmres_solution_keeps_its_bits(gpu_lib, i):
+    """The same solutions by GMRES in FP64, bit for bit: the back substitution rounds as in its former shape
+    whatever the compiler makes of the present one."""
+    g = np.load(GOLDEN)
+    leaf, f, aca = g[f"par{i}"]
+    bem = DiffBEM(int(leaf), 2.0, [f], 1, aca, aca, 1e-6, precision="fp64", incident=("plane", (0.3, -1.0, 0.2)))
+    bem.silent = True
+    bem.set_krylov("gmres")
+    bem.set_mesh(g[f"Ps{i}"], g[f"Es{i}"])
+    assert np.array_equal(bem.surface_vals(f), g[f"x{i}"])
