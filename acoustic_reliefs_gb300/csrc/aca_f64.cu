@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(T) aca_f64_kernel(AcaF64Args A) {
       if (tid < C && c < n) {
         const cd v = f64_finish(items, tid, coef, toff, A.pool + m + c, nst);
         vnew[c] = v;
-        const double a = wide ? f64_abs2(v.re, v.im) : f64_abs2(v.im, v.re);
+        const double a = f64_abs2(wide ? v.re : v.im, wide ? v.im : v.re);
         if (a > best) {
           best = a;
           bidx = c;
